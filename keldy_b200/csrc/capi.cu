@@ -810,6 +810,21 @@ static ItemDev make_item(const kb_model *m, const kb_integrand *f, int order) {
   return it;
 }
 
+// Points per scheduling chunk of a work item of n points: `most` (the context's chunk size for
+// its order, autotuned or kb_context_set_launch), halved while the item would have fewer chunks
+// than half the resident tree warps, so that a small item is spread over the GPU instead of a
+// few warps walking long chunks (a batch of many small items keeps larger chunks than one
+// small item alone would need). Not below the size at which a group's set-up is a small part
+// of its work: 8 points up to order 5, 4 up to order 8, then 2 and 1. It depends on the item
+// alone: a batch adds each item's points in the order of a call of its own.
+static int item_chunk(const kb_context *ctx, int order, int64_t n, int most) {
+  int c = most;
+  const int64_t want = std::min((int64_t)ctx->sm_count * ctx->ctas_per_sm * TREE_WARPS / 2, MAX_SPLIT_CHUNKS);
+  const int least = order <= 5 ? 8 : order <= 8 ? 4 : order == 9 ? 2 : 1;
+  while (c > least && (n + c - 1) / c < want) c >>= 1;
+  return c;
+}
+
 // Runs the tree (or direct) kernel over `count` points of one item in an evaluation
 // mode, then re-evaluates points the tree flagged with the pivoted-LU kernel.
 static int run_eval(kb_context *ctx, ItemDev it, int mode, int64_t count, const double *in_host, int keep,
@@ -824,7 +839,8 @@ static int run_eval(kb_context *ctx, ItemDev it, int mode, int64_t count, const 
   const bool use_tree = (algo == KB_ALGO_TREE) || (algo == KB_ALGO_AUTO && it.spin_symmetric);
   if (algo == KB_ALGO_TREE && !it.spin_symmetric)
     return fail(KB_E_INVALID, "the tree algorithm needs equal spin-up and spin-down g0 tables");
-  long long nchunks = (count + CHUNK_POINTS - 1) / CHUNK_POINTS;
+  if (use_tree) it.chunk_points = item_chunk(ctx, N, count, 32); // a warp per chunk: 32 points fill its lanes
+  long long nchunks = (count + it.chunk_points - 1) / it.chunk_points;
   long long offs[2] = {0, nchunks};
   DevBuf ditem, doff, dcnt, din, dval, djac, ddom, dscale, dflag;
   KB_CUDA(ditem.alloc(sizeof(ItemDev), st));
@@ -875,7 +891,7 @@ static int run_eval(kb_context *ctx, ItemDev it, int mode, int64_t count, const 
       DevBuf didx;
       KB_CUDA(didx.alloc(idx.size() * sizeof(int), st));
       KB_CUDA(cudaMemcpyAsync(didx.p, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-      long long nc2 = ((long long)idx.size() + CHUNK_POINTS - 1) / CHUNK_POINTS;
+      long long nc2 = ((long long)idx.size() + it.chunk_points - 1) / it.chunk_points;
       long long offs2[2] = {0, nc2};
       KB_CUDA(cudaMemcpyAsync(doff.p, offs2, sizeof(offs2), cudaMemcpyHostToDevice, st));
       KB_CUDA(cudaMemsetAsync(dcnt.p, 0, sizeof(int), st));
@@ -1141,19 +1157,6 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
 constexpr int64_t FLOW_PIECE = 1 << 22;            // points per flow-mapped piece
 constexpr size_t FLOW_ROUND_BYTES = (size_t)1 << 30; // flow-mapped points held at once
 
-// Points per scheduling chunk of a work item of n points: the context's chunk size for its
-// order (autotuned or kb_context_set_launch), halved (down to 8) while the item would have
-// fewer chunks than half the resident tree CTAs, so that a small item is spread over the
-// GPU instead of a few CTAs walking long chunks one point after another (a batch of many
-// small items keeps larger chunks than one small item alone would need). It depends on
-// the item alone: a batch adds each item's points in the order of a call of its own.
-int item_chunk(const kb_context *ctx, int order, int64_t n) {
-  int c = ctx->chunk_points[order];
-  const int64_t want = (int64_t)ctx->sm_count * ctx->ctas_per_sm / 2;
-  while (c > 8 && (n + c - 1) / c < want) c >>= 1;
-  return c;
-}
-
 // Checks of a work item shared by kb_integrate and kb_plan_create; fills `it`.
 int work_item(kb_context *ctx, const kb_work &w, int algo, ItemDev &it, int &tree) {
   int st = check_integrand(w.m, &w.f, w.order);
@@ -1178,7 +1181,7 @@ int work_item(kb_context *ctx, const kb_work &w, int algo, ItemDev &it, int &tre
   it.rng = sobol_dev(w.rng);
   it.k_first = w.k_first;
   it.n_points = w.n_points;
-  it.chunk_points = item_chunk(ctx, w.order, w.n_points);
+  it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order]);
   if (w.flow && w.flow->layout.kind == FLOW_KIND_SPLINE) it.spline_knots = w.flow->knots; // mapped in line
   if (w.flow && w.flow->layout.kind == FLOW_KIND_AR_SPLINE) it.ar_spline = w.flow->master; // mapped in line
   if (algo == KB_ALGO_TREE && !it.spin_symmetric)
@@ -1846,8 +1849,11 @@ constexpr size_t NOALLOC_OFFS_OFF = NOALLOC_ITEMS_OFF + sizeof(ItemDev) * KB_NOA
 constexpr size_t NOALLOC_ACC_OFF = ((NOALLOC_OFFS_OFF + sizeof(long long) * (KB_NOALLOC_MAX_ITEMS + 1)) + 255) / 256 * 256;
 constexpr size_t NOALLOC_CNT_OFF = NOALLOC_ACC_OFF + sizeof(kb_accum) * 2 * KB_NOALLOC_MAX_ITEMS;
 constexpr size_t NOALLOC_PART_OFF = (NOALLOC_CNT_OFF + sizeof(int) + 255) / 256 * 256;
+// An item's chunks number at most its chunks in the documented unit (noalloc_unit), or twice
+// MAX_SPLIT_CHUNKS where item_chunk split a small item further.
+constexpr size_t NOALLOC_PARTIALS = KB_NOALLOC_MAX_CHUNKS + KB_NOALLOC_MAX_ITEMS * 2 * MAX_SPLIT_CHUNKS;
 constexpr size_t NOALLOC_PTS_OFF =
-    (NOALLOC_PART_OFF + sizeof(ChunkPartial) * (size_t)KB_NOALLOC_MAX_CHUNKS + 255) / 256 * 256;
+    (NOALLOC_PART_OFF + sizeof(ChunkPartial) * (size_t)NOALLOC_PARTIALS + 255) / 256 * 256;
 constexpr size_t NOALLOC_PTS_SLOTS = (KB_NOALLOC_SCRATCH_BYTES - NOALLOC_PTS_OFF) / (PTS_SLOT * sizeof(double));
 // one set-up slot per resident tree CTA of a 148-SM B200 at the most CTAs per SM the
 // launch shape allows; a device with more SMs runs the tree with a grid capped at the slots
@@ -1855,6 +1861,15 @@ constexpr size_t NOALLOC_B200_TREE_CTAS = 148 * 4;
 static_assert(NOALLOC_PTS_SLOTS >= NOALLOC_B200_TREE_CTAS, "scratch too small for one set-up slot per resident CTA");
 
 static __device__ __align__(256) unsigned char kb_noalloc_scratch[KB_NOALLOC_SCRATCH_BYTES];
+
+// The unit of the call's documented chunk limit: the context's chunk size of the order, halved
+// (down to 8) while the item would have fewer chunks than half the resident tree CTAs.
+int noalloc_unit(const kb_context *ctx, int order, int64_t n) {
+  int c = ctx->chunk_points[order];
+  const int64_t want = (int64_t)ctx->sm_count * ctx->ctas_per_sm / 2;
+  while (c > 8 && (n + c - 1) / c < want) c >>= 1;
+  return c;
+}
 
 std::mutex g_noalloc_mu;
 unsigned char *g_noalloc_addr[NOALLOC_MAX_DEVICES] = {};
@@ -1908,8 +1923,9 @@ extern "C" int kb_integrate_noalloc(kb_context *ctx, const kb_work *work, int n_
     group_of[i] = it.spin_symmetric ? 0 : 1;
     // the same scheduling chunks as kb_integrate (the context's launch shape of the order,
     // smaller for a small item), so that the sums are added in the same order
-    it.chunk_points = item_chunk(ctx, w.order, w.n_points);
-    chunks_total += (w.n_points + it.chunk_points - 1) / it.chunk_points;
+    it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order]);
+    const int64_t unit = noalloc_unit(ctx, w.order, w.n_points);
+    chunks_total += (w.n_points + unit - 1) / unit;
   }
   if (chunks_total > KB_NOALLOC_MAX_CHUNKS)
     return fail(KB_E_INVALID, "kb_integrate_noalloc: more than KB_NOALLOC_MAX_CHUNKS (65,536) scheduling chunks in "

@@ -23,44 +23,20 @@ struct ChunkPartial {
 };
 
 constexpr int CHUNK_POINTS = 128; // points per scheduling chunk (<= 128: two 64-bit masks)
-// Per-CTA slot of the tree kernel in global memory (L2-resident): the chunk's set-up,
-// PTS_ROWS doubles (coordinates [MAX_ORDER][CHUNK_POINTS], then the Jacobians and the
-// domain flags of the chunk's points; with time bins also each point's bin code (2 bin + 1
-// when its value is added, 2 bin when only counted, -1 when dropped) and its f*J (re,
-// im)), then G_STAGE complex entries of staged G matrices (a G-batch, tree_gbatch).
-constexpr int PTS_ROWS = CHUNK_POINTS * (MAX_ORDER + 5);
-constexpr int G_STAGE = 4096;
-// Frontier entries at the start of a buffer that the tree's fused bottom uses for its
-// per-point sums (CTA_THREADS double2 and CTA_THREADS / 2 double2 of doubles).
-constexpr int BOTTOM_SCRATCH = CTA_THREADS + CTA_THREADS / 2;
-constexpr int PTS_SLOT = PTS_ROWS + 2 * G_STAGE;
-// Per-CTA slot of the kernel-method tree: the chunk's set-up rows only.
-constexpr int KM_SLOT = PTS_ROWS;
+// The tree kernel (wick_tree.cu): warps of a CTA, resident CTAs per SM (12 warps: 168 registers
+// per thread and 18.7 KB of shared memory per warp), and the complex entries of a warp's global
+// scratch (L2-resident): the nodes of orders 9..16 above level 8, sum_{m=9..16} (m+1)^2.
+constexpr int TREE_WARPS = 3;
+constexpr int TREE_CTAS_PER_SM = 4;
+constexpr int TREE_STACK = 1500;
+constexpr int PTS_SLOT = TREE_WARPS * TREE_STACK * 2; // doubles per CTA
+// A small work item is split into finer scheduling chunks only while it has fewer than this.
+constexpr int64_t MAX_SPLIT_CHUNKS = 888;
+// Per-CTA slot of the kernel-method tree: the chunk's set-up (coordinates
+// [MAX_ORDER][CHUNK_POINTS], then Jacobians, domain flags and bin codes).
+constexpr int KM_SLOT = CHUNK_POINTS * (MAX_ORDER + 5);
 // Resident CTAs per SM of the kernel-method tree (256 threads, ~114 KB of shared memory).
 constexpr int KM_CTAS_PER_SM = 2;
-static_assert(PTS_ROWS % 2 == 0 && PTS_SLOT % 2 == 0, "staged G on 16-byte boundaries");
-
-// Points per G-batch of the tree kernel at order N: their (2N+1)^2 matrices G fit the
-// staging area, their coordinates the kernel's 256-entry shared array, and the count is a
-// multiple of the sub-batch size tree_points_per_chunk(N).
-__host__ __device__ inline int tree_gbatch(int N) {
-  const int P = tree_points_per_chunk(N);
-  const int M = 2 * N + 1;
-  // orders above TREE_MAX_SUB keep up to four subtree roots (17 x 17) and their prefix
-  // determinants after the batch's G matrices
-  const int R = 2 * TREE_MAX_SUB + 1, reserve = N > TREE_MAX_SUB ? 4 * R * R + 4 : 0;
-  int g = CHUNK_POINTS;
-  if (N > 0 && 256 / N < g) g = 256 / N;
-  if ((G_STAGE - reserve) / (M * M) < g) g = (G_STAGE - reserve) / (M * M);
-  g -= g % P;
-  return g > 0 ? g : P;
-}
-
-// Orders whose G-batch is a single sub-batch (1..4) gain nothing from staging G in global
-// memory: the tree kernel builds their G directly in shared memory.
-__host__ __device__ inline bool tree_direct(int N) {
-  return N <= TREE_MAX_SUB && tree_gbatch(N) <= tree_points_per_chunk(N);
-}
 
 struct Launch {
   const ItemDev *items; // device
@@ -79,8 +55,7 @@ struct Launch {
   int *out_dom;
   double *out_scale;
   int *out_flag;        // tree: 1 = point needs the pivoted-LU kernel
-  // tree kernel: gridDim.x * PTS_SLOT doubles of set-up and staging scratch (kernel-method
-  // tree: gridDim.x * KM_SLOT)
+  // gridDim.x * PTS_SLOT doubles of scratch (tree kernel) or KM_SLOT (kernel-method tree)
   double *pts;
   // IN_SOBOL
   ChunkPartial *partials; // [n_chunks]
@@ -112,9 +87,9 @@ inline int items_any_cubic(const ItemDev *items, size_t n) {
   return 0;
 }
 
-size_t tree_smem_bytes();
 // sets the kernels' shared-memory attributes (before any stream capture)
 cudaError_t configure_kernels();
+cudaError_t configure_tree_kernels(); // the tree kernel's part
 cudaError_t launch_tree(const Launch &L, int grid, cudaStream_t st);
 cudaError_t launch_direct(const Launch &L, int grid, cudaStream_t st);
 // pivoted-LU evaluation of the points marked in the chunk partials' fb_mask

@@ -7,18 +7,6 @@
 // principal submatrix of one (2n+1)^2 matrix G (vertex j forward = row 2j, backward =
 // row 2j+1, external = row 2n).
 //
-// Tree kernel: Gaussian elimination of G with the pivot of vertex k taken on the
-// diagonal entry of the chosen copy (2k or 2k+1) visits all 2^n configurations as the
-// leaves of a binary tree; the Schur complement of a node is shared by its whole
-// subtree. At a leaf, det(s2_a) is the product of the pivots along the path (spin
-// symmetric models) and the remaining 1x1 Schur complement of the external corner is
-// det(s1_a)/det(s2_a). Cost O(2^n) complex FMAs per point instead of O(2^n n^3).
-// The top levels run breadth-first in shared memory (two 20.7 KB frontier buffers,
-// ping-pong), the last three (two at orders 3 and 4) per thread in registers. Orders above
-// 8 walk their first n-8 levels one root-to-subtree path at a time. Per G-batch of points
-// every table lookup is issued at once and G staged in global memory; each sub-batch's G
-// is copied into shared memory asynchronously while the previous sub-batch's bottom runs.
-//
 // Direct kernel: keldy's own algorithm, one partial-pivot LU pair per configuration
 // (pivot = first maximum of |re|+|im|, as LAPACK's zgetf2). It serves models whose
 // spin-down tables differ from spin-up ones, points whose tree pivots fall below the
@@ -38,23 +26,6 @@ constexpr int NT = CTA_THREADS;
 // first of the set-up slot's three rows of per-point bin data (after the coordinates,
 // the Jacobians and the flags)
 constexpr int BIN_CODE_ROW = MAX_ORDER + 2;
-// Threads of a tree-kernel CTA: eight per 9x9 node (16 nodes per sub-batch at orders 5..8),
-// four per 7x7 node (up to 32 at orders 3 and 4).
-constexpr int TREE_THREADS = CTA_THREADS;
-
-struct TreeShared {
-  double2 buf[2][FRONTIER];
-  double2 D[2][NT];  // prefix determinant per node (ping-pong with the frontier)
-  double2 tmp[NT];   // pivot reciprocals during a level; per-node partial sums after the bottom
-  double u[256];     // vertex times, u[j * np + p]
-  double jac[NT];
-  double2 fval[NT];
-  double fscale[NT];
-  int flag[NT];      // bit 0: out of domain, bit 1: needs the pivoted-LU kernel
-  double2 wsum[TREE_THREADS / 32]; // per-warp partial sums of the per-point reduction
-  double wscale[TREE_THREADS / 32];
-};
-
 __device__ __forceinline__ int find_item(const long long *off, int n_items, long long c) {
   int lo = 0, hi = n_items; // off[lo] <= c < off[hi]
   while (hi - lo > 1) {
@@ -313,621 +284,6 @@ __device__ void build_G_any(const ItemDev &it, int N, int np, const double *u, c
     build_G<false, GK>(it, N, np, u, flag, buf, spin, bad);
 }
 
-// 16-byte asynchronous copies global -> shared (the L2-only variant: the source was
-// written by this CTA moments before), and the wait for the calling thread's copies.
-__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// Copies n complex entries (the staged G of a sub-batch) into shared memory, spread over
-// the CTA's threads; completed by cp_async_wait_all and a barrier.
-__device__ __forceinline__ void copy_roots(double2 *dst, const double2 *src, int n) {
-  for (int e = threadIdx.x; e < n; e += blockDim.x) cp_async16(dst + e, src + e);
-}
-
-// One breadth-first level, both children of a node from one read of its rows: thread r
-// takes row i of parent `par` and writes row i of children 2 par (pivot on row 0) and
-// 2 par + 1 (pivot on row 1). Nodes per point = 2^lg_npp; m >= 9.
-__device__ void tree_level2(const double2 *cur, double2 *nxt, const double2 *Dc, double2 *Dn, double2 *inv,
-                            int *flag, int nodes, int lg_npp, int m, double floor_) {
-  const int mc = m - 2, mm = m * m, mcc = mc * mc;
-  for (int c = threadIdx.x; c < 2 * nodes; c += blockDim.x) {
-    int par = c >> 1, b = c & 1;
-    double2 piv = cur[par * mm + b * (m + 1)];
-    if (!(cabs1(piv) >= floor_)) flag[par >> lg_npp] |= 2;
-    inv[c] = crcp(piv);
-    Dn[c] = cmul(Dc[par], piv);
-  }
-  __syncthreads();
-  const unsigned rows = (unsigned)(nodes * mc);
-  const unsigned magic = 0xFFFFFFFFu / (unsigned)mc + 1u; // r / mc == umulhi(r, magic) for r < 2^20, mc <= 31
-  // split rows into column segments of at least 4 columns while the CTA has idle threads
-  int lgseg = 0;
-  while ((rows << (lgseg + 1)) <= blockDim.x && (mc >> (lgseg + 1)) >= 4) ++lgseg;
-  const int seglen = (mc + (1 << lgseg) - 1) >> lgseg;
-  const unsigned items = rows << lgseg;
-  for (unsigned t = threadIdx.x; t < items; t += blockDim.x) {
-    const unsigned r = t >> lgseg;
-    const int j0 = (int)(t & ((1u << lgseg) - 1)) * seglen, j1 = min(mc, j0 + seglen);
-    const unsigned par = __umulhi(r, magic);
-    const unsigned i = r - par * (unsigned)mc;
-    const double2 *S = cur + par * mm;
-    const double2 L0 = cmul(S[(i + 2) * m], inv[2 * par]);
-    const double2 L1 = cmul(S[(i + 2) * m + 1], inv[2 * par + 1]);
-    const double2 *srow = S + (i + 2) * m + 2, *p0 = S + 2, *p1 = S + m + 2;
-    double2 *o0 = nxt + (2 * par) * mcc + i * mc, *o1 = o0 + mcc;
-#pragma unroll 4
-    for (int j = j0; j < j1; ++j) {
-      const double2 v = srow[j];
-      o0[j] = cfms(v, L0, p0[j]);
-      o1[j] = cfms(v, L1, p1[j]);
-    }
-  }
-  __syncthreads();
-}
-
-// Two breadth-first levels at once: node `par` (m x m) into its four grandchildren
-// 4 par + 2 b + bp (pivot on row b, then on row bp of that child), (m-4) x (m-4) each,
-// every entry formed exactly as two tree_level2 steps form it. A pre-pass forms each
-// parent's pivot quantities once (one thread per (parent, b, b'), into pv); then each item
-// (grandchild row i of a parent, one first pivot b, a column segment) forms the entries of
-// child b it needs itself and writes row i of grandchildren (b, 0) and (b, 1), so the pair
-// takes two barriers and never stores the children. (Items of both first pivots, twice the
-// work per item and half the items, were 6 % slower at order 8 and 3-5 % at orders 6, 7,
-// 9 and 10: the first pair of a one-point sub-batch had 26 busy threads of 128. Items
-// that formed the pivot quantities themselves, six reciprocals each, with one barrier per
-// pair, were slower again, 4-13 % at orders 6-10. A pre-pass that also formed the
-// grandchildren's pivot rows, three complex products per column and item instead of five,
-// was slower as well: four loads per three products, less work in flight per thread.)
-__device__ void tree_level4(const double2 *cur, double2 *nxt, const double2 *Dc, double2 *Dn, int *flag, int nodes,
-                            int lg_npp, int m, double floor_, double2 *pv) {
-  const int mg = m - 4, mm = m * m, mgg = mg * mg;
-  // the pivot quantities of every (parent, b, b') once, before the rows (pv: 12 entries
-  // per parent): the first pivot's reciprocal, child row b''s factor and the second
-  // pivot's reciprocal; the guard flags and the grandchildren's prefix determinants
-  for (int c = threadIdx.x; c < nodes * 4; c += blockDim.x) {
-    const int par = c >> 2, b = (c >> 1) & 1, bp = c & 1;
-    const double2 *S = cur + par * mm;
-    const double2 piv = S[b * (m + 1)];
-    const double2 ibv = crcp(piv);
-    const double2 Lpv = cmul(S[(2 + bp) * m + b], ibv); // child row bp's factor
-    const double2 cpv = cfms(S[(2 + bp) * m + 2 + bp], Lpv, S[b * m + 2 + bp]);
-    pv[c * 3 + 0] = ibv;
-    pv[c * 3 + 1] = Lpv;
-    pv[c * 3 + 2] = crcp(cpv);
-    if (!(cabs1(piv) >= floor_) || !(cabs1(cpv) >= floor_)) flag[par >> lg_npp] |= 2;
-    Dn[c] = cmul(cmul(Dc[par], piv), cpv);
-  }
-  __syncthreads();
-  if (nodes == 1) {
-    // a single parent (the first pair of a one-point sub-batch, orders 8 and up): items of
-    // one row, one b and one b', each writing one grandchild's row, so that 104 threads
-    // work at order 8 instead of 52 (order 8 -0.7 %, order 10 -3 %)
-    int lgs = 0;
-    while (((4 * mg) << (lgs + 1)) <= (int)blockDim.x && (mg >> (lgs + 1)) >= 4) ++lgs;
-    const int sl = (mg + (1 << lgs) - 1) >> lgs;
-    const int nit = (4 * mg) << lgs;
-    for (int t = threadIdx.x; t < nit; t += blockDim.x) {
-      const int q4 = t >> lgs;
-      const int j0 = (t & ((1 << lgs) - 1)) * sl, j1 = min(mg, j0 + sl);
-      const int c = q4 & 3, b = c >> 1, bp = c & 1, i = q4 >> 2;
-      const double2 *S = cur;
-      const double2 Lr = cmul(S[(i + 4) * m + b], pv[(2 * b) * 3]);
-      const double2 Lp = pv[c * 3 + 1];
-      const double2 Lg = cmul(cfms(S[(i + 4) * m + 2 + bp], Lr, S[b * m + 2 + bp]), pv[c * 3 + 2]);
-      const double2 *sr = S + (i + 4) * m + 4, *sb = S + b * m + 4, *sa = S + (2 + bp) * m + 4;
-      double2 *o = nxt + c * mgg + i * mg;
-#pragma unroll 3
-      for (int j = j0; j < j1; ++j) {
-        const double2 pb = sb[j];
-        const double2 cij = cfms(sr[j], Lr, pb); // child b, row i + 2
-        const double2 cc = cfms(sa[j], Lp, pb);  // child b, row b' (the second pivot row)
-        o[j] = cfms(cij, Lg, cc);
-      }
-    }
-    __syncthreads();
-    return;
-  }
-  const unsigned rows = (unsigned)(nodes * mg);
-  const unsigned magic = 0xFFFFFFFFu / (unsigned)mg + 1u; // r / mg == umulhi(r, magic) for r < 2^20, mg <= 31
-  // column segments of at least two columns while the CTA has idle threads; four for a
-  // single node (a one-point sub-batch's first pair, orders 8 and up), where fewer, longer
-  // segments repeat each item's own quantities (Lr, the child-row entries, Lg) less often
-  const int minc = nodes == 1 ? 4 : 2;
-  int lgseg = 0;
-  while (((2 * rows) << (lgseg + 1)) <= blockDim.x && (mg >> (lgseg + 1)) >= minc) ++lgseg;
-  const int seglen = (mg + (1 << lgseg) - 1) >> lgseg;
-  const unsigned items = (2 * rows) << lgseg;
-  for (unsigned t = threadIdx.x; t < items; t += blockDim.x) {
-    const unsigned rb2 = t >> lgseg;
-    const int j0 = (int)(t & ((1u << lgseg) - 1)) * seglen, j1 = min(mg, j0 + seglen);
-    const int b = (int)(rb2 & 1u);
-    const unsigned r = rb2 >> 1;
-    const unsigned par = __umulhi(r, magic);
-    const int i = (int)(r - par * (unsigned)mg);
-    const double2 *S = cur + par * mm;
-    const double2 ib = pv[(par * 4 + 2 * b) * 3];
-    const double2 Lr = cmul(S[(i + 4) * m + b], ib);
-    const double2 Lp0 = pv[(par * 4 + 2 * b) * 3 + 1], Lp1 = pv[(par * 4 + 2 * b + 1) * 3 + 1];
-    const double2 Lg0 = cmul(cfms(S[(i + 4) * m + 2], Lr, S[b * m + 2]), pv[(par * 4 + 2 * b) * 3 + 2]);
-    const double2 Lg1 = cmul(cfms(S[(i + 4) * m + 3], Lr, S[b * m + 3]), pv[(par * 4 + 2 * b + 1) * 3 + 2]);
-    const double2 *sr = S + (i + 4) * m + 4, *sb = S + b * m + 4, *s2 = S + 2 * m + 4, *s3 = S + 3 * m + 4;
-    double2 *o = nxt + (4 * par + 2 * b) * mgg + i * mg;
-    // (unrolled by 2 the kernel spilled five times as many bytes and ran 3-16 % slower)
-#pragma unroll 3
-    for (int j = j0; j < j1; ++j) {
-      const double2 v = sr[j], pb = sb[j], a2 = s2[j], a3 = s3[j];
-      const double2 cij = cfms(v, Lr, pb);  // child b, row i + 2
-      const double2 c0 = cfms(a2, Lp0, pb); // child b, row 0 (pivot row of b' = 0)
-      const double2 c1 = cfms(a3, Lp1, pb); // child b, row 1
-      o[j] = cfms(cij, Lg0, c0);
-      o[mgg + j] = cfms(cij, Lg1, c1);
-    }
-  }
-  __syncthreads();
-}
-
-
-// One step down a fixed path (single point): pivot on row b, drop rows 0 and 1.
-__device__ void tree_path_step(const double2 *cur, double2 *nxt, const double2 *Dc, double2 *Dn, int *flag, int m,
-                               int b, double floor_) {
-  const int mc = m - 2;
-  // every thread forms the pivot's reciprocal itself: no barrier before the row updates
-  const double2 piv = cur[b * m + b];
-  const double2 inv = crcp(piv);
-  if (threadIdx.x == 0) {
-    if (!(cabs1(piv) >= floor_)) flag[0] |= 2;
-    Dn[0] = cmul(Dc[0], piv);
-  }
-  const unsigned magic = 0xFFFFFFFFu / (unsigned)mc + 1u; // r / mc == umulhi(r, magic) for r < 2^20, mc >= 2
-  for (int r = threadIdx.x; r < mc * mc; r += blockDim.x) {
-    const int i = (int)__umulhi((unsigned)r, magic), j = r - i * mc;
-    double2 Lf = cmul(cur[(i + 2) * m + b], inv);
-    nxt[r] = cfms(cur[(i + 2) * m + j + 2], Lf, cur[b * m + j + 2]);
-  }
-  __syncthreads();
-}
-
-// Last two levels of a 5x5 node in registers: children on pivots 0/1, then the four
-// leaves, each leaf term (-1)^|a| det(s2)^2 * (1x1 Schur complement) written without
-// division as Db^2 T_cc (T_cc T_ee - T_ce T_ec).
-__device__ __forceinline__ void tree_bottom5r(const double2 (&s)[25], double2 D, int parity, double floor_,
-                                              bool want_scale, double2 &sum, double &scale, bool &guard) {
-  sum = c2(0.0, 0.0);
-  scale = 0.0;
-#pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    double2 piv = s[b * 6];
-    if (!(cabs1(piv) >= floor_)) guard = true;
-    double2 inv = crcp(piv);
-    double2 Db = cmul(D, piv);
-    double2 T[9];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      double2 Lf = cmul(s[(i + 2) * 5 + b], inv);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) T[i * 3 + j] = cfms(s[(i + 2) * 5 + j + 2], Lf, s[b * 5 + j + 2]);
-    }
-    double2 Db2 = cmul(Db, Db);
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      double2 q = cmul(T[c * 4], cfms(cmul(T[c * 4], T[8]), T[c * 3 + 2], T[6 + c]));
-      double2 term = cmul(Db2, q);
-      if ((b ^ c) & 1)
-        sum = c2(sum.x - term.x, sum.y - term.y);
-      else
-        sum = cadd(sum, term);
-      if (want_scale) scale += cabs(term);
-    }
-  }
-  if (parity & 1) sum = c2(-sum.x, -sum.y);
-}
-
-__device__ __forceinline__ void tree_bottom5(const double2 *R, double2 D, int parity, double floor_, bool want_scale,
-                                             double2 &sum, double &scale, bool &guard) {
-  double2 s[25];
-#pragma unroll
-  for (int i = 0; i < 25; ++i) s[i] = R[i];
-  tree_bottom5r(s, D, parity, floor_, want_scale, sum, scale, guard);
-}
-
-// Grandchild (b, bp) of a 7x7 node (shared memory; rows 0,1: vertex k, 2,3: vertex k+1,
-// 4,5: vertex k+2, 6: external) in registers: eliminate row b, then row 2 + bp of the
-// child, leaving the 3x3 Schur complement T over rows {4, 5, 6}; then its two leaves,
-// each (-1)^|a| det(s2)^2 T_cc (T_cc T_ee - T_ce T_ec). Only the child's entries that T
-// needs are formed (rows and columns 2 + bp, 4, 5, 6), each as the two-level scheme forms it.
-__device__ __forceinline__ void tree_bottom7q(const double2 *S, double2 D, int b, int bp, int parity, double floor_,
-                                              bool want_scale, double2 &sum, double &scale, bool &guard) {
-  const double2 p1 = S[b * 8];
-  if (!(cabs1(p1) >= floor_)) guard = true;
-  const double2 i1 = crcp(p1);
-  const int c0 = 2 + bp;
-  // child row c0 at columns c0, 4, 5, 6
-  double2 a0[4];
-  {
-    const double2 Lf = cmul(S[c0 * 7 + b], i1);
-    a0[0] = cfms(S[c0 * 7 + c0], Lf, S[b * 7 + c0]);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) a0[j + 1] = cfms(S[c0 * 7 + 4 + j], Lf, S[b * 7 + 4 + j]);
-  }
-  const double2 p2 = a0[0];
-  if (!(cabs1(p2) >= floor_)) guard = true;
-  const double2 i2 = crcp(p2);
-  double2 T[9];
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    const int ri = 4 + r;
-    const double2 Lf = cmul(S[ri * 7 + b], i1);
-    const double2 ar0 = cfms(S[ri * 7 + c0], Lf, S[b * 7 + c0]);
-    const double2 L2 = cmul(ar0, i2);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) T[r * 3 + j] = cfms(cfms(S[ri * 7 + 4 + j], Lf, S[b * 7 + 4 + j]), L2, a0[j + 1]);
-  }
-  const double2 Db = cmul(cmul(D, p1), p2);
-  const double2 Db2 = cmul(Db, Db);
-  sum = c2(0.0, 0.0);
-  scale = 0.0;
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    const double2 q = cmul(T[c * 4], cfms(cmul(T[c * 4], T[8]), T[c * 3 + 2], T[6 + c]));
-    const double2 term = cmul(Db2, q);
-    if ((b ^ bp ^ c) & 1)
-      sum = c2(sum.x - term.x, sum.y - term.y);
-    else
-      sum = cadd(sum, term);
-    if (want_scale) scale += cabs(term);
-  }
-  if (parity & 1) sum = c2(-sum.x, -sum.y);
-}
-
-// Sums (v, sc) over aligned groups of G consecutive threads (G a power of two <= TREE_THREADS)
-// and adds group g's sum to fval[g], fscale[g] for g < ngroups. Fixed shuffle pattern:
-// deterministic. Every thread of the CTA calls it.
-__device__ void group_sum(double2 v, double sc, int G, int ngroups, double2 *fval, double *fscale, double2 *wsum,
-                          double *wscale) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int gw = G < 32 ? G : 32;
-  for (int off = 1; off < gw; off <<= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
-    sc += __shfl_xor_sync(0xffffffffu, sc, off);
-  }
-  if (G <= 32) {
-    const int g = tid / G;
-    if ((lane & (G - 1)) == 0 && g < ngroups) {
-      fval[g] = cadd(fval[g], v);
-      fscale[g] += sc;
-    }
-    __syncthreads();
-  } else {
-    if (lane == 0) {
-      wsum[warp] = v;
-      wscale[warp] = sc;
-    }
-    __syncthreads();
-    const int wpg = G / 32;
-    if (tid < ngroups) {
-      double2 f = fval[tid];
-      double s2 = fscale[tid];
-      for (int w = tid * wpg; w < (tid + 1) * wpg; ++w) {
-        f = cadd(f, wsum[w]);
-        s2 += wscale[w];
-      }
-      fval[tid] = f;
-      fscale[tid] = s2;
-    }
-    __syncthreads();
-  }
-}
-
-// Great-grandchild (b, bp, bq) of a 9x9 node (shared memory; rows 0,1: vertex k, 2,3:
-// vertex k+1, 4,5: vertex k+2, 6,7: vertex k+3, 8: external) in registers: the
-// eliminations of row b, then 2 + bp, then 4 + bq, every entry formed as the breadth-first
-// levels and tree_bottom7q form it (so each leaf term is the same number), leaving the
-// 3x3 Schur complement T over rows {6, 7, 8}; then its two leaves,
-// each (-1)^|a| det(s2)^2 T_cc (T_cc T_ee - T_ce T_ec).
-__device__ __forceinline__ void tree_bottom9(const double2 *S, double2 D, int b, int bp, int bq, int parity,
-                                             double floor_, bool want_scale, double2 &sum, double &scale,
-                                             bool &guard) {
-  constexpr int W = 9;
-  const int c = 2 + bp, d = 4 + bq;
-  const int cols[5] = {c, d, 6, 7, 8};
-  const double2 p1 = S[b * W + b];
-  if (!(cabs1(p1) >= floor_)) guard = true;
-  const double2 i1 = crcp(p1);
-  double2 rb[5]; // row b at the columns that remain needed
-#pragma unroll
-  for (int k = 0; k < 5; ++k) rb[k] = S[b * W + cols[k]];
-  // child row c (first elimination) at columns {c, d, 6, 7, 8}
-  double2 rc[5];
-  {
-    const double2 Lf = cmul(S[c * W + b], i1);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) rc[k] = cfms(S[c * W + cols[k]], Lf, rb[k]);
-  }
-  const double2 p2 = rc[0];
-  if (!(cabs1(p2) >= floor_)) guard = true;
-  const double2 i2 = crcp(p2);
-  // grandchild row d (second elimination) at columns {d, 6, 7, 8}
-  double2 rd[4];
-  {
-    const double2 Lf = cmul(S[d * W + b], i1);
-    const double2 a = cfms(S[d * W + c], Lf, rb[0]);
-    const double2 L2 = cmul(a, i2);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) rd[k] = cfms(cfms(S[d * W + cols[k + 1]], Lf, rb[k + 1]), L2, rc[k + 1]);
-  }
-  const double2 p3 = rd[0];
-  if (!(cabs1(p3) >= floor_)) guard = true;
-  const double2 i3 = crcp(p3);
-  // T row r - 6 at columns {6, 7, 8} (third elimination)
-  double2 T[9];
-#pragma unroll
-  for (int rr = 0; rr < 3; ++rr) {
-    const int r = 6 + rr;
-    const double2 Lf = cmul(S[r * W + b], i1);
-    const double2 a0 = cfms(S[r * W + c], Lf, rb[0]);
-    const double2 L2 = cmul(a0, i2);
-    const double2 a1 = cfms(cfms(S[r * W + d], Lf, rb[1]), L2, rc[1]);
-    const double2 L3 = cmul(a1, i3);
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-      T[rr * 3 + j] = cfms(cfms(cfms(S[r * W + 6 + j], Lf, rb[2 + j]), L2, rc[2 + j]), L3, rd[1 + j]);
-  }
-  const double2 Db = cmul(cmul(cmul(D, p1), p2), p3);
-  const double2 Db2 = cmul(Db, Db);
-  sum = c2(0.0, 0.0);
-  scale = 0.0;
-#pragma unroll
-  for (int cc = 0; cc < 2; ++cc) {
-    const double2 q = cmul(T[cc * 4], cfms(cmul(T[cc * 4], T[8]), T[cc * 3 + 2], T[6 + cc]));
-    const double2 term = cmul(Db2, q);
-    if ((b ^ bp ^ bq ^ cc) & 1)
-      sum = c2(sum.x - term.x, sum.y - term.y);
-    else
-      sum = cadd(sum, term);
-    if (want_scale) scale += cabs(term);
-  }
-  if (parity & 1) sum = c2(-sum.x, -sum.y);
-}
-
-// Per-point sums of the fused bottom (thread q * NODES + node, 2^lg nodes per point): lane
-// groups of consecutive nodes by shuffles, then each point's groups and the
-// TREE_THREADS / NODES descendant slots q in a fixed order by thread p; adds to fval[p],
-// fscale[p]. Every thread calls it; scratch: 256 double2 + 256 double of free shared memory
-// (BOTTOM_SCRATCH entries), read until the caller's next barrier.
-template <int NODES>
-__device__ void bottom_sum(double2 v, double sc, int lg, int np, double2 *fval, double *fscale, double2 *scratch) {
-  static_assert(NODES >= 16 && NODES * (TREE_THREADS / NODES) == TREE_THREADS, "descendant slots of the CTA");
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int g = lg < 5 ? (1 << lg) : 32;
-  for (int off = 1; off < g; off <<= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
-    sc += __shfl_xor_sync(0xffffffffu, sc, off);
-  }
-  double *sscale = reinterpret_cast<double *>(scratch + TREE_THREADS);
-  if ((lane & (g - 1)) == 0) {
-    scratch[tid] = v;
-    sscale[tid] = sc;
-  }
-  __syncthreads();
-  if (tid < np) {
-    const int per = 1 << lg;
-    double2 f = fval[tid];
-    double s2 = fscale[tid];
-    for (int q = 0; q < TREE_THREADS / NODES; ++q)
-      for (int nd = tid * per; nd < (tid + 1) * per; nd += g) {
-        f = cadd(f, scratch[q * NODES + nd]);
-        s2 += sscale[q * NODES + nd];
-      }
-    fval[tid] = f;
-    fscale[tid] = s2;
-  }
-}
-
-// Order 1: the 3x3 root's two leaves directly.
-__device__ __forceinline__ void tree_bottom3(const double2 *R, double2 &sum, double &scale, bool want_scale) {
-  sum = c2(0.0, 0.0);
-  scale = 0.0;
-#pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    double2 piv = R[b * 4];
-    double2 term = cmul(piv, cfms(cmul(piv, R[8]), R[b * 3 + 2], R[6 + b]));
-    if (b)
-      sum = c2(sum.x - term.x, sum.y - term.y);
-    else
-      sum = cadd(sum, term);
-    if (want_scale) scale += cabs(term);
-  }
-}
-
-// One sub-batch of np points (N <= TREE_MAX_SUB, or the subtree of a path pass) whose
-// root matrices sit at `root` in frontier buffer rb, with S.D[rb][node] their prefix
-// determinants: the breadth-first levels, then the fused bottom, each point's sum added
-// to fval[p] (fscale[p]) and bit 1 of flag[p] set where a pivot fell below the guard.
-// pf_n > 0: copies pf_n staged entries from pf_src to the buffer the bottom does not read
-// (at offset roff, past the bottom's scratch) while the bottom runs, for the next
-// sub-batch. Returns the buffer the bottom read. The per-point sums are read from the
-// bottom's scratch until the caller's next barrier.
-__device__ int tree_sub(TreeShared &S, int N, int np, int rb, const double2 *root, int *flag, double2 *fval,
-                        double *fscale, double floor_, bool want_scale, int parity0, const double2 *pf_src,
-                        int pf_n, int roff) {
-  const int tid = threadIdx.x;
-  // breadth-first levels down to 9x9 nodes, then the fused bottom of three eliminations;
-  // orders 3 and 4 go down to 7x7 nodes and a bottom of two (three were 4 % slower at 4)
-  const int LB = N >= 5 ? N - 4 : (N >= 3 ? N - 3 : 0);
-  int m = 2 * N + 1, cur = rb, nodes = np, lg = 0;
-  const double2 *src = root;
-  for (int k = 0; k + 1 < LB; k += 2) { // pairs of levels, then a last single one
-    tree_level4(src, S.buf[cur ^ 1], S.D[cur], S.D[cur ^ 1], flag, nodes, lg, m, floor_, S.tmp);
-    nodes *= 4;
-    lg += 2;
-    m -= 4;
-    cur ^= 1;
-    src = S.buf[cur];
-  }
-  if (LB & 1) {
-    tree_level2(src, S.buf[cur ^ 1], S.D[cur], S.D[cur ^ 1], S.tmp, flag, nodes, lg, m, floor_);
-    nodes *= 2;
-    lg += 1;
-    m -= 2;
-    cur ^= 1;
-    src = S.buf[cur];
-  }
-  if (pf_n > 0) copy_roots(S.buf[cur ^ 1] + roff, pf_src, pf_n);
-  double2 v = c2(0.0, 0.0);
-  double sc = 0.0;
-  bool guard = false;
-  int p = 0;
-  if (m == 7) { // four threads per 7x7 node: grandchild tid >> 5 of node tid & 31, so that a
-                // warp's lanes read consecutive nodes (49-entry stride: no bank conflicts)
-    const int node = tid & 31, q = tid >> 5;
-    if (node < nodes) {
-      p = node >> lg;
-      const int parity = __popc(node & ((1 << lg) - 1)) + parity0;
-      tree_bottom7q(src + node * 49, S.D[cur][node], q >> 1, q & 1, parity, floor_, want_scale, v, sc, guard);
-    }
-    if (guard) flag[p] |= 2;
-    bottom_sum<32>(v, sc, lg, np, fval, fscale, S.buf[cur ^ 1]);
-  } else if (m == 9) { // eight threads per 9x9 node: great-grandchild tid >> 4 of node tid & 15
-    const int node = tid & 15, q = tid >> 4;
-    if (node < nodes) {
-      p = node >> lg;
-      const int parity = __popc(node & ((1 << lg) - 1)) + parity0;
-      tree_bottom9(src + node * 81, S.D[cur][node], q >> 2, (q >> 1) & 1, q & 1, parity, floor_, want_scale, v, sc,
-                   guard);
-    }
-    if (guard) flag[p] |= 2;
-    bottom_sum<16>(v, sc, lg, np, fval, fscale, S.buf[cur ^ 1]);
-  } else { // orders 1 and 2: the root itself, one thread per point
-    if (tid < nodes) {
-      p = tid;
-      if (m == 5)
-        tree_bottom5(src + tid * 25, S.D[cur][tid], parity0, floor_, want_scale, v, sc, guard);
-      else
-        tree_bottom3(src + tid * 9, v, sc, want_scale);
-    }
-    if (guard) flag[p] |= 2;
-    group_sum(v, sc, 1, np, fval, fscale, S.wsum, S.wscale);
-  }
-  return cur;
-}
-
-// Where a sub-batch's roots go when they are copied while the previous sub-batch's bottom
-// runs: past the bottom's scratch (orders 3 and up) of the buffer the bottom does not read.
-// -1: they do not fit beside it (order 3); those sub-batches copy theirs after a barrier.
-__device__ __forceinline__ int tree_prefetch_offset(int N, int P) {
-  const int off = N >= 3 ? BOTTOM_SCRATCH : 0;
-  return off + P * (2 * N + 1) * (2 * N + 1) <= FRONTIER ? off : -1;
-}
-
-// The G-batch's points (gb, staged G at gst: point p at p M^2): the integrand of each,
-// added to S.fval[p] (S.fscale[p]) with bit 1 of S.flag[p] set where a pivot fell below
-// the guard. S.D and the frontier buffers are free on entry; the caller's barrier follows.
-__device__ void tree_gbatch_points(TreeShared &S, const ItemDev &it, int N, int gb, double2 *gst,
-                                   bool want_scale, bool direct, int *bad) {
-  const int tid = threadIdx.x;
-  const int M = 2 * N + 1, MM = M * M;
-  const double floor_ = it.model.pivot_floor;
-  if (N == 0) {
-    if (tid < gb && !(S.flag[tid] & 1)) {
-      kb_gf_index a = it.f.A, b = it.f.B;
-      a.timesplit = 0;
-      b.timesplit = 0;
-      double2 v = g0_contour(it.model, a, b, 0, bad);
-      S.fval[tid] = v;
-      S.fscale[tid] = cabs(v);
-    }
-    return;
-  }
-  if (N > TREE_MAX_SUB) {
-    // one point at a time: the K0 = N - 8 levels above the order-8 subtrees. The last one
-    // (order 9) or two of them run breadth-first (tree_level2 / tree_level4 on one node) into
-    // the staging area after the batch's G matrices, 2^Kb subtree roots of 17 x 17 and their
-    // prefix determinants; the Kp levels before them are walked one root-to-node path at a
-    // time (2^Kp passes, the point's G copied again for each). Against walking all K0 levels
-    // by paths: orders 10 / 12 -4 / -20 %, order 9 +7 % (its one breadth-first level computes
-    // what its two paths did, through the staging area; the code that kept paths for order 9
-    // compiled into a kernel 13 % slower at order 10). Each subtree root is copied into shared memory
-    // asynchronously while the previous subtree's bottom runs. Subtrees are summed in the
-    // order of their path bits, first level first, as walking all K0 levels by paths would.
-    const int K0 = N - TREE_MAX_SUB;
-    const int Kb = K0 >= 2 ? 2 : 1, Kp = K0 - Kb, NS = 1 << Kb;
-    constexpr int R = 2 * TREE_MAX_SUB + 1, RR = R * R;
-    double2 *gsub = gst + (size_t)gb * MM;
-    double2 *gD = gsub + (size_t)NS * RR;
-    const int pf = tree_prefetch_offset(TREE_MAX_SUB, 1);
-    for (int p = 0; p < gb; ++p) {
-      for (int sub = 0; sub < (1 << Kp); ++sub) {
-        copy_roots(S.buf[0], gst + (size_t)p * MM, MM);
-        if (tid == 0) S.D[0][0] = c2(1.0, 0.0);
-        cp_async_wait_all();
-        __syncthreads();
-        int m = M, cur = 0;
-        for (int k = 0; k < Kp; ++k) {
-          const int b = (sub >> (Kp - 1 - k)) & 1;
-          tree_path_step(S.buf[cur], S.buf[cur ^ 1], S.D[cur], S.D[cur ^ 1], S.flag + p, m, b, floor_);
-          m -= 2;
-          cur ^= 1;
-        }
-        if (Kb == 2)
-          tree_level4(S.buf[cur], gsub, S.D[cur], gD, S.flag + p, 1, 0, m, floor_, S.tmp);
-        else
-          tree_level2(S.buf[cur], gsub, S.D[cur], gD, S.tmp, S.flag + p, 1, 0, m, floor_);
-        int rb = 0, roff = 0;
-        for (int g = 0; g < NS; ++g) {
-          if (g == 0) {
-            copy_roots(S.buf[0], gsub, RR);
-            if (tid == 0) S.D[0][0] = gD[0];
-            cp_async_wait_all();
-            __syncthreads();
-          }
-          const bool prefetch = pf >= 0 && g + 1 < NS;
-          const int bot = tree_sub(S, TREE_MAX_SUB, 1, rb, S.buf[rb] + roff, S.flag + p, S.fval + p, S.fscale + p,
-                                   floor_, want_scale, __popc(sub) + __popc(g), gsub + (size_t)(g + 1) * RR,
-                                   prefetch ? RR : 0, pf);
-          if (prefetch) {
-            rb = bot ^ 1;
-            roff = pf;
-            if (tid == 0) S.D[rb][0] = gD[g + 1];
-            cp_async_wait_all();
-          }
-          __syncthreads();
-        }
-      }
-    }
-    return;
-  }
-  const int P = tree_points_per_chunk(N);
-  const int pf = tree_prefetch_offset(N, P);
-  int rb = 0, roff = 0;
-  for (int sb = 0; sb < gb; sb += P) {
-    const int np = min(P, gb - sb);
-    if (sb == 0 || pf < 0) { // copy this sub-batch's roots now (direct: built there already)
-      rb = 0;
-      roff = 0;
-      if (!direct) copy_roots(S.buf[0], gst + (size_t)sb * MM, np * MM);
-      if (tid < np) S.D[0][tid] = c2(1.0, 0.0);
-      cp_async_wait_all();
-      __syncthreads();
-    }
-    const int nsb = sb + P, nnp = min(P, gb - nsb);
-    const bool prefetch = pf >= 0 && nnp > 0;
-    const int bot = tree_sub(S, N, np, rb, S.buf[rb] + roff, S.flag + sb, S.fval + sb, S.fscale + sb, floor_,
-                             want_scale, 0, gst + (size_t)nsb * MM, prefetch ? nnp * MM : 0, pf);
-    if (prefetch) {
-      rb = bot ^ 1;
-      roff = pf;
-      if (tid < nnp) S.D[rb][tid] = c2(1.0, 0.0);
-      cp_async_wait_all();
-    }
-    __syncthreads();
-  }
-}
-
 __device__ __forceinline__ double2 apply_cutoff(double2 f, double cutoff) {
   return (cabs(f) < cutoff) ? c2(0.0, 0.0) : f;
 }
@@ -940,198 +296,6 @@ __device__ __forceinline__ void clear_bins(const Launch &L, int c) {
     L.bin_counts[(size_t)c * L.nbins + b] = 0u;
   }
   if (threadIdx.x == 0) L.bin_dropped[c] = 0u;
-}
-
-// Persistent CTAs pull chunks of up to 128 points. Per chunk: the points' set-up (Sobol
-// coordinates or given inputs, warper chain, domain flag: one thread per point) into the
-// CTA's global slot; then per G-batch of tree_gbatch(N) points: every table lookup of the
-// batch in flight at once (build_G into the slot's staging area), then the trees of its
-// sub-batches, each sub-batch's G copied into shared memory asynchronously while the
-// previous sub-batch's bottom runs; then the batch's values in point order.
-template <bool EVAL, bool ANY_CUBIC>
-__global__ void __launch_bounds__(TREE_THREADS, 4) tree_kernel(Launch L) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TreeShared &S = *reinterpret_cast<TreeShared *>(smem_raw);
-  __shared__ int s_chunk;
-  __shared__ int s_bad;
-  // the chunk's partial sums and dropped count (thread 0), in shared memory so that they
-  // hold no registers through the tree
-  __shared__ ChunkPartial s_part;
-  __shared__ unsigned s_drop;
-  __shared__ unsigned s_bal[3][TREE_THREADS / 32]; // per warp: in-domain, guarded and dropped points of a batch
-  const int tid = threadIdx.x;
-  if (tid == 0) s_bad = 0;
-  for (;;) {
-    if (tid == 0) {
-      s_chunk = atomicAdd(L.chunk_counter, 1);
-      s_part.sum_re = s_part.sum_im = 0.0;
-      s_part.n_in_domain = s_part.n_fallback = 0;
-      s_part.fb_mask[0] = s_part.fb_mask[1] = 0;
-      s_drop = 0;
-    }
-    __syncthreads();
-    const int c = s_chunk;
-    if (c >= L.n_chunks) break;
-    const int item = find_item(L.chunk_offsets, L.n_items, c);
-    const ItemDev &it = L.items[item];
-    const long long cfirst = (long long)(c - L.chunk_offsets[item]) * it.chunk_points;
-    const long long total = EVAL ? (L.index ? (long long)L.n_index : it.n_points) : it.n_points;
-    const int ccount = (int)min((long long)it.chunk_points, total - cfirst);
-    const int N = it.order;
-    const int GB = tree_gbatch(N);
-    const bool keep = (L.mode == IN_SOBOL) ? true : (L.keep_u_hypercube != 0);
-    const bool want_scale = EVAL && L.out_scale != nullptr;
-    double *slot = L.pts + (size_t)blockIdx.x * PTS_SLOT;
-    double2 *gst = reinterpret_cast<double2 *>(slot + PTS_ROWS);
-    if (tid < ccount) prepare_point(L, it, N, cfirst + tid, keep, slot, tid);
-    __syncthreads();
-    for (int g0 = 0; g0 < ccount; g0 += GB) {
-      const int gb = min(GB, ccount - g0);
-      if (tid < gb) {
-        for (int j = 0; j < N; ++j) S.u[j * gb + tid] = slot[j * CHUNK_POINTS + g0 + tid];
-        S.jac[tid] = slot[MAX_ORDER * CHUNK_POINTS + g0 + tid];
-        S.flag[tid] = (int)slot[(MAX_ORDER + 1) * CHUNK_POINTS + g0 + tid];
-        S.fval[tid] = c2(0.0, 0.0);
-        S.fscale[tid] = 0.0;
-      }
-      __syncthreads();
-      const bool direct = tree_direct(N);
-      if (N > 0) {
-        if (direct) // the batch is one sub-batch: G straight into the frontier buffer
-          build_G_any<ANY_CUBIC, 2>(it, N, gb, S.u, S.flag, S.buf[0], it.f.A.spin, &s_bad);
-        else
-          build_G_any<ANY_CUBIC, 4>(it, N, gb, S.u, S.flag, gst, it.f.A.spin, &s_bad);
-        __syncthreads();
-      }
-      tree_gbatch_points(S, it, N, gb, gst, want_scale, direct, &s_bad);
-      if (EVAL) {
-        if (tid < gb) {
-          const long long o = cfirst + g0 + tid;
-          int fl = S.flag[tid];
-          const double2 fv = S.fval[tid];
-          if (!isfinite(fv.x) || !isfinite(fv.y)) fl |= 2;
-          const bool dom = !(fl & 1);
-          const double2 f = dom ? apply_cutoff(fv, it.f.cutoff) : c2(0.0, 0.0);
-          const double j = S.jac[tid];
-          L.out_val[o] = c2(f.x * j, f.y * j);
-          if (L.out_jac) L.out_jac[o] = j;
-          if (L.out_dom) L.out_dom[o] = dom ? 1 : 0;
-          if (L.out_scale) L.out_scale[o] = dom ? S.fscale[tid] * fabs(j) : 0.0;
-          if (L.out_flag) L.out_flag[o] = (dom && (fl & 2)) ? 1 : 0;
-        }
-      } else {
-        // the batch's point values, one thread per point; then each warp's sum in a fixed
-        // shuffle order, and thread 0 adds the warps in order (deterministic)
-        const int lane = tid & 31, w = tid >> 5;
-        bool dom = false, fb = false, drop = false;
-        double2 fj = c2(0.0, 0.0);
-        if (tid < gb) {
-          int fl = S.flag[tid];
-          const double2 fv = S.fval[tid];
-          if (!isfinite(fv.x) || !isfinite(fv.y)) fl |= 2;
-          const int q = g0 + tid;
-          int bin = -2;
-          if (L.nbins) { // the code prepare_point stored: 2 bin, or -1 when dropped
-            const double code = slot[BIN_CODE_ROW * CHUNK_POINTS + q];
-            bin = code < 0.0 ? -1 : (int)code >> 1;
-            drop = bin < 0;
-          }
-          if (!(fl & 1)) {
-            dom = true;
-            fb = (fl & 2) != 0;
-            if (!fb) {
-              const double2 f = apply_cutoff(fv, it.f.cutoff);
-              const double j = S.jac[tid];
-              fj = c2(f.x * j, f.y * j);
-              if (bin >= 0) {
-                slot[BIN_CODE_ROW * CHUNK_POINTS + q] = (double)(2 * bin + 1);
-                slot[(BIN_CODE_ROW + 1) * CHUNK_POINTS + q] = fj.x;
-                slot[(BIN_CODE_ROW + 2) * CHUNK_POINTS + q] = fj.y;
-              }
-            }
-          }
-        }
-        for (int off = 16; off > 0; off >>= 1) {
-          fj.x += __shfl_xor_sync(0xffffffffu, fj.x, off);
-          fj.y += __shfl_xor_sync(0xffffffffu, fj.y, off);
-        }
-        const unsigned bdom = __ballot_sync(0xffffffffu, dom), bfb = __ballot_sync(0xffffffffu, fb);
-        const unsigned bdrop = __ballot_sync(0xffffffffu, drop);
-        if (lane == 0) {
-          S.wsum[w] = fj;
-          s_bal[0][w] = bdom;
-          s_bal[1][w] = bfb;
-          s_bal[2][w] = bdrop;
-        }
-        __syncthreads();
-        if (tid == 0) {
-          double2 csum = c2(s_part.sum_re, s_part.sum_im);
-          unsigned long long cdom = s_part.n_in_domain, cfb = s_part.n_fallback;
-          unsigned long long mask0 = s_part.fb_mask[0], mask1 = s_part.fb_mask[1];
-          unsigned cdrop = s_drop;
-          for (int k = 0; k < TREE_THREADS / 32; ++k) {
-            csum = cadd(csum, S.wsum[k]);
-            cdom += __popc(s_bal[0][k]);
-            cfb += __popc(s_bal[1][k]);
-            cdrop += __popc(s_bal[2][k]);
-            // guarded points' chunk bits: point q = g0 + 32 k + lane
-            const unsigned long long m = s_bal[1][k];
-            const int b0 = g0 + 32 * k;
-            if (m && b0 < 64) {
-              mask0 |= m << b0;
-              if (b0 > 32) mask1 |= m >> (64 - b0);
-            } else if (m) {
-              mask1 |= m << (b0 - 64);
-            }
-          }
-          s_part.sum_re = csum.x;
-          s_part.sum_im = csum.y;
-          s_part.n_in_domain = cdom;
-          s_part.n_fallback = cfb;
-          s_part.fb_mask[0] = mask0;
-          s_part.fb_mask[1] = mask1;
-          s_drop = cdrop;
-        }
-      }
-      __syncthreads();
-    }
-    if (!EVAL && L.nbins) {
-      // the chunk's bins with its points added in point order (the order of one thread
-      // walking the chunk): one thread per bin for up to 512 bins, else one thread over the
-      // points; the pivoted-LU pass adds its points later
-      const double *code = slot + BIN_CODE_ROW * CHUNK_POINTS;
-      const double *vre = code + CHUNK_POINTS, *vim = vre + CHUNK_POINTS;
-      if (L.nbins <= 512) {
-        for (int b = tid; b < L.nbins; b += blockDim.x) {
-          double2 bs = c2(0.0, 0.0);
-          unsigned cnt = 0;
-          for (int q = 0; q < ccount; ++q) {
-            if (code[q] < 0.0 || (int)code[q] >> 1 != b) continue;
-            cnt++;
-            if ((int)code[q] & 1) bs = c2(bs.x + vre[q], bs.y + vim[q]);
-          }
-          L.bin_sums[(size_t)c * L.nbins + b] = bs;
-          L.bin_counts[(size_t)c * L.nbins + b] = cnt;
-        }
-      } else {
-        clear_bins(L, c);
-        __syncthreads();
-        if (tid == 0)
-          for (int q = 0; q < ccount; ++q) {
-            if (code[q] < 0.0) continue;
-            const int b = (int)code[q] >> 1;
-            L.bin_counts[(size_t)c * L.nbins + b]++;
-            if ((int)code[q] & 1) {
-              double2 &bs = L.bin_sums[(size_t)c * L.nbins + b];
-              bs = c2(bs.x + vre[q], bs.y + vim[q]);
-            }
-          }
-      }
-      if (tid == 0) L.bin_dropped[c] = s_drop;
-    }
-    if (!EVAL && tid == 0) L.partials[c] = s_part;
-  }
-  if (tid == 0 && s_bad) atomicOr(L.err, 1);
 }
 
 // ---------------------------------------------------------------- direct kernel
@@ -2138,22 +1302,8 @@ cudaError_t launch_reduce_bins(const Launch &L, double2 *sums, unsigned long lon
   return cudaGetLastError();
 }
 
-size_t tree_smem_bytes() { return sizeof(TreeShared); }
-
-// Shared-memory limit of the four tree-kernel instantiations.
-static cudaError_t configure_tree(int smem) {
-  cudaError_t e = cudaFuncSetAttribute(tree_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tree_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tree_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tree_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  return e;
-}
-
 cudaError_t configure_kernels() {
-  cudaError_t e = configure_tree((int)sizeof(TreeShared));
+  cudaError_t e = configure_tree_kernels();
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DirectShared));
   if (e == cudaSuccess)
@@ -2164,22 +1314,6 @@ cudaError_t configure_kernels() {
 }
 
 static size_t direct_smem_bytes() { return sizeof(DirectShared); }
-
-cudaError_t launch_tree(const Launch &L, int grid, cudaStream_t st) {
-  const size_t smem = tree_smem_bytes();
-  if (L.mode == IN_SOBOL) {
-    if (L.any_cubic)
-      tree_kernel<false, true><<<grid, TREE_THREADS, smem, st>>>(L);
-    else
-      tree_kernel<false, false><<<grid, TREE_THREADS, smem, st>>>(L);
-  } else {
-    if (L.any_cubic)
-      tree_kernel<true, true><<<grid, TREE_THREADS, smem, st>>>(L);
-    else
-      tree_kernel<true, false><<<grid, TREE_THREADS, smem, st>>>(L);
-  }
-  return cudaGetLastError();
-}
 
 cudaError_t launch_direct(const Launch &L, int grid, cudaStream_t st) {
   direct_kernel<<<grid, NT, direct_smem_bytes(), st>>>(L);

@@ -1,0 +1,60 @@
+"""The warp-per-group tree kernel where its layout changes: point counts around a pass (256 >> n
+points), a group (32, 16 above order 8) and a chunk, at every order's first level; times equal
+to each other and to the external times, and vertices later than one or both external points on
+either branch. Against the CPU oracle; |gpu - cpu| <= 1e-12 sum_a |det up det down|, as for the
+other integrand tests."""
+import numpy as np
+import pytest
+
+from keldy_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+ENDS = [((7.0, 0, 0, 0, 0), (7.0, 0, 1, 0, 0)), ((6.0, 0, 1, 0, 0), (3.0, 0, 0, 0, 0)),
+        ((2.5, 1, 0, 0, 0), (8.0, 1, 0, 0, 0)), ((5.0, 0, 1, 0, 0), (5.0, 0, 1, 0, 0))]
+
+
+def _models(ctx, oracle, golden, alpha=0.4):
+    le, gr = golden["table_beta20_lesser"], golden["table_beta20_greater"]
+    return ctx.model(10.0, le, gr, alpha), oracle.model(10.0, le, gr, alpha)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 6, 7, 8, 9, 11])
+def test_point_counts_ties_and_external_order(ctx, oracle, golden, n):
+    gm, om = _models(ctx, oracle, golden)
+    rng = np.random.default_rng(40 + n)
+    per_pass = 32 if n <= 3 else max(1, 256 >> n)
+    counts = {1, per_pass + 1, 33, 2 * per_pass - 1} if n <= 8 else {1, 2, 17} if n == 9 else {2}
+    for k, count in enumerate(sorted(counts)):
+        A, B = ENDS[(n + k) % len(ENDS)]
+        t = rng.random((count, n)) * 10.0
+        if n > 1:
+            t[::2, n - 1] = t[::2, 0]  # equal vertex times
+        t[-1, 0] = A[0]  # a vertex at each external time
+        t[-1, n // 2] = B[0]
+        for scale in (False, True):
+            v, d, *gsc = gm.integrand(A, B, t, algo=capi.ALGO_TREE, want_scale=scale)
+            w, dw, sc = oracle.integrand(om, A, B, t)
+            np.testing.assert_array_equal(d, dw)
+            assert np.all(np.abs(v - w) <= 1e-12 * sc), (n, count, scale)
+            if scale:
+                np.testing.assert_allclose(gsc[0], sc, rtol=1e-9)
+
+
+@pytest.mark.parametrize("chunk", [1, 13, 33, 100, 128])
+def test_chunk_sizes(ctx, oracle, golden, chunk):
+    """Ragged chunks and groups of an integration, with out-of-domain points among the others."""
+    gm, om = _models(ctx, oracle, golden, 0.0)
+    chain = [(capi.WARPER_PLASMA_UV, 10.0, 0.0), (capi.WARPER_INVERSE, 10.0, 2.0)]
+    A, B = (10.0, 0, 0, 0, 0), (10.0, 0, 1, 0, 0)
+    before = ctx.get_launch(3)
+    try:
+        ctx.set_launch(-1, chunk)
+        for n, npts in ((1, 301), (3, 301), (5, 203), (8, 101), (9, 35)):
+            (s, np_, nd, nfb), = capi.integrate(ctx, [dict(model=gm, rng=ctx.sobol(n), chain=chain, A=A, B=B, order=n,
+                                                           k_first=29, n_points=npts)])
+            w, onp, ond, sc = oracle.integrate(om, A, B, [(1, 10.0, 0.0), (3, 10.0, 2.0)], n, npts, seed=28)
+            assert (np_, nd, nfb) == (onp, ond, 0)
+            assert abs(s - w) <= 1e-12 * sc, (n, abs(s - w) / sc)
+    finally:
+        ctx.set_launch(-1, *before)
