@@ -811,17 +811,20 @@ static ItemDev make_item(const kb_model *m, const kb_integrand *f, int order) {
 }
 
 // Points per scheduling chunk of a work item of n points: `most` (the context's chunk size for
-// its order, autotuned or kb_context_set_launch), halved while the item would have fewer chunks
-// than half the resident tree warps, so that a small item is spread over the GPU instead of a
-// few warps walking long chunks (a batch of many small items keeps larger chunks than one
-// small item alone would need). Not below the size at which a group's set-up is a small part
-// of its work: 8 points up to order 5, 4 up to order 8, then 2 and 1. It depends on the item
+// its order, autotuned or kb_context_set_launch), halved down to a full group (32 points, 16 above
+// order 8) while the item would have fewer than eight chunks per resident tree warp (at most
+// `limit`), so that the last chunks of a large item leave no warp idle for long: 2^18 points of
+// order 7 in 2,048 chunks of 128 on 1,776 warps were two rounds for 1.15. A smaller group costs:
+// with 8 points per chunk instead of 32, order 8 takes 26 %, order 6 48 % and order 2 three times
+// as long, so below a full group (down to 8 points, 4 from order 6 on, 1 from order 10 on) only
+// while the item would have fewer chunks than an eighth of the warps. It depends on the item
 // alone: a batch adds each item's points in the order of a call of its own.
-static int item_chunk(const kb_context *ctx, int order, int64_t n, int most) {
+static int item_chunk(const kb_context *ctx, int order, int64_t n, int most, int64_t limit) {
   int c = most;
-  const int64_t want = std::min((int64_t)ctx->sm_count * ctx->ctas_per_sm * TREE_WARPS / 2, MAX_SPLIT_CHUNKS);
-  const int least = order <= 5 ? 8 : order <= 8 ? 4 : order == 9 ? 2 : 1;
-  while (c > least && (n + c - 1) / c < want) c >>= 1;
+  const int64_t warps = (int64_t)ctx->sm_count * ctx->ctas_per_sm * TREE_WARPS;
+  const int full = order <= 8 ? 32 : 16, least = order <= 5 ? 8 : order <= 8 ? 4 : order == 9 ? 2 : 1;
+  while (c > full && (n + c - 1) / c < std::min(8 * warps, limit)) c >>= 1;
+  while (c > least && (n + c - 1) / c < warps / 8) c >>= 1;
   return c;
 }
 
@@ -839,7 +842,7 @@ static int run_eval(kb_context *ctx, ItemDev it, int mode, int64_t count, const 
   const bool use_tree = (algo == KB_ALGO_TREE) || (algo == KB_ALGO_AUTO && it.spin_symmetric);
   if (algo == KB_ALGO_TREE && !it.spin_symmetric)
     return fail(KB_E_INVALID, "the tree algorithm needs equal spin-up and spin-down g0 tables");
-  if (use_tree) it.chunk_points = item_chunk(ctx, N, count, 32); // a warp per chunk: 32 points fill its lanes
+  if (use_tree) it.chunk_points = item_chunk(ctx, N, count, 32, INT64_MAX); // a warp per chunk: 32 points fill its lanes
   long long nchunks = (count + it.chunk_points - 1) / it.chunk_points;
   long long offs[2] = {0, nchunks};
   DevBuf ditem, doff, dcnt, din, dval, djac, ddom, dscale, dflag;
@@ -1181,7 +1184,7 @@ int work_item(kb_context *ctx, const kb_work &w, int algo, ItemDev &it, int &tre
   it.rng = sobol_dev(w.rng);
   it.k_first = w.k_first;
   it.n_points = w.n_points;
-  it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order]);
+  it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order], INT64_MAX);
   if (w.flow && w.flow->layout.kind == FLOW_KIND_SPLINE) it.spline_knots = w.flow->knots; // mapped in line
   if (w.flow && w.flow->layout.kind == FLOW_KIND_AR_SPLINE) it.ar_spline = w.flow->master; // mapped in line
   if (algo == KB_ALGO_TREE && !it.spin_symmetric)
@@ -1850,8 +1853,9 @@ constexpr size_t NOALLOC_ACC_OFF = ((NOALLOC_OFFS_OFF + sizeof(long long) * (KB_
 constexpr size_t NOALLOC_CNT_OFF = NOALLOC_ACC_OFF + sizeof(kb_accum) * 2 * KB_NOALLOC_MAX_ITEMS;
 constexpr size_t NOALLOC_PART_OFF = (NOALLOC_CNT_OFF + sizeof(int) + 255) / 256 * 256;
 // An item's chunks number at most its chunks in the documented unit (noalloc_unit), or twice
-// MAX_SPLIT_CHUNKS where item_chunk split a small item further.
-constexpr size_t NOALLOC_PARTIALS = KB_NOALLOC_MAX_CHUNKS + KB_NOALLOC_MAX_ITEMS * 2 * MAX_SPLIT_CHUNKS;
+// NOALLOC_SPLIT_CHUNKS where item_chunk split a small item further.
+constexpr int64_t NOALLOC_SPLIT_CHUNKS = 888;
+constexpr size_t NOALLOC_PARTIALS = KB_NOALLOC_MAX_CHUNKS + KB_NOALLOC_MAX_ITEMS * 2 * NOALLOC_SPLIT_CHUNKS;
 constexpr size_t NOALLOC_PTS_OFF =
     (NOALLOC_PART_OFF + sizeof(ChunkPartial) * (size_t)NOALLOC_PARTIALS + 255) / 256 * 256;
 constexpr size_t NOALLOC_PTS_SLOTS = (KB_NOALLOC_SCRATCH_BYTES - NOALLOC_PTS_OFF) / (PTS_SLOT * sizeof(double));
@@ -1921,9 +1925,8 @@ extern "C" int kb_integrate_noalloc(kb_context *ctx, const kb_work *work, int n_
     it.k_first = w.k_first;
     it.n_points = w.n_points;
     group_of[i] = it.spin_symmetric ? 0 : 1;
-    // the same scheduling chunks as kb_integrate (the context's launch shape of the order,
-    // smaller for a small item), so that the sums are added in the same order
-    it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order]);
+    // kb_integrate's rule for a small item's scheduling chunks, but at most as many as the array holds
+    it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order], NOALLOC_SPLIT_CHUNKS);
     const int64_t unit = noalloc_unit(ctx, w.order, w.n_points);
     chunks_total += (w.n_points + unit - 1) / unit;
   }

@@ -24,14 +24,12 @@ struct ChunkPartial {
 
 constexpr int CHUNK_POINTS = 128; // points per scheduling chunk (<= 128: two 64-bit masks)
 // The tree kernel (wick_tree.cu): warps of a CTA, resident CTAs per SM (12 warps: 168 registers
-// per thread and 18.7 KB of shared memory per warp), and the complex entries of a warp's global
-// scratch (L2-resident): the nodes of orders 9..16 above level 8, sum_{m=9..16} (m+1)^2.
+// per thread and 19 KB of shared memory per warp), and the complex entries of a warp's global
+// scratch (L2-resident): the nodes of orders 9..16 above level 8, sum_{m=9..16} (m+1)^2 + 2 * 81.
 constexpr int TREE_WARPS = 3;
 constexpr int TREE_CTAS_PER_SM = 4;
-constexpr int TREE_STACK = 1500;
+constexpr int TREE_STACK = 1662;
 constexpr int PTS_SLOT = TREE_WARPS * TREE_STACK * 2; // doubles per CTA
-// A small work item is split into finer scheduling chunks only while it has fewer than this.
-constexpr int64_t MAX_SPLIT_CHUNKS = 888;
 // Per-CTA slot of the kernel-method tree: the chunk's set-up (coordinates
 // [MAX_ORDER][CHUNK_POINTS], then Jacobians, domain flags and bin codes).
 constexpr int KM_SLOT = CHUNK_POINTS * (MAX_ORDER + 5);

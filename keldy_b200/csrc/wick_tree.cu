@@ -27,10 +27,15 @@
 //
 // Work split: a level of 256 >> m nodes with m vertices left fills a warp from m = 8 (one
 // node, one point) down to m = 3 (32 nodes, one per lane), whatever the order: order n starts
-// at level n with 2^(8-n) points per warp. Levels 8..5 go through shared memory with the lanes
-// of a node splitting its children; the last three vertices run in registers. Orders above 8
-// walk the first n - 8 levels depth first, one node per level kept. Warps never wait for each
-// other: no CTA barrier in the kernel.
+// at level n with 2^(8-n) points per warp. Levels 8 to 5 go through shared memory with the lanes
+// of a node splitting its children; the last five vertices run in registers. Orders above 8
+// walk the levels above 9 depth first. Warps never wait for each other: no CTA barrier.
+//
+// Bound: latency. Order 8 (2^20 points): 3.6 ms, FP64 pipe 42 % busy, 1,590 instructions per point,
+// of them 800 FP64, shared memory 50 %; the stalls are fixed latencies of dependent FP64
+// instructions and shared-memory loads at 12 warps per SM. Splitting a level's nodes over fewer
+// lanes with more registers (512 >> m nodes, 255 registers, 8 warps) took 4.6 ms, 15 warps at
+// 128 registers 4.8 (spills), an elimination of both vertices 8 and 7 per step 4.1.
 #include <cuda_runtime.h>
 
 #include "kb_device.cuh"
@@ -43,35 +48,91 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// Row width and node size of a node with m vertices left (m+1 rows): the row widths and sizes
-// are chosen so that the eight lanes of a 128-bit shared-memory phase hit different banks in
-// the levels' reads and writes.
-__host__ __device__ constexpr int node_w(int m) { return m == 7 ? 9 : m + 1; }
+// Row width and node size of a node with m vertices left (m+1 rows). A 16-byte shared-memory read
+// takes two cycles when each half-warp reads at most eight distinct words in different 16-byte
+// banks and four when all words differ; the widths, the sizes and the lanes' blocks are chosen
+// for that in the reads of levels 6 and 5.
+__host__ __device__ constexpr int node_w(int m) { return m == 7 ? 9 : m == 6 ? 10 : m + 1; }
 __host__ __device__ constexpr int node_sz(int m) {
-  return m == 1 ? 5 : m == 2 ? 9 : m == 3 ? 17 : m == 4 ? 26 : m == 5 ? 36 : m == 6 ? 49 : m == 7 ? 72 : (m + 1) * (m + 1);
+  return m == 1 ? 5 : m == 2 ? 9 : m == 3 ? 17 : m == 4 ? 25 : m == 5 ? 37 : m == 6 ? 76 : m == 7 ? 72 : (m + 1) * (m + 1);
 }
-// Complex entries of a warp's node buffers: level m's nodes start at NODES_ODD for odd m >= 5,
-// at 0 otherwise; the point differences delta start after the buffers the order uses.
-constexpr int NODES_ODD = 16 * 26;                     // behind the 16 nodes of level 4
-constexpr int NODES_END = NODES_ODD + 8 * 36;          // behind the 8 nodes of level 5
-constexpr int WARP_BUF = NODES_END + 272;              // delta of order 16: 16 * 17
-__host__ __device__ constexpr int node_base(int m) { return (m & 1) && m >= 5 ? NODES_ODD : 0; }
-__host__ __device__ constexpr int delta_base(int n) { return n >= 5 ? NODES_END : n == 4 ? NODES_ODD : 32 * 17; }
+// Complex entries of a warp's buffers: the nodes of odd levels (and the roots of orders 1..4) at 0,
+// those of levels 6 and 8 behind level 5's, then the point differences delta, then the nodes of
+// levels 8 and 9 that orders above 8 keep.
+constexpr int NODES6 = 8 * 37;
+constexpr int NODES_END = NODES6 + 4 * 76;
+constexpr int WARP_BUF = 960;
+__host__ __device__ constexpr int node_base(int m) { return m == 6 || m == 8 ? NODES6 : 0; }
+__host__ __device__ constexpr int delta_base(int n) { return n >= 6 ? NODES_END : n == 5 ? NODES6 : n == 4 ? 16 * 25 : 32 * 17; }
 // delta of a point, in shells: vertex k (1 = latest) holds its k column entries (i, k), i < k,
 // at k(k-1), then its k row entries (k, j), j < k, at k*k.
 __host__ __device__ constexpr int delta_sz(int n) { return n < 8 ? n * (n + 1) + 1 : n * (n + 1); }
-static_assert(delta_base(3) + 32 * delta_sz(3) <= WARP_BUF && delta_base(5) + 8 * delta_sz(5) <= WARP_BUF &&
-                  delta_base(4) + 16 * delta_sz(4) <= WARP_BUF && delta_base(8) + 16 * 17 <= WARP_BUF,
-              "differences fit behind the nodes");
+// Points of a pass (2^(n-3) lanes per point, at most one point per lane), and of a group.
+__host__ __device__ constexpr int pass_points(int n) { return n <= 3 ? 32 : n >= 8 ? 1 : 256 >> n; }
+__host__ __device__ constexpr int group_lg(int n) { return n <= 8 ? 5 : 4; }
+static_assert(delta_base(3) + 32 * delta_sz(3) <= WARP_BUF && delta_base(4) + 16 * delta_sz(4) <= WARP_BUF &&
+                  delta_base(5) + 8 * delta_sz(5) <= WARP_BUF && delta_base(6) + 4 * delta_sz(6) <= WARP_BUF &&
+                  delta_base(16) + delta_sz(16) <= WARP_BUF && 2 * 256 <= WARP_BUF,
+              "differences (and the set-up's factors) fit in a warp's buffers");
+// The lookups of a pass: entry (p, i, j), i != j, of point p's root (position 0: external row A or
+// column B; 1..n: the vertices, latest first). Fields: index of the times of positions i and j in
+// the group's array, place in the roots and in the differences, kind (0: j the earlier vertex,
+// 1: i the earlier, 2: row A, 3: column B).
+constexpr int lookup_first(int n) { // entries of orders below n
+  int s = 0;
+  for (int k = 1; k < n; ++k) s += pass_points(k) * k * (k + 1);
+  return s;
+}
+struct LookupTable {
+  unsigned long long e[lookup_first(MAX_ORDER + 1)];
+  int first[MAX_ORDER + 1];
+  constexpr LookupTable() : e(), first() {
+    int r = 0;
+    for (int n = 1; n <= MAX_ORDER; ++n) {
+      first[n] = r;
+      const int ssz = n > 8 ? 0 : node_sz(n), w = n > 8 ? n + 1 : node_w(n), st = 1 << group_lg(n);
+      for (int p = 0; p < pass_points(n); ++p)
+        for (int i = 0; i <= n; ++i)
+          for (int j = 0; j <= n; ++j) {
+            if (i == j) continue;
+            const unsigned long long ui = i * st + p, uj = (j ? j : n + 1) * st + p;
+            const unsigned long long so = p * ssz + i * w + j, dof = p * delta_sz(n) + (i < j ? j * (j - 1) + i : i * i + j);
+            const unsigned long long kind = i == 0 ? 2 : j == 0 ? 3 : i < j ? 0 : 1;
+            e[r++] = ui | uj << 10 | so << 20 | dof << 32 | kind << 42;
+          }
+    }
+  }
+};
+__device__ const LookupTable lookups = LookupTable();
+
+// What an entry's value is made of, by its kind: the table, and the copies as a word: the high word
+// of delta's sign (+1, -1: forward minus backward copy is g^> - g^< or the opposite; 0: both copies
+// are one function), bit 0: the backward copy is g^>, bit 1: there is no table. `alt`: for a
+// vertex on the other side of the external time.
+struct EntryKind {
+  const double2 *tab;
+  unsigned w, alt;
+};
+
+// What the passes read of their work item, kept in shared memory: with the kernel's shared memory
+// most of the L1, a global load is often an L2 round trip.
+struct ItemConst {
+  EntryKind kind[4];
+  double2 eq; // equal contour points
+  double xmin, delta, rdelta, floor_;
+  const unsigned long long *lookup;
+  int last; // first mesh point of the last interval
+  int cubic;
+};
 
 template <bool SCALE>
 struct WarpShared {
   double2 buf[WARP_BUF];
-  double u[256];      // the group's vertex times, u[j * gp + p] (sorted, latest first)
+  double u[320];      // the group's times, u[i * gp + p]: A, the vertices latest first, B
   double2 fval[32];   // the group's values
-  double2 D2[2][16];  // squared prefix determinant of every node (by parity of its level)
-  double2 Dst[8];     // the same of the depth-first levels above 8
-  int fl[32];         // a guarded pivot in the point's tree
+  ItemConst k;
+  double2 D2[24];     // squared prefix determinants: level 5's nodes at 0, 6's at 8, 7's and 8's at
+                      // 12, the depth-first levels' above 8 at 16
   double fscale[SCALE ? 32 : 2];
 };
 
@@ -80,6 +141,20 @@ __device__ __forceinline__ double2 cfma(double2 c, double2 a, double2 b) {
 }
 // s + f d, f = 1 (the forward copy) or 0
 __device__ __forceinline__ double2 copyof(double2 s, double2 d, double f) { return c2(fma(d.x, f, s.x), fma(d.y, f, s.y)); }
+
+// 1 / a for a pivot: the squared modulus' reciprocal by one third-order Newton-Raphson (Householder)
+// step from the hardware's 20-bit seed, y (1 + e + e^2) with e = 1 - x y: error e^3 < 2^-57 plus
+// the last rounding. Three dependent multiply-adds and no special-case branch, where the IEEE
+// quotient 1.0 / x takes a longer chain on each level's critical path. A zero, overflowed or
+// not finite modulus gives a NaN or an infinity, which the guard catches.
+__device__ __forceinline__ double2 pivot_rcp(double2 a) {
+  const double x = fma(a.x, a.x, a.y * a.y);
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  y = fma(y, fma(e, e, e), y);
+  return c2(a.x * y, -a.y * y);
+}
 
 __device__ __forceinline__ int find_chunk_item(const long long *off, int n_items, long long c) {
   int lo = 0, hi = n_items; // off[lo] <= c < off[hi]
@@ -123,8 +198,8 @@ __device__ __forceinline__ void sobol_group(const SobolDev &s, uint32_t k0, int 
 // point's Jacobian and domain flag. The product warpers, whose logarithms and exponentials
 // dominate, run over (coordinate, point) pairs so that small groups fill the warp; a point's
 // Jacobian is the product of its factors in coordinate order.
-__device__ void setup_group(const Launch &L, const ItemDev &it, int N, int lg, long long gp0, int cnt, bool keep,
-                            double *u, double *fac, int lane, double &jac, bool &dom) {
+__device__ __noinline__ void setup_group(const Launch &L, const ItemDev &it, int N, int lg, long long gp0, int cnt, bool keep,
+                            double *u, double *fac, int lane, double &jac, bool &dom, bool &sorted) {
   jac = 1.0;
   int top = 0;
   const bool mine = lane < cnt;
@@ -180,6 +255,12 @@ __device__ void setup_group(const Launch &L, const ItemDev &it, int N, int lg, l
         double t;
         f = table_reverse(wd.tab[wd.ntab == 1 ? 0 : j], x, t);
         x = t;
+      } else if (wd.kind == KB_WARPER_EXPONENTIAL) {
+        // u = u_max - w log(1 + c0 l), so 1 / f1(u) = c1 exp(u / w) = c1 (1 + c0) / (1 + c0 l) without
+        // the exponential (and without the rounding of u in its argument)
+        const double a = wd.c[0] * x;
+        x = wd.u_max - wd.w * log1p(a);
+        f = wd.c[1] * ((1.0 + wd.c[0]) / (1.0 + a));
       } else {
         const double t = warper_Finv(wd, x);
         x = t;
@@ -197,9 +278,17 @@ __device__ void setup_group(const Launch &L, const ItemDev &it, int N, int lg, l
   }
   jac *= cj;
   dom = it.f.A.spin == it.f.B.spin;
-  if (mine && keep)
-    for (int j = 0; j < N; ++j)
-      if (u[(j << lg) + lane] < 0.0) dom = false;
+  sorted = true;
+  if (mine) {
+    double before = u[lane];
+    if (keep && before < 0.0) dom = false;
+    for (int j = 1; j < N; ++j) {
+      const double x = u[(j << lg) + lane];
+      if (keep && x < 0.0) dom = false;
+      if (!(x <= before)) sorted = false;
+      before = x;
+    }
+  }
 }
 
 // Bin of the earliest vertex time (binner_t::in_bounds and coord2index, binner.hpp:163-176:
@@ -213,8 +302,8 @@ __device__ __forceinline__ int earliest_bin(const Launch &L, const double *u, in
   return min((int)((t - L.bin_xmin) / L.bin_size), L.nbins - 1);
 }
 
-// Sorts a point's times (stride st), latest first; of equal times the higher vertex index
-// counts as the later one on the contour (compare_3way's timesplit).
+// Sorts a point's times (stride st), latest first (of equal times the higher vertex index counts
+// as the later one on the contour, compare_3way's timesplit: their order changes nothing here).
 __device__ __forceinline__ void sort_times(double *u, int st, int N) {
   for (int i = 1; i < N; ++i) {
     const double v = u[i * st];
@@ -227,154 +316,176 @@ __device__ __forceinline__ void sort_times(double *u, int st, int N) {
   }
 }
 
-// Root matrices and differences of np points (columns p0.. of u): entry (i, j), i != j, of
-// position i (0: the external row A or column B, 1..N: the vertices, latest first) is one table
-// lookup of g^< and g^> at one time difference: S = the copy of Keldysh index 1 (backward) of
-// the pair's earlier vertex, delta = forward copy - S. Each lane starts GK lookups before it
-// uses the first, so that their L2 round trips overlap.
-template <bool CUBIC, int GK>
-__device__ void build_roots(const ItemDev &it, int N, int np, const double *u, int st, unsigned dommask, double2 eq,
-                            double2 *S, int ssz, int sw, double2 *dl, int dsz, int lane, bool &bad) {
+// dx / delta correctly rounded, from rdelta = 1 / delta rounded: the product and one residual step
+// (Markstein's theorem).
+__device__ __forceinline__ double mesh_position(double dx, double delta, double rdelta) {
+  const double q = __dmul_rn(dx, rdelta);
+  return fma(fma(-q, delta, dx), rdelta, q);
+}
+
+// Whether every lookup of a point (sorted times, stride st) lies inside the tabulated window. The
+// mesh position grows with the time difference, so the extreme differences decide.
+__device__ __forceinline__ bool in_window(const ItemDev &it, int N, const double *u, int st, double rdelta) {
   const ModelDev &m = it.model;
-  const kb_gf_index &A = it.f.A, &B = it.f.B;
-  const int spin = A.spin;
-  const double2 *t00 = m.tab[spin][0][0];
-  const double2 *trow = m.tab[spin][A.orbital][0];
-  const double2 *tcol = m.tab[spin][0][B.orbital];
-  const int per = N * (N + 1), total = np * per;
-  // quotients by multiply-high with 2^32 / d rounded up (exact: r < 2^16, d <= 272); 0 = d is 1
-  const unsigned mper = 0xFFFFFFFFu / (unsigned)per + 1u;
-  const unsigned mn = N > 1 ? 0xFFFFFFFFu / (unsigned)N + 1u : 0u;
+  const int spin = it.f.A.spin;
+  const double hi = u[0], lo = u[(N - 1) * st];
+  auto inside = [&](double x) {
+    const double a = mesh_position(__dsub_rn(x, m.xmin), m.delta, rdelta);
+    return a >= 0.0 && a <= (double)(m.npts - 1);
+  };
+  bool ok = true;
+  for (int j = 0; j < N; ++j) ok = ok && u[j * st] == u[j * st];
+  if (N > 1 && m.tab[spin][0][0]) ok = ok && inside(hi - lo) && inside(lo - hi);
+  if (m.tab[spin][it.f.A.orbital][0]) ok = ok && inside(it.f.A.time - lo) && inside(it.f.A.time - hi);
+  if (m.tab[spin][0][it.f.B.orbital]) ok = ok && inside(hi - it.f.B.time) && inside(lo - it.f.B.time);
+  return ok;
+}
+
+// What the lookups of an absent block read.
+__device__ __align__(128) const double2 no_table[8] = {};
+
+// Root matrices and differences of the np points of a pass from column s0 of u: S = the copy of
+// Keldysh index 1 (backward) of an entry's earlier vertex, delta = forward copy - S. Each entry
+// is one lookup of g^< and g^> at one time difference; each lane starts GK of them, without a
+// branch between them, before it uses the first, so that their L2 round trips overlap. The
+// gathers do not allocate in the little L1 that shared memory leaves, which then holds the
+// entry list, the item and the Sobol matrices (order 8 -6 %, order 5 -13 %). The position's whole
+// part comes from rounding a - 1/2 (at a mesh point either interval gives the mesh value).
+template <bool CUBIC, int GK>
+__device__ __forceinline__ void build_roots(const ItemConst &K, int N, int np, const double *u, double2 *S, int ssz,
+                                            int sw, double2 *dl, int lane) {
+  const double xmin = K.xmin, delta = K.delta, rdelta = K.rdelta;
+  const int last = K.last, total = np * N * (N + 1);
+  const unsigned long long *lt = K.lookup;
   for (int base = 0; base < total; base += 32 * GK) {
-    int so[GK], dof[GK], ix[GK], how[GK]; // how: bit 0 forward copy is g^>, bit 1 backward copy is g^>, 4 none, 8 zero
+    unsigned lo[GK], hi[GK], word[GK];
     double wt[GK];
     const double2 *tb[GK];
 #pragma unroll
+    for (int k = 0; k < GK; ++k) { // idle lanes repeat the last entry
+      const unsigned long long e = __ldg(lt + min(base + 32 * k + lane, total - 1));
+      lo[k] = (unsigned)e;
+      hi[k] = (unsigned)(e >> 32);
+    }
+#pragma unroll
     for (int k = 0; k < GK; ++k) {
-      const int r = base + 32 * k + lane;
-      how[k] = 4;
-      tb[k] = nullptr;
-      ix[k] = so[k] = dof[k] = 0;
-      wt[k] = 0.0;
-      if (r >= total) continue;
-      const int p = (int)__umulhi((unsigned)r, mper), q = r - p * per;
-      const int i = mn ? (int)__umulhi((unsigned)q, mn) : q;
-      const int jj = q - i * N, j = jj + (jj >= i ? 1 : 0);
-      so[k] = p * ssz + i * sw + j;
-      dof[k] = p * dsz + (i < j ? j * (j - 1) + i : i * i + j);
-      if (!((dommask >> p) & 1u)) { // out of domain: identity, its value is discarded
-        how[k] = 8;
-        continue;
-      }
-      double dt;
-      if (i == 0) {
-        const double uj = u[(j - 1) * st + p];
-        dt = A.time - uj;
-        tb[k] = trow;
-        // A later than the vertex (or at its time): forward g^>, backward g^<; earlier: A's branch decides
-        how[k] = A.time < uj ? (A.k_idx ? 3 : 0) : 1;
-      } else if (j == 0) {
-        const double ui = u[(i - 1) * st + p];
-        dt = ui - B.time;
-        tb[k] = tcol;
-        how[k] = ui > B.time ? (B.k_idx ? 0 : 3) : 2;
+      const int kind = (hi[k] >> 10) & 3;
+      const EntryKind ek = K.kind[kind];
+      const double d = __dsub_rn(u[lo[k] & 1023], u[(lo[k] >> 10) & 1023]);
+      // the other side: A earlier than the vertex (d < 0), the vertex later than B (d > 0)
+      const unsigned dh = (unsigned)__double2hiint(d) ^ ((unsigned)kind << 31);
+      word[k] = dh > 0x80000000u ? ek.alt : ek.w;
+      const double a = mesh_position(__dsub_rn(d, xmin), delta, rdelta);
+      const double t52 = __dadd_rn(a - 0.5, 6755399441055744.0); // 1.5 * 2^52: the sum's low word is the integer
+      int ix = (int)min((unsigned)__double2loint(t52), (unsigned)last);
+      if (CUBIC) ix = max(0, min(ix - 1, last - 2)); // first of the four mesh points
+      wt[k] = a - (__hiloint2double(0x43380000, ix) - 6755399441055744.0);
+      tb[k] = ek.tab + 2 * ((word[k] & 2u) ? 0 : ix);
+    }
+    double2 v[GK][CUBIC ? 8 : 4];
+#pragma unroll
+    for (int k = 0; k < GK; ++k)
+#pragma unroll
+      for (int e = 0; e < (CUBIC ? 4 : 2); ++e)
+        asm volatile("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(v[k][2 * e].x), "=d"(v[k][2 * e].y), "=d"(v[k][2 * e + 1].x), "=d"(v[k][2 * e + 1].y)
+                     : "l"(tb[k] + 2 * e));
+#pragma unroll
+    for (int k = 0; k < GK; ++k) {
+      double2 gl, gg;
+      if (CUBIC) { // Lagrange through the four mesh points, as interp_pair_cubic
+        const double x = wt[k], am = x - 1.0, bm = x - 2.0, cm = x - 3.0;
+        const double n0 = am * bm * cm, n3 = x * am * bm;
+        const double w[4] = {-mesh_position(n0, 6.0, 1.0 / 6.0), 0.5 * (x * bm * cm), -0.5 * (x * am * cm),
+                             mesh_position(n3, 6.0, 1.0 / 6.0)};
+        gl = gg = c2(0.0, 0.0);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const double2 l = v[k][2 * e], g = v[k][2 * e + 1];
+          gl = c2(fma(w[e], l.x, gl.x), fma(w[e], l.y, gl.y));
+          gg = c2(fma(w[e], g.x, gg.x), fma(w[e], g.y, gg.y));
+        }
       } else {
-        dt = u[(i - 1) * st + p] - u[(j - 1) * st + p];
-        tb[k] = t00;
-        how[k] = i < j ? 1 : 2;
+        const double w = wt[k];
+        const double2 l0 = v[k][0], g0 = v[k][1], l1 = v[k][2], g1 = v[k][3];
+        gl = c2(fma(w, l1.x - l0.x, l0.x), fma(w, l1.y - l0.y, l0.y));
+        gg = c2(fma(w, g1.x - g0.x, g0.x), fma(w, g1.y - g0.y, g0.y));
       }
-      if (tb[k] && !interp_index(m, dt, ix[k], wt[k])) {
-        bad = true;
-        ix[k] = 0;
-        wt[k] = 0.0;
-      }
-    }
-    double2 gl[GK], gg[GK];
-#pragma unroll
-    for (int k = 0; k < GK; ++k) {
-      if (tb[k] && CUBIC)
-        interp_pair_cubic(tb[k], m.npts, ix[k], wt[k], gl[k], gg[k]);
-      else if (tb[k])
-        interp_pair(tb[k], ix[k], wt[k], gl[k], gg[k]);
-      else
-        gl[k] = gg[k] = c2(0.0, 0.0);
-    }
-#pragma unroll
-    for (int k = 0; k < GK; ++k) {
-      if (how[k] == 4) continue;
-      const double2 f = (how[k] & 1) ? gg[k] : gl[k], b = (how[k] & 2) ? gg[k] : gl[k];
-      S[so[k]] = b;
-      dl[dof[k]] = c2(f.x - b.x, f.y - b.y);
+      const double sg = __hiloint2double(word[k] & 0xFFF00000u, 0);
+      S[lo[k] >> 20] = (word[k] & 1u) ? gg : gl;
+      dl[hi[k] & 1023] = c2(sg * (gg.x - gl.x), sg * (gg.y - gl.y));
     }
   }
   // diagonals (equal contour points) and the external corner
+  const unsigned md = 0xFFFFFFFFu / (unsigned)(N + 1) + 1u; // e / (N + 1) by multiply-high
+  const double2 eq = K.eq;
   for (int e = lane; e < np * (N + 1); e += 32) {
-    const int p = e / (N + 1), i = e - p * (N + 1);
-    const bool in = (dommask >> p) & 1u;
-    S[p * ssz + i * sw + i] = i == 0 ? c2(0.0, 0.0) : (in ? eq : c2(1.0, 0.0));
+    const int p = (int)__umulhi((unsigned)e, md), i = e - p * (N + 1);
+    S[p * ssz + i * (sw + 1)] = i == 0 ? c2(0.0, 0.0) : eq;
   }
 }
 
 // ------------------------------------------------------------------ the tree
 
-// Level m (4 < m <= 8): the children of this lane's node. Nodes of a level, and the lanes
-// of a node, are numbered so that a point's nodes stay in its own lanes: node lane >> (m-3),
-// child lane >> (m-4), whose low bit is the copy of vertex m it eliminates (1: backward).
-template <int m>
-__device__ __forceinline__ void level(double2 *buf, const double2 *dl, const double2 *D2p, double2 *D2c, int lane,
-                                      double floor_, bool &guard) {
-  constexpr int W = node_w(m), WC = node_w(m - 1), LC = m - 4; // 2^LC lanes per child
-  const int child = lane >> LC, l = lane & ((1 << LC) - 1);
-  const double2 *S = buf + node_base(m) + (child >> 1) * node_sz(m);
-  double2 *o = buf + node_base(m - 1) + child * node_sz(m - 1);
-  const double2 *dc = dl + m * (m - 1), *dr = dl + m * m;
-  const double f = (child & 1) ? 0.0 : 1.0;
-  const double2 p = S[m * W + m];
+// Nodes of a level, and the lanes of a node, are numbered so that a point's nodes stay in its
+// own lanes: with m vertices left, node lane >> (m-3), whose low bit is the copy of vertex m+1
+// that led to it (1: backward).
+
+// Level 8 (node S, 9 x 9) to level 7: half a row of its child per lane.
+__device__ __forceinline__ void level8(const double2 *S, double2 *buf, const double2 *dl, double2 D2, double2 *D2c,
+                                       int lane, double floor_, bool &guard) {
+  constexpr int W = node_w(8), WC = node_w(7);
+  const int child = lane >> 4, l = lane & 15, i = l >> 1, j0 = (l & 1) * 4;
+  const double2 *dc = dl + 56, *dr = dl + 64;
+  const double f = child ? 0.0 : 1.0;
+  const double2 p = S[8 * W + 8], ip = pivot_rcp(p);
   if (!(cabs1(p) >= floor_)) guard = true;
-  const double2 ip = crcp(p);
+  if (l == 0) D2c[child] = cmul(D2, cmul(p, p));
+  const double2 Lf = cmul(copyof(S[i * W + 8], dc[i], f), ip);
+  double2 *o = buf + node_base(7) + child * node_sz(7) + i * WC + j0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) o[q] = cfms(S[i * W + j0 + q], Lf, copyof(S[8 * W + j0 + q], dr[j0 + q], f));
+}
+
+// Level 7 to level 6: a row of its child per lane.
+__device__ __forceinline__ void level7(double2 *buf, const double2 *dl, const double2 *D2p, double2 *D2c, int lane, double floor_, bool &guard) {
+  constexpr int W = node_w(7), WC = node_w(6);
+  const int child = lane >> 3, i = lane & 7;
+  const double2 *S = buf + node_base(7) + (child >> 1) * node_sz(7);
+  const double2 *dc = dl + 42, *dr = dl + 49;
+  const double f = (child & 1) ? 0.0 : 1.0;
+  const double2 p = S[7 * W + 7], ip = pivot_rcp(p);
+  if (!(cabs1(p) >= floor_)) guard = true;
+  if (i < 7) {
+    const double2 Lf = cmul(copyof(S[i * W + 7], dc[i], f), ip);
+    double2 *o = buf + node_base(6) + child * node_sz(6) + i * WC;
+#pragma unroll
+    for (int j = 0; j < 7; ++j) o[j] = cfms(S[i * W + j], Lf, copyof(S[7 * W + j], dr[j], f));
+  } else {
+    D2c[child] = cmul(D2p[child >> 1], cmul(p, p));
+  }
+}
+
+// Level 6 to level 5: a 3 x 3 block of its child per lane.
+__device__ __forceinline__ void level6(double2 *buf, const double2 *dl, const double2 *D2p, double2 *D2c, int lane,
+                                       double floor_, bool &guard) {
+  constexpr int W = node_w(6), WC = node_w(5);
+  const int child = lane >> 2, l = lane & 3, i0 = (l >> 1) * 3, j0 = (l & 1) * 3;
+  const double2 *S = buf + node_base(6) + (child >> 1) * node_sz(6);
+  const double2 *dc = dl + 30, *dr = dl + 36;
+  const double f = (child & 1) ? 0.0 : 1.0;
+  const double2 p = S[6 * W + 6], ip = pivot_rcp(p);
+  if (!(cabs1(p) >= floor_)) guard = true;
   if (l == 0) D2c[child] = cmul(D2p[child >> 1], cmul(p, p));
-  if constexpr (m == 8) { // 8 x 8: half a row per lane
-    const int i = l >> 1, j0 = (l & 1) * 4;
-    const double2 Lf = cmul(copyof(S[i * W + m], dc[i], f), ip);
+  double2 r[3];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int j = j0 + q;
-      o[i * WC + j] = cfms(S[i * W + j], Lf, copyof(S[m * W + j], dr[j], f));
-    }
-  } else if constexpr (m == 7) { // 7 x 7: a row per lane
-    if (l < 7) {
-      const double2 Lf = cmul(copyof(S[l * W + m], dc[l], f), ip);
+  for (int j = 0; j < 3; ++j) r[j] = copyof(S[6 * W + j0 + j], dr[j0 + j], f);
+  double2 *o = buf + node_base(5) + child * node_sz(5) + i0 * WC + j0;
 #pragma unroll
-      for (int j = 0; j < 7; ++j) o[l * WC + j] = cfms(S[l * W + j], Lf, copyof(S[m * W + j], dr[j], f));
-    }
-  } else if constexpr (m == 6) { // 6 x 6: a 3 x 3 block per lane
-    const int i0 = (l >> 1) * 3, j0 = (l & 1) * 3;
-    double2 r[3];
+  for (int i = 0; i < 3; ++i) {
+    const double2 Lf = cmul(copyof(S[(i0 + i) * W + 6], dc[i0 + i], f), ip);
 #pragma unroll
-    for (int j = 0; j < 3; ++j) r[j] = copyof(S[m * W + j0 + j], dr[j0 + j], f);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const double2 Lf = cmul(copyof(S[(i0 + i) * W + m], dc[i0 + i], f), ip);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) o[(i0 + i) * WC + j0 + j] = cfms(S[(i0 + i) * W + j0 + j], Lf, r[j]);
-    }
-  } else { // 5 x 5: rows 0, 1 or 3, 4 per lane, and its side of row 2
-    const int i0 = l * 3, j0 = l * 2;
-    double2 r[5];
-#pragma unroll
-    for (int j = 0; j < 5; ++j) r[j] = copyof(S[m * W + j], dr[j], f);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const double2 Lf = cmul(copyof(S[(i0 + i) * W + m], dc[i0 + i], f), ip);
-#pragma unroll
-      for (int j = 0; j < 5; ++j) o[(i0 + i) * WC + j] = cfms(S[(i0 + i) * W + j], Lf, r[j]);
-    }
-    const double2 Lf = cmul(copyof(S[2 * W + m], dc[2], f), ip);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const double2 rj = l ? r[j + 2] : r[j];
-      o[2 * WC + j0 + j] = cfms(S[2 * W + j0 + j], Lf, rj);
-    }
+    for (int j = 0; j < 3; ++j) o[i * WC + j] = cfms(S[(i0 + i) * W + j0 + j], Lf, r[j]);
   }
 }
 
@@ -396,7 +507,7 @@ __device__ __forceinline__ double2 leaf2(const double2 (&T)[9], double2 dX, doub
   const double2 tf = cmul(cfms(P, c1, r1), cfms(cfms(Q, cadd(g, g2), r1), cadd(h, h2), c1));
   if constexpr (SCALE) {
     if (!(cabs1(T[8]) >= floor_)) guard = true;
-    const double2 ip = crcp(T[8]);
+    const double2 ip = pivot_rcp(T[8]);
 #pragma unroll
     for (int a2 = 0; a2 < 2; ++a2) {
       const double2 c0 = a2 ? T[2] : cadd(T[2], d2[0]), r0 = a2 ? T[6] : cadd(T[6], d2[2]);
@@ -420,7 +531,7 @@ __device__ __forceinline__ double2 leaf3(const double2 (&s)[16], const double2 *
                                          bool &guard, double &scale) {
   const double2 p = s[15];
   if (!(cabs1(p) >= floor_)) guard = true;
-  const double2 ip = crcp(p);
+  const double2 ip = pivot_rcp(p);
   const double2 dX = dl[0], dY = dl[1];
   const double2 d2[4] = {dl[2], dl[3], dl[4], dl[5]};
   const double2 g2 = cmul(d2[0], dY), h2 = cmul(dX, d2[2]);
@@ -447,16 +558,46 @@ __device__ __forceinline__ double2 leaf3(const double2 (&s)[16], const double2 *
   return cmul(Dn, acc);
 }
 
-// Level 4's child of this lane (child index = lane) in registers, then leaf3.
+// Level 5 to this lane's node s of level 3 (index = lane), both eliminations in registers; returns
+// its D^2. (Through level-4 nodes in shared memory, two lanes sharing each elimination, order 8 takes
+// 6 % longer.)
 template <bool SCALE>
-__device__ __forceinline__ double2 level4_leaves(const double2 *buf, const double2 *dl, const double2 *D2p, int lane,
-                                                 double floor_, bool &guard, double &scale) {
+__device__ __forceinline__ double2 level5(double2 (&s)[16], const double2 *buf, const double2 *dl, const double2 *D2p,
+                                          int lane, double floor_, bool &guard) {
+  constexpr int W = node_w(5);
+  const double2 *S = buf + node_base(5) + (lane >> 2) * node_sz(5);
+  const double f5 = (lane & 2) ? 0.0 : 1.0, f4 = (lane & 1) ? 0.0 : 1.0;
+  const double2 p5 = S[5 * W + 5], i5 = pivot_rcp(p5);
+  double2 r5[5], r4[4];
+#pragma unroll
+  for (int j = 0; j < 5; ++j) r5[j] = copyof(S[5 * W + j], dl[25 + j], f5);
+  const double2 L54 = cmul(copyof(S[4 * W + 5], dl[24], f5), i5);
+  const double2 p4 = cfms(S[4 * W + 4], L54, r5[4]), i4 = pivot_rcp(p4);
+  if (!(cabs1(p5) >= floor_) || !(cabs1(p4) >= floor_)) guard = true;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) r4[j] = copyof(cfms(S[4 * W + j], L54, r5[j]), dl[16 + j], f4);
+  s[0] = c2(0.0, 0.0);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const double2 L5 = cmul(copyof(S[i * W + 5], dl[20 + i], f5), i5);
+    const double2 L4 = cmul(copyof(cfms(S[i * W + 4], L5, r5[4]), dl[12 + i], f4), i4);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (SCALE || i + j > 0) s[4 * i + j] = cfms(cfms(S[i * W + j], L5, r5[j]), L4, r4[j]);
+  }
+  const double2 pp = cmul(p5, p4);
+  return cmul(D2p[lane >> 2], cmul(pp, pp));
+}
+
+// Order 4's child s of this lane (child index = lane) in registers; returns its D^2.
+template <bool SCALE>
+__device__ __forceinline__ double2 level4(double2 (&s)[16], const double2 *buf, const double2 *dl, const double2 *D2p,
+                                          int lane, double floor_, bool &guard) {
   const double2 *S = buf + (lane >> 1) * node_sz(4);
   const double f = (lane & 1) ? 0.0 : 1.0;
-  const double2 p = S[24];
+  const double2 p = S[24], ip = pivot_rcp(p);
   if (!(cabs1(p) >= floor_)) guard = true;
-  const double2 ip = crcp(p);
-  double2 r[4], s[16];
+  double2 r[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) r[j] = copyof(S[20 + j], dl[16 + j], f);
   s[0] = c2(0.0, 0.0);
@@ -467,173 +608,228 @@ __device__ __forceinline__ double2 level4_leaves(const double2 *buf, const doubl
     for (int j = 0; j < 4; ++j)
       if (SCALE || i + j > 0) s[4 * i + j] = cfms(S[5 * i + j], Lf, r[j]);
   }
-  return leaf3<SCALE>(s, dl, cmul(D2p[lane >> 1], cmul(p, p)), floor_, guard, scale);
+  return cmul(D2p[lane >> 1], cmul(p, p));
 }
 
-// The tree below the nodes of level min(n, 8) in the buffers (their D^2 set): this lane's
-// value, with the sign of its copies of the vertices down to 4.
+// The tree below the roots of order n <= 8 in the buffers, or below the node of level 8 at
+// T.buf[node8] with D^2 = D8 (orders 8 and up): this lane's value, with the sign of its copies of the
+// vertices down to 4.
 template <bool SCALE>
-__device__ __forceinline__ double2 subtree(WarpShared<SCALE> &T, const double2 *dl, int n, int lane, double floor_,
-                                           bool &guard, double &scale) {
-  if (n >= 8) {
-    level<8>(T.buf, dl, T.D2[0], T.D2[1], lane, floor_, guard);
-    __syncwarp();
-  }
-  if (n >= 7) {
-    level<7>(T.buf, dl, T.D2[1], T.D2[0], lane, floor_, guard);
-    __syncwarp();
-  }
-  if (n >= 6) {
-    level<6>(T.buf, dl, T.D2[0], T.D2[1], lane, floor_, guard);
-    __syncwarp();
-  }
-  if (n >= 5) {
-    level<5>(T.buf, dl, T.D2[1], T.D2[0], lane, floor_, guard);
-    __syncwarp();
-  }
-  double2 v;
-  if (n >= 4) {
-    v = level4_leaves<SCALE>(T.buf, dl, T.D2[0], lane, floor_, guard, scale);
-  } else {
-    double2 s[16];
+__device__ __forceinline__ double2 subtree(WarpShared<SCALE> &T, int node8, double2 D8, const double2 *dl, int n, int lane,
+                                           double floor_, bool &guard, double &scale) {
+  double2 s[16], D2 = c2(1.0, 0.0);
+  if (n <= 3) {
     const double2 *S = T.buf + lane * node_sz(3);
 #pragma unroll
     for (int e = 0; e < 16; ++e) s[e] = S[e];
-    v = leaf3<SCALE>(s, dl, c2(1.0, 0.0), floor_, guard, scale);
+  } else {
+    if (n >= 8) {
+      level8(T.buf + node8, T.buf, dl, D8, T.D2 + 12, lane, floor_, guard);
+      __syncwarp();
+    }
+    if (n >= 7) level7(T.buf, dl, T.D2 + 12, T.D2 + 8, lane, floor_, guard);
+    if (n >= 6) {
+      __syncwarp();
+      level6(T.buf, dl, T.D2 + 8, T.D2, lane, floor_, guard);
+      __syncwarp();
+    }
+    if (n == 4)
+      D2 = level4<SCALE>(s, T.buf, dl, T.D2, lane, floor_, guard);
+    else
+      D2 = level5<SCALE>(s, T.buf, dl, T.D2, lane, floor_, guard);
   }
-  const int lg = min(n, 8) - 3;
-  if (__popc(lane & ((1 << lg) - 1)) & 1) v = c2(-v.x, -v.y);
-  return v;
+  const double2 v = leaf3<SCALE>(s, dl, D2, floor_, guard, scale);
+  const int lg = n <= 3 ? 0 : min(n, 8) - 3;
+  return (__popc(lane & ((1 << lg) - 1)) & 1) ? c2(-v.x, -v.y) : v;
 }
 
-// One depth-first step above level 8: node S (m vertices left, m+1 wide) to its child of copy
-// a, written to o (m wide). All lanes; the caller's __syncwarp follows.
+// One step above level 8: node S (m vertices left, m+1 wide) to its child of copy a, or PAIR: to both
+// children (copy 0 by the lower half-warp at o, copy 1 by the upper one behind it), m wide. A column
+// per lane; its rows' loads are issued together, as S may lie in global scratch. D2n: the
+// children's D^2. The caller's __syncwarp follows.
+template <bool PAIR>
 __device__ __forceinline__ void step_down(const double2 *S, double2 *o, const double2 *dl, int m, int a, int lane,
                                           double2 D2, double2 &D2n, double floor_, bool &guard) {
-  const int W = m + 1;
+  const int W = m + 1, j = lane & 15, half = lane >> 4;
   const double2 p = S[m * W + m];
-  if (!(cabs1(p) >= floor_)) guard = true;
-  const double2 ip = crcp(p);
-  D2n = cmul(D2, cmul(p, p));
-  const double f = a ? 0.0 : 1.0;
   const double2 *dc = dl + m * (m - 1), *dr = dl + m * m;
-  const unsigned magic = 0xFFFFFFFFu / (unsigned)m + 1u; // e / m == umulhi(e, magic) for e < 2^16
-  for (int e = lane; e < m * m; e += 32) {
-    const int i = (int)__umulhi((unsigned)e, magic), j = e - i * m;
-    const double2 Lf = cmul(copyof(S[i * W + m], dc[i], f), ip);
-    o[e] = cfms(S[i * W + j], Lf, copyof(S[m * W + j], dr[j], f));
+  const double f = (PAIR ? half : a) ? 0.0 : 1.0;
+  const int col = min(j, m - 1); // idle lanes repeat the last column's loads
+  const double2 r = copyof(S[m * W + col], dr[col], f);
+  if (!(cabs1(p) >= floor_)) guard = true;
+  const double2 ip = pivot_rcp(p);
+  D2n = cmul(D2, cmul(p, p));
+  if (PAIR) o += half * m * m;
+  constexpr int ROWS = 5, STEP = PAIR ? 1 : 2;
+  for (int i0 = PAIR ? 0 : half; i0 < m; i0 += ROWS * STEP) {
+    double2 c[ROWS], x[ROWS];
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const int i = min(i0 + k * STEP, m - 1);
+      c[k] = copyof(S[i * W + m], dc[i], f);
+      x[k] = S[i * W + col];
+    }
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const int i = i0 + k * STEP;
+      if (i < m && j < m) o[i * m + j] = cfms(x[k], cmul(c[k], ip), r);
+    }
   }
 }
 
-// A group's points in passes of P, each point's value into T.fval (guarded: T.fl).
+// a on lanes with bit `bit` clear, b on the others, each summed over the lane pair.
+__device__ __forceinline__ double2 merge_lanes(double2 a, double2 b, int bit, int lane) {
+  const bool up = lane & bit;
+  const double2 keep = up ? b : a, send = up ? a : b;
+  return c2(keep.x + __shfl_xor_sync(FULL, send.x, bit), keep.y + __shfl_xor_sync(FULL, send.y, bit));
+}
+
+// A group's points in passes, each point's value into T.fval; returns the points with a guarded
+// pivot (bit per point of the group).
 template <bool SCALE, bool ANY_CUBIC>
-__device__ void group_values(WarpShared<SCALE> &T, const ItemDev &it, int n, int lgp, int cnt, unsigned dommask,
-                             double2 eq, double2 *stack, int lane, bool &bad) {
-  const double floor_ = it.model.pivot_floor;
-  const int P = n <= 3 ? 32 : (n >= 8 ? 1 : 256 >> n);
-  const int lg = n < 3 ? 0 : min(n, 8) - 3; // lanes per point
-  const int st = 1 << lgp;
+__device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int n, int cnt, unsigned inmask, double2 *stack,
+                                                 int lane) {
+  const double floor_ = T.k.floor_;
+  const int P = pass_points(n);
+  const int lg = n <= 3 ? 0 : min(n, 8) - 3; // lanes per point
   double2 *dl0 = T.buf + delta_base(n);
   const int dsz = delta_sz(n);
-  // orders above 8: the nodes of the depth-first levels, the deepest behind the differences in
-  // shared memory when it fits, the others in global scratch
-  double2 *node9 = nullptr;
-  int soff = 0;
+  // orders above 8: the depth-first levels' nodes, level 8's pair and then level 9's node behind the
+  // differences in shared memory where they fit, the others in global scratch
+  double2 *pair8 = nullptr, *node9 = nullptr;
+  int pair_at = 0;
   if (n > 8) {
-    const bool fits = n * (n + 1) + 100 <= WARP_BUF - NODES_END;
+    int room = WARP_BUF - delta_base(n) - dsz;
+    double2 *at = dl0 + dsz;
+    int soff = 0;
     for (int m = n; m > 9; --m) soff += (m + 1) * (m + 1);
-    node9 = fits ? dl0 + n * (n + 1) : stack + soff;
-  }
-  for (int s0 = 0; s0 < cnt; s0 += P) {
-    const int np = min(P, cnt - s0);
-    const unsigned dm = (dommask >> s0) & (np >= 32 ? FULL : (1u << np) - 1u);
-    if (P == 1 && !dm) {
-      if (lane == 0) {
-        T.fval[s0] = c2(0.0, 0.0);
-        T.fl[s0] = 0;
-        if (SCALE) T.fscale[s0] = 0.0;
-      }
-      continue;
+    pair8 = stack + TREE_STACK - 162;
+    node9 = stack + soff;
+    if (room >= 162) {
+      pair8 = at;
+      pair_at = (int)(at - T.buf);
+      at += 162;
+      room -= 162;
     }
-    double2 *root = n > 9 ? stack : (n == 9 ? node9 : T.buf + node_base(n));
-    const int rsz = n > 8 ? 0 : node_sz(n), rw = n > 8 ? n + 1 : node_w(n);
-    if (ANY_CUBIC && it.model.interp == 3)
-      build_roots<true, 2>(it, n, np, T.u + s0, st, dm, eq, root, rsz, rw, dl0, dsz, lane, bad);
-    else
-      build_roots<false, 4>(it, n, np, T.u + s0, st, dm, eq, root, rsz, rw, dl0, dsz, lane, bad);
-    if (n >= 4 && lane < 16) T.D2[n > 8 ? 0 : n & 1][lane] = c2(1.0, 0.0);
-    __syncwarp();
+    if (room >= 100) node9 = at;
+  }
+  const int K0 = max(n - 9, 0); // K0 depth-first levels above level 9
+  double2 *root = n > 9 ? stack : (n == 9 ? node9 : T.buf + node_base(n));
+  const int rsz = n > 8 ? 0 : node_sz(n), rw = n > 8 ? n + 1 : node_w(n);
+  unsigned guarded = 0;
+  double2 h0 = c2(0.0, 0.0), h1 = c2(0.0, 0.0); // values of earlier passes of a quad, not yet summed over lanes
+  for (int s0 = 0, t = 0; s0 < cnt || (lg >= 2 && (t & 3)); s0 += P, ++t) {
+    const int np = min(P, cnt - s0);
+    const unsigned in = np <= 0 ? 0u : (inmask >> s0) & (np >= 32 ? FULL : (1u << np) - 1u);
     bool guard = false;
     double scale = 0.0;
     double2 v = c2(0.0, 0.0);
-    if (n > 8) {
-      const int K0 = n - 8;
-      for (int sub = 0; sub < (1 << K0); ++sub) {
-        // the levels whose copy changed since the last subtree, down to level 8
-        const int first = sub == 0 ? 0 : K0 - 1 - (__ffs(sub) - 1);
-        const double2 *src = stack;
-        int off = 0;
-        for (int d = 0; d < K0; ++d) {
-          const int m = n - d;
-          const double2 *S = m == 9 ? node9 : stack + off;
-          off += (m + 1) * (m + 1);
-          if (d < first) continue;
-          double2 *o = m - 1 == 8 ? T.buf : (m - 1 == 9 ? node9 : stack + off);
-          double2 D2n;
-          step_down(S, o, dl0, m, (sub >> (K0 - 1 - d)) & 1, lane, d == 0 ? c2(1.0, 0.0) : T.Dst[d - 1], D2n, floor_,
-                    guard);
-          __syncwarp();
-          if (lane == 0) {
-            if (m - 1 == 8)
-              T.D2[0][0] = D2n;
-            else
-              T.Dst[d] = D2n;
+    if (in) {
+      if (ANY_CUBIC && T.k.cubic)
+        build_roots<true, 2>(T.k, n, np, T.u + s0, root, rsz, rw, dl0, lane);
+      else
+        build_roots<false, 3>(T.k, n, np, T.u + s0, root, rsz, rw, dl0, lane);
+      if (n <= 7 && n >= 4) {
+        if (n >= 5 && lane < 8) T.D2[n == 7 ? 12 + (lane & 1) : n == 6 ? 8 + (lane & 3) : lane] = c2(1.0, 0.0);
+        if (n == 4 && lane < 16) T.D2[lane] = c2(1.0, 0.0);
+      }
+      __syncwarp();
+      if (n >= 3) {
+        // orders above 8: 2^K0 subtrees of level 9's node, each its two children's; else one tree
+        const double2 *dl = n >= 8 ? dl0 : dl0 + min(lane >> lg, np - 1) * dsz; // (idle lanes: the last point's)
+        double2 D8 = c2(1.0, 0.0);
+        const int trees = n > 8 ? 2 << K0 : 1;
+        for (int tr = 0; tr < trees; ++tr) {
+          int node8 = node_base(8);
+          if (n > 8) {
+            if (pair_at) {
+              node8 = pair_at + 81 * (tr & 1);
+            }
+            if ((tr & 1) == 0) {
+              // the levels whose copy changed since the last subtree, down to level 9
+              const int sub = tr >> 1, first = sub == 0 ? 0 : K0 - __ffs(sub);
+              int off = 0;
+              for (int d = 0; d <= K0; ++d) {
+                const int m = n - d;
+                const double2 *S = d == K0 ? node9 : stack + off;
+                off += (m + 1) * (m + 1);
+                if (d < first) continue;
+                const double2 D2 = d == 0 ? c2(1.0, 0.0) : T.D2[15 + d];
+                if (d == K0)
+                  step_down<true>(S, pair8, dl0, 9, 0, lane, D2, D8, floor_, guard);
+                else
+                  step_down<false>(S, d + 1 == K0 ? node9 : stack + off, dl0, m, (sub >> (K0 - 1 - d)) & 1, lane, D2, D8,
+                                   floor_, guard);
+                if (lane == 0) T.D2[16 + d] = D8;
+                __syncwarp();
+              }
+            }
+            if (!pair_at) { // orders 15 and 16: level 8's node from global scratch
+              for (int e = lane; e < 81; e += 32) T.buf[node_base(8) + e] = pair8[81 * (tr & 1) + e];
+              __syncwarp();
+            }
           }
+          const double2 w = subtree<SCALE>(T, node8, D8, dl, n, lane, floor_, guard, scale);
+          v = (__popc(tr) & 1) ? c2(v.x - w.x, v.y - w.y) : cadd(v, w);
           __syncwarp();
         }
-        (void)src;
-        const double2 w = subtree<SCALE>(T, dl0, 8, lane, floor_, guard, scale);
-        v = (__popc(sub) & 1) ? c2(v.x - w.x, v.y - w.y) : cadd(v, w);
-        __syncwarp();
-      }
-    } else if (n >= 3) {
-      const int p = min(lane >> lg, np - 1); // idle lanes of a short pass repeat its last point's differences
-      v = subtree<SCALE>(T, dl0 + p * dsz, n, lane, floor_, guard, scale);
-    } else if (n == 2) {
-      if (lane < np) {
-        double2 s[9], d2[4];
-        const double2 *S = T.buf + lane * node_sz(2), *dl = dl0 + lane * dsz;
+      } else if (n == 2) {
+        if (lane < np) {
+          double2 s[9], d2[4];
+          const double2 *S = T.buf + lane * node_sz(2), *dl = dl0 + lane * dsz;
 #pragma unroll
-        for (int e = 0; e < 9; ++e) s[e] = S[e];
+          for (int e = 0; e < 9; ++e) s[e] = S[e];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) d2[e] = dl[2 + e];
-        if (!(cabs1(s[8]) >= floor_)) guard = true;
-        v = leaf2<SCALE>(s, dl[0], dl[1], d2, cmul(d2[0], dl[1]), cmul(dl[0], d2[2]), scale, floor_, guard);
+          for (int e = 0; e < 4; ++e) d2[e] = dl[2 + e];
+          if (!(cabs1(s[8]) >= floor_)) guard = true;
+          v = leaf2<SCALE>(s, dl[0], dl[1], d2, cmul(d2[0], dl[1]), cmul(dl[0], d2[2]), scale, floor_, guard);
+        }
+      } else if (lane < np) { // order 1: -p (X_f Y_f - X_b Y_b)
+        const double2 *S = T.buf + lane * node_sz(1), *dl = dl0 + lane * dsz;
+        const double2 dX = dl[0], dY = dl[1];
+        v = cmul(S[3], cfma(cmul(S[1], dY), dX, cadd(S[2], dY)));
+        v = c2(-v.x, -v.y);
+        if (SCALE) {
+          const double2 xb = S[1], yb = S[2], xf = cadd(xb, dX), yf = cadd(yb, dY);
+          scale = cabs(cmul(S[3], cfms(cmul(S[3], S[0]), xf, yf))) + cabs(cmul(S[3], cfms(cmul(S[3], S[0]), xb, yb)));
+        }
       }
-    } else if (lane < np) { // order 1: -p (X_f Y_f - X_b Y_b)
-      const double2 *S = T.buf + lane * node_sz(1), *dl = dl0 + lane * dsz;
-      const double2 dX = dl[0], dY = dl[1];
-      v = cmul(S[3], cfma(cmul(S[1], dY), dX, cadd(S[2], dY)));
-      v = c2(-v.x, -v.y);
-      if (SCALE) {
-        const double2 xb = S[1], yb = S[2], xf = cadd(xb, dX), yf = cadd(yb, dY);
-        scale = cabs(cmul(S[3], cfms(cmul(S[3], S[0]), xf, yf))) + cabs(cmul(S[3], cfms(cmul(S[3], S[0]), xb, yb)));
+      const unsigned gm = __ballot_sync(FULL, guard);
+      if (gm) {
+        const unsigned mine = lg == 5 ? gm : (gm >> ((lane << lg) & 31)) & ((1u << (1 << lg)) - 1u);
+        guarded |= __ballot_sync(FULL, lane < np && mine) << s0;
       }
     }
-    for (int off = 1; off < (1 << lg); off <<= 1) {
-      v.x += __shfl_xor_sync(FULL, v.x, off);
-      v.y += __shfl_xor_sync(FULL, v.y, off);
-      if (SCALE) scale += __shfl_xor_sync(FULL, scale, off);
+    if (SCALE) {
+      for (int off = 1; off < (1 << lg); off <<= 1) scale += __shfl_xor_sync(FULL, scale, off);
+      if ((lane & ((1 << lg) - 1)) == 0 && (lane >> lg) < np) T.fscale[s0 + (lane >> lg)] = scale;
     }
-    const unsigned gm = __ballot_sync(FULL, guard);
-    const int p = lane >> lg;
-    if ((lane & ((1 << lg) - 1)) == 0 && p < np) {
-      T.fval[s0 + p] = v;
-      T.fl[s0 + p] = ((gm >> lane) & (lg == 5 ? FULL : (1u << (1 << lg)) - 1u)) != 0u;
-      if (SCALE) T.fscale[s0 + p] = scale;
+    // sums over a point's lanes. Of four passes at a time (4 lanes per point and up): the first two
+    // rounds leave the lanes of each residue mod 4 with one pass's value, the others sum those
+    if (lg >= 2) {
+      if ((t & 1) == 0) {
+        h0 = v;
+      } else if ((t & 3) == 1) {
+        h1 = merge_lanes(h0, v, 1, lane);
+      } else {
+        v = merge_lanes(h1, merge_lanes(h0, v, 1, lane), 2, lane);
+        for (int off = 4; off < (1 << lg); off <<= 1) {
+          v.x += __shfl_xor_sync(FULL, v.x, off);
+          v.y += __shfl_xor_sync(FULL, v.y, off);
+        }
+        const int q = (t - 3 + (lane & 3)) * P + (lane >> lg);
+        if ((lane & ((1 << lg) - 4)) == 0 && q < cnt) T.fval[q] = v;
+      }
+    } else {
+      if (lg == 1) {
+        v.x += __shfl_xor_sync(FULL, v.x, 1);
+        v.y += __shfl_xor_sync(FULL, v.y, 1);
+      }
+      if ((lane & ((1 << lg) - 1)) == 0 && (lane >> lg) < np) T.fval[s0 + (lane >> lg)] = v;
     }
     __syncwarp();
   }
+  return guarded;
 }
 
 __device__ __forceinline__ double2 cut_off(double2 f, double cutoff) { return cabs(f) < cutoff ? c2(0.0, 0.0) : f; }
@@ -641,7 +837,6 @@ __device__ __forceinline__ double2 cut_off(double2 f, double cutoff) { return ca
 // Persistent warps pull scheduling chunks (it.chunk_points points of one item) and walk them
 // in groups of up to 32 points (16 above order 8): set-up, values, then the group's sum in a
 // fixed shuffle order, so that results do not depend on which warp ran what.
-// Bound: FP64 issue and shared-memory reads of the levels; 12 warps per SM at 168 registers.
 template <bool EVAL, bool ANY_CUBIC, bool SCALE>
 __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel(Launch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -649,24 +844,50 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
   WarpShared<SCALE> &T = reinterpret_cast<WarpShared<SCALE> *>(smem_raw)[warp];
   double2 *stack = reinterpret_cast<double2 *>(L.pts) + (size_t)(blockIdx.x * TREE_WARPS + warp) * TREE_STACK;
   bool bad = false;
+  int item = -1, next = 0;
+  if (lane == 0) next = atomicAdd(L.chunk_counter, 1);
   for (;;) {
-    int c = 0;
-    if (lane == 0) c = atomicAdd(L.chunk_counter, 1);
-    c = __shfl_sync(FULL, c, 0);
+    const int c = __shfl_sync(FULL, next, 0);
     if (c >= L.n_chunks) break;
-    const int item = find_chunk_item(L.chunk_offsets, L.n_items, c);
+    if (lane == 0) next = atomicAdd(L.chunk_counter, 1); // the chunk after this one, ahead of its use
+    bool fresh = item < 0;
+    if (fresh || c >= L.chunk_offsets[item + 1]) {
+      item = find_chunk_item(L.chunk_offsets, L.n_items, c);
+      fresh = true;
+    }
     const ItemDev &it = L.items[item];
     const long long cfirst = (long long)(c - L.chunk_offsets[item]) * it.chunk_points;
     const int ccount = (int)min((long long)it.chunk_points, (long long)it.n_points - cfirst);
     const int N = it.order;
     const bool keep = EVAL ? (L.keep_u_hypercube != 0) : true;
-    const int lgp = N <= 8 ? 5 : 4;
-    double2 eq = c2(0.0, 0.0);
-    if (N > 0) {
+    const int lgp = group_lg(N);
+    const double rdelta = 1.0 / it.model.delta;
+    __syncwarp();
+    if (fresh && lane == 0 && N > 0) { // what the passes read of the item
+      const ModelDev &m = it.model;
+      const int spin = it.f.A.spin;
       double2 gl, gg;
       int b0 = 0;
-      g0_pair(it.model, it.model.tab[it.f.A.spin][0][0], 0.0, gl, gg, &b0);
-      eq = c2(gl.x, gl.y - it.model.alpha);
+      g0_pair(m, m.tab[spin][0][0], 0.0, gl, gg, &b0);
+      T.k.eq = c2(gl.x, gl.y - m.alpha);
+      const double2 *tab[4] = {m.tab[spin][0][0], m.tab[spin][0][0], m.tab[spin][it.f.A.orbital][0],
+                               m.tab[spin][0][it.f.B.orbital]};
+      // A later than the vertex (or at its time): forward copy g^>, backward g^<; earlier: A's branch
+      // decides. B likewise; of two vertices the earlier one's index.
+      constexpr unsigned GREATER = 0x3FF00000u, LESSER = 0xBFF00001u;
+      const unsigned w[4] = {GREATER, LESSER, GREATER, LESSER};
+      const unsigned alt[4] = {GREATER, LESSER, it.f.A.k_idx ? 1u : 0u, it.f.B.k_idx ? 0u : 1u};
+      for (int k = 0; k < 4; ++k) {
+        const unsigned none = tab[k] ? 0u : 2u;
+        T.k.kind[k] = EntryKind{tab[k] ? tab[k] : no_table, w[k] | none, alt[k] | none};
+      }
+      T.k.xmin = m.xmin;
+      T.k.delta = m.delta;
+      T.k.rdelta = rdelta;
+      T.k.floor_ = m.pivot_floor;
+      T.k.lookup = lookups.e + lookups.first[N];
+      T.k.last = m.npts - 2;
+      T.k.cubic = m.interp == 3;
     }
     if (!EVAL && L.nbins) {
       for (int b = lane; b < L.nbins; b += 32) {
@@ -682,15 +903,31 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
       const int cnt = min(1 << lgp, ccount - g0);
       const bool mine = lane < cnt;
       double jac;
-      bool dom;
-      setup_group(L, it, N, lgp, cfirst + g0, cnt, keep, T.u, reinterpret_cast<double *>(T.buf), lane, jac, dom);
+      bool dom, sorted;
+      setup_group(L, it, N, lgp, cfirst + g0, cnt, keep, T.u + (1 << lgp), reinterpret_cast<double *>(T.buf), lane, jac, dom, sorted);
       int bin = -1;
-      if (!EVAL && L.nbins && mine) bin = earliest_bin(L, T.u + lane, 1 << lgp, N);
-      if (mine) sort_times(T.u + lane, 1 << lgp, N);
+      if (!EVAL && L.nbins && mine) bin = earliest_bin(L, T.u + (1 << lgp) + lane, 1 << lgp, N);
       const unsigned dommask = __ballot_sync(FULL, mine && dom);
+      unsigned guarded = 0;
       if (N > 0) {
+        bool in = mine && dom;
+        double *ul = T.u + (1 << lgp) + lane;
+        if (!sorted) sort_times(ul, 1 << lgp, N); // (the plasma warper's times come sorted)
+        if (in && !in_window(it, N, ul, 1 << lgp, rdelta)) {
+          bad = true;
+          in = false;
+        }
+        if (mine) {
+          // a point that is not evaluated still takes its place in a pass: at A's time, inside the window
+          const double tA = it.f.A.time;
+          if (!in)
+            for (int j = 0; j < N; ++j) ul[j << lgp] = tA;
+          T.u[lane] = tA;
+          T.u[((N + 1) << lgp) + lane] = it.f.B.time;
+        }
+        const unsigned inmask = __ballot_sync(FULL, in);
         __syncwarp();
-        group_values<SCALE, ANY_CUBIC>(T, it, N, lgp, cnt, dommask, eq, stack, lane, bad);
+        guarded = group_values<SCALE, ANY_CUBIC>(T, N, cnt, inmask, stack, lane);
       } else if (mine) { // order 0: g0(A, B)
         kb_gf_index a = it.f.A, b = it.f.B;
         a.timesplit = b.timesplit = 0;
@@ -698,13 +935,12 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
         const double2 v = dom ? g0_contour(it.model, a, b, 0, &b0) : c2(0.0, 0.0);
         bad = bad || b0;
         T.fval[lane] = v;
-        T.fl[lane] = 0;
         if (SCALE) T.fscale[lane] = cabs(v);
       }
       __syncwarp();
       const double2 fv = mine ? T.fval[lane] : c2(0.0, 0.0);
       const bool ok = mine && dom;
-      const bool fb = ok && (T.fl[lane] || !isfinite(fv.x) || !isfinite(fv.y));
+      const bool fb = ok && (((guarded >> lane) & 1u) || !isfinite(fv.x) || !isfinite(fv.y));
       if (EVAL) {
         if (mine) {
           const long long o = cfirst + g0 + lane;
