@@ -1252,8 +1252,9 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
     if (st) return st;
     KB_CHECK(work[i].order <= KM_MAX_ORDER, "the kernel method runs orders 1..10");
     KB_CHECK(!work[i].flow, "the kernel method does not take a learned flow");
-    items[(size_t)i].chunk_points = 16; // a CTA evaluates its chunk's points one after another
-    offs.push_back(offs.back() + (items[(size_t)i].n_points + 15) / 16);
+    const int64_t cp = items[(size_t)i].chunk_points =
+        item_chunk(ctx, work[i].order, items[(size_t)i].n_points, CHUNK_POINTS, INT64_MAX);
+    offs.push_back(offs.back() + (items[(size_t)i].n_points + cp - 1) / cp);
   }
   const long long nchunks = offs.back();
   if (nchunks > INT32_MAX) return fail(KB_E_INVALID, "too many points in one call");
@@ -1309,13 +1310,14 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
   KB_CUDA(dpts.alloc((size_t)kgrid * KM_SLOT * sizeof(double), st));
   L.pts = dpts.as<double>();
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[0], st));
-  KB_CUDA(launch_kernel_method(L, kgrid, st));
+  KB_CUDA(launch_km_tree(L, kgrid, st));
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[1], st));
+  KB_CUDA(launch_km_fallback(L, ctx->sm_count * 4, st));
   KB_CUDA(launch_reduce(L, dacc.as<kb_accum>(), st));
   if (nb)
     KB_CUDA(launch_reduce_bins(L, dos.as<double2>(), doc.as<unsigned long long>(), dod.as<unsigned long long>(), st));
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[2], st));
-  ctx->last_launches = nb ? 3 : 2;
+  ctx->last_launches = nb ? 4 : 3;
   std::vector<kb_accum> part(items.size());
   std::vector<double> hbs(items.size() * nb * 2);
   std::vector<unsigned long long> hbc(items.size() * nb), hbd(items.size());
@@ -1385,14 +1387,15 @@ int kb_integrand_kernel_eval(kb_context *ctx, const kb_model *m, const kb_gf_ind
   if (count == 0) return KB_OK;
   ItemDev it = make_item(m, &f, order);
   it.n_points = count;
-  it.chunk_points = 16;
+  it.chunk_points = item_chunk(ctx, order, count, 32, INT64_MAX);
   std::lock_guard<std::mutex> lk(ctx->mu);
   KB_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
-  const long long nchunks = (count + 15) / 16;
+  const long long nchunks = (count + it.chunk_points - 1) / it.chunk_points;
   long long offs[2] = {0, nchunks};
-  DevBuf ditem, doff, dcnt, din, dout, ddom;
+  DevBuf ditem, doff, dcnt, din, dout, ddom, dpart;
   KB_CUDA(ditem.alloc(sizeof(ItemDev), s));
+  KB_CUDA(dpart.alloc((size_t)nchunks * sizeof(ChunkPartial), s));
   KB_CUDA(doff.alloc(sizeof(offs), s));
   KB_CUDA(dcnt.alloc(sizeof(int), s));
   KB_CUDA(din.alloc((size_t)count * order * sizeof(double), s));
@@ -1414,6 +1417,7 @@ int kb_integrand_kernel_eval(kb_context *ctx, const kb_model *m, const kb_gf_ind
   L.mode = IN_TIMES;
   L.keep_u_hypercube = keep_u_hypercube;
   L.in = din.as<double>();
+  L.partials = dpart.as<ChunkPartial>();
   L.out_kvals = dout.as<double2>();
   L.out_dom = ddom.as<int>();
   L.err = ctx->d_err;
@@ -1421,7 +1425,8 @@ int kb_integrand_kernel_eval(kb_context *ctx, const kb_model *m, const kb_gf_ind
   DevBuf dpts;
   KB_CUDA(dpts.alloc((size_t)kgrid * KM_SLOT * sizeof(double), s));
   L.pts = dpts.as<double>();
-  KB_CUDA(launch_kernel_method(L, kgrid, s));
+  KB_CUDA(launch_km_tree(L, kgrid, s));
+  KB_CUDA(launch_km_fallback(L, (int)std::min<long long>(nchunks, ctx->sm_count * 4), s));
   int err = 0;
   KB_CUDA(cudaMemcpyAsync(out, dout.p, (size_t)count * 2 * order * sizeof(double2), cudaMemcpyDeviceToHost, s));
   if (in_domain) KB_CUDA(cudaMemcpyAsync(in_domain, ddom.p, (size_t)count * sizeof(int), cudaMemcpyDeviceToHost, s));

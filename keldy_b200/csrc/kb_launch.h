@@ -30,11 +30,14 @@ constexpr int TREE_WARPS = 3;
 constexpr int TREE_CTAS_PER_SM = 4;
 constexpr int TREE_STACK = 1662;
 constexpr int PTS_SLOT = TREE_WARPS * TREE_STACK * 2; // doubles per CTA
-// Per-CTA slot of the kernel-method tree: the chunk's set-up (coordinates
-// [MAX_ORDER][CHUNK_POINTS], then Jacobians, domain flags and bin codes).
-constexpr int KM_SLOT = CHUNK_POINTS * (MAX_ORDER + 5);
-// Resident CTAs per SM of the kernel-method tree (256 threads, ~114 KB of shared memory).
-constexpr int KM_CTAS_PER_SM = 2;
+// The kernel-method tree (km_tree.cu): warps of a CTA, resident CTAs per SM (8 warps: 255 registers
+// per thread, 25 KB of shared memory per warp), and a warp's global scratch (complex entries): the
+// nodes of orders 9 and 10 above level 8.
+constexpr int KM_MAX_ORDER = 10;
+constexpr int KM_WARPS = 2;
+constexpr int KM_CTAS_PER_SM = 4;
+constexpr int KM_STACK = 11 * 12 + 10 * 11;
+constexpr int KM_SLOT = KM_WARPS * KM_STACK * 2; // doubles per CTA
 
 struct Launch {
   const ItemDev *items; // device
@@ -98,8 +101,10 @@ cudaError_t launch_reduce(const Launch &L, kb_accum *acc_dev, cudaStream_t st);
 // over the item's chunks in chunk order (written, not added)
 // keldy's kernel-method integrand (integrand_g_kernel): IN_SOBOL with time bins of 2
 // columns, or IN_TIMES into out_kvals. Orders 1..KM_MAX_ORDER.
-constexpr int KM_MAX_ORDER = 10;
-cudaError_t launch_kernel_method(const Launch &L, int grid, cudaStream_t st);
+cudaError_t configure_km_kernel();
+cudaError_t launch_km_tree(const Launch &L, int grid, cudaStream_t st);
+// the pivoted-LU evaluation of the points it marked (chunk partials' fb_mask)
+cudaError_t launch_km_fallback(const Launch &L, int grid, cudaStream_t st);
 cudaError_t launch_reduce_bins(const Launch &L, double2 *sums, unsigned long long *counts,
                                unsigned long long *dropped, cudaStream_t st);
 

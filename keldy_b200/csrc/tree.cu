@@ -23,9 +23,7 @@ namespace kb {
 namespace {
 
 constexpr int NT = CTA_THREADS;
-// first of the set-up slot's three rows of per-point bin data (after the coordinates,
-// the Jacobians and the flags)
-constexpr int BIN_CODE_ROW = MAX_ORDER + 2;
+
 __device__ __forceinline__ int find_item(const long long *off, int n_items, long long c) {
   int lo = 0, hi = n_items; // off[lo] <= c < off[hi]
   while (hi - lo > 1) {
@@ -95,41 +93,6 @@ __device__ __forceinline__ int time_bin(const Launch &L, const double *u, int st
   if (!(L.bin_xmin <= t && t <= L.bin_xmax)) return -1;
   if (t == L.bin_xmax) return L.nbins - 1;
   return min((int)((t - L.bin_xmin) / L.bin_size), L.nbins - 1);
-}
-
-// One point of a chunk, on one thread: Sobol coordinates (or the given inputs), the
-// warper chain, the domain flag; written to the CTA's set-up slot at column t.
-__device__ void prepare_point(const Launch &L, const ItemDev &it, int N, long long gp, bool keep, double *slot,
-                              int t) {
-  double x[MAX_ORDER];
-  double jac = 1.0;
-  if (L.mode == IN_SOBOL) {
-    if (it.flow_x) { // Sobol point already mapped by the learned flow
-      for (int j = 0; j < N; ++j) x[j] = it.flow_x[gp * N + j];
-      jac = it.flow_jac[gp];
-    } else {
-      const uint32_t k = it.k_first + (uint32_t)gp;
-      for (int j = 0; j < N; ++j) x[j] = sobol_coord(it.rng, k, j);
-      if (it.spline_knots) jac = spline_flow_point(it.spline_knots, N, x, 1);
-      if (it.ar_spline) jac = ar_spline_point(it.ar_spline, N, x, 1);
-    }
-    jac *= chain_reverse(it.chain, it.chain_len, 0, N, x, 1);
-  } else {
-    const long long src = L.index ? (long long)L.index[gp] : gp;
-    for (int j = 0; j < N; ++j) x[j] = L.in[src * N + j];
-    if (L.mode == IN_LI) jac = chain_reverse(it.chain, it.chain_start, 0, N, x, 1);
-  }
-  int dom = (it.f.A.spin == it.f.B.spin) ? 1 : 0;
-  if (keep)
-    for (int j = 0; j < N; ++j)
-      if (x[j] < 0.0) dom = 0;
-  for (int j = 0; j < N; ++j) slot[j * CHUNK_POINTS + t] = x[j];
-  slot[MAX_ORDER * CHUNK_POINTS + t] = jac;
-  slot[(MAX_ORDER + 1) * CHUNK_POINTS + t] = dom ? 0.0 : 1.0;
-  if (L.nbins) { // the time bin of the earliest vertex: code 2 bin, or -1 when dropped
-    const int bin = time_bin(L, x, 1, N);
-    slot[BIN_CODE_ROW * CHUNK_POINTS + t] = bin < 0 ? -1.0 : (double)(2 * bin);
-  }
 }
 
 // G (row-major, M = 2N+1) of np points: G[p*M*M + r*M + c]. Out-of-domain points get
@@ -504,9 +467,10 @@ __global__ void __launch_bounds__(NT) direct_kernel(Launch L) {
 __device__ __forceinline__ int next_guarded(const Launch &L, long long first, int step, int after, unsigned *found) {
   if (after < 0) {
     const long long c = first + (long long)threadIdx.x * step;
-    const unsigned m = __ballot_sync(0xffffffffu, c < L.n_chunks && L.partials[c].n_fallback != 0);
+    const unsigned m =
+        __ballot_sync(0xffffffffu, threadIdx.x < NT && c < L.n_chunks && L.partials[c].n_fallback != 0);
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) found[threadIdx.x >> 5] = m;
+    if ((threadIdx.x & 31) == 0 && threadIdx.x < NT) found[threadIdx.x >> 5] = m;
     __syncthreads();
   }
   for (int k = after + 1; k < NT; k = (k | 31) + 1) {
@@ -617,16 +581,13 @@ __global__ void __launch_bounds__(RT) reduce_kernel(Launch L, kb_accum *acc) {
 }
 
 // ------------------------------------------------------------ kernel method
-// keldy's integrand_g_kernel (impurity_oneband/wick_kernel.cpp:42-138): with the fixed
-// point X in the external slot, for every Keldysh configuration a the matrix s1 (X first,
-// then the vertex copies picked by a; keldy zeroes its entry (n, n)) is factored with
-// partial pivoting and the first row of its cofactor matrix is found by solving
-// s1 x = det(s1) e_0 (first_row_expansion, det_expansion.hpp:44-74). Vertex i's term is
-// x_{i+1} (-1)^|a| det(s2_a), accumulated at (vertex time, a_i). Here the terms of a point
-// are summed per (vertex i, Keldysh index k) in configuration order (2n sums), then
-// binned; keldy accumulates them one by one into the same bins.
-// Threads of a km_tree_kernel CTA (two CTAs per SM: 16 warps); the points per pass stay
-// sized for 128 (km_points_per_pass), the extra warps hide the levels' latency.
+// keldy's integrand_g_kernel (impurity_oneband/wick_kernel.cpp:42-138) as keldy computes it: with
+// the fixed point X in the external slot, for every Keldysh configuration a the matrix s1 (X first,
+// then the vertex copies picked by a; keldy zeroes its entry (n, n)) is factored with partial
+// pivoting and the first row of its cofactor matrix is found by solving s1 x = det(s1) e_0
+// (first_row_expansion, det_expansion.hpp:44-74). Vertex i's term is x_{i+1} (-1)^|a| det(s2_a),
+// accumulated at (vertex time, a_i). For points with a guarded pivot in the tree form
+// (km_tree.cu) and models whose spins differ.
 constexpr int KM_THREADS = 256;
 struct KernelShared {
   double2 G1[(2 * KM_MAX_ORDER + 1) * (2 * KM_MAX_ORDER + 1)];
@@ -761,539 +722,72 @@ __device__ double2 kernel_point(KernelShared &K, const ItemDev &it, int N, int *
   return acc;
 }
 
-// ------------------------------------------------------------ kernel method, tree form
-// For spin-symmetric models det(s2_a) = det(V_a), V_a the vertex block of G picked by a,
-// and keldy's s1_a = [[g_XX, r], [c, W_a]] with W_a = V_a except its last vertex's
-// diagonal entry set to 0. The first-row cofactors of s1_a are x_0 = det(W_a) and
-// x_{i+1} = -det(W_a) (W_a^-1 c)_i (block inverse), so only the vertex block and the X
-// column enter. Gauss-Jordan elimination of the vertices in order 0..n-1, pivoting on the
-// diagonal entry of the chosen copy and carrying the X column, visits the 2^n
-// configurations as the leaves of a binary tree that shares its prefixes, as the direct
-// integrand's tree does; a node after j eliminations holds the j eliminated rows (pivot
-// rows normalised by their pivots), both copies' rows of the remaining vertices, and the
-// columns of the remaining copies plus the X column. At a leaf (copy b of the last
-// vertex), with D the product of the earlier pivots, p the last pivot and p_W = p minus
-// that copy's original diagonal entry (the Schur complement is affine in it with
-// coefficient 1), c_b the carried X entry of the last row and (e_j, f_j) an eliminated
-// row's last-copy and X entries:
-//   x_n = -D c_b,  x_{j+1} = -D (p_W f_j - e_j c_b),  det(V_a) = D p,
-// with no division by p_W (W_a may be singular, as for n = 1). Cost O(2^n n) per point
-// after the shared levels, instead of 2^n pivoted LU pairs. A point whose pivot falls
-// below the guard (or a model whose spins differ) takes keldy's pivoted-LU path,
-// kernel_point above, with the same per-(vertex, index) sums.
-
-// Sized for two CTAs per SM: at most 64 points per pass, 64 nodes per level, 128 vertex
-// times; the per-warp partial sums of the leaves' reduction live in the frontier buffer
-// that the last level leaves free.
-constexpr int KM_MAX_PASS = 64;
-// Complex entries per frontier buffer of the kernel-method tree: its widest level (64 nodes
-// of 10 x 5 at order 8, one point per pass) is larger than the direct tree's.
-constexpr int KM_FRONTIER = 3200;
-
-struct KMTreeShared {
-  union {
-    double2 buf[2][KM_FRONTIER];
-    KernelShared K; // the pivoted-LU path of a guarded point (after the tree pass)
-  };
-  double2 D[2][KM_MAX_PASS];
-  double2 inv[KM_MAX_PASS];
-  double u[2 * KM_MAX_PASS];   // vertex times, u[j * np + p]
-  double jac[KM_MAX_PASS];
-  int flag[KM_MAX_PASS];       // bit 0: out of domain, bit 1: a guarded pivot
-  double2 gd[KM_MAX_PASS][2];  // original diagonal entries of the last vertex's two copies, per point
-  double2 S[256];              // per point the 2n sums, S[p * 2n + 2i + k]
-  int bidx[256];               // per (point, vertex) the time bin (-1 dropped, -2 out of domain)
-};
-
-// Points per pass of the tree form: 2^(n-1) threads per point (one per configuration of
-// the first n-1 vertices; two for n = 1) up to the CTA's 128; orders 9 and 10 walk their first 2 and 3
-// levels one path at a time so that the widest level fits a frontier buffer.
-__host__ __device__ inline int km_points_per_pass(int n) { return n == 1 ? 64 : n <= 8 ? (128 >> (n - 1)) : 1; }
-__host__ __device__ inline int km_path_levels(int n) { return n <= 8 ? 0 : n - 7; }
-
-// Orders with path levels run 2^K0 passes from the same G (one point per pass). It stays
-// at the end of the frontier buffer that no level of a pass writes that far (level j
-// writes buffer (j + 1) & 1 from its start; the leaves' reduction scratch takes the first
-// 160 entries of the free buffer). Returns that buffer, or -1 (single pass, or no room).
-__host__ __device__ inline int km_root_buffer(int N) {
-  const int K0 = km_path_levels(N);
-  if (K0 == 0) return -1;
-  const int root = (2 * N + 1) * (2 * N + 1);
-  int use[2] = {0, 0}, nodes = 1;
-  for (int j = 0; j < N - 2; ++j) {
-    if (j >= K0) nodes *= 2;
-    const int sz = nodes * (2 * N - j - 1) * (2 * (N - j) - 1);
-    if (use[(j + 1) & 1] < sz) use[(j + 1) & 1] = sz;
-  }
-  const int b = use[0] <= use[1] ? 0 : 1;
-  return (use[b] + root <= KM_FRONTIER && root + 160 <= KM_FRONTIER) ? b : -1;
-}
-
-// One elimination level: vertex j of every node (rows 2n - j, columns 2(n - j) + 1,
-// stride `cs` elements per node) into its children (rows 2n - j - 1, columns
-// 2(n - j) - 1). bsel < 0: both children (child 2 par + b pivots on copy b); otherwise
-// the single child on copy bsel. inv and Dn get the children's pivot reciprocals and
-// prefix determinants. (Each item forming its own reciprocals instead, without the
-// barrier after them, was 2-5 % slower at orders 6-8; levels fused in pairs as in the
-// direct tree, with a pivot pre-pass and the children never stored, were 6-16 % slower at
-// orders 5-8: the kept rows make each grandchild entry cost 2.5 complex FMAs there
-// against 1.5 in two single levels.)
-__device__ void km_level(const double2 *cur, int cs, double2 *nxt, const double2 *Dc, double2 *Dn, double2 *inv,
-                         int *flag, int nodes, int lg_npp, int j, int n, int bsel, double floor_) {
-  const int R = 2 * n - j, C = 2 * (n - j) + 1;
-  const int R1 = R - 1, C1 = C - 2;
-  const int nch = bsel < 0 ? 2 : 1;
-  for (int c = threadIdx.x; c < nodes * nch; c += blockDim.x) {
-    const int par = bsel < 0 ? c >> 1 : c, b = bsel < 0 ? (c & 1) : bsel;
-    const double2 piv = cur[par * cs + (j + b) * C + b];
-    if (!(cabs1(piv) >= floor_)) flag[par >> lg_npp] |= 2;
-    inv[c] = crcp(piv);
-    Dn[c] = cmul(Dc[par], piv);
-  }
-  __syncthreads();
-  // rows split into column segments while the CTA has idle threads: of at least 4 columns,
-  // down to single columns when a pass holds at most 4 points (orders 6 and up, whose top
-  // levels have few rows: order 8 7 % faster, orders 9 / 10 6 / 5 %; orders 4-5 2 % slower)
-  const int rows = nodes * R1;
-  const int minc = (nodes >> lg_npp) <= 4 ? 1 : 4;
-  int lgseg = 0;
-  while ((rows << (lgseg + 1)) <= (int)blockDim.x && (C1 >> (lgseg + 1)) >= minc) ++lgseg;
-  const int seglen = (C1 + (1 << lgseg) - 1) >> lgseg;
-  const unsigned magic = 0xFFFFFFFFu / (unsigned)R1 + 1u; // r / R1 == umulhi(r, magic) for r < 2^20, R1 >= 3
-  for (int t = threadIdx.x; t < (rows << lgseg); t += blockDim.x) {
-    const int r = t >> lgseg;
-    const int q0 = (t & ((1 << lgseg) - 1)) * seglen, q1 = min(C1, q0 + seglen);
-    const int par = (int)__umulhi((unsigned)r, magic), ri = r - par * R1;
-    const double2 *S = cur + par * cs;
-    for (int k = 0; k < nch; ++k) {
-      const int b = bsel < 0 ? k : bsel;
-      const int ci = par * nch + k;
-      const double2 *prow = S + (j + b) * C + 2;
-      double2 *o = nxt + (size_t)ci * (R1 * C1) + ri * C1;
-      const double2 iv = inv[ci];
-      if (ri == j) {
-        for (int q = q0; q < q1; ++q) o[q] = cmul(prow[q], iv);
-      } else {
-        const int old = ri < j ? ri : ri + 1;
-        const double2 *srow = S + old * C;
-        const double2 Lf = cmul(srow[b], iv);
-#pragma unroll 4
-        for (int q = q0; q < q1; ++q) o[q] = cfms(srow[q + 2], Lf, prow[q]);
-      }
-    }
-  }
-  __syncthreads();
-}
-
-// The leaves under a node after n-2 eliminations (rows: n-2 eliminated, then vertex
-// n-2's two copies, then vertex n-1's; columns: the four copies, then X), on thread b
-// (copy of vertex n-2): the last elimination in registers, then both leaves. Adds the
-// terms into v[2i + k] (vertex i, Keldysh index k). path: the copies of vertices
-// 0..n-3 (bit n-3-i for vertex i), parity their count.
-template <int n>
-__device__ __forceinline__ void km_leaves2(const double2 *S, double2 D, const double2 *gd, int b, unsigned path,
-                                           int parity, double floor_, bool &guard, double2 (&v)[2 * n]) {
-  const int C = 5;
-  const double2 p1 = S[(n - 2 + b) * C + b];
-  if (!(cabs1(p1) >= floor_)) guard = true;
-  const double2 i1 = crcp(p1);
-  const double2 D1 = cmul(D, p1);
-  double2 prow[3];
-#pragma unroll
-  for (int q = 0; q < 3; ++q) prow[q] = cmul(S[(n - 2 + b) * C + 2 + q], i1);
-  // rows of vertex n-1's copies after the elimination: pivot, X entry, W pivot
-  double2 p[2], cb[2], pw[2];
-#pragma unroll
-  for (int bp = 0; bp < 2; ++bp) {
-    const double2 *r = S + (n + bp) * C;
-    const double2 Lf = r[b]; // prow is normalised by the pivot already
-    p[bp] = cfms(r[2 + bp], Lf, prow[bp]);
-    cb[bp] = cfms(r[4], Lf, prow[2]);
-    pw[bp] = c2(p[bp].x - gd[bp].x, p[bp].y - gd[bp].y);
-    if (!(cabs1(p[bp]) >= floor_)) guard = true;
-  }
-  // coefficient of each leaf: -D1 * det(V) * sign = -D1^2 p (-1)^(parity + b + bp)
-  double2 coef[2];
-#pragma unroll
-  for (int bp = 0; bp < 2; ++bp) {
-    double2 t = cmul(cmul(D1, D1), p[bp]);
-    if ((parity + b + bp) & 1) t = c2(-t.x, -t.y);
-    coef[bp] = c2(-t.x, -t.y);
-  }
-  // vertex n-1: x_n = -D1 c_b (the D1 factor is in coef)
-#pragma unroll
-  for (int bp = 0; bp < 2; ++bp) {
-    const double2 t = cmul(coef[bp], cb[bp]);
-    v[2 * (n - 1) + bp] = cadd(v[2 * (n - 1) + bp], t);
-  }
-  // eliminated rows: vertices 0..n-3 (rows 0..n-3), then vertex n-2 (the pivot row)
-#pragma unroll
-  for (int i = 0; i <= n - 2; ++i) {
-    double2 r0, r1, rx; // the child's row i at vertex n-1's copies and X
-    if (i == n - 2) {
-      r0 = prow[0];
-      r1 = prow[1];
-      rx = prow[2];
-    } else {
-      const double2 *r = S + i * C;
-      const double2 Lf = r[b];
-      r0 = cfms(r[2], Lf, prow[0]);
-      r1 = cfms(r[3], Lf, prow[1]);
-      rx = cfms(r[4], Lf, prow[2]);
-    }
-    const int k = (i == n - 2) ? b : (int)((path >> (n - 3 - i)) & 1u);
-    double2 acc = c2(0.0, 0.0);
-#pragma unroll
-    for (int bp = 0; bp < 2; ++bp) {
-      // x_{i+1} / D1 = p_W f - e c_b
-      const double2 x = cfms(cmul(pw[bp], rx), bp ? r1 : r0, cb[bp]);
-      acc = cadd(acc, cmul(coef[bp], x));
-    }
-    // to (i, k), written without a dynamic index so that v stays in registers
-    v[2 * i] = cadd(v[2 * i], k ? c2(0.0, 0.0) : acc);
-    v[2 * i + 1] = cadd(v[2 * i + 1], k ? acc : c2(0.0, 0.0));
-  }
-}
-
-// Sums the 2n values v[] over aligned groups of G consecutive threads (G a power of two)
-// into S[g * 2n + q] for group g < ngroups; fixed shuffle pattern (deterministic).
-template <int n2>
-__device__ void km_group_sum(double2 (&v)[n2], int G, int ngroups, double2 *S, double2 (*red)[2 * KM_MAX_ORDER]) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int gw = G < 32 ? G : 32;
-#pragma unroll
-  for (int q = 0; q < n2; ++q)
-    for (int off = 1; off < gw; off <<= 1) {
-      v[q].x += __shfl_xor_sync(0xffffffffu, v[q].x, off);
-      v[q].y += __shfl_xor_sync(0xffffffffu, v[q].y, off);
-    }
-  if (G <= 32) {
-    const int g = tid / G;
-    if ((lane & (G - 1)) == 0 && g < ngroups)
-#pragma unroll
-      for (int q = 0; q < n2; ++q) S[g * n2 + q] = cadd(S[g * n2 + q], v[q]);
-    __syncthreads();
-  } else {
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < n2; ++q) red[warp][q] = v[q];
-    __syncthreads();
-    const int wpg = G / 32;
-    for (int e = tid; e < ngroups * n2; e += blockDim.x) {
-      const int g = e / n2, q = e - g * n2;
-      double2 s = S[e];
-      for (int w = g * wpg; w < (g + 1) * wpg; ++w) s = cadd(s, red[w][q]);
-      S[e] = s;
-    }
-    __syncthreads();
-  }
-}
-
-// Per-point sums S of np points whose inputs are in K.u, K.flag (tree form; flag bit 1
-// marks points to redo on the pivoted-LU path).
-template <int N>
-__device__ void km_tree_points(KMTreeShared &K, const ItemDev &it, int np, int *bad) {
-  const int tid = threadIdx.x;
-  const int n2 = 2 * N;
-  for (int e = tid; e < np * n2; e += blockDim.x) K.S[e] = c2(0.0, 0.0);
-  __syncthreads();
-  const double floor_ = it.model.pivot_floor;
-  const int spin = it.f.A.spin;
-  const int K0 = km_path_levels(N);
-  const int M = 2 * N + 1;
-  // G built once for all passes (one point per pass) when it fits at a buffer's end
-  const int rb = km_root_buffer(N);
-  double2 *root = rb >= 0 ? K.buf[rb] + (KM_FRONTIER - M * M) : K.buf[0];
-  for (int sub = 0; sub < (1 << K0); ++sub) {
-    if (rb < 0 || sub == 0) build_G_any<true>(it, N, np, K.u, K.flag, root, spin, bad);
-    __syncthreads();
-    for (int p = tid; p < np; p += blockDim.x) {
-      K.D[0][p] = c2(1.0, 0.0);
-      const double2 *G = root + (size_t)p * M * M;
-      K.gd[p][0] = G[(2 * N - 2) * M + 2 * N - 2];
-      K.gd[p][1] = G[(2 * N - 1) * M + 2 * N - 1];
-    }
-    __syncthreads();
-    double2 v[2 * N];
-#pragma unroll
-    for (int q = 0; q < 2 * N; ++q) v[q] = c2(0.0, 0.0);
-    if (N == 1) {
-      // the leaves of the root itself: x_1 = -c_b, det(V) = p
-      if (tid < 2 * np) {
-        const int p = tid >> 1, b = tid & 1;
-        const double2 *G = K.buf[0] + (size_t)p * M * M;
-        const double2 piv = G[b * M + b], cb = G[b * M + 2];
-        double2 t = cmul(piv, cb);
-        if (!b) t = c2(-t.x, -t.y); // -(-1)^b p c_b
-        v[0] = b ? c2(0.0, 0.0) : t;
-        v[1] = b ? t : c2(0.0, 0.0);
-      }
-      km_group_sum<2 * N>(v, 2, np, K.S, reinterpret_cast<double2(*)[2 * KM_MAX_ORDER]>(K.buf[1]));
-      continue;
-    }
-    int cur = 0, cs = M * M, nodes = np, lg = 0;
-    for (int j = 0; j < N - 2; ++j) {
-      const int bsel = j < K0 ? (int)((sub >> (K0 - 1 - j)) & 1u) : -1;
-      km_level(j == 0 ? root : K.buf[cur], cs, K.buf[cur ^ 1], K.D[cur], K.D[cur ^ 1], K.inv, K.flag, nodes, lg, j,
-               N, bsel, floor_);
-      if (bsel < 0) {
-        nodes *= 2;
-        lg += 1;
-      }
-      cur ^= 1;
-      cs = (2 * N - j - 1) * (2 * (N - j) - 1);
-    }
-    // nodes after N-2 eliminations: 2 threads each
-    bool guard = false;
-    int p = 0;
-    if (tid < 2 * nodes) {
-      const int node = tid >> 1, b = tid & 1;
-      p = node >> lg;
-      const unsigned pathbits = ((unsigned)sub << lg) | (unsigned)(node & ((1 << lg) - 1));
-      if constexpr (N >= 2)
-        km_leaves2<N>(K.buf[cur] + (size_t)node * cs, K.D[cur][node], K.gd[p], b, pathbits, __popc(pathbits), floor_,
-                      guard, v);
-    }
-    if (guard) K.flag[p] |= 2;
-    km_group_sum<2 * N>(v, 2 << lg, np, K.S, reinterpret_cast<double2(*)[2 * KM_MAX_ORDER]>(K.buf[cur ^ 1]));
-  }
-}
-
-__device__ void km_tree_points_any(KMTreeShared &K, const ItemDev &it, int N, int np, int *bad) {
-  switch (N) {
-  case 1: km_tree_points<1>(K, it, np, bad); break;
-  case 2: km_tree_points<2>(K, it, np, bad); break;
-  case 3: km_tree_points<3>(K, it, np, bad); break;
-  case 4: km_tree_points<4>(K, it, np, bad); break;
-  case 5: km_tree_points<5>(K, it, np, bad); break;
-  case 6: km_tree_points<6>(K, it, np, bad); break;
-  case 7: km_tree_points<7>(K, it, np, bad); break;
-  case 8: km_tree_points<8>(K, it, np, bad); break;
-  case 9: km_tree_points<9>(K, it, np, bad); break;
-  default: km_tree_points<10>(K, it, np, bad); break;
-  }
-}
-
-// A pass's point values (one per thread, f, in the domain or not, with its dropped bin
-// terms) into the chunk's sums: each warp's by a fixed xor-shuffle pattern, then thread 0
-// adds the warps in order (deterministic). Every thread calls it; the caller's barrier
-// follows before the next pass.
-__device__ __noinline__ void km_pass_sum(double2 f, bool dom, unsigned long long drop, double2 &csum,
-                                         unsigned long long &cdom, unsigned *dropped) {
-  __shared__ double2 wsum[KM_THREADS / 32];
-  __shared__ unsigned wdom[KM_THREADS / 32];
-  __shared__ unsigned long long wdrop[KM_THREADS / 32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int off = 16; off > 0; off >>= 1) {
-    f.x += __shfl_xor_sync(0xffffffffu, f.x, off);
-    f.y += __shfl_xor_sync(0xffffffffu, f.y, off);
-    drop += __shfl_xor_sync(0xffffffffu, drop, off);
-  }
-  const unsigned bdom = __ballot_sync(0xffffffffu, dom);
-  if (lane == 0) {
-    wsum[w] = f;
-    wdom[w] = bdom;
-    wdrop[w] = drop;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long d = 0;
-    for (int k = 0; k < KM_THREADS / 32; ++k) {
-      csum = cadd(csum, wsum[k]);
-      cdom += __popc(wdom[k]);
-      d += wdrop[k];
-    }
-    if (dropped) *dropped += (unsigned)d;
-  }
-}
-
-// integrand_g_kernel_single_omega (wick_kernel_single_omega.cpp:126-135): point p's terms
-// weighted by e^{i omega t} of their vertex, in vertex order, times its Jacobian.
-__device__ __forceinline__ double2 km_fourier_value(const KMTreeShared &K, const Launch &L, int p, int np, int N) {
-  const int n2 = 2 * N;
-  double2 f = c2(0.0, 0.0);
-  for (int i = 0; i < N; ++i) {
-    double sn, cs;
-    sincos(L.km_omega * K.u[i * np + p], &sn, &cs);
-    const double2 sv = cadd(K.S[p * n2 + 2 * i], K.S[p * n2 + 2 * i + 1]);
-    f = cadd(f, cmul(sv, c2(cs, sn)));
-  }
-  const double j = K.jac[p];
-  return c2(f.x * j, f.y * j);
-}
-
-__global__ void __launch_bounds__(KM_THREADS, KM_CTAS_PER_SM) km_tree_kernel(Launch L) {
+// The points the tree form marked (fb_mask of the chunks' partials), one by one: their 2n sums to
+// out_kvals (IN_TIMES), or times their Jacobian to the chunk's bins and sum.
+__global__ void __launch_bounds__(KM_THREADS) km_fallback_kernel(Launch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  KMTreeShared &K = *reinterpret_cast<KMTreeShared *>(smem_raw);
-  __shared__ int s_chunk;
+  KernelShared &K = *reinterpret_cast<KernelShared *>(smem_raw);
   __shared__ int s_bad;
+  __shared__ unsigned s_found[NT / 32];
   const int tid = threadIdx.x;
   if (tid == 0) s_bad = 0;
+  __syncthreads();
   const bool eval = L.mode != IN_SOBOL;
-  const int nb = L.nbins * L.bin_cols;
-  for (;;) {
-    if (tid == 0) s_chunk = atomicAdd(L.chunk_counter, 1);
-    __syncthreads();
-    const int c = s_chunk;
-    if (c >= L.n_chunks) break;
+  const bool keep = eval ? (L.keep_u_hypercube != 0) : true;
+  const int nb = L.nbins * 2;
+  const long long step = gridDim.x;
+  int k = -1;
+  for (long long c0 = blockIdx.x; c0 < L.n_chunks;) {
+    k = next_guarded(L, c0, gridDim.x, k, s_found);
+    if (k < 0) {
+      c0 += NT * step;
+      continue;
+    }
+    const int c = (int)(c0 + k * step);
+    ChunkPartial pr = L.partials[c];
     const int item = find_item(L.chunk_offsets, L.n_items, c);
     const ItemDev &it = L.items[item];
+    const int N = it.order, n2 = 2 * N;
+    const unsigned half = 1u << (N - 1);
     const long long cfirst = (long long)(c - L.chunk_offsets[item]) * it.chunk_points;
-    const int ccount = (int)min((long long)it.chunk_points, it.n_points - cfirst);
-    const int N = it.order;
-    const int n2 = 2 * N;
-    const bool keep = L.mode == IN_SOBOL ? true : (L.keep_u_hypercube != 0);
-    if (!eval && nb) {
-      for (int b = tid; b < nb; b += blockDim.x) {
-        L.bin_sums[(size_t)c * nb + b] = c2(0.0, 0.0);
-        L.bin_counts[(size_t)c * nb + b] = 0u;
-      }
-      if (tid == 0) L.bin_dropped[c] = 0u;
-    }
-    double2 csum = c2(0.0, 0.0);
-    unsigned long long cdom = 0;
-    const int P = it.spin_symmetric ? km_points_per_pass(N) : 1;
-    // passes of at most 8 points (orders 5 and up): the chunk's points are set up at once
-    // (Sobol coordinates or given inputs, warper chain, domain flag: one thread per point)
-    // into the CTA's slot and each pass reads its own, instead of a pass's few threads
-    // walking the chain for its points while the others wait
-    const bool staged = P <= 8;
-    double *slot = L.pts + (size_t)blockIdx.x * KM_SLOT;
-    if (staged) {
-      if (tid < ccount) prepare_point(L, it, N, cfirst + tid, keep, slot, tid);
+    for (int bit = 0; bit < it.chunk_points; ++bit) {
+      if (!((pr.fb_mask[bit >> 6] >> (bit & 63)) & 1ull)) continue;
       __syncthreads();
-    }
-    for (int sb = 0; sb < ccount; sb += P) {
-      const int np = min(P, ccount - sb);
-      if (!staged) {
-        load_points(L, it, N, np, cfirst + sb, K.u, K.jac, K.flag, keep);
-      } else if (tid < np) {
-        for (int j = 0; j < N; ++j) K.u[j * np + tid] = slot[j * CHUNK_POINTS + sb + tid];
-        K.jac[tid] = slot[MAX_ORDER * CHUNK_POINTS + sb + tid];
-        K.flag[tid] = (int)slot[(MAX_ORDER + 1) * CHUNK_POINTS + sb + tid];
-      }
+      load_points(L, it, N, 1, cfirst + bit, K.u, K.jac, K.flag, keep);
       __syncthreads();
-      if (it.spin_symmetric) {
-        km_tree_points_any(K, it, N, np, &s_bad);
-      } else {
-        for (int e = tid; e < np * n2; e += blockDim.x) K.S[e] = c2(0.0, 0.0);
-        if (tid < np) K.flag[tid] |= (K.flag[tid] & 1) ? 0 : 2;
-        __syncthreads();
-      }
-      // guarded points (and the spin-asymmetric ones): keldy's pivoted-LU path, one by one
-      bool g = false; // any guarded point (every warp finds the same answer, no barrier)
-      for (int p = tid & 31; p < np; p += 32) g = g || (K.flag[p] & 3) == 2;
-      const bool any_guarded = __any_sync(0xffffffffu, g);
-      for (int p = 0; any_guarded && p < np; ++p) {
-        if ((K.flag[p] & 3) != 2) continue;
-        double ut[KM_MAX_ORDER];
-        for (int j = 0; j < N; ++j) ut[j] = K.u[j * np + p];
-        __syncthreads();
-        if (tid < N) K.K.u[tid] = ut[tid];
-        if (tid == 0) K.K.flag[0] = 0;
-        __syncthreads();
-        const double2 s = kernel_point(K.K, it, N, &s_bad);
-        if (tid < n2) K.S[p * n2 + tid] = s;
-        __syncthreads();
-      }
+      const double2 s = kernel_point(K, it, N, &s_bad);
+      if (tid < n2) K.S[tid] = s;
+      __syncthreads();
+      const double j = K.jac[0];
       if (eval) {
-        for (int e = tid; e < np * n2; e += blockDim.x) {
-          const int p = e / n2, q = e - p * n2;
-          const long long gp = cfirst + sb + p;
-          const bool dom = !(K.flag[p] & 1);
-          const double j = K.jac[p];
-          L.out_kvals[gp * n2 + q] = dom ? c2(K.S[e].x * j, K.S[e].y * j) : c2(0.0, 0.0);
-          if (q == 0) {
-            if (L.out_jac) L.out_jac[gp] = j;
-            if (L.out_dom) L.out_dom[gp] = dom ? 1 : 0;
+        if (tid < n2) L.out_kvals[(cfirst + bit) * n2 + tid] = c2(s.x * j, s.y * j);
+      } else if (tid == 0) {
+        for (int i = 0; i < N; ++i) {
+          if (L.km_fourier) {
+            double sn, cs;
+            sincos(L.km_omega * K.u[i], &sn, &cs);
+            const double2 v = cmul(cadd(K.S[2 * i], K.S[2 * i + 1]), c2(cs, sn));
+            pr.sum_re += v.x * j;
+            pr.sum_im += v.y * j;
+            continue;
           }
-        }
-      } else if (L.km_fourier) {
-        // integrand_g_kernel_single_omega (wick_kernel_single_omega.cpp:126-135): the
-        // point's terms weighted by e^{i omega t} of their vertex, in point and vertex order
-        // passes of more than two points: one thread per point, then km_pass_sum; one or
-        // two points: thread 0 in point order (no extra barrier)
-        if (P > 2) {
-          const bool dom = tid < np && !(K.flag[tid] & 1);
-          const double2 f = dom ? km_fourier_value(K, L, tid, np, N) : c2(0.0, 0.0);
-          km_pass_sum(f, dom, 0ull, csum, cdom, nullptr);
-        } else if (tid == 0) {
-          for (int p = 0; p < np; ++p) {
-            if (K.flag[p] & 1) continue;
-            cdom++;
-            csum = cadd(csum, km_fourier_value(K, L, p, np, N));
-          }
-        }
-      } else {
-        // bin of every (point, vertex); then one thread per (bin, index) adds the pass's
-        // terms in point and vertex order, as one thread walking them would
-        for (int e = tid; e < np * N; e += blockDim.x) {
-          const int p = e / N, i = e - p * N;
-          K.bidx[e] = (K.flag[p] & 1) ? -2 : time_bin(L, K.u + i * np + p, 1, 1);
-        }
-        __syncthreads();
-        const unsigned half = 1u << (N - 1);
-        for (int bk = tid; bk < nb; bk += blockDim.x) {
-          const int bin = bk >> 1, k = bk & 1;
-          double2 bs = L.bin_sums[(size_t)c * nb + bk];
-          unsigned cnt = 0;
-          bool any = false;
-          for (int p = 0; p < np; ++p) {
-            const double j = K.jac[p];
-            for (int i = 0; i < N; ++i)
-              if (K.bidx[p * N + i] == bin) {
-                const double2 sv = K.S[p * n2 + 2 * i + k];
-                bs = c2(bs.x + sv.x * j, bs.y + sv.y * j);
-                cnt += half;
-                any = true;
-              }
-          }
-          if (any) {
-            L.bin_sums[(size_t)c * nb + bk] = bs;
-            L.bin_counts[(size_t)c * nb + bk] += cnt;
-          }
-        }
-        if (P > 2) { // as above: one thread per point, then km_pass_sum
-          double2 f = c2(0.0, 0.0);
-          unsigned long long drop = 0;
-          const bool dom = tid < np && !(K.flag[tid] & 1);
-          if (dom) {
-            const double j = K.jac[tid];
-            for (int i = 0; i < N; ++i) {
-              if (K.bidx[tid * N + i] < 0) drop += 2 * half;
-              for (int k = 0; k < 2; ++k) {
-                const double2 sv = K.S[tid * n2 + 2 * i + k];
-                f = c2(f.x + sv.x * j, f.y + sv.y * j);
-              }
-            }
-          }
-          km_pass_sum(f, dom, drop, csum, cdom, L.bin_dropped + c);
-        } else if (tid == 0) {
-          for (int p = 0; p < np; ++p) {
-            if (K.flag[p] & 1) continue;
-            cdom++;
-            const double j = K.jac[p];
-            for (int i = 0; i < N; ++i) {
-              if (K.bidx[p * N + i] < 0) L.bin_dropped[c] += 2 * half;
-              for (int k = 0; k < 2; ++k) {
-                const double2 sv = K.S[p * n2 + 2 * i + k];
-                csum = c2(csum.x + sv.x * j, csum.y + sv.y * j);
-              }
-            }
+          const int bin = time_bin(L, K.u + i, 1, 1);
+          if (bin < 0) L.bin_dropped[c] += 2 * half;
+          for (int q = 0; q < 2; ++q) {
+            const double2 v = c2(K.S[2 * i + q].x * j, K.S[2 * i + q].y * j);
+            pr.sum_re += v.x;
+            pr.sum_im += v.y;
+            if (bin < 0) continue;
+            const size_t b = (size_t)c * nb + 2 * bin + q;
+            L.bin_sums[b] = cadd(L.bin_sums[b], v);
+            L.bin_counts[b] += half;
           }
         }
       }
-      __syncthreads();
     }
-    if (!eval && tid == 0) {
-      ChunkPartial pr;
-      pr.sum_re = csum.x;
-      pr.sum_im = csum.y;
-      pr.n_in_domain = cdom;
-      pr.n_fallback = 0;
-      pr.fb_mask[0] = pr.fb_mask[1] = 0;
-      L.partials[c] = pr;
-    }
+    __syncthreads();
+    if (tid == 0) L.partials[c] = pr;
+    __syncthreads();
   }
   if (tid == 0 && s_bad) atomicOr(L.err, 1);
 }
@@ -1347,8 +841,8 @@ __global__ void __launch_bounds__(32 * BW) reduce_bins_kernel(Launch L, double2 
 // The launchers rely on configure_kernels() having set the kernels' shared-memory limits
 // on the launching device: kb_context_create calls it, with the context's device current,
 // for every context (the attribute belongs to each device's context, not to the process).
-cudaError_t launch_kernel_method(const Launch &L, int grid, cudaStream_t st) {
-  km_tree_kernel<<<grid, KM_THREADS, (int)sizeof(KMTreeShared), st>>>(L);
+cudaError_t launch_km_fallback(const Launch &L, int grid, cudaStream_t st) {
+  km_fallback_kernel<<<grid, KM_THREADS, (int)sizeof(KernelShared), st>>>(L);
   return cudaGetLastError();
 }
 
@@ -1367,7 +861,8 @@ cudaError_t configure_kernels() {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(fallback_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DirectShared));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(km_tree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KMTreeShared));
+    e = cudaFuncSetAttribute(km_fallback_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KernelShared));
+  if (e == cudaSuccess) e = configure_km_kernel();
   return e;
 }
 

@@ -1,0 +1,48 @@
+"""The kernel method's tree kernel where its layout changes: point counts around a pass (256 >> n
+points) and a group, at every order's first level; the zeroed vertex (the last one) at any place in
+time, equal times, vertices later than X, X on either branch; and points handed to the pivoted
+LU next to others. Against the CPU oracle, |gpu - cpu| <= 1e-12 of the point's sum of |terms|."""
+import numpy as np
+import pytest
+
+from keldy_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 6, 7, 8, 9, 10])
+def test_point_counts_places_and_branches(ctx, oracle, golden, n):
+    le, gr = golden["table_beta20_lesser"], golden["table_beta20_greater"]
+    gm, om = ctx.model(10.0, le, gr, 0.4), oracle.model(10.0, le, gr, 0.4)
+    rng = np.random.default_rng(60 + n)
+    per_pass = 32 if n <= 3 else max(1, 256 >> n)
+    counts = {1, per_pass + 1, 33} if n <= 6 else {1, per_pass + 1, 17} if n <= 8 else {2}
+    for k, count in enumerate(sorted(counts)):
+        X = (6.0, 0, (n + k) % 2, 0, 0)
+        t = rng.random((count, n)) * 10.0
+        if n > 1:
+            t[::2, n - 1] = t[::2, 0]  # the zeroed vertex at another one's time
+        t[-1, 0] = X[0]
+        got, dom = gm.integrand_kernel(X, t)
+        want, odom, sc = oracle.integrand_kernel(om, X, t)
+        assert np.array_equal(dom, odom)
+        assert np.all(np.abs(got - want).max(axis=(1, 2)) <= 1e-12 * np.maximum(sc, 1e-300)), (n, count)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 6])
+def test_guarded_points_among_others(ctx, oracle, n):
+    """A table whose g(0) is small but not zero for some copies: every point of it goes to the
+    pivoted LU; in one call with an ordinary model's item, both sums equal the oracle's."""
+    t = np.linspace(-10, 10, 2001)
+    le = 1j * t * np.exp(-t * t / 8) + 0.2 * np.sin(t)
+    odd = (le, -np.conj(le[::-1]))
+    le2 = 0.5j * np.exp(-np.abs(t)) + 0.1 * np.sin(t) * np.exp(-np.abs(t))
+    plain = (le2, -np.conj(le2))
+    X = (10.0, 0, 0, 0, 0)
+    chain = [(capi.WARPER_PLASMA_UV, 10.0, 0.0), (capi.WARPER_EXPONENTIAL, 10.0, 1.0)]
+    items = [dict(model=ctx.model(10.0, *m), rng=ctx.sobol(n), chain=chain, A=X, order=n, k_first=5, n_points=151)
+             for m in (odd, plain)]
+    for (s, npt, nd, bins, cnt, drop), m in zip(capi.integrate_kernel(ctx, items, 7, 1.0, 9.0), (odd, plain)):
+        ws, onp, ond, sc, ob, oc, od = oracle.integrate_kernel(oracle.model(10.0, *m), X, chain, n, 151, 7, 1.0, 9.0, seed=4)
+        assert (npt, nd, drop) == (onp, ond, od) and np.array_equal(cnt, oc)
+        assert np.abs(bins - ob).max() <= 1e-12 * sc and abs(s - ws) <= 1e-12 * sc
