@@ -828,6 +828,30 @@ static int item_chunk(const kb_context *ctx, int order, int64_t n, int most, int
   return c;
 }
 
+} // extern "C"
+
+// Places in one device block: an allocation, an upload and a download per call instead of one per
+// array (each costs the host 2 to 5 us, most of a small call).
+namespace {
+struct Block {
+  size_t size = 0;
+  size_t take(size_t bytes) {
+    const size_t at = size;
+    size += (bytes + 255) / 256 * 256;
+    return at;
+  }
+};
+// The tree kernel's global scratch: only orders above 9 keep nodes there.
+size_t tree_scratch(int grid, int max_order) {
+  return max_order > 9 ? (size_t)grid * PTS_SLOT * sizeof(double) : 0;
+}
+template <typename T> T *place(const DevBuf &b, size_t at) {
+  return reinterpret_cast<T *>(static_cast<unsigned char *>(b.p) + at);
+}
+} // namespace
+
+extern "C" {
+
 // Runs the tree (or direct) kernel over `count` points of one item in an evaluation
 // mode, then re-evaluates points the tree flagged with the pivoted-LU kernel.
 static int run_eval(kb_context *ctx, ItemDev it, int mode, int64_t count, const double *in_host, int keep,
@@ -845,77 +869,84 @@ static int run_eval(kb_context *ctx, ItemDev it, int mode, int64_t count, const 
   if (use_tree) it.chunk_points = item_chunk(ctx, N, count, 32, INT64_MAX); // a warp per chunk: 32 points fill its lanes
   long long nchunks = (count + it.chunk_points - 1) / it.chunk_points;
   long long offs[2] = {0, nchunks};
-  DevBuf ditem, doff, dcnt, din, dval, djac, ddom, dscale, dflag;
-  KB_CUDA(ditem.alloc(sizeof(ItemDev), st));
-  KB_CUDA(doff.alloc(sizeof(offs), st));
-  KB_CUDA(dcnt.alloc(sizeof(int), st));
-  size_t inbytes = (size_t)count * N * sizeof(double);
-  KB_CUDA(din.alloc(inbytes, st));
-  KB_CUDA(dval.alloc(count * sizeof(double2), st));
-  KB_CUDA(djac.alloc(count * sizeof(double), st));
-  KB_CUDA(ddom.alloc(count * sizeof(int), st));
-  KB_CUDA(dflag.alloc(count * sizeof(int), st));
-  if (scale) KB_CUDA(dscale.alloc(count * sizeof(double), st));
-  KB_CUDA(cudaMemcpyAsync(ditem.p, &it, sizeof(ItemDev), cudaMemcpyHostToDevice, st));
-  KB_CUDA(cudaMemcpyAsync(doff.p, offs, sizeof(offs), cudaMemcpyHostToDevice, st));
-  if (inbytes) KB_CUDA(cudaMemcpyAsync(din.p, in_host, inbytes, cudaMemcpyHostToDevice, st));
-  KB_CUDA(cudaMemsetAsync(dcnt.p, 0, sizeof(int), st));
-  KB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), st));
+  const int grid = (int)std::min<long long>(nchunks, use_tree ? ctx->tree_grid : ctx->sm_count * 4);
+  const size_t inbytes = (size_t)count * N * sizeof(double);
+  struct Head { // uploaded in one piece
+    ItemDev it;
+    long long offs[2];
+    int counter, flagged, err, pad;
+  } head;
+  memset(&head, 0, sizeof(head));
+  head.it = it;
+  memcpy(head.offs, offs, sizeof(offs));
+  Block B;
+  const size_t a_head = B.take(sizeof(Head)), a_in = B.take(inbytes), a_val = B.take(count * sizeof(double2)),
+               a_jac = B.take(count * sizeof(double)), a_dom = B.take(count * sizeof(int)),
+               a_flag = B.take(count * sizeof(int)), a_scale = B.take(scale ? count * sizeof(double) : 0),
+               a_pts = B.take(use_tree ? tree_scratch(grid, N) : 0);
+  DevBuf buf;
+  KB_CUDA(buf.alloc(B.size, st));
+  Head *dh = place<Head>(buf, a_head);
+  KB_CUDA(cudaMemcpyAsync(dh, &head, sizeof(head), cudaMemcpyHostToDevice, st));
+  if (inbytes) KB_CUDA(cudaMemcpyAsync(place<double>(buf, a_in), in_host, inbytes, cudaMemcpyHostToDevice, st));
   Launch L;
   memset(&L, 0, sizeof(L));
-  L.items = ditem.as<ItemDev>();
+  L.items = &dh->it;
   L.n_items = 1;
   L.any_cubic = items_any_cubic(&it, 1);
-  L.chunk_offsets = doff.as<long long>();
+  L.chunk_offsets = dh->offs;
   L.n_chunks = (int)nchunks;
-  L.chunk_counter = dcnt.as<int>();
+  L.chunk_counter = &dh->counter;
   L.mode = mode;
   L.keep_u_hypercube = keep;
-  L.in = din.as<double>();
-  L.out_val = dval.as<double2>();
-  L.out_jac = djac.as<double>();
-  L.out_dom = ddom.as<int>();
-  L.out_scale = scale ? dscale.as<double>() : nullptr;
-  L.out_flag = dflag.as<int>();
-  L.err = ctx->d_err;
-  int grid = (int)std::min<long long>(nchunks, use_tree ? ctx->tree_grid : ctx->sm_count * 4);
-  if (use_tree) {
-    DevBuf dpts;
-    KB_CUDA(dpts.alloc((size_t)grid * PTS_SLOT * sizeof(double), st));
-    L.pts = dpts.as<double>();
+  L.in = place<double>(buf, a_in);
+  L.out_val = place<double2>(buf, a_val);
+  L.out_jac = place<double>(buf, a_jac);
+  L.out_dom = place<int>(buf, a_dom);
+  L.out_scale = scale ? place<double>(buf, a_scale) : nullptr;
+  L.out_flag = place<int>(buf, a_flag);
+  L.n_flagged = &dh->flagged;
+  L.pts = place<double>(buf, a_pts);
+  L.err = &dh->err;
+  if (use_tree)
     KB_CUDA(launch_tree(L, grid, st));
+  else
+    KB_CUDA(launch_direct(L, grid, st));
+  auto download = [&]() -> int {
+    KB_CUDA(cudaMemcpyAsync(&head, dh, sizeof(head), cudaMemcpyDeviceToHost, st));
+    KB_CUDA(cudaMemcpyAsync(out, L.out_val, count * sizeof(double2), cudaMemcpyDeviceToHost, st));
+    if (jac) KB_CUDA(cudaMemcpyAsync(jac, L.out_jac, count * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (in_domain) KB_CUDA(cudaMemcpyAsync(in_domain, L.out_dom, count * sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (scale) KB_CUDA(cudaMemcpyAsync(scale, L.out_scale, count * sizeof(double), cudaMemcpyDeviceToHost, st));
+    KB_CUDA(cudaStreamSynchronize(st));
+    return KB_OK;
+  };
+  int rc = download();
+  if (rc) return rc;
+  if (use_tree && head.flagged) {
+    // the points the tree flagged, with the pivoted LU
     std::vector<int> flags((size_t)count);
-    KB_CUDA(cudaMemcpyAsync(flags.data(), dflag.p, count * sizeof(int), cudaMemcpyDeviceToHost, st));
+    KB_CUDA(cudaMemcpyAsync(flags.data(), L.out_flag, count * sizeof(int), cudaMemcpyDeviceToHost, st));
     KB_CUDA(cudaStreamSynchronize(st));
     std::vector<int> idx;
     for (int64_t i = 0; i < count; ++i)
       if (flags[(size_t)i]) idx.push_back((int)i);
-    if (!idx.empty()) {
-      DevBuf didx;
-      KB_CUDA(didx.alloc(idx.size() * sizeof(int), st));
-      KB_CUDA(cudaMemcpyAsync(didx.p, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-      long long nc2 = ((long long)idx.size() + it.chunk_points - 1) / it.chunk_points;
-      long long offs2[2] = {0, nc2};
-      KB_CUDA(cudaMemcpyAsync(doff.p, offs2, sizeof(offs2), cudaMemcpyHostToDevice, st));
-      KB_CUDA(cudaMemsetAsync(dcnt.p, 0, sizeof(int), st));
-      Launch L2 = L;
-      L2.index = didx.as<int>();
-      L2.n_index = (int)idx.size();
-      L2.n_chunks = (int)nc2;
-      KB_CUDA(launch_direct(L2, (int)std::min<long long>(nc2, ctx->sm_count * 4), st));
-      KB_CUDA(cudaStreamSynchronize(st));
-    }
-  } else {
-    KB_CUDA(launch_direct(L, grid, st));
+    DevBuf didx;
+    KB_CUDA(didx.alloc(idx.size() * sizeof(int), st));
+    KB_CUDA(cudaMemcpyAsync(didx.p, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+    const long long nc2 = ((long long)idx.size() + it.chunk_points - 1) / it.chunk_points;
+    const long long offs2[2] = {0, nc2};
+    KB_CUDA(cudaMemcpyAsync(dh->offs, offs2, sizeof(offs2), cudaMemcpyHostToDevice, st));
+    KB_CUDA(cudaMemsetAsync(&dh->counter, 0, sizeof(int), st));
+    Launch L2 = L;
+    L2.index = didx.as<int>();
+    L2.n_index = (int)idx.size();
+    L2.n_chunks = (int)nc2;
+    KB_CUDA(launch_direct(L2, (int)std::min<long long>(nc2, ctx->sm_count * 4), st));
+    rc = download();
+    if (rc) return rc;
   }
-  int err = 0;
-  KB_CUDA(cudaMemcpyAsync(out, dval.p, count * sizeof(double2), cudaMemcpyDeviceToHost, st));
-  if (jac) KB_CUDA(cudaMemcpyAsync(jac, djac.p, count * sizeof(double), cudaMemcpyDeviceToHost, st));
-  if (in_domain) KB_CUDA(cudaMemcpyAsync(in_domain, ddom.p, count * sizeof(int), cudaMemcpyDeviceToHost, st));
-  if (scale) KB_CUDA(cudaMemcpyAsync(scale, dscale.p, count * sizeof(double), cudaMemcpyDeviceToHost, st));
-  KB_CUDA(cudaMemcpyAsync(&err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  KB_CUDA(cudaStreamSynchronize(st));
-  if (err & 1) return fail(KB_E_RANGE, "g0 evaluated outside its tabulated time window");
+  if (head.err & 1) return fail(KB_E_RANGE, "g0 evaluated outside its tabulated time window");
   return KB_OK;
 }
 
@@ -1029,9 +1060,9 @@ struct TimeBins {
 
 // One batched pass over `items`: two groups (tree / pivoted LU), each one persistent
 // launch over its items, heaviest orders first. Sums are added to acc[acc_index[i]]
-// (and to the time bins of that work item when `bins` is given).
+// (and to the time bins of that work item when `bins` is given), the kernels' error bits to err.
 int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std::vector<int> &use_tree,
-                  const std::vector<int> &acc_index, kb_accum *acc, const TimeBins *bins = nullptr) {
+                  const std::vector<int> &acc_index, kb_accum *acc, int &err, const TimeBins *bins = nullptr) {
   cudaStream_t st = ctx->stream;
   const int n_work = (int)items.size();
   for (int group = 0; group < 2; ++group) {
@@ -1049,50 +1080,47 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
     }
     const long long nchunks = offs.back();
     if (nchunks > INT32_MAX) return fail(KB_E_INVALID, "too many points in one kb_integrate call");
-    DevBuf ditems, doff, dcnt, dpart, dacc_s;
-    KB_CUDA(ditems.alloc(sorted.size() * sizeof(ItemDev), st));
-    KB_CUDA(doff.alloc(offs.size() * sizeof(long long), st));
-    KB_CUDA(dcnt.alloc(sizeof(int), st));
-    KB_CUDA(dpart.alloc((size_t)nchunks * sizeof(ChunkPartial), st));
-    KB_CUDA(dacc_s.alloc(sorted.size() * sizeof(kb_accum), st));
-    KB_CUDA(cudaMemcpyAsync(ditems.p, sorted.data(), sorted.size() * sizeof(ItemDev), cudaMemcpyHostToDevice, st));
-    KB_CUDA(cudaMemcpyAsync(doff.p, offs.data(), offs.size() * sizeof(long long), cudaMemcpyHostToDevice, st));
-    KB_CUDA(cudaMemsetAsync(dcnt.p, 0, sizeof(int), st));
-    KB_CUDA(cudaMemsetAsync(dacc_s.p, 0, sorted.size() * sizeof(kb_accum), st));
+    const int tgrid = (int)std::min<long long>(nchunks, (long long)ctx->sm_count * ctx->ctas_per_sm);
+    const size_t ni = sorted.size(), nb = bins ? (size_t)bins->nbins : 0;
+    // one block: the upload (items, chunk offsets, the scheduling counter, zeroed sums and error
+    // flag), from the sums on also the download (and the bins), then what the device keeps
+    Block B;
+    const size_t a_items = B.take(ni * sizeof(ItemDev)), a_offs = B.take(offs.size() * sizeof(long long)),
+                 a_cnt = B.take(sizeof(int)), a_acc = B.take(ni * sizeof(kb_accum)), a_err = B.take(sizeof(int)),
+                 up_end = B.size, a_os = B.take(ni * nb * sizeof(double2)),
+                 a_oc = B.take(ni * nb * sizeof(unsigned long long)), a_od = B.take(nb ? ni * sizeof(unsigned long long) : 0),
+                 down_end = B.size, a_part = B.take((size_t)nchunks * sizeof(ChunkPartial)),
+                 a_bs = B.take((size_t)nchunks * nb * sizeof(double2)),
+                 a_bc = B.take((size_t)nchunks * nb * sizeof(unsigned)),
+                 a_bd = B.take(nb ? (size_t)nchunks * sizeof(unsigned) : 0),
+                 a_pts = B.take(group == 0 ? tree_scratch(tgrid, sorted[0].order) : 0);
+    std::vector<unsigned char> host(down_end, 0);
+    memcpy(host.data() + a_items, sorted.data(), ni * sizeof(ItemDev));
+    memcpy(host.data() + a_offs, offs.data(), offs.size() * sizeof(long long));
+    DevBuf buf;
+    KB_CUDA(buf.alloc(B.size, st));
+    KB_CUDA(cudaMemcpyAsync(buf.p, host.data(), up_end, cudaMemcpyHostToDevice, st));
     Launch L;
     memset(&L, 0, sizeof(L));
-    L.items = ditems.as<ItemDev>();
-    L.n_items = (int)sorted.size();
-    L.any_cubic = items_any_cubic(sorted.data(), sorted.size());
-    L.chunk_offsets = doff.as<long long>();
+    L.items = place<ItemDev>(buf, a_items);
+    L.n_items = (int)ni;
+    L.any_cubic = items_any_cubic(sorted.data(), ni);
+    L.chunk_offsets = place<long long>(buf, a_offs);
     L.n_chunks = (int)nchunks;
-    L.chunk_counter = dcnt.as<int>();
+    L.chunk_counter = place<int>(buf, a_cnt);
     L.mode = IN_SOBOL;
-    L.partials = dpart.as<ChunkPartial>();
-    L.err = ctx->d_err;
-    DevBuf dbs, dbc, dbd, dos, doc, dod;
+    L.partials = place<ChunkPartial>(buf, a_part);
+    L.pts = place<double>(buf, a_pts);
+    L.err = place<int>(buf, a_err);
     if (bins) {
-      const size_t nb = (size_t)bins->nbins;
-      KB_CUDA(dbs.alloc((size_t)nchunks * nb * sizeof(double2), st));
-      KB_CUDA(dbc.alloc((size_t)nchunks * nb * sizeof(unsigned), st));
-      KB_CUDA(dbd.alloc((size_t)nchunks * sizeof(unsigned), st));
-      KB_CUDA(dos.alloc(sorted.size() * nb * sizeof(double2), st));
-      KB_CUDA(doc.alloc(sorted.size() * nb * sizeof(unsigned long long), st));
-      KB_CUDA(dod.alloc(sorted.size() * sizeof(unsigned long long), st));
       L.nbins = bins->nbins;
       L.bin_cols = 1;
       L.bin_xmin = bins->xmin;
       L.bin_xmax = bins->xmax;
       L.bin_size = (bins->xmax - bins->xmin) / bins->nbins;
-      L.bin_sums = dbs.as<double2>();
-      L.bin_counts = dbc.as<unsigned>();
-      L.bin_dropped = dbd.as<unsigned>();
-    }
-    DevBuf dpts;
-    const int tgrid = (int)std::min<long long>(nchunks, (long long)ctx->sm_count * ctx->ctas_per_sm);
-    if (group == 0) {
-      KB_CUDA(dpts.alloc((size_t)tgrid * PTS_SLOT * sizeof(double), st));
-      L.pts = dpts.as<double>();
+      L.bin_sums = place<double2>(buf, a_bs);
+      L.bin_counts = place<unsigned>(buf, a_bc);
+      L.bin_dropped = place<unsigned>(buf, a_bd);
     }
     if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[0], st));
     if (group == 0)
@@ -1105,27 +1133,21 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
       ctx->last_launches++;
     }
     if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[2], st));
-    KB_CUDA(launch_reduce(L, dacc_s.as<kb_accum>(), st));
+    KB_CUDA(launch_reduce(L, place<kb_accum>(buf, a_acc), st));
     if (bins) {
-      KB_CUDA(launch_reduce_bins(L, dos.as<double2>(), doc.as<unsigned long long>(), dod.as<unsigned long long>(), st));
+      KB_CUDA(launch_reduce_bins(L, place<double2>(buf, a_os), place<unsigned long long>(buf, a_oc),
+                                 place<unsigned long long>(buf, a_od), st));
       ctx->last_launches++;
     }
     if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[3], st));
     ctx->last_launches += 2;
-    std::vector<kb_accum> part(sorted.size());
-    KB_CUDA(cudaMemcpyAsync(part.data(), dacc_s.p, part.size() * sizeof(kb_accum), cudaMemcpyDeviceToHost, st));
-    std::vector<double> hbs;
-    std::vector<unsigned long long> hbc, hbd;
-    if (bins) {
-      const size_t nb = (size_t)bins->nbins;
-      hbs.resize(sorted.size() * nb * 2);
-      hbc.resize(sorted.size() * nb);
-      hbd.resize(sorted.size());
-      KB_CUDA(cudaMemcpyAsync(hbs.data(), dos.p, hbs.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-      KB_CUDA(cudaMemcpyAsync(hbc.data(), doc.p, hbc.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-      KB_CUDA(cudaMemcpyAsync(hbd.data(), dod.p, hbd.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    }
+    KB_CUDA(cudaMemcpyAsync(host.data() + a_acc, place<unsigned char>(buf, a_acc), down_end - a_acc, cudaMemcpyDeviceToHost, st));
     KB_CUDA(cudaStreamSynchronize(st));
+    const kb_accum *part = reinterpret_cast<const kb_accum *>(host.data() + a_acc);
+    const double *hbs = reinterpret_cast<const double *>(host.data() + a_os);
+    const unsigned long long *hbc = reinterpret_cast<const unsigned long long *>(host.data() + a_oc);
+    const unsigned long long *hbd = reinterpret_cast<const unsigned long long *>(host.data() + a_od);
+    err |= *reinterpret_cast<const int *>(host.data() + a_err);
     if (ctx->timing) {
       float a = 0, b = 0, c = 0;
       KB_CUDA(cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[1]));
@@ -1144,7 +1166,6 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
       a.n_in_domain += part[j].n_in_domain;
       a.n_fallback += part[j].n_fallback;
       if (bins) {
-        const size_t nb = (size_t)bins->nbins;
         for (size_t b = 0; b < nb; ++b) {
           bins->sums[2 * ((size_t)w * nb + b)] += hbs[2 * (j * nb + b)];
           bins->sums[2 * ((size_t)w * nb + b) + 1] += hbs[2 * (j * nb + b) + 1];
@@ -1262,74 +1283,65 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
   std::lock_guard<std::mutex> lk(ctx->mu);
   KB_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
-  const size_t nb = bins ? 2 * (size_t)bins->nbins : 0;
-  DevBuf ditems, doff, dcnt, dpart, dacc, dbs, dbc, dbd, dos, doc, dod;
-  KB_CUDA(ditems.alloc(items.size() * sizeof(ItemDev), st));
-  KB_CUDA(doff.alloc(offs.size() * sizeof(long long), st));
-  KB_CUDA(dcnt.alloc(sizeof(int), st));
-  KB_CUDA(dpart.alloc((size_t)nchunks * sizeof(ChunkPartial), st));
-  KB_CUDA(dacc.alloc(items.size() * sizeof(kb_accum), st));
-  if (nb) {
-    KB_CUDA(dbs.alloc((size_t)nchunks * nb * sizeof(double2), st));
-    KB_CUDA(dbc.alloc((size_t)nchunks * nb * sizeof(unsigned), st));
-    KB_CUDA(dbd.alloc((size_t)nchunks * sizeof(unsigned), st));
-    KB_CUDA(dos.alloc(items.size() * nb * sizeof(double2), st));
-    KB_CUDA(doc.alloc(items.size() * nb * sizeof(unsigned long long), st));
-    KB_CUDA(dod.alloc(items.size() * sizeof(unsigned long long), st));
-  }
-  KB_CUDA(cudaMemcpyAsync(ditems.p, items.data(), items.size() * sizeof(ItemDev), cudaMemcpyHostToDevice, st));
-  KB_CUDA(cudaMemcpyAsync(doff.p, offs.data(), offs.size() * sizeof(long long), cudaMemcpyHostToDevice, st));
-  KB_CUDA(cudaMemsetAsync(dcnt.p, 0, sizeof(int), st));
-  KB_CUDA(cudaMemsetAsync(dacc.p, 0, items.size() * sizeof(kb_accum), st));
-  KB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), st));
+  const size_t nb = bins ? 2 * (size_t)bins->nbins : 0, ni = items.size();
+  const int kgrid = (int)std::min<long long>(nchunks, (long long)ctx->sm_count * KM_CTAS_PER_SM);
+  // one block, as run_integrate's
+  Block B;
+  const size_t a_items = B.take(ni * sizeof(ItemDev)), a_offs = B.take(offs.size() * sizeof(long long)),
+               a_cnt = B.take(sizeof(int)), a_acc = B.take(ni * sizeof(kb_accum)), a_err = B.take(sizeof(int)),
+               up_end = B.size, a_os = B.take(ni * nb * sizeof(double2)),
+               a_oc = B.take(ni * nb * sizeof(unsigned long long)), a_od = B.take(nb ? ni * sizeof(unsigned long long) : 0),
+               down_end = B.size, a_part = B.take((size_t)nchunks * sizeof(ChunkPartial)),
+               a_bs = B.take((size_t)nchunks * nb * sizeof(double2)), a_bc = B.take((size_t)nchunks * nb * sizeof(unsigned)),
+               a_bd = B.take(nb ? (size_t)nchunks * sizeof(unsigned) : 0),
+               a_pts = B.take((size_t)kgrid * KM_SLOT * sizeof(double));
+  std::vector<unsigned char> host(down_end, 0);
+  memcpy(host.data() + a_items, items.data(), ni * sizeof(ItemDev));
+  memcpy(host.data() + a_offs, offs.data(), offs.size() * sizeof(long long));
+  DevBuf buf;
+  KB_CUDA(buf.alloc(B.size, st));
+  KB_CUDA(cudaMemcpyAsync(buf.p, host.data(), up_end, cudaMemcpyHostToDevice, st));
   Launch L;
   memset(&L, 0, sizeof(L));
-  L.items = ditems.as<ItemDev>();
+  L.items = place<ItemDev>(buf, a_items);
   L.n_items = n_work;
-  L.chunk_offsets = doff.as<long long>();
+  L.chunk_offsets = place<long long>(buf, a_offs);
   L.n_chunks = (int)nchunks;
-  L.chunk_counter = dcnt.as<int>();
+  L.chunk_counter = place<int>(buf, a_cnt);
   L.mode = IN_SOBOL;
-  L.partials = dpart.as<ChunkPartial>();
+  L.partials = place<ChunkPartial>(buf, a_part);
   if (bins) {
     L.nbins = bins->nbins;
     L.bin_cols = 2;
     L.bin_xmin = bins->xmin;
     L.bin_xmax = bins->xmax;
     L.bin_size = (bins->xmax - bins->xmin) / bins->nbins;
-    L.bin_sums = dbs.as<double2>();
-    L.bin_counts = dbc.as<unsigned>();
-    L.bin_dropped = dbd.as<unsigned>();
+    L.bin_sums = place<double2>(buf, a_bs);
+    L.bin_counts = place<unsigned>(buf, a_bc);
+    L.bin_dropped = place<unsigned>(buf, a_bd);
   } else {
     L.km_fourier = 1;
     L.km_omega = *omega;
   }
-  L.err = ctx->d_err;
-  const int kgrid = (int)std::min<long long>(nchunks, (long long)ctx->sm_count * KM_CTAS_PER_SM);
-  DevBuf dpts;
-  KB_CUDA(dpts.alloc((size_t)kgrid * KM_SLOT * sizeof(double), st));
-  L.pts = dpts.as<double>();
+  L.err = place<int>(buf, a_err);
+  L.pts = place<double>(buf, a_pts);
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[0], st));
   KB_CUDA(launch_km_tree(L, kgrid, st));
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[1], st));
   KB_CUDA(launch_km_fallback(L, ctx->sm_count * 4, st));
-  KB_CUDA(launch_reduce(L, dacc.as<kb_accum>(), st));
+  KB_CUDA(launch_reduce(L, place<kb_accum>(buf, a_acc), st));
   if (nb)
-    KB_CUDA(launch_reduce_bins(L, dos.as<double2>(), doc.as<unsigned long long>(), dod.as<unsigned long long>(), st));
+    KB_CUDA(launch_reduce_bins(L, place<double2>(buf, a_os), place<unsigned long long>(buf, a_oc),
+                               place<unsigned long long>(buf, a_od), st));
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[2], st));
   ctx->last_launches = nb ? 4 : 3;
-  std::vector<kb_accum> part(items.size());
-  std::vector<double> hbs(items.size() * nb * 2);
-  std::vector<unsigned long long> hbc(items.size() * nb), hbd(items.size());
-  KB_CUDA(cudaMemcpyAsync(part.data(), dacc.p, part.size() * sizeof(kb_accum), cudaMemcpyDeviceToHost, st));
-  if (nb) {
-    KB_CUDA(cudaMemcpyAsync(hbs.data(), dos.p, hbs.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    KB_CUDA(cudaMemcpyAsync(hbc.data(), doc.p, hbc.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    KB_CUDA(cudaMemcpyAsync(hbd.data(), dod.p, hbd.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  }
-  int err = 0;
-  KB_CUDA(cudaMemcpyAsync(&err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  KB_CUDA(cudaMemcpyAsync(host.data() + a_acc, place<unsigned char>(buf, a_acc), down_end - a_acc, cudaMemcpyDeviceToHost, st));
   KB_CUDA(cudaStreamSynchronize(st));
+  const kb_accum *part = reinterpret_cast<const kb_accum *>(host.data() + a_acc);
+  const double *hbs = reinterpret_cast<const double *>(host.data() + a_os);
+  const unsigned long long *hbc = reinterpret_cast<const unsigned long long *>(host.data() + a_oc);
+  const unsigned long long *hbd = reinterpret_cast<const unsigned long long *>(host.data() + a_od);
+  const int err = *reinterpret_cast<const int *>(host.data() + a_err);
   if (ctx->timing) {
     float a = 0, c = 0;
     KB_CUDA(cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[1]));
@@ -1457,13 +1469,14 @@ int integrate_impl(kb_context *ctx, const kb_work *work, int n_work, int algo, k
   cudaStream_t st = ctx->stream;
   ctx->last_ms[0] = ctx->last_ms[1] = ctx->last_ms[2] = 0.0;
   ctx->last_launches = 0;
-  KB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), st));
+  int err = 0;
+  if (any_flow) KB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), st)); // the flow kernels' error bits
   {
     int rc = spline_knots_for(work, n_work, st, &ctx->last_launches);
     if (rc) return rc;
   }
   if (!any_flow) {
-    int rc = run_integrate(ctx, items, use_tree, index, acc, tb);
+    int rc = run_integrate(ctx, items, use_tree, index, acc, err, tb);
     if (rc) return rc;
   } else {
     // Items with a flow run in pieces whose flow-mapped points (li, Jacobian) are made by
@@ -1519,14 +1532,17 @@ int integrate_impl(kb_context *ctx, const kb_work *work, int n_work, int algo, k
         rtree.push_back(p.tree);
         racc.push_back(p.acc);
       }
-      int rc = run_integrate(ctx, ritems, rtree, racc, acc, tb);
+      int rc = run_integrate(ctx, ritems, rtree, racc, acc, err, tb);
       if (rc) return rc;
       first_round = false;
     }
   }
-  int err = 0;
-  KB_CUDA(cudaMemcpyAsync(&err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  KB_CUDA(cudaStreamSynchronize(st));
+  if (any_flow) {
+    int flow_err = 0;
+    KB_CUDA(cudaMemcpyAsync(&flow_err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    KB_CUDA(cudaStreamSynchronize(st));
+    err |= flow_err;
+  }
   if (err & 1) return fail(KB_E_RANGE, "g0 evaluated outside its tabulated time window");
   if (err & 2) return fail(KB_E_CUDA, "a flow kernel's wait on the tensor cores ran out");
   return KB_OK;
@@ -1548,8 +1564,13 @@ struct kb_plan {
     int *d_cnt = nullptr;
     ChunkPartial *d_part = nullptr;
     double *d_pts = nullptr;
-    kb_accum *d_acc = nullptr;
+    kb_accum *d_acc = nullptr; // in d_result
   } g[2];
+  // cleared by one memset and read back by one copy: both groups' sums, their chunk counters, the
+  // kernels' error bits
+  unsigned char *d_result = nullptr;
+  size_t result_bytes = 0;
+  int *d_err = nullptr;
   int n_work = 0;
   std::vector<int> where_group, where_pos; // work index -> (group, sorted position)
   std::vector<const kb_sobol *> rng;
@@ -1574,11 +1595,10 @@ static void plan_free(kb_plan *p) {
   for (auto &g : p->g) {
     cudaFree(g.d_items);
     cudaFree(g.d_offs);
-    cudaFree(g.d_cnt);
     cudaFree(g.d_part);
     cudaFree(g.d_pts);
-    cudaFree(g.d_acc);
   }
+  cudaFree(p->d_result);
   for (auto &f : p->fills) cudaFree(f.buf);
   delete p;
 }
@@ -1655,10 +1675,9 @@ int kb_plan_create(kb_context *ctx, const kb_work *work, int n_work, int algo, k
                                                           : (long long)ctx->sm_count * 4);
     cudaError_t e = device_malloc(&g.d_items, sizeof(ItemDev) * g.n_items);
     if (e == cudaSuccess) e = device_malloc(&g.d_offs, sizeof(long long) * offs.size());
-    if (e == cudaSuccess) e = device_malloc(&g.d_cnt, sizeof(int));
     if (e == cudaSuccess) e = device_malloc(&g.d_part, sizeof(ChunkPartial) * (size_t)g.n_chunks);
-    if (e == cudaSuccess && gi == 0) e = device_malloc(&g.d_pts, sizeof(double) * PTS_SLOT * (size_t)g.grid);
-    if (e == cudaSuccess) e = device_malloc(&g.d_acc, sizeof(kb_accum) * g.n_items);
+    const size_t scratch = gi == 0 ? tree_scratch(g.grid, g.items[0].order) : 0;
+    if (e == cudaSuccess && scratch) e = device_malloc(&g.d_pts, scratch);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(g.d_items, g.items.data(), sizeof(ItemDev) * g.n_items, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess)
@@ -1669,6 +1688,23 @@ int kb_plan_create(kb_context *ctx, const kb_work *work, int n_work, int algo, k
       return fail(KB_E_NOMEM, std::string("kb_plan_create: ") + cudaGetErrorString(e));
     }
   }
+  {
+    Block B;
+    const size_t a_acc[2] = {B.take(sizeof(kb_accum) * (size_t)p->g[0].n_items), B.take(sizeof(kb_accum) * (size_t)p->g[1].n_items)};
+    const size_t a_err = B.take(3 * sizeof(int));
+    p->result_bytes = a_err + 3 * sizeof(int);
+    cudaError_t e = device_malloc(&p->d_result, p->result_bytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p->d_result, 0, p->result_bytes, ctx->stream);
+    if (e != cudaSuccess) {
+      plan_free(p);
+      return fail(KB_E_NOMEM, std::string("kb_plan_create: ") + cudaGetErrorString(e));
+    }
+    p->d_err = reinterpret_cast<int *>(p->d_result + a_err);
+    for (int gi = 0; gi < 2; ++gi) {
+      p->g[gi].d_acc = reinterpret_cast<kb_accum *>(p->d_result + a_acc[gi]);
+      p->g[gi].d_cnt = p->d_err + 1 + gi;
+    }
+  }
   for (auto &f : p->fills) f.pos = p->where_pos[(size_t)f.pos];
   *out = p;
   return KB_OK;
@@ -1676,17 +1712,16 @@ int kb_plan_create(kb_context *ctx, const kb_work *work, int n_work, int algo, k
 
 // The launch sequence of one run (captured into the plan's graph).
 static int plan_enqueue(kb_context *ctx, kb_plan *p, cudaStream_t st) {
+  KB_CUDA(cudaMemsetAsync(p->d_result, 0, p->result_bytes, st));
   for (const kb_flow *f : p->splines) KB_CUDA(launch_spline_knots(f->master, f->dim, f->knots, st));
   for (const auto &f : p->fills) {
     const uint32_t *kf = &p->g[f.gi].d_items[f.pos].k_first;
-    KB_CUDA(launch_flow_map(f.layout, 1, f.n, nullptr, f.rng, 0, kf, 1, f.buf, f.buf + (size_t)f.n * f.order, ctx->d_err,
+    KB_CUDA(launch_flow_map(f.layout, 1, f.n, nullptr, f.rng, 0, kf, 1, f.buf, f.buf + (size_t)f.n * f.order, p->d_err,
                             ctx->sm_count, st));
   }
   for (int gi = 0; gi < 2; ++gi) {
     auto &g = p->g[gi];
     if (!g.n_items) continue;
-    KB_CUDA(cudaMemsetAsync(g.d_acc, 0, sizeof(kb_accum) * g.n_items, st));
-    KB_CUDA(cudaMemsetAsync(g.d_cnt, 0, sizeof(int), st));
     Launch L;
     memset(&L, 0, sizeof(L));
     L.items = g.d_items;
@@ -1698,7 +1733,7 @@ static int plan_enqueue(kb_context *ctx, kb_plan *p, cudaStream_t st) {
     L.mode = IN_SOBOL;
     L.partials = g.d_part;
     L.pts = g.d_pts;
-    L.err = ctx->d_err;
+    L.err = p->d_err;
     if (gi == 0) {
       KB_CUDA(launch_tree(L, g.grid, st));
       KB_CUDA(launch_fallback(L, ctx->sm_count * 4, st));
@@ -1729,7 +1764,6 @@ int kb_plan_launch(kb_context *ctx, kb_plan *plan) {
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return fail(KB_E_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
   }
-  KB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), st));
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[0], st));
   KB_CUDA(cudaGraphLaunch(plan->exec, st));
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[1], st));
@@ -1741,15 +1775,8 @@ int kb_plan_result(kb_context *ctx, kb_plan *plan, kb_accum *acc) {
   std::lock_guard<std::mutex> lk(ctx->mu);
   KB_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
-  std::vector<kb_accum> part[2];
-  for (int gi = 0; gi < 2; ++gi) {
-    part[gi].resize((size_t)plan->g[gi].n_items);
-    if (plan->g[gi].n_items)
-      KB_CUDA(cudaMemcpyAsync(part[gi].data(), plan->g[gi].d_acc, sizeof(kb_accum) * plan->g[gi].n_items,
-                              cudaMemcpyDeviceToHost, st));
-  }
-  int err = 0;
-  KB_CUDA(cudaMemcpyAsync(&err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  std::vector<unsigned char> host(plan->result_bytes);
+  KB_CUDA(cudaMemcpyAsync(host.data(), plan->d_result, host.size(), cudaMemcpyDeviceToHost, st));
   KB_CUDA(cudaStreamSynchronize(st));
   if (ctx->timing) {
     float ms = 0;
@@ -1758,12 +1785,14 @@ int kb_plan_result(kb_context *ctx, kb_plan *plan, kb_accum *acc) {
       ctx->last_ms[1] = ctx->last_ms[2] = 0.0;
     }
   }
+  const int err = *reinterpret_cast<const int *>(host.data() + ((unsigned char *)plan->d_err - plan->d_result));
   if (err & 1) return fail(KB_E_RANGE, "g0 evaluated outside its tabulated time window");
   if (err & 2) return fail(KB_E_CUDA, "a flow kernel's wait on the tensor cores ran out");
   for (int gi = 0; gi < 2; ++gi)
     for (int j = 0; j < plan->g[gi].n_items; ++j) {
       kb_accum &a = acc[plan->g[gi].ids[(size_t)j]];
-      const kb_accum &q = part[gi][(size_t)j];
+      const kb_accum &q =
+          reinterpret_cast<const kb_accum *>(host.data() + ((unsigned char *)plan->g[gi].d_acc - plan->d_result))[j];
       a.sum_re += q.sum_re;
       a.sum_im += q.sum_im;
       a.n_points += q.n_points;

@@ -629,6 +629,8 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
           if (SCALE) L.out_scale[o] = dom ? T.fscale[lane] * fabs(jac) : 0.0;
           if (L.out_flag) L.out_flag[o] = fb ? 1 : 0;
         }
+        const unsigned nf = __popc(__ballot_sync(FULL, fb));
+        if (nf && lane == 0) atomicAdd(L.n_flagged, (int)nf);
         __syncwarp();
         continue;
       }
