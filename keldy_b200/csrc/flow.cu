@@ -201,15 +201,22 @@ __device__ __forceinline__ unsigned char *row_ptr(unsigned char *buf, int t) {
 }
 
 // Hat features of the conditioning dims of x into row t of buffer `buf`; feature
-// 16*T_l[0] is the constant 1.
-__device__ void encode_row(const FlowDev &f, int l, const float (&x)[FLOW_MAX_DIM], unsigned char *buf, int t) {
+// 16*T_l[0] is the constant 1. With PARTS threads per row, thread `part` does its part of the
+// columns (as in epi_relu).
+template <int PARTS>
+__device__ void encode_row(const FlowDev &f, int l, const float (&x)[FLOW_MAX_DIM], unsigned char *buf, int t,
+                           int part) {
   unsigned char *row = row_ptr(buf, t);
   const unsigned tm = f.tmask[l];
   const int t0 = f.tdim[l][0];
 #pragma unroll
-  for (int i = 0; i < FLOW_MAX_DIM; ++i) {
+  for (int k = 0; k < FLOW_MAX_DIM / PARTS; ++k) {
+    const int i = part * (FLOW_MAX_DIM / PARTS) + k;
+    float xi = x[k];
+#pragma unroll
+    for (int q = 1; q < PARTS; ++q) xi = part == q ? x[q * (FLOW_MAX_DIM / PARTS) + k] : xi;
     const bool cond = i < f.dim && !((tm >> i) & 1u);
-    float u = x[i] * (float)FLOW_BLOB - 0.5f;
+    float u = xi * (float)FLOW_BLOB - 0.5f;
     const float fl = floorf(u);
     const int j0 = cond ? (int)fl : -100;
     const float fr = u - fl;
@@ -230,10 +237,12 @@ __device__ void encode_row(const FlowDev &f, int l, const float (&x)[FLOW_MAX_DI
 }
 
 // Accumulator row -> ReLU -> bf16 row t of `buf`, hidden unit 127 set to 1.
-__device__ void epi_relu(uint32_t trow, unsigned char *buf, int t) {
+template <int PARTS>
+__device__ void epi_relu(uint32_t trow, unsigned char *buf, int t, int part) {
   unsigned char *row = row_ptr(buf, t);
 #pragma unroll
-  for (int c4 = 0; c4 < 4; ++c4) {
+  for (int c = 0; c < 4 / PARTS; ++c) {
+    const int c4 = part * (4 / PARTS) + c;
     float v[32];
     tmem_ld32(trow + 32 * c4, v);
 #pragma unroll
@@ -254,18 +263,19 @@ __device__ void epi_relu(uint32_t trow, unsigned char *buf, int t) {
 // The three conditioner products of layer l on the features already in act[0]:
 // h1 -> act[1], h2 -> act[h2buf], logits left in the accumulator. Weight slots are
 // refilled with matrix j of layer `next` (-1: none) after product j.
+template <int PARTS>
 __device__ bool conditioner(Pipe &P, unsigned char *act, int h2buf, int next, uint32_t trow) {
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, row = t & (NT - 1), part = t / NT;
   Mma none = {};
   Mma m = {P.tmem, act_addr(P, 0), w_addr(P, 0), 0, 0, 0};
   if (!mma_step(P, 0, m, none, 1)) return false;
   if (t == 0 && next >= 0) load_weight(P, 0, 3 * next + 0);
-  epi_relu(trow, act + MAT_BYTES, t);
+  epi_relu<PARTS>(trow, act + MAT_BYTES, row, part);
   m.a = act_addr(P, 1);
   m.b = w_addr(P, 1);
   if (!mma_step(P, 1, m, none, 1)) return false;
   if (t == 0 && next >= 0) load_weight(P, 1, 3 * next + 1);
-  epi_relu(trow, act + (size_t)h2buf * MAT_BYTES, t);
+  epi_relu<PARTS>(trow, act + (size_t)h2buf * MAT_BYTES, row, part);
   m.a = act_addr(P, h2buf);
   m.b = w_addr(P, 2);
   if (!mma_step(P, 2, m, none, 1)) return false;
@@ -393,7 +403,7 @@ __global__ void __launch_bounds__(NT, 2)
       float xf[FLOW_MAX_DIM];
 #pragma unroll
       for (int d = 0; d < FLOW_MAX_DIM; ++d) xf[d] = (float)x[d];
-      encode_row(f, l, xf, act, t);
+      encode_row<1>(f, l, xf, act, t, 0);
       // the layer's three products: features -> h1 -> h2 -> logits, all in one buffer
       for (int j = 0; j < 3 && ok; ++j, ++q) {
         const int slot = (int)(q & 1);
@@ -401,7 +411,7 @@ __global__ void __launch_bounds__(NT, 2)
         ok = mma_step(P, slot, m, none, 1);
         if (!ok) break;
         if (t == 0 && q + 2 < nq) load_weight(P, slot, mat_of(q + 2));
-        if (j < 2) epi_relu(trow, act, t);
+        if (j < 2) epi_relu<1>(trow, act, t, 0);
       }
       if (!ok) break;
 #pragma unroll
@@ -467,7 +477,15 @@ __global__ void __launch_bounds__(NT, 2)
 
 // ------------------------------------------------------------ training step
 // TMEM columns: [0,128) working accumulator, [128,256) dW1, [256,384) dW2, [384,512) dW3.
-__global__ void __launch_bounds__(NT, 1)
+// Bound: a CTA's chain of 71 products per tile, each waited for, with an epilogue between two: a
+// batch of 8,192 points is 64 tiles, so the chain's length is the step's time. Four threads per
+// point (warps w, w + 4, w + 8, w + 12 on TMEM lane quadrant w) take one slot, or a quarter of an
+// epilogue's columns, each: with one thread per point a step of 8,192 points took 248 us, with two
+// 152 us, with four 150 us. The coordinates and their gradients that the other threads made
+// are exchanged in shared memory once per layer.
+constexpr int TRAIN_PARTS = 4;
+constexpr int TRAIN_NT = TRAIN_PARTS * NT;
+__global__ void __launch_bounds__(TRAIN_NT, 1)
     flow_train_kernel(FlowDev f, long long count, const float *xin, const float *win, const int *index,
                       float inv_batch, float *partials, float *loss_part, float *xs, int *err) {
   extern __shared__ unsigned char smem_raw[];
@@ -476,11 +494,12 @@ __global__ void __launch_bounds__(NT, 1)
   SmemHead *head;
   Pipe P;
   pipe_init(P, base, 3, head, f.img, 512);
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const uint32_t trow = P.tmem + ((uint32_t)(warp * 32) << 16);
+  __shared__ float s_x[FLOW_MAX_DIM][NT], s_l[FLOW_SLOTS][NT];
+  const int tid = threadIdx.x, t = tid & (NT - 1), part = tid / NT, warp = tid >> 5, lane = tid & 31;
+  const uint32_t trow = P.tmem + ((uint32_t)((warp & 3) * 32) << 16);
   const long long ntiles = (count + NT - 1) / NT;
   const int N = f.dim;
-  if (t == 0 && blockIdx.x < ntiles)
+  if (tid == 0 && blockIdx.x < ntiles)
     for (int j = 0; j < 3; ++j) load_weight(P, j, j);
   bool ok = true;
   bool first = true;
@@ -496,14 +515,15 @@ __global__ void __launch_bounds__(NT, 1)
     float lq = 0.0f;
     // forward, saving each layer's input
     for (int l = 0; l < FLOW_LAYERS && ok; ++l) {
-      if (valid)
+      if (valid && part == 0)
 #pragma unroll
         for (int d = 0; d < FLOW_MAX_DIM; ++d) xs[((size_t)l * FLOW_MAX_DIM + d) * count + p] = x[d];
-      encode_row(f, l, x, act, t);
-      ok = conditioner(P, act, 2, l + 1 < FLOW_LAYERS ? l + 1 : -1, trow);
+      encode_row<TRAIN_PARTS>(f, l, x, act, t, part);
+      ok = conditioner<TRAIN_PARTS>(P, act, 2, l + 1 < FLOW_LAYERS ? l + 1 : -1, trow);
       if (!ok) break;
 #pragma unroll
-      for (int s = 0; s < FLOW_SLOTS; ++s) {
+      for (int s2 = 0; s2 < FLOW_SLOTS / TRAIN_PARTS; ++s2) {
+        const int s = part * (FLOW_SLOTS / TRAIN_PARTS) + s2;
         if (s >= f.ntr[l]) break;
         const int d = f.tdim[l][s];
         float v[32];
@@ -527,18 +547,25 @@ __global__ void __launch_bounds__(NT, 1)
           if (j < b) cb += pj;
           if (j == b) pb = pj;
         }
-        set_dim(x, d, cb + (u - (float)b) * pb);
-        lq += logf(FLOW_BINS * pb);
+        s_x[d][t] = cb + (u - (float)b) * pb;
+        s_l[s][t] = logf(FLOW_BINS * pb);
       }
+      __syncthreads();
+      if (part == 0) // a point's log terms in slot order
+        for (int s = 0; s < f.ntr[l]; ++s) lq += s_l[s][t];
+      const unsigned tm = f.tmask[l];
+#pragma unroll
+      for (int d = 0; d < FLOW_MAX_DIM; ++d)
+        if ((tm >> d) & 1u) x[d] = s_x[d][t];
     }
     if (!ok) break;
-    // loss of the tile
+    // loss of the tile (the first thread of each point holds its sum)
     float lv = valid ? -w * lq * inv_batch : 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lv += __shfl_xor_sync(0xffffffffu, lv, o);
-    if (lane == 0) head->red[warp] = lv;
+    if (part == 0 && lane == 0) head->red[warp] = lv;
     __syncthreads();
-    if (t == 0) {
+    if (tid == 0) {
       const float tot = head->red[0] + head->red[1] + head->red[2] + head->red[3];
       loss_part[blockIdx.x] = first ? tot : loss_part[blockIdx.x] + tot;
     }
@@ -550,13 +577,14 @@ __global__ void __launch_bounds__(NT, 1)
       if (valid)
 #pragma unroll
         for (int d = 0; d < FLOW_MAX_DIM; ++d) x[d] = xs[((size_t)l * FLOW_MAX_DIM + d) * count + p];
-      encode_row(f, l, x, act, t);
-      ok = conditioner(P, act, 2, -1, trow);
+      encode_row<TRAIN_PARTS>(f, l, x, act, t, part);
+      ok = conditioner<TRAIN_PARTS>(P, act, 2, -1, trow);
       if (!ok) break;
       // logit gradients -> act[0] (the features are no longer needed)
       unsigned char *row0 = row_ptr(act, t);
 #pragma unroll
-      for (int s = 0; s < FLOW_SLOTS; ++s) {
+      for (int s2 = 0; s2 < FLOW_SLOTS / TRAIN_PARTS; ++s2) {
+        const int s = part * (FLOW_SLOTS / TRAIN_PARTS) + s2;
         float g[32];
         if (s < f.ntr[l]) {
           const int d = f.tdim[l][s];
@@ -591,7 +619,7 @@ __global__ void __launch_bounds__(NT, 1)
           }
 #pragma unroll
           for (int j = 0; j < 32; ++j) g[j] = v[j] * (g[j] - dot);
-          set_dim(gx, d, gz * FLOW_BINS * pb);
+          s_x[d][t] = gz * FLOW_BINS * pb;
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) g[j] = 0.0f;
@@ -606,7 +634,7 @@ __global__ void __launch_bounds__(NT, 1)
       Mma mw = {P.tmem + 384, act_addr(P, 0), act_addr(P, 2), 1, 1, 0};
       Mma mx_ = {P.tmem, act_addr(P, 0), w_addr(P, 2), 0, 1, 0};
       if (!(ok = mma_step(P, 2, mw, mx_, 2))) break;
-      if (t == 0 && l > 0) load_weight(P, 2, 3 * (l - 1) + 2);
+      if (tid == 0 && l > 0) load_weight(P, 2, 3 * (l - 1) + 2);
       // g2 = dh2 * [h2 > 0] (unit 127: 0) -> act[2]
       unsigned char *row2 = row_ptr(act + 2 * MAT_BYTES, t);
       unsigned char *row1 = row_ptr(act + MAT_BYTES, t);
@@ -614,7 +642,8 @@ __global__ void __launch_bounds__(NT, 1)
       for (int pass = 0; pass < 2; ++pass) {
         unsigned char *rowh = pass == 0 ? row2 : row1;
 #pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4) {
+        for (int c = 0; c < 4 / TRAIN_PARTS; ++c) {
+          const int c4 = part * (4 / TRAIN_PARTS) + c;
           float v[32];
           tmem_ld32(trow + 32 * c4, v);
 #pragma unroll
@@ -637,28 +666,29 @@ __global__ void __launch_bounds__(NT, 1)
           Mma a = {P.tmem + 256, act_addr(P, 2), act_addr(P, 1), 1, 1, 0};
           Mma b = {P.tmem, act_addr(P, 2), w_addr(P, 1), 0, 1, 0};
           if (!(ok = mma_step(P, 1, a, b, 2))) break;
-          if (t == 0 && l > 0) load_weight(P, 1, 3 * (l - 1) + 1);
+          if (tid == 0 && l > 0) load_weight(P, 1, 3 * (l - 1) + 1);
         }
       }
       if (!ok) break;
       // the features again -> act[0]; dW1 = g1^T e ; de = g1 W1
-      encode_row(f, l, x, act, t);
+      encode_row<TRAIN_PARTS>(f, l, x, act, t, part);
       Mma a = {P.tmem + 128, act_addr(P, 1), act_addr(P, 0), 1, 1, 0};
       Mma b = {P.tmem, act_addr(P, 1), w_addr(P, 0), 0, 1, 0};
       if (!(ok = mma_step(P, 0, a, b, l > 0 ? 2 : 1))) break;
-      if (t == 0 && l > 0) load_weight(P, 0, 3 * (l - 1) + 0);
+      if (tid == 0 && l > 0) load_weight(P, 0, 3 * (l - 1) + 0);
       if (l > 0) {
         // gradient of the conditioning dims through the hat features
         const unsigned tm = f.tmask[l];
 #pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4) {
+        for (int c = 0; c < 4 / TRAIN_PARTS; ++c) {
           float v[32];
-          tmem_ld32(trow + 32 * c4, v);
+          tmem_ld32(trow + 32 * (part * (4 / TRAIN_PARTS) + c), v);
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
-            const int i = 2 * c4 + h;
+            const int i = part * (FLOW_MAX_DIM / TRAIN_PARTS) + 2 * c + h;
             if (i < N && !((tm >> i) & 1u)) {
-              const float u = x[i] * (float)FLOW_BLOB - 0.5f;
+              const float xi = get_dim(x, i), gi = get_dim(gx, i);
+              const float u = xi * (float)FLOW_BLOB - 0.5f;
               const int j0 = (int)floorf(u);
               float gsum = 0.0f;
 #pragma unroll
@@ -666,17 +696,21 @@ __global__ void __launch_bounds__(NT, 1)
                 if (j == j0) gsum -= v[16 * h + j];
                 if (j == j0 + 1) gsum += v[16 * h + j];
               }
-              gx[i] += (float)FLOW_BLOB * gsum;
+              s_x[i][t] = gi + (float)FLOW_BLOB * gsum;
             }
           }
         }
+        __syncthreads();
+#pragma unroll
+        for (int d = 0; d < FLOW_MAX_DIM; ++d)
+          if (d < N) gx[d] = s_x[d][t];
       }
       // this tile's weight gradients of layer l -> the CTA's partial sums
 #pragma unroll 1
       for (int mtx = 0; mtx < 3; ++mtx) {
         float *dst = partials + (size_t)blockIdx.x * FLOW_NPARAM + (size_t)(3 * l + mtx) * FLOW_MAT;
 #pragma unroll 1
-        for (int c4 = 0; c4 < 4; ++c4) {
+        for (int c4 = part * (4 / TRAIN_PARTS); c4 < (part + 1) * (4 / TRAIN_PARTS); ++c4) {
           float v[32];
           tmem_ld32(trow + 128 * (1 + mtx) + 32 * c4, v);
 #pragma unroll
@@ -688,7 +722,7 @@ __global__ void __launch_bounds__(NT, 1)
       }
     }
   }
-  if (!ok && t == 0) atomicOr(err, FLOW_ERR_TIMEOUT);
+  if (!ok && tid == 0) atomicOr(err, FLOW_ERR_TIMEOUT);
   pipe_finish(P, 512, err);
 }
 
@@ -801,7 +835,7 @@ cudaError_t launch_flow_train(const FlowDev &f, long long count, const float *x,
   if (count <= 0) return cudaSuccess;
   const long long tiles = (count + NT - 1) / NT;
   if (grid > tiles) grid = (int)tiles;
-  flow_train_kernel<<<grid, NT, flow_train_smem_bytes(), st>>>(f, count, x, w, index, inv_batch, partials, loss_part,
+  flow_train_kernel<<<grid, TRAIN_NT, flow_train_smem_bytes(), st>>>(f, count, x, w, index, inv_batch, partials, loss_part,
                                                                xs, err);
   return cudaGetLastError();
 }
