@@ -41,9 +41,9 @@ int flow_error(kb_context *ctx) {
 
 // Loss partials and weight-gradient partials of `count` points (device x, w, index).
 int train_pass(kb_flow *f, long long count, const float *dx, const float *dw, const int *dindex, float *partials,
-               float *loss_part, float *xs, int grid) {
+               float *loss_part, float *xs, uint16_t *hidden, int grid) {
   kb_context *ctx = f->ctx;
-  KB_CUDA(launch_flow_train(f->layout, count, dx, dw, dindex, 1.0f / (float)count, partials, loss_part, xs, ctx->d_err,
+  KB_CUDA(launch_flow_train(f->layout, count, dx, dw, dindex, 1.0f / (float)count, partials, loss_part, xs, hidden, ctx->d_err,
                             grid, ctx->stream));
   return KB_OK;
 }
@@ -396,20 +396,21 @@ int kb_flow_gradient(kb_flow *f, int64_t count, const double *x, const double *w
     return KB_OK;
   }
   const int grid = train_grid(f, count);
-  DevBuf dx, dw, di, dpart, dloss, dxs, dgrad;
+  DevBuf dx, dw, di, dpart, dloss, dxs, dhid, dgrad;
   KB_CUDA(dx.alloc(hx.size() * sizeof(float), st));
   KB_CUDA(dw.alloc(hw.size() * sizeof(float), st));
   KB_CUDA(di.alloc(idx.size() * sizeof(int), st));
   KB_CUDA(dpart.alloc((size_t)grid * FLOW_NPARAM * sizeof(float), st));
   KB_CUDA(dloss.alloc((size_t)grid * sizeof(float), st));
   KB_CUDA(dxs.alloc((size_t)count * FLOW_LAYERS * FLOW_MAX_DIM * sizeof(float), st));
+  KB_CUDA(dhid.alloc((size_t)grid * FLOW_HIDDEN * sizeof(uint16_t), st));
   KB_CUDA(dgrad.alloc((size_t)FLOW_NPARAM * sizeof(float), st));
   KB_CUDA(cudaMemcpyAsync(dx.p, hx.data(), hx.size() * sizeof(float), cudaMemcpyHostToDevice, st));
   KB_CUDA(cudaMemcpyAsync(dw.p, hw.data(), hw.size() * sizeof(float), cudaMemcpyHostToDevice, st));
   KB_CUDA(cudaMemcpyAsync(di.p, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice, st));
   KB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), st));
   int rc = train_pass(f, count, dx.as<float>(), dw.as<float>(), di.as<int>(), dpart.as<float>(), dloss.as<float>(),
-                      dxs.as<float>(), grid);
+                      dxs.as<float>(), dhid.as<uint16_t>(), grid);
   if (rc) return rc;
   KB_CUDA(launch_flow_reduce(dpart.as<float>(), grid, dgrad.as<float>(), st));
   std::vector<float> inr((size_t)FLOW_NPARAM), lp((size_t)grid);
@@ -459,13 +460,14 @@ int kb_flow_train(kb_flow *f, int64_t count, const double *x, const double *w, c
   if (param_flow(f)) return spline_train(f, count, hx, hw, cfg, batch, per_epoch, steps, loss_hist,
                                                                n_steps);
   const int grid = train_grid(f, batch);
-  DevBuf dx, dw, di, dpart, dlp, dxs, dhist;
+  DevBuf dx, dw, di, dpart, dlp, dxs, dhid, dhist;
   KB_CUDA(dx.alloc(hx.size() * sizeof(float), st));
   KB_CUDA(dw.alloc(hw.size() * sizeof(float), st));
   KB_CUDA(di.alloc((size_t)count * sizeof(int), st));
   KB_CUDA(dpart.alloc((size_t)grid * FLOW_NPARAM * sizeof(float), st));
   KB_CUDA(dlp.alloc((size_t)grid * sizeof(float), st));
   KB_CUDA(dxs.alloc((size_t)batch * FLOW_LAYERS * FLOW_MAX_DIM * sizeof(float), st));
+  KB_CUDA(dhid.alloc((size_t)grid * FLOW_HIDDEN * sizeof(uint16_t), st));
   KB_CUDA(dhist.alloc((size_t)steps * sizeof(float), st));
   KB_CUDA(cudaMemcpyAsync(dx.p, hx.data(), hx.size() * sizeof(float), cudaMemcpyHostToDevice, st));
   KB_CUDA(cudaMemcpyAsync(dw.p, hw.data(), hw.size() * sizeof(float), cudaMemcpyHostToDevice, st));
@@ -482,7 +484,7 @@ int kb_flow_train(kb_flow *f, int64_t count, const double *x, const double *w, c
     KB_CUDA(cudaMemcpyAsync(di.p, perm.data(), perm.size() * sizeof(int), cudaMemcpyHostToDevice, st));
     for (int64_t b = 0; b < per_epoch; ++b, ++s) {
       int rc = train_pass(f, batch, dx.as<float>(), dw.as<float>(), di.as<int>() + b * batch, dpart.as<float>(),
-                          dlp.as<float>(), dxs.as<float>(), grid);
+                          dlp.as<float>(), dxs.as<float>(), dhid.as<uint16_t>(), grid);
       if (rc) return rc;
       const int64_t t = ++f->adam_step;
       const double lr = cfg->lr_final + 0.5 * (cfg->lr - cfg->lr_final) * (1.0 + std::cos(pi * (double)s / (double)steps));

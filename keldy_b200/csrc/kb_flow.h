@@ -74,10 +74,12 @@ cudaError_t launch_flow_map(const FlowDev &f, int direction, long long count, co
                             int *err, int grid, cudaStream_t st);
 // Loss and gradient partials of one batch: point p of the batch is index[p] of x/w
 // (x: [*][dim] float, w: weights). partials [grid][FLOW_NPARAM] in the internal order
-// [matrix][in][out]; loss_part[grid] = sum w (-log q) * inv_batch; xs: 48 floats per point.
+// [matrix][in][out]; loss_part[grid] = sum w (-log q) * inv_batch; xs: 48 floats per point;
+// hidden: FLOW_HIDDEN bf16 values per CTA of the grid.
+constexpr int FLOW_HIDDEN = 2 * FLOW_LAYERS * FLOW_MAT;
 cudaError_t launch_flow_train(const FlowDev &f, long long count, const float *x, const float *w, const int *index,
-                              float inv_batch, float *partials, float *loss_part, float *xs, int *err, int grid,
-                              cudaStream_t st);
+                              float inv_batch, float *partials, float *loss_part, float *xs, uint16_t *hidden, int *err,
+                              int grid, cudaStream_t st);
 // Sum of the partials (grid rows) into grad [FLOW_NPARAM] (internal order).
 cudaError_t launch_flow_reduce(const float *partials, int nparts, float *grad, cudaStream_t st);
 // Adam step on the fp32 master weights (internal order) from the summed partials; writes
