@@ -1128,21 +1128,34 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
     else
       KB_CUDA(launch_direct(L, (int)std::min<long long>(nchunks, ctx->sm_count * 4), st));
     if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[1], st));
-    if (group == 0) {
+    // sums, bins and the error flag to the host
+    auto finish = [&]() -> int {
+      if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[2], st));
+      KB_CUDA(launch_reduce(L, place<kb_accum>(buf, a_acc), st));
+      if (bins)
+        KB_CUDA(launch_reduce_bins(L, place<double2>(buf, a_os), place<unsigned long long>(buf, a_oc),
+                                   place<unsigned long long>(buf, a_od), st));
+      ctx->last_launches += bins ? 2 : 1;
+      if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[3], st));
+      KB_CUDA(cudaMemcpyAsync(host.data() + a_acc, place<unsigned char>(buf, a_acc), down_end - a_acc,
+                              cudaMemcpyDeviceToHost, st));
+      KB_CUDA(cudaStreamSynchronize(st));
+      return KB_OK;
+    };
+    ctx->last_launches++;
+    int rc = finish();
+    if (rc) return rc;
+    // guarded points are rare: their pass is launched when the sums say that there are some (the
+    // launch is a seventh of a small call), and the sums are formed again with them
+    bool guarded = false;
+    for (size_t j = 0; j < ni; ++j) guarded = guarded || reinterpret_cast<const kb_accum *>(host.data() + a_acc)[j].n_fallback;
+    if (group == 0 && guarded) {
+      KB_CUDA(cudaMemsetAsync(place<kb_accum>(buf, a_acc), 0, ni * sizeof(kb_accum), st));
       KB_CUDA(launch_fallback(L, ctx->sm_count * 4, st));
       ctx->last_launches++;
+      rc = finish();
+      if (rc) return rc;
     }
-    if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[2], st));
-    KB_CUDA(launch_reduce(L, place<kb_accum>(buf, a_acc), st));
-    if (bins) {
-      KB_CUDA(launch_reduce_bins(L, place<double2>(buf, a_os), place<unsigned long long>(buf, a_oc),
-                                 place<unsigned long long>(buf, a_od), st));
-      ctx->last_launches++;
-    }
-    if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[3], st));
-    ctx->last_launches += 2;
-    KB_CUDA(cudaMemcpyAsync(host.data() + a_acc, place<unsigned char>(buf, a_acc), down_end - a_acc, cudaMemcpyDeviceToHost, st));
-    KB_CUDA(cudaStreamSynchronize(st));
     const kb_accum *part = reinterpret_cast<const kb_accum *>(host.data() + a_acc);
     const double *hbs = reinterpret_cast<const double *>(host.data() + a_os);
     const unsigned long long *hbc = reinterpret_cast<const unsigned long long *>(host.data() + a_oc);
@@ -1328,15 +1341,29 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[0], st));
   KB_CUDA(launch_km_tree(L, kgrid, st));
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[1], st));
-  KB_CUDA(launch_km_fallback(L, ctx->sm_count * 4, st));
-  KB_CUDA(launch_reduce(L, place<kb_accum>(buf, a_acc), st));
-  if (nb)
-    KB_CUDA(launch_reduce_bins(L, place<double2>(buf, a_os), place<unsigned long long>(buf, a_oc),
-                               place<unsigned long long>(buf, a_od), st));
-  if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[2], st));
-  ctx->last_launches = nb ? 4 : 3;
-  KB_CUDA(cudaMemcpyAsync(host.data() + a_acc, place<unsigned char>(buf, a_acc), down_end - a_acc, cudaMemcpyDeviceToHost, st));
-  KB_CUDA(cudaStreamSynchronize(st));
+  auto finish = [&]() -> int { // as run_integrate's
+    KB_CUDA(launch_reduce(L, place<kb_accum>(buf, a_acc), st));
+    if (nb)
+      KB_CUDA(launch_reduce_bins(L, place<double2>(buf, a_os), place<unsigned long long>(buf, a_oc),
+                                 place<unsigned long long>(buf, a_od), st));
+    if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[2], st));
+    ctx->last_launches += nb ? 2 : 1;
+    KB_CUDA(cudaMemcpyAsync(host.data() + a_acc, place<unsigned char>(buf, a_acc), down_end - a_acc, cudaMemcpyDeviceToHost, st));
+    KB_CUDA(cudaStreamSynchronize(st));
+    return KB_OK;
+  };
+  ctx->last_launches = 1;
+  int rc = finish();
+  if (rc) return rc;
+  bool guarded = false;
+  for (size_t j = 0; j < ni; ++j) guarded = guarded || reinterpret_cast<const kb_accum *>(host.data() + a_acc)[j].n_fallback;
+  if (guarded) {
+    KB_CUDA(cudaMemsetAsync(place<kb_accum>(buf, a_acc), 0, ni * sizeof(kb_accum), st));
+    KB_CUDA(launch_km_fallback(L, ctx->sm_count * 4, st));
+    ctx->last_launches++;
+    rc = finish();
+    if (rc) return rc;
+  }
   const kb_accum *part = reinterpret_cast<const kb_accum *>(host.data() + a_acc);
   const double *hbs = reinterpret_cast<const double *>(host.data() + a_os);
   const unsigned long long *hbc = reinterpret_cast<const unsigned long long *>(host.data() + a_oc);
