@@ -51,16 +51,51 @@ __device__ __forceinline__ double2 pivot_rcp(double2 a) {
   return c2(a.x * y, -a.y * y);
 }
 
-__device__ __forceinline__ int find_chunk_item(const long long *off, int n_items, long long c) {
-  int lo = 0, hi = n_items; // off[lo] <= c < off[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (off[mid] <= c)
-      lo = mid;
-    else
-      hi = mid;
+// The latency of a small call is a chain of round trips to the L2 (300 to 700 cycles each): what
+// follows keeps their number down. 1,000 points of order 2: the kernel took 18,900 cycles, 9,400 of
+// them in the item's search, constants and set-up.
+
+// The warps take their first chunk by their place (first warps of all CTAs, then second ones) and
+// later ones from the counter, each one chunk ahead of its use. (As plain PTX: atomicAdd's
+// compiled form hands the result through a shuffle, which waits for it at once.)
+__device__ __forceinline__ int first_chunk() { return (threadIdx.x >> 5) * gridDim.x + blockIdx.x; }
+__device__ __forceinline__ int later_chunk(int *counter, int warps, int lane) {
+  int next = 0;
+  if (lane == 0) asm volatile("atom.global.add.s32 %0, [%1], 1;" : "=r"(next) : "l"(counter) : "memory");
+  return next + (int)gridDim.x * warps;
+}
+
+// The item of chunk c (the last with off[item] <= c), by all lanes: a 32nd of the list per round.
+__device__ __forceinline__ int find_chunk_item(const long long *off, int n_items, long long c, int lane) {
+  int lo = 0, len = n_items; // off[lo] <= c < off[lo + len]
+  while (len > 1) {
+    const int step = (len + 31) >> 5, p = lane * step;
+    const unsigned le = __ballot_sync(FULL, p < len && off[lo + p] <= c);
+    const int k = 31 - __clz(le);
+    lo += k * step;
+    len = min(step, len - k * step);
   }
   return lo;
+}
+
+// A copy of an item in a warp's buffers, behind the set-up's factors, for the set-up of a group: the
+// some fifty reads of its fields there were L2 round trips (little L1 beside the shared memory, and
+// the spilled registers go through it).
+constexpr int ITEM_AT = 128; // complex entries: order << lg factors are at most 256 doubles
+constexpr int ITEM_END = ITEM_AT + (int)(sizeof(ItemDev) + 15) / 16;
+__device__ __forceinline__ const ItemDev &stage_item(double2 *buf, const ItemDev *src, int lane) {
+  constexpr int WORDS = (int)sizeof(ItemDev) / 8, R = (WORDS + 31) / 32;
+  static_assert(sizeof(ItemDev) % 8 == 0, "whole words");
+  unsigned long long w[R];
+  unsigned long long *dst = reinterpret_cast<unsigned long long *>(buf + ITEM_AT);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (32 * r + lane < WORDS) w[r] = reinterpret_cast<const unsigned long long *>(src)[32 * r + lane];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (32 * r + lane < WORDS) dst[32 * r + lane] = w[r];
+  __syncwarp();
+  return *reinterpret_cast<const ItemDev *>(dst);
 }
 
 // ------------------------------------------------------------------ a group's set-up
@@ -73,19 +108,30 @@ __device__ __forceinline__ void sobol_group(const SobolDev &s, uint32_t k0, int 
   const uint32_t k = k0 + lane, b0 = k0 >> 5, b1 = b0 + 1;
   const uint32_t g0 = (b0 << 5) ^ (b0 << 4), g1 = (b1 << 5) ^ (b1 << 4);
   const uint32_t r = k & 31u, gr = r ^ (r >> 1);
-  for (int j = 0; j < N; ++j) {
-    const uint32_t *C = s.Csr + j * s.m;
-    // column b of the matrix; Gray bit m (point 2^m) folds into column 0
-    const uint32_t col = lane < s.m ? __ldg(C + lane) : (lane == s.m ? __ldg(C) : 0u);
-    const uint32_t x0 = __reduce_xor_sync(FULL, ((g0 >> lane) & 1u) ? col : 0u);
-    const uint32_t x1 = __reduce_xor_sync(FULL, ((g1 >> lane) & 1u) ? col : 0u);
-    uint32_t cur = (k >> 5) == b0 ? x0 : x1;
+  for (int j0 = 0; j0 < N; j0 += 4) { // four coordinates' columns in flight
+    uint32_t cols[4], sh[4];
 #pragma unroll
-    for (int b = 0; b < 5; ++b) {
-      const uint32_t cb = __shfl_sync(FULL, col, b);
-      if ((gr >> b) & 1u) cur ^= cb;
+    for (int q = 0; q < 4; ++q) {
+      const int j = min(j0 + q, N - 1);
+      const uint32_t *C = s.Csr + j * s.m;
+      // column b of the matrix; Gray bit m (point 2^m) folds into column 0
+      cols[q] = lane < s.m ? __ldg(C + lane) : (lane == s.m ? __ldg(C) : 0u);
+      sh[q] = __ldg(s.shfr + j);
     }
-    if (lane < (1 << lg)) u[(j << lg) + lane] = 2.3283064365386963e-10 * (double)(cur ^ __ldg(s.shfr + j));
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (j0 + q >= N) break;
+      const uint32_t col = cols[q];
+      const uint32_t x0 = __reduce_xor_sync(FULL, ((g0 >> lane) & 1u) ? col : 0u);
+      const uint32_t x1 = __reduce_xor_sync(FULL, ((g1 >> lane) & 1u) ? col : 0u);
+      uint32_t cur = (k >> 5) == b0 ? x0 : x1;
+#pragma unroll
+      for (int b = 0; b < 5; ++b) {
+        const uint32_t cb = __shfl_sync(FULL, col, b);
+        if ((gr >> b) & 1u) cur ^= cb;
+      }
+      if (lane < (1 << lg)) u[((j0 + q) << lg) + lane] = 2.3283064365386963e-10 * (double)(cur ^ sh[q]);
+    }
   }
 }
 
@@ -93,12 +139,16 @@ __device__ __forceinline__ void sobol_group(const SobolDev &s, uint32_t k0, int 
 // point's Jacobian and domain flag. The product warpers, whose logarithms and exponentials
 // dominate, run over (coordinate, point) pairs so that small groups fill the warp; a point's
 // Jacobian is the product of its factors in coordinate order.
-__device__ __noinline__ void setup_group(const Launch &L, const ItemDev &it, int N, int lg, long long gp0, int cnt, bool keep,
-                            double *u, double *fac, int lane, double &jac, bool &dom, bool &sorted) {
-  jac = 1.0;
+struct GroupSetup {
+  double jac;
+  bool dom, sorted; // inside the domain; the times latest first
+};
+__device__ __noinline__ GroupSetup setup_group(int mode, const double *in, const ItemDev &it, int N, int lg, long long gp0,
+                                               int cnt, bool keep, double *u, double *fac, int lane) {
+  double jac = 1.0;
   int top = 0;
   const bool mine = lane < cnt;
-  if (L.mode == IN_SOBOL) {
+  if (mode == IN_SOBOL) {
     top = it.chain_len;
     if (it.flow_x) { // Sobol points already mapped by the learned flow
       for (int j = 0; j < N; ++j)
@@ -126,8 +176,8 @@ __device__ __noinline__ void setup_group(const Launch &L, const ItemDev &it, int
     }
   } else {
     for (int j = 0; j < N; ++j)
-      if (mine) u[(j << lg) + lane] = L.in[(gp0 + lane) * N + j];
-    if (L.mode == IN_LI) top = it.chain_start;
+      if (mine) u[(j << lg) + lane] = in[(gp0 + lane) * N + j];
+    if (mode == IN_LI) top = it.chain_start;
   }
   __syncwarp();
   int lc = 0;
@@ -172,8 +222,7 @@ __device__ __noinline__ void setup_group(const Launch &L, const ItemDev &it, int
     __syncwarp();
   }
   jac *= cj;
-  dom = it.f.A.spin == it.f.B.spin;
-  sorted = true;
+  bool dom = it.f.A.spin == it.f.B.spin, sorted = true;
   if (mine) {
     double before = u[lane];
     if (keep && before < 0.0) dom = false;
@@ -184,6 +233,7 @@ __device__ __noinline__ void setup_group(const Launch &L, const ItemDev &it, int
       before = x;
     }
   }
+  return GroupSetup{jac, dom, sorted};
 }
 
 // Bin of the earliest vertex time (binner_t::in_bounds and coord2index, binner.hpp:163-176:
@@ -239,25 +289,23 @@ __device__ __forceinline__ bool in_window(const ItemDev &it, int N, const double
 // What the lookups of an absent block read.
 __device__ __align__(128) const double2 no_table[8] = {};
 
-// One lane fills an item's constants.
-__device__ void fill_item(ItemConst &K, const ItemDev &it, double rdelta, const unsigned long long *lookup) {
+// An item's constants: a kind of entry per lane, the rest by lane 0.
+__device__ __forceinline__ void fill_item(ItemConst &K, const ItemDev &it, double rdelta, const unsigned long long *lookup, int lane) {
+  if (lane >= 4) return;
   const ModelDev &m = it.model;
   const int spin = it.f.A.spin;
-  double2 gl, gg;
-  int b0 = 0;
-  g0_pair(m, m.tab[spin][0][0], 0.0, gl, gg, &b0);
-  K.eq = c2(gl.x, gl.y - m.alpha);
-  const double2 *tab[4] = {m.tab[spin][0][0], m.tab[spin][0][0], m.tab[spin][it.f.A.orbital][0],
-                           m.tab[spin][0][it.f.B.orbital]};
   // A later than the vertex (or at its time): forward copy g^>, backward g^<; earlier: A's branch
   // decides. B likewise; of two vertices the earlier one's index.
   constexpr unsigned GREATER = 0x3FF00000u, LESSER = 0xBFF00001u;
-  const unsigned w[4] = {GREATER, LESSER, GREATER, LESSER};
-  const unsigned alt[4] = {GREATER, LESSER, it.f.A.k_idx ? 1u : 0u, it.f.B.k_idx ? 0u : 1u};
-  for (int k = 0; k < 4; ++k) {
-    const unsigned none = tab[k] ? 0u : 2u;
-    K.kind[k] = EntryKind{tab[k] ? tab[k] : no_table, w[k] | none, alt[k] | none};
-  }
+  const double2 *tab = m.tab[spin][lane == 2 ? it.f.A.orbital : 0][lane == 3 ? it.f.B.orbital : 0];
+  const unsigned w = (lane & 1) ? LESSER : GREATER, none = tab ? 0u : 2u;
+  const unsigned alt = lane == 2 ? (it.f.A.k_idx ? 1u : 0u) : lane == 3 ? (it.f.B.k_idx ? 0u : 1u) : w;
+  K.kind[lane] = EntryKind{tab ? tab : no_table, w | none, alt | none};
+  if (lane) return;
+  double2 gl, gg;
+  int b0 = 0;
+  g0_pair(m, tab, 0.0, gl, gg, &b0);
+  K.eq = c2(gl.x, gl.y - m.alpha);
   K.xmin = m.xmin;
   K.delta = m.delta;
   K.rdelta = rdelta;

@@ -460,25 +460,24 @@ __global__ void __launch_bounds__(KM_WARPS * 32, KM_CTAS_PER_SM) km_tree_kernel(
   const bool eval = L.mode != IN_SOBOL;
   const int nb = L.nbins * 2;
   bool bad = false;
-  int item = -1, next = 0;
-  if (lane == 0) next = atomicAdd(L.chunk_counter, 1);
+  int item = -1, next = first_chunk();
   for (;;) {
     const int c = __shfl_sync(FULL, next, 0);
     if (c >= L.n_chunks) break;
-    if (lane == 0) next = atomicAdd(L.chunk_counter, 1);
+    next = later_chunk(L.chunk_counter, KM_WARPS, lane); // the chunk after this one, ahead of its use
     bool fresh = item < 0;
     if (fresh || c >= L.chunk_offsets[item + 1] || c < L.chunk_offsets[item]) {
-      item = find_chunk_item(L.chunk_offsets, L.n_items, c);
+      item = find_chunk_item(L.chunk_offsets, L.n_items, c, lane);
       fresh = true;
     }
-    const ItemDev &it = L.items[item];
+    const ItemDev &it = L.items[item]; // (a copy as the integrand's kernel keeps doubles the spills: +20 %)
     const long long cfirst = (long long)(c - L.chunk_offsets[item]) * it.chunk_points;
     const int ccount = (int)min((long long)it.chunk_points, (long long)it.n_points - cfirst);
     const int N = it.order, n2 = 2 * N, P = km_pass(N), lgp = km_group_lg(N), st = 1 << lgp, lg = max(min(N, 8) - 3, 0);
     const bool keep = eval ? (L.keep_u_hypercube != 0) : true;
     const double rdelta = 1.0 / it.model.delta;
     __syncwarp();
-    if (fresh && lane == 0) fill_item(T.k, it, rdelta, km_lookups.e + km_lookups.first[N]);
+    if (fresh) fill_item(T.k, it, rdelta, km_lookups.e + km_lookups.first[N], lane);
     if (!eval && L.nbins) {
       for (int b = lane; b < nb; b += 32) {
         L.bin_sums[(size_t)c * nb + b] = c2(0.0, 0.0);
@@ -498,10 +497,12 @@ __global__ void __launch_bounds__(KM_WARPS * 32, KM_CTAS_PER_SM) km_tree_kernel(
     for (int g0 = 0; g0 < ccount; g0 += st) {
       const int cnt = min(st, ccount - g0);
       const bool mine = lane < cnt;
-      double jac;
-      bool dom, sorted;
       double *ul = T.u + st + lane;
-      setup_group(L, it, N, lgp, cfirst + g0, cnt, keep, T.u + st, reinterpret_cast<double *>(T.buf), lane, jac, dom, sorted);
+      const GroupSetup su =
+          setup_group(L.mode, L.in, it, N, lgp, cfirst + g0, cnt, keep, T.u + st, reinterpret_cast<double *>(T.buf), lane);
+      const double jac = su.jac;
+      const bool dom = su.dom;
+      bool sorted = su.sorted;
       bool in = mine && dom;
       if (mine) {
         // (equal times need the vertices' order: the set-up's `sorted` lets them pass)

@@ -543,6 +543,11 @@ __global__ void __launch_bounds__(RT) reduce_kernel(Launch L, kb_accum *acc) {
   const long long c0 = L.chunk_offsets[item], c1 = L.chunk_offsets[item + 1];
   double re = 0.0, im = 0.0;
   unsigned long long dom = 0, fb = 0;
+  kb_accum a;
+  if (threadIdx.x == 0) { // read ahead of the sums
+    a = acc[item];
+    a.n_points += (uint64_t)L.items[item].n_points;
+  }
 #pragma unroll 4
   for (long long c = c0 + threadIdx.x; c < c1; c += RT) {
     const ChunkPartial &pr = L.partials[c];
@@ -572,11 +577,11 @@ __global__ void __launch_bounds__(RT) reduce_kernel(Launch L, kb_accum *acc) {
       dom += s_dom[t];
       fb += s_fb[t];
     }
-    acc[item].sum_re += re;
-    acc[item].sum_im += im;
-    acc[item].n_points += (uint64_t)L.items[item].n_points;
-    acc[item].n_in_domain += dom;
-    acc[item].n_fallback += fb;
+    a.sum_re += re;
+    a.sum_im += im;
+    a.n_in_domain += dom;
+    a.n_fallback += fb;
+    acc[item] = a;
   }
 }
 

@@ -31,7 +31,7 @@
 // of a node splitting its children; the last five vertices run in registers. Orders above 8
 // walk the levels above 9 depth first. Warps never wait for each other: no CTA barrier.
 //
-// Bound: latency. Order 8 (2^20 points): 3.6 ms, FP64 pipe 42 % busy, 1,590 instructions per point,
+// Bound: latency. Order 8 (2^20 points): 3.3 ms, FP64 pipe 42 % busy, 1,590 instructions per point,
 // of them 800 FP64, shared memory 50 %; the stalls are fixed latencies of dependent FP64
 // instructions and shared-memory loads at 12 warps per SM. Splitting a level's nodes over fewer
 // lanes with more registers (512 >> m nodes, 255 registers, 8 warps) took 4.6 ms, 15 warps at
@@ -68,7 +68,7 @@ __host__ __device__ constexpr int pass_points(int n) { return n <= 3 ? 32 : n >=
 __host__ __device__ constexpr int group_lg(int n) { return n <= 8 ? 5 : 4; }
 static_assert(delta_base(3) + 32 * delta_sz(3) <= WARP_BUF && delta_base(4) + 16 * delta_sz(4) <= WARP_BUF &&
                   delta_base(5) + 8 * delta_sz(5) <= WARP_BUF && delta_base(6) + 4 * delta_sz(6) <= WARP_BUF &&
-                  delta_base(16) + delta_sz(16) <= WARP_BUF && 2 * 256 <= WARP_BUF,
+                  delta_base(16) + delta_sz(16) <= WARP_BUF && ITEM_END <= WARP_BUF,
               "differences (and the set-up's factors) fit in a warp's buffers");
 // The lookups of a pass: entry (p, i, j), i != j, of point p's root (position 0: external row A or
 // column B; 1..n: the vertices, latest first). Fields: index of the times of positions i and j in
@@ -101,6 +101,16 @@ struct LookupTable {
 };
 __device__ const LookupTable lookups = LookupTable();
 
+// What a warp keeps of its chunk from group to group: the same in all lanes, where a spilled register
+// is 128 bytes and an L2 round trip (with the item's copy: order 1 0.18 -> 0.13 ms, order 2 0.25 -> 0.19).
+struct ChunkState {
+  double2 sum;
+  unsigned long long fb0, fb1; // the guarded points' bits
+  long long first;             // first point of the chunk within its item
+  int chunk, item, count, order;
+  unsigned ndom, nfb, ndrop;
+};
+
 template <bool SCALE>
 struct WarpShared {
   double2 buf[WARP_BUF];
@@ -109,7 +119,9 @@ struct WarpShared {
   ItemConst k;
   double2 D2[24];     // squared prefix determinants: level 5's nodes at 0, 6's at 8, 7's and 8's at
                       // 12, the depth-first levels' above 8 at 16
-  double fscale[SCALE ? 32 : 2];
+  double cutoff;
+  ChunkState s;
+  double fscale[SCALE ? 32 : 1];
 };
 
 // Root matrices and differences of the np points of a pass (u: their times).
@@ -386,20 +398,25 @@ __device__ __forceinline__ double2 merge_lanes(double2 a, double2 b, int bit, in
 }
 
 // A group's points in passes, each point's value into T.fval; returns the points with a guarded
-// pivot (bit per point of the group).
-template <bool SCALE, bool ANY_CUBIC>
-__device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int n, int cnt, unsigned inmask, double2 *stack,
+// pivot (bit per point of the group). ORDER: 1..8, 0 for the orders above. Compiled per order, as
+// the places, strides and the levels that an order has are then constants: 2^20 points of order 8 3.54 ->
+// 3.25 ms, of order 5 0.68 -> 0.61, and the orders above, without the branches of the others, 5 to
+// 10 % less.
+template <bool SCALE, bool ANY_CUBIC, int ORDER>
+__device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int order, int cnt, unsigned inmask, double2 *stack,
                                                  int lane) {
+  constexpr bool DEEP = ORDER == 0;
+  const int n = DEEP ? order : ORDER;
   const double floor_ = T.k.floor_;
   const int P = pass_points(n);
   const int lg = n <= 3 ? 0 : min(n, 8) - 3; // lanes per point
-  double2 *dl0 = T.buf + delta_base(n);
+  double2 *dl0 = T.buf + delta_base(DEEP ? 9 : n);
   const int dsz = delta_sz(n);
   // orders above 8: the depth-first levels' nodes, level 8's pair and then level 9's node behind the
   // differences in shared memory where they fit, the others in global scratch
   double2 *pair8 = nullptr, *node9 = nullptr;
   int pair_at = 0;
-  if (n > 8) {
+  if constexpr (DEEP) {
     int room = WARP_BUF - delta_base(n) - dsz;
     double2 *at = dl0 + dsz;
     int soff = 0;
@@ -415,8 +432,8 @@ __device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int n, in
     if (room >= 100) node9 = at;
   }
   const int K0 = max(n - 9, 0); // K0 depth-first levels above level 9
-  double2 *root = n > 9 ? stack : (n == 9 ? node9 : T.buf + node_base(n));
-  const int rsz = n > 8 ? 0 : node_sz(n), rw = n > 8 ? n + 1 : node_w(n);
+  double2 *root = DEEP ? (n > 9 ? stack : node9) : T.buf + node_base(n);
+  const int rsz = DEEP ? 0 : node_sz(n), rw = DEEP ? n + 1 : node_w(n);
   unsigned guarded = 0;
   double2 h0 = c2(0.0, 0.0), h1 = c2(0.0, 0.0); // values of earlier passes of a quad, not yet summed over lanes
   for (int s0 = 0, t = 0; s0 < cnt || (lg >= 2 && (t & 3)); s0 += P, ++t) {
@@ -430,19 +447,19 @@ __device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int n, in
         build_roots<true, 2>(T.k, n, np, T.u + s0, root, rsz, rw, dl0, lane);
       else
         build_roots<false, 3>(T.k, n, np, T.u + s0, root, rsz, rw, dl0, lane);
-      if (n <= 7 && n >= 4) {
+      if (!DEEP && n <= 7 && n >= 4) {
         if (n >= 5 && lane < 8) T.D2[n == 7 ? 12 + (lane & 1) : n == 6 ? 8 + (lane & 3) : lane] = c2(1.0, 0.0);
         if (n == 4 && lane < 16) T.D2[lane] = c2(1.0, 0.0);
       }
       __syncwarp();
-      if (n >= 3) {
+      if (DEEP || n >= 3) {
         // orders above 8: 2^K0 subtrees of level 9's node, each its two children's; else one tree
-        const double2 *dl = n >= 8 ? dl0 : dl0 + min(lane >> lg, np - 1) * dsz; // (idle lanes: the last point's)
+        const double2 *dl = DEEP || n >= 8 ? dl0 : dl0 + min(lane >> lg, np - 1) * dsz; // (idle lanes: the last point's)
         double2 D8 = c2(1.0, 0.0);
-        const int trees = n > 8 ? 2 << K0 : 1;
+        const int trees = DEEP ? 2 << K0 : 1;
         for (int tr = 0; tr < trees; ++tr) {
           int node8 = node_base(8);
-          if (n > 8) {
+          if constexpr (DEEP) {
             if (pair_at) {
               node8 = pair_at + 81 * (tr & 1);
             }
@@ -470,7 +487,7 @@ __device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int n, in
               __syncwarp();
             }
           }
-          const double2 w = subtree<SCALE>(T, node8, D8, dl, n, lane, floor_, guard, scale);
+          const double2 w = subtree<SCALE>(T, node8, D8, dl, DEEP ? 8 : n, lane, floor_, guard, scale);
           v = (__popc(tr) & 1) ? c2(v.x - w.x, v.y - w.y) : cadd(v, w);
           __syncwarp();
         }
@@ -533,7 +550,17 @@ __device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int n, in
   return guarded;
 }
 
-__device__ __forceinline__ double2 cut_off(double2 f, double cutoff) { return cabs(f) < cutoff ? c2(0.0, 0.0) : f; }
+__device__ __forceinline__ double2 cut_off(double2 f, double cutoff) { return cutoff > 0.0 && cabs(f) < cutoff ? c2(0.0, 0.0) : f; }
+
+// Order 0: g0(A, B).
+__device__ __noinline__ double2 order0(const ItemDev &it, int *err) {
+  kb_gf_index a = it.f.A, b = it.f.B;
+  a.timesplit = b.timesplit = 0;
+  int b0 = 0;
+  const double2 v = g0_contour(it.model, a, b, 0, &b0);
+  if (b0) atomicOr(err, 1);
+  return v;
+}
 
 // Persistent warps pull scheduling chunks (it.chunk_points points of one item) and walk them
 // in groups of up to 32 points (16 above order 8): set-up, values, then the group's sum in a
@@ -544,28 +571,29 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpShared<SCALE> &T = reinterpret_cast<WarpShared<SCALE> *>(smem_raw)[warp];
   double2 *stack = reinterpret_cast<double2 *>(L.pts) + (size_t)(blockIdx.x * TREE_WARPS + warp) * TREE_STACK;
-  bool bad = false;
-  int item = -1, next = 0;
-  if (lane == 0) next = atomicAdd(L.chunk_counter, 1);
+  if (lane == 0) T.s.item = -1;
+  int next = first_chunk();
   for (;;) {
     const int c = __shfl_sync(FULL, next, 0);
     if (c >= L.n_chunks) break;
-    if (lane == 0) next = atomicAdd(L.chunk_counter, 1); // the chunk after this one, ahead of its use
+    next = later_chunk(L.chunk_counter, TREE_WARPS, lane); // the chunk after this one, ahead of its use
+    __syncwarp();
+    int item = T.s.item;
     bool fresh = item < 0;
     if (fresh || c >= L.chunk_offsets[item + 1]) {
-      item = find_chunk_item(L.chunk_offsets, L.n_items, c);
+      item = find_chunk_item(L.chunk_offsets, L.n_items, c, lane);
       fresh = true;
     }
-    const ItemDev &it = L.items[item];
+    const ItemDev &it = stage_item(T.buf, L.items + item, lane); // until group_values
     const long long cfirst = (long long)(c - L.chunk_offsets[item]) * it.chunk_points;
-    const int ccount = (int)min((long long)it.chunk_points, (long long)it.n_points - cfirst);
+    if (lane == 0)
+      T.s = ChunkState{c2(0.0, 0.0), 0, 0, cfirst, c, item, (int)min((long long)it.chunk_points, (long long)it.n_points - cfirst), it.order, 0, 0, 0};
     const int N = it.order;
     const bool keep = EVAL ? (L.keep_u_hypercube != 0) : true;
     const int lgp = group_lg(N);
-    const double rdelta = 1.0 / it.model.delta;
-    __syncwarp();
-    if (fresh && lane == 0 && N > 0) { // what the passes read of the item
-      fill_item(T.k, it, rdelta, lookups.e + lookups.first[N]);
+    if (fresh) { // what the passes read of the item
+      if (N > 0) fill_item(T.k, it, 1.0 / it.model.delta, lookups.e + lookups.first[N], lane);
+      if (lane == 0) T.cutoff = it.f.cutoff;
     }
     if (!EVAL && L.nbins) {
       for (int b = lane; b < L.nbins; b += 32) {
@@ -574,25 +602,27 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
       }
       __syncwarp();
     }
-    double2 csum = c2(0.0, 0.0);
-    unsigned ndom = 0, nfb = 0, ndrop = 0;
-    unsigned long long fbm0 = 0, fbm1 = 0;
-    for (int g0 = 0; g0 < ccount; g0 += 1 << lgp) {
-      const int cnt = min(1 << lgp, ccount - g0);
+    __syncwarp();
+    for (int g0 = 0; g0 < T.s.count; g0 += 1 << lgp) {
+      const int cnt = min(1 << lgp, T.s.count - g0);
       const bool mine = lane < cnt;
-      double jac;
-      bool dom, sorted;
-      setup_group(L, it, N, lgp, cfirst + g0, cnt, keep, T.u + (1 << lgp), reinterpret_cast<double *>(T.buf), lane, jac, dom, sorted);
+      const int N = T.s.order;
+      if (g0) stage_item(T.buf, L.items + T.s.item, lane);
+      const GroupSetup su = setup_group(L.mode, L.in, it, N, lgp, T.s.first + g0, cnt, keep, T.u + (1 << lgp),
+                                        reinterpret_cast<double *>(T.buf), lane);
+      const double jac = su.jac;
+      const bool dom = su.dom;
       int bin = -1;
       if (!EVAL && L.nbins && mine) bin = earliest_bin(L, T.u + (1 << lgp) + lane, 1 << lgp, N);
       const unsigned dommask = __ballot_sync(FULL, mine && dom);
+      if (lane == 0) T.s.ndom += __popc(dommask);
       unsigned guarded = 0;
       if (N > 0) {
         bool in = mine && dom;
         double *ul = T.u + (1 << lgp) + lane;
-        if (!sorted) sort_times(ul, 1 << lgp, N); // (the plasma warper's times come sorted)
-        if (in && !in_window(it, N, ul, 1 << lgp, rdelta)) {
-          bad = true;
+        if (!su.sorted) sort_times(ul, 1 << lgp, N); // (the plasma warper's times come sorted)
+        if (in && !in_window(it, N, ul, 1 << lgp, T.k.rdelta)) {
+          atomicOr(L.err, 1);
           in = false;
         }
         if (mine) {
@@ -605,13 +635,19 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
         }
         const unsigned inmask = __ballot_sync(FULL, in);
         __syncwarp();
-        guarded = group_values<SCALE, ANY_CUBIC>(T, N, cnt, inmask, stack, lane);
+        switch (N) {
+          case 1: guarded = group_values<SCALE, ANY_CUBIC, 1>(T, N, cnt, inmask, stack, lane); break;
+          case 2: guarded = group_values<SCALE, ANY_CUBIC, 2>(T, N, cnt, inmask, stack, lane); break;
+          case 3: guarded = group_values<SCALE, ANY_CUBIC, 3>(T, N, cnt, inmask, stack, lane); break;
+          case 4: guarded = group_values<SCALE, ANY_CUBIC, 4>(T, N, cnt, inmask, stack, lane); break;
+          case 5: guarded = group_values<SCALE, ANY_CUBIC, 5>(T, N, cnt, inmask, stack, lane); break;
+          case 6: guarded = group_values<SCALE, ANY_CUBIC, 6>(T, N, cnt, inmask, stack, lane); break;
+          case 7: guarded = group_values<SCALE, ANY_CUBIC, 7>(T, N, cnt, inmask, stack, lane); break;
+          case 8: guarded = group_values<SCALE, ANY_CUBIC, 8>(T, N, cnt, inmask, stack, lane); break;
+          default: guarded = group_values<SCALE, ANY_CUBIC, 0>(T, N, cnt, inmask, stack, lane);
+        }
       } else if (mine) { // order 0: g0(A, B)
-        kb_gf_index a = it.f.A, b = it.f.B;
-        a.timesplit = b.timesplit = 0;
-        int b0 = 0;
-        const double2 v = dom ? g0_contour(it.model, a, b, 0, &b0) : c2(0.0, 0.0);
-        bad = bad || b0;
+        const double2 v = dom ? order0(it, L.err) : c2(0.0, 0.0);
         T.fval[lane] = v;
         if (SCALE) T.fscale[lane] = cabs(v);
       }
@@ -621,8 +657,8 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
       const bool fb = ok && (((guarded >> lane) & 1u) || !isfinite(fv.x) || !isfinite(fv.y));
       if (EVAL) {
         if (mine) {
-          const long long o = cfirst + g0 + lane;
-          const double2 f = ok ? cut_off(fv, it.f.cutoff) : c2(0.0, 0.0);
+          const long long o = T.s.first + g0 + lane;
+          const double2 f = ok ? cut_off(fv, T.cutoff) : c2(0.0, 0.0);
           L.out_val[o] = c2(f.x * jac, f.y * jac);
           if (L.out_jac) L.out_jac[o] = jac;
           if (L.out_dom) L.out_dom[o] = dom ? 1 : 0;
@@ -636,7 +672,7 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
       }
       double2 fj = c2(0.0, 0.0);
       if (ok && !fb) {
-        const double2 f = cut_off(fv, it.f.cutoff);
+        const double2 f = cut_off(fv, T.cutoff);
         fj = c2(f.x * jac, f.y * jac);
       }
       if (L.nbins) {
@@ -647,12 +683,14 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
         const unsigned same = __match_any_sync(FULL, mine ? bin : -2);
         __syncwarp();
         if (mine && bin >= 0 && (same & ((1u << lane) - 1u)) == 0u) {
-          double2 s = L.bin_sums[(size_t)c * L.nbins + bin];
+          const size_t o = (size_t)T.s.chunk * L.nbins + bin;
+          double2 s = L.bin_sums[o];
           for (unsigned r = same; r; r &= r - 1) s = cadd(s, T.fval[__ffs(r) - 1]);
-          L.bin_sums[(size_t)c * L.nbins + bin] = s;
-          L.bin_counts[(size_t)c * L.nbins + bin] += __popc(same);
+          L.bin_sums[o] = s;
+          L.bin_counts[o] += __popc(same);
         }
-        ndrop += __popc(__ballot_sync(FULL, mine && bin < 0));
+        const unsigned nd = __popc(__ballot_sync(FULL, mine && bin < 0));
+        if (lane == 0) T.s.ndrop += nd;
         __syncwarp();
       }
       const unsigned fbm = __ballot_sync(FULL, fb);
@@ -660,30 +698,28 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
         fj.x += __shfl_xor_sync(FULL, fj.x, off);
         fj.y += __shfl_xor_sync(FULL, fj.y, off);
       }
-      csum = cadd(csum, fj);
-      ndom += __popc(dommask);
-      nfb += __popc(fbm);
-      // the guarded points' bits of the chunk: g0 is a multiple of 16
-      if (g0 < 64)
-        fbm0 |= (unsigned long long)fbm << g0;
-      if (g0 > 32 && g0 < 64)
-        fbm1 |= (unsigned long long)fbm >> (64 - g0);
-      if (g0 >= 64) fbm1 |= (unsigned long long)fbm << (g0 - 64);
+      if (lane == 0) {
+        T.s.sum = cadd(T.s.sum, fj);
+        T.s.nfb += __popc(fbm);
+        // the guarded points' bits of the chunk: g0 is a multiple of 16
+        if (g0 < 64) T.s.fb0 |= (unsigned long long)fbm << g0;
+        if (g0 > 32 && g0 < 64) T.s.fb1 |= (unsigned long long)fbm >> (64 - g0);
+        if (g0 >= 64) T.s.fb1 |= (unsigned long long)fbm << (g0 - 64);
+      }
       __syncwarp();
     }
     if (!EVAL && lane == 0) {
       ChunkPartial pr;
-      pr.sum_re = csum.x;
-      pr.sum_im = csum.y;
-      pr.n_in_domain = ndom;
-      pr.n_fallback = nfb;
-      pr.fb_mask[0] = fbm0;
-      pr.fb_mask[1] = fbm1;
-      L.partials[c] = pr;
-      if (L.nbins) L.bin_dropped[c] = ndrop;
+      pr.sum_re = T.s.sum.x;
+      pr.sum_im = T.s.sum.y;
+      pr.n_in_domain = T.s.ndom;
+      pr.n_fallback = T.s.nfb;
+      pr.fb_mask[0] = T.s.fb0;
+      pr.fb_mask[1] = T.s.fb1;
+      L.partials[T.s.chunk] = pr;
+      if (L.nbins) L.bin_dropped[T.s.chunk] = T.s.ndrop;
     }
   }
-  if (__any_sync(FULL, bad) && lane == 0) atomicOr(L.err, 1);
 }
 
 template <bool SCALE>
