@@ -448,6 +448,99 @@ __device__ __noinline__ void km_deep(KmShared &T, double2 *stack, const double2 
   }
 }
 
+// A group's passes: the points' sums, scaled by their Jacobians, to the bins, the sum or the output;
+// returns the points for the pivoted-LU pass. ORDER: 1..8, 0 for the orders above: compiled per
+// order, as the integrand's passes are.
+template <int ORDER>
+__device__ __forceinline__ unsigned km_passes(const Launch &L, KmShared &T, int order, bool symmetric, int cnt, unsigned inmask,
+                                              unsigned dommask, long long first, int c, double2 *stack, int lane,
+                                              double2 &csum, unsigned &ndrop) {
+  const int N = ORDER ? ORDER : order, n2 = 2 * N, P = km_pass(N), lgp = km_group_lg(N), lg = max(min(N, 8) - 3, 0);
+  const bool eval = L.mode != IN_SOBOL;
+  const int nb = L.nbins * 2;
+  const double floor_ = T.k.floor_;
+  double2 *dl0 = T.buf + km_delta(N);
+  const int dsz = km_delta_sz(N);
+  double2 *root = N > 8 ? stack : T.buf + km_base(N);
+  const int rsz = N > 8 ? 0 : km_sz(N);
+  double2 *out = N > 8 ? T.out : T.buf;
+  unsigned guarded = symmetric ? 0u : dommask;
+  for (int s0 = 0; s0 < cnt; s0 += P) {
+    const int np = min(P, cnt - s0);
+    const unsigned some = (inmask >> s0) & (np >= 32 ? FULL : (1u << np) - 1u);
+    bool guard = false;
+    unsigned good = 0; // points of the pass with values
+    if (some && symmetric) {
+      if (T.k.cubic)
+        build_entries<true, 2>(T.k, np * N * N, T.u + s0, root, dl0, lane);
+      else
+        build_entries<false, 3>(T.k, np * N * N, T.u + s0, root, dl0, lane);
+      km_fixed_entries(T, N, np, s0, lgp, root, rsz, lane);
+      if (N <= 8 && N >= 4) T.D2[lane] = c2(1.0, 0.0);
+      __syncwarp();
+      double2 h[8], g;
+      if (N > 8)
+        km_deep(T, stack, dl0, N, lane, floor_, guard);
+      else
+        km_subtree(T, out, dl0 + min(lane >> lg, np - 1) * dsz, N, np, false, lane, floor_, guard, h, g);
+      const unsigned gm = __ballot_sync(FULL, guard);
+      const unsigned pm = lg == 5 ? gm : (gm >> ((lane << lg) & 31)) & ((1u << (1 << lg)) - 1u);
+      // a value that is not finite goes to the pivoted-LU pass as a guarded one does
+      bool nonfinite = false;
+      if (lane < np)
+        for (int q = 0; q < n2; ++q) {
+          const double2 v = out[lane * n2 + q];
+          nonfinite = nonfinite || !isfinite(v.x) || !isfinite(v.y);
+        }
+      const unsigned flagged = __ballot_sync(FULL, lane < np && (pm || nonfinite)) & some;
+      guarded |= flagged << s0;
+      good = some & ~flagged;
+    }
+    // every (point, position, index) of the pass: e = p 2N + 2 (i - 1) + k
+    for (int e0 = 0; e0 < np * n2; e0 += 32) {
+      const int e = e0 + lane;
+      const bool have = e < np * n2;
+      const int ee = have ? e : 0, p = ee / n2, q = ee - p * n2, i = q >> 1; // idle lanes: the first
+      const bool ok = have && ((good >> p) & 1u);
+      const double j = T.jac[s0 + p], t = T.u[((i + 1) << lgp) + s0 + p];
+      double2 v = ok ? out[ee] : c2(0.0, 0.0);
+      v = c2(v.x * j, v.y * j);
+      if (eval) {
+        if (have && !((guarded >> (s0 + p)) & 1u))
+          L.out_kvals[(first + s0 + p) * n2 + 2 * T.place[(i << lgp) + s0 + p] + (q & 1)] = v;
+        continue;
+      }
+      if (L.km_fourier) {
+        double sn, cs;
+        sincos(L.km_omega * t, &sn, &cs);
+        csum = cadd(csum, ok ? cmul(v, c2(cs, sn)) : c2(0.0, 0.0));
+        continue;
+      }
+      int bin = -1;
+      if (L.bin_xmin <= t && t <= L.bin_xmax)
+        bin = t == L.bin_xmax ? L.nbins - 1 : min((int)((t - L.bin_xmin) / L.bin_size), L.nbins - 1);
+      csum = cadd(csum, v);
+      // each bin's lowest lane adds the lanes' terms in order
+      const unsigned same = __match_any_sync(FULL, ok && bin >= 0 ? 2 * bin + (q & 1) : -1 - lane);
+      double2 s = v;
+      for (unsigned r = same & (same - 1u); __any_sync(FULL, r != 0u); r &= r - 1u) {
+        const int from = r ? __ffs(r) - 1 : lane;
+        const double2 w = c2(__shfl_sync(FULL, v.x, from), __shfl_sync(FULL, v.y, from));
+        if (r) s = cadd(s, w);
+      }
+      if (ok && bin >= 0 && lane == __ffs(same) - 1) {
+        const size_t b = (size_t)c * nb + 2 * bin + (q & 1);
+        L.bin_sums[b] = cadd(L.bin_sums[b], s);
+        L.bin_counts[b] += (unsigned)__popc(same) << (N - 1);
+      }
+      ndrop += __popc(__ballot_sync(FULL, ok && bin < 0)) << (N - 1);
+      __syncwarp();
+    }
+    __syncwarp();
+  }
+  return guarded;
+}
+
 // Persistent warps pull scheduling chunks and walk them in groups (32 points up to order 3, then 16):
 // set-up, then passes of km_pass points, each pass's 2n sums per point to the outputs (IN_TIMES), the
 // chunk's bins, or weighted by e^{i omega t} (km_fourier) to the chunk's sum. Points with a guarded
@@ -473,7 +566,7 @@ __global__ void __launch_bounds__(KM_WARPS * 32, KM_CTAS_PER_SM) km_tree_kernel(
     const ItemDev &it = L.items[item]; // (a copy as the integrand's kernel keeps doubles the spills: +20 %)
     const long long cfirst = (long long)(c - L.chunk_offsets[item]) * it.chunk_points;
     const int ccount = (int)min((long long)it.chunk_points, (long long)it.n_points - cfirst);
-    const int N = it.order, n2 = 2 * N, P = km_pass(N), lgp = km_group_lg(N), st = 1 << lgp, lg = max(min(N, 8) - 3, 0);
+    const int N = it.order, lgp = km_group_lg(N), st = 1 << lgp;
     const bool keep = eval ? (L.keep_u_hypercube != 0) : true;
     const double rdelta = 1.0 / it.model.delta;
     __syncwarp();
@@ -488,12 +581,6 @@ __global__ void __launch_bounds__(KM_WARPS * 32, KM_CTAS_PER_SM) km_tree_kernel(
     double2 csum = c2(0.0, 0.0);
     unsigned ndom = 0, nfb = 0, ndrop = 0;
     unsigned long long fbm[2] = {0, 0};
-    const double floor_ = T.k.floor_;
-    double2 *dl0 = T.buf + km_delta(N);
-    const int dsz = km_delta_sz(N);
-    double2 *root = N > 8 ? stack : T.buf + km_base(N);
-    const int rsz = N > 8 ? 0 : km_sz(N);
-    double2 *out = N > 8 ? T.out : T.buf;
     for (int g0 = 0; g0 < ccount; g0 += st) {
       const int cnt = min(st, ccount - g0);
       const bool mine = lane < cnt;
@@ -526,79 +613,17 @@ __global__ void __launch_bounds__(KM_WARPS * 32, KM_CTAS_PER_SM) km_tree_kernel(
           for (int j = 0; j < N; ++j) T.u[((j + 1) << lgp) + lane] = dom && !it.spin_symmetric ? ul[j << lgp] : tX;
       }
       __syncwarp();
-      unsigned guarded = it.spin_symmetric ? 0u : dommask;
-      for (int s0 = 0; s0 < cnt; s0 += P) {
-        const int np = min(P, cnt - s0);
-        const unsigned some = (inmask >> s0) & (np >= 32 ? FULL : (1u << np) - 1u);
-        bool guard = false;
-        unsigned good = 0; // points of the pass with values
-        if (some && it.spin_symmetric) {
-          if (T.k.cubic)
-            build_entries<true, 2>(T.k, np * N * N, T.u + s0, root, dl0, lane);
-          else
-            build_entries<false, 3>(T.k, np * N * N, T.u + s0, root, dl0, lane);
-          km_fixed_entries(T, N, np, s0, lgp, root, rsz, lane);
-          if (N <= 8 && N >= 4) T.D2[lane] = c2(1.0, 0.0);
-          __syncwarp();
-          double2 h[8], g;
-          if (N > 8)
-            km_deep(T, stack, dl0, N, lane, floor_, guard);
-          else
-            km_subtree(T, out, dl0 + min(lane >> lg, np - 1) * dsz, N, np, false, lane, floor_, guard, h, g);
-          const unsigned gm = __ballot_sync(FULL, guard);
-          const unsigned pm = lg == 5 ? gm : (gm >> ((lane << lg) & 31)) & ((1u << (1 << lg)) - 1u);
-          // a value that is not finite goes to the pivoted-LU pass as a guarded one does
-          bool nonfinite = false;
-          if (lane < np)
-            for (int q = 0; q < n2; ++q) {
-              const double2 v = out[lane * n2 + q];
-              nonfinite = nonfinite || !isfinite(v.x) || !isfinite(v.y);
-            }
-          const unsigned flagged = __ballot_sync(FULL, lane < np && (pm || nonfinite)) & some;
-          guarded |= flagged << s0;
-          good = some & ~flagged;
-        }
-        // every (point, position, index) of the pass: e = p 2N + 2 (i - 1) + k
-        for (int e0 = 0; e0 < np * n2; e0 += 32) {
-          const int e = e0 + lane;
-          const bool have = e < np * n2;
-          const int ee = have ? e : 0, p = ee / n2, q = ee - p * n2, i = q >> 1; // idle lanes: the first
-          const bool ok = have && ((good >> p) & 1u);
-          const double j = T.jac[s0 + p], t = T.u[((i + 1) << lgp) + s0 + p];
-          double2 v = ok ? out[ee] : c2(0.0, 0.0);
-          v = c2(v.x * j, v.y * j);
-          if (eval) {
-            if (have && !((guarded >> (s0 + p)) & 1u))
-              L.out_kvals[(cfirst + g0 + s0 + p) * n2 + 2 * T.place[(i << lgp) + s0 + p] + (q & 1)] = v;
-            continue;
-          }
-          if (L.km_fourier) {
-            double sn, cs;
-            sincos(L.km_omega * t, &sn, &cs);
-            csum = cadd(csum, ok ? cmul(v, c2(cs, sn)) : c2(0.0, 0.0));
-            continue;
-          }
-          int bin = -1;
-          if (L.bin_xmin <= t && t <= L.bin_xmax)
-            bin = t == L.bin_xmax ? L.nbins - 1 : min((int)((t - L.bin_xmin) / L.bin_size), L.nbins - 1);
-          csum = cadd(csum, v);
-          // each bin's lowest lane adds the lanes' terms in order
-          const unsigned same = __match_any_sync(FULL, ok && bin >= 0 ? 2 * bin + (q & 1) : -1 - lane);
-          double2 s = v;
-          for (unsigned r = same & (same - 1u); __any_sync(FULL, r != 0u); r &= r - 1u) {
-            const int from = r ? __ffs(r) - 1 : lane;
-            const double2 w = c2(__shfl_sync(FULL, v.x, from), __shfl_sync(FULL, v.y, from));
-            if (r) s = cadd(s, w);
-          }
-          if (ok && bin >= 0 && lane == __ffs(same) - 1) {
-            const size_t b = (size_t)c * nb + 2 * bin + (q & 1);
-            L.bin_sums[b] = cadd(L.bin_sums[b], s);
-            L.bin_counts[b] += (unsigned)__popc(same) << (N - 1);
-          }
-          ndrop += __popc(__ballot_sync(FULL, ok && bin < 0)) << (N - 1);
-          __syncwarp();
-        }
-        __syncwarp();
+      unsigned guarded;
+      switch (N) {
+        case 1: guarded = km_passes<1>(L, T, N, it.spin_symmetric, cnt, inmask, dommask, cfirst + g0, c, stack, lane, csum, ndrop); break;
+        case 2: guarded = km_passes<2>(L, T, N, it.spin_symmetric, cnt, inmask, dommask, cfirst + g0, c, stack, lane, csum, ndrop); break;
+        case 3: guarded = km_passes<3>(L, T, N, it.spin_symmetric, cnt, inmask, dommask, cfirst + g0, c, stack, lane, csum, ndrop); break;
+        case 4: guarded = km_passes<4>(L, T, N, it.spin_symmetric, cnt, inmask, dommask, cfirst + g0, c, stack, lane, csum, ndrop); break;
+        case 5: guarded = km_passes<5>(L, T, N, it.spin_symmetric, cnt, inmask, dommask, cfirst + g0, c, stack, lane, csum, ndrop); break;
+        case 6: guarded = km_passes<6>(L, T, N, it.spin_symmetric, cnt, inmask, dommask, cfirst + g0, c, stack, lane, csum, ndrop); break;
+        case 7: guarded = km_passes<7>(L, T, N, it.spin_symmetric, cnt, inmask, dommask, cfirst + g0, c, stack, lane, csum, ndrop); break;
+        case 8: guarded = km_passes<8>(L, T, N, it.spin_symmetric, cnt, inmask, dommask, cfirst + g0, c, stack, lane, csum, ndrop); break;
+        default: guarded = km_passes<0>(L, T, N, it.spin_symmetric, cnt, inmask, dommask, cfirst + g0, c, stack, lane, csum, ndrop);
       }
       if (eval && mine) {
         const long long o = cfirst + g0 + lane;
