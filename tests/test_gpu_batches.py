@@ -1,0 +1,65 @@
+"""Batches and groups of the integration where the kernels' schedule branches: the search of a chunk's
+item over one, two and three rounds of 32, items without points among others, ordinary items beside
+items whose points all go to the pivoted LU (their pass follows only when the sums count some), and
+groups of several quads of passes at every compiled order. A batch's sums are those of separate
+calls, bit for bit; against the CPU oracle, |gpu - cpu| <= 1e-12 of the sum of |terms|."""
+import numpy as np
+import pytest
+
+from keldy_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+INVERSE = [(capi.WARPER_PLASMA_UV, 10.0, 0.0), (capi.WARPER_INVERSE, 10.0, 2.0)]  # few points in the domain above order 8
+EXPONENTIAL = [(capi.WARPER_PLASMA_UV, 10.0, 0.0), (capi.WARPER_EXPONENTIAL, 10.0, 1.0)]
+A, B = (10.0, 0, 0, 0, 0), (10.0, 0, 1, 0, 0)
+
+
+def _tables(kind):
+    t = np.linspace(-10, 10, 2001)
+    if kind == "guarded":  # g(0) = 0: a zero pivot at every point
+        le = 1j * t * np.exp(-t * t / 8) + 0.2 * np.sin(t)
+    else:
+        le = 0.5j * np.exp(-np.abs(t)) + 0.1 * np.sin(t) * np.exp(-np.abs(t))
+    return le, -np.conj(le[::-1])
+
+
+def _item(model, rng, order, npts, k_first, chain=INVERSE):
+    return dict(model=model, rng=rng, chain=chain, A=A, B=B, order=order, k_first=k_first, n_points=npts)
+
+
+@pytest.mark.parametrize("count", [2, 31, 33, 1023, 1025])
+def test_batch_equals_calls(ctx, count):
+    m = ctx.model(10.0, *_tables("plain"))
+    rngs = {n: ctx.sobol(n) for n in (1, 2, 3, 5)}
+    items = [_item(m, rngs[(1, 2, 3, 5)[i % 4]], (1, 2, 3, 5)[i % 4], (i * 7) % 23, 1 + i) for i in range(count)]
+    batch = capi.integrate(ctx, items)
+    for i in sorted({0, 1, count // 3, count // 2, count - 2, count - 1}):
+        single, = capi.integrate(ctx, [items[i]])
+        assert single == batch[i], i
+    assert [r[1] for r in batch] == [it["n_points"] for it in items]
+
+
+@pytest.mark.parametrize("chain", [INVERSE, EXPONENTIAL])
+@pytest.mark.parametrize("order", [1, 2, 4, 6, 9])
+def test_guarded_items_among_others(ctx, oracle, order, chain):
+    rng = ctx.sobol(order)
+    items, want = [], []
+    for i, kind in enumerate(("plain", "guarded", "plain")):
+        items.append(_item(ctx.model(10.0, *_tables(kind)), rng, order, 37 + i, 3 + i, chain))
+        want.append(oracle.integrate(oracle.model(10.0, *_tables(kind)), A, B, chain, order, 37 + i, seed=2 + i))
+    for (s, npt, nd, nfb), (w, onp, ond, sc), kind in zip(capi.integrate(ctx, items), want, ("plain", "guarded", "plain")):
+        assert (npt, nd) == (onp, ond)
+        assert (nfb > 0) == (kind == "guarded" and order > 1 and ond > 0)
+        assert abs(s - w) <= 1e-12 * sc, (kind, abs(s - w) / sc)
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 5, 6, 7, 8, 9, 10])
+def test_groups_of_several_quads(ctx, oracle, order):
+    """Enough points for full groups: fewer are spread over the warps in smaller ones."""
+    npts = 7203 if order <= 6 else 3601
+    m = ctx.model(10.0, *_tables("plain"))
+    (s, npt, nd, nfb), = capi.integrate(ctx, [_item(m, ctx.sobol(order), order, npts, 6, EXPONENTIAL)])
+    w, onp, ond, sc = oracle.integrate(oracle.model(10.0, *_tables("plain")), A, B, EXPONENTIAL, order, npts, seed=5)
+    assert (npt, nd, nfb) == (onp, ond, 0) and nd > npts // 2
+    assert abs(s - w) <= 1e-12 * sc
