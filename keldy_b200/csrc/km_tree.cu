@@ -49,6 +49,11 @@ __host__ __device__ constexpr int km_delta(int n) {
 // entries (k, j); behind all shells the n entries of column C.
 __host__ __device__ constexpr int km_delta_sz(int n) { return n * n + (n < 8 && n % 2 == 0 ? 1 : 0); }
 __host__ __device__ constexpr int km_pass(int n) { return n <= 3 ? 32 : n >= 8 ? 1 : 256 >> n; }
+// Lookups in flight per lane (whole rounds of lanes for a pass's n^2 entries per point; 0: the orders above 8).
+__host__ __device__ constexpr int km_flight(int n) {
+  constexpr int FLIGHT[] = {4, 1, 4, 5, 4, 4, 5, 4, 2};
+  return FLIGHT[n];
+}
 __host__ __device__ constexpr int km_group_lg(int n) { return n <= 3 ? 5 : 4; }
 static_assert(km_delta(3) + 32 * km_delta_sz(3) <= KM_BUF && km_delta(4) + 16 * km_delta_sz(4) <= KM_BUF &&
                   km_delta(5) + 8 * km_delta_sz(5) <= KM_BUF && km_delta(6) + 4 * km_delta_sz(6) <= KM_BUF &&
@@ -474,7 +479,7 @@ __device__ __forceinline__ unsigned km_passes(const Launch &L, KmShared &T, int 
       if (T.k.cubic)
         build_entries<true, 2>(T.k, np * N * N, T.u + s0, root, dl0, lane);
       else
-        build_entries<false, 3>(T.k, np * N * N, T.u + s0, root, dl0, lane);
+        build_entries<false, km_flight(ORDER)>(T.k, np * N * N, T.u + s0, root, dl0, lane);
       km_fixed_entries(T, N, np, s0, lgp, root, rsz, lane);
       if (N <= 8 && N >= 4) T.D2[lane] = c2(1.0, 0.0);
       __syncwarp();

@@ -65,10 +65,21 @@ __host__ __device__ constexpr int delta_base(int n) { return n >= 6 ? NODES_END 
 __host__ __device__ constexpr int delta_sz(int n) { return n < 8 ? n * (n + 1) + 1 : n * (n + 1); }
 // Points of a pass (2^(n-3) lanes per point, at most one point per lane), and of a group.
 __host__ __device__ constexpr int pass_points(int n) { return n <= 3 ? 32 : n >= 8 ? 1 : 256 >> n; }
+// Points whose roots are built together: a pass's, but two of order 8 (72 entries a point leave the
+// lanes' second and third lookup idle: 3.25 -> 3.16 ms). Lookups in flight per lane: with whole rounds
+// of lanes for the build's entries (3 at every order: order 7's 112 took two rounds, 1.89 ms for 1.78;
+// order 10 13.3 for 12.9).
+__host__ __device__ constexpr int build_points(int n) { return n == 8 ? 2 : pass_points(n); }
+__host__ __device__ constexpr int build_flight(int n) {
+  constexpr int FLIGHT[] = {4, 2, 3, 6, 5, 4, 3, 4, 5}; // (0: the orders above 8)
+  return FLIGHT[n];
+}
+// A root's place: its level's, order 8's two behind the differences.
+__host__ __device__ constexpr int root_base(int n) { return n == 8 ? NODES_END + 2 * 72 : node_base(n); }
 __host__ __device__ constexpr int group_lg(int n) { return n <= 8 ? 5 : 4; }
 static_assert(delta_base(3) + 32 * delta_sz(3) <= WARP_BUF && delta_base(4) + 16 * delta_sz(4) <= WARP_BUF &&
                   delta_base(5) + 8 * delta_sz(5) <= WARP_BUF && delta_base(6) + 4 * delta_sz(6) <= WARP_BUF &&
-                  delta_base(16) + delta_sz(16) <= WARP_BUF && ITEM_END <= WARP_BUF,
+                  delta_base(16) + delta_sz(16) <= WARP_BUF && root_base(8) + 2 * 81 <= WARP_BUF && ITEM_END <= WARP_BUF,
               "differences (and the set-up's factors) fit in a warp's buffers");
 // The lookups of a pass: entry (p, i, j), i != j, of point p's root (position 0: external row A or
 // column B; 1..n: the vertices, latest first). Fields: index of the times of positions i and j in
@@ -76,7 +87,7 @@ static_assert(delta_base(3) + 32 * delta_sz(3) <= WARP_BUF && delta_base(4) + 16
 // 1: i the earlier, 2: row A, 3: column B).
 constexpr int lookup_first(int n) { // entries of orders below n
   int s = 0;
-  for (int k = 1; k < n; ++k) s += pass_points(k) * k * (k + 1);
+  for (int k = 1; k < n; ++k) s += build_points(k) * k * (k + 1);
   return s;
 }
 struct LookupTable {
@@ -86,8 +97,8 @@ struct LookupTable {
     int r = 0;
     for (int n = 1; n <= MAX_ORDER; ++n) {
       first[n] = r;
-      const int ssz = n > 8 ? 0 : node_sz(n), w = n > 8 ? n + 1 : node_w(n), st = 1 << group_lg(n);
-      for (int p = 0; p < pass_points(n); ++p)
+      const int ssz = n > 8 ? 0 : n == 8 ? 81 : node_sz(n), w = n > 8 ? n + 1 : node_w(n), st = 1 << group_lg(n);
+      for (int p = 0; p < build_points(n); ++p)
         for (int i = 0; i <= n; ++i)
           for (int j = 0; j <= n; ++j) {
             if (i == j) continue;
@@ -432,8 +443,8 @@ __device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int order
     if (room >= 100) node9 = at;
   }
   const int K0 = max(n - 9, 0); // K0 depth-first levels above level 9
-  double2 *root = DEEP ? (n > 9 ? stack : node9) : T.buf + node_base(n);
-  const int rsz = DEEP ? 0 : node_sz(n), rw = DEEP ? n + 1 : node_w(n);
+  double2 *root = DEEP ? (n > 9 ? stack : node9) : T.buf + root_base(n);
+  const int rsz = DEEP ? 0 : n == 8 ? 81 : node_sz(n), rw = DEEP ? n + 1 : node_w(n);
   unsigned guarded = 0;
   double2 h0 = c2(0.0, 0.0), h1 = c2(0.0, 0.0); // values of earlier passes of a quad, not yet summed over lanes
   for (int s0 = 0, t = 0; s0 < cnt || (lg >= 2 && (t & 3)); s0 += P, ++t) {
@@ -442,11 +453,14 @@ __device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int order
     bool guard = false;
     double scale = 0.0;
     double2 v = c2(0.0, 0.0);
+    const bool second = ORDER == 8 && (t & 1) && ((inmask >> (s0 - 1)) & 1u);
     if (in) {
-      if (ANY_CUBIC && T.k.cubic)
-        build_roots<true, 2>(T.k, n, np, T.u + s0, root, rsz, rw, dl0, lane);
+      const int nb = ORDER == 8 ? min(2, cnt - s0) : np;
+      if (second) { // built with the point before
+      } else if (ANY_CUBIC && T.k.cubic)
+        build_roots<true, 2>(T.k, n, nb, T.u + s0, root, rsz, rw, dl0, lane);
       else
-        build_roots<false, 3>(T.k, n, np, T.u + s0, root, rsz, rw, dl0, lane);
+        build_roots<false, build_flight(ORDER)>(T.k, n, nb, T.u + s0, root, rsz, rw, dl0, lane);
       if (!DEEP && n <= 7 && n >= 4) {
         if (n >= 5 && lane < 8) T.D2[n == 7 ? 12 + (lane & 1) : n == 6 ? 8 + (lane & 3) : lane] = c2(1.0, 0.0);
         if (n == 4 && lane < 16) T.D2[lane] = c2(1.0, 0.0);
@@ -454,11 +468,11 @@ __device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int order
       __syncwarp();
       if (DEEP || n >= 3) {
         // orders above 8: 2^K0 subtrees of level 9's node, each its two children's; else one tree
-        const double2 *dl = DEEP || n >= 8 ? dl0 : dl0 + min(lane >> lg, np - 1) * dsz; // (idle lanes: the last point's)
+        const double2 *dl = DEEP || n >= 8 ? dl0 + dsz * second : dl0 + min(lane >> lg, np - 1) * dsz; // (idle lanes: the last point's)
         double2 D8 = c2(1.0, 0.0);
         const int trees = DEEP ? 2 << K0 : 1;
         for (int tr = 0; tr < trees; ++tr) {
-          int node8 = node_base(8);
+          int node8 = ORDER == 8 ? root_base(8) + 81 * second : node_base(8);
           if constexpr (DEEP) {
             if (pair_at) {
               node8 = pair_at + 81 * (tr & 1);
