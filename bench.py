@@ -36,8 +36,8 @@ GAMMA, EPS_D, BIAS, BETA, T_MAX, NPTS = 1.0, 0.0, 0.0, 50.0, 20.0, 40001
 # order 8) from an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum), keyed by
 # the hash of the kernel's code (tree_source_hash, comments stripped) at the time of the capture. A build
 # whose sources hash differently reports no traffic figure until it is captured again.
-TREE_DRAM_CAPTURES = {"e99222e79bec14ce": 2335744 + 204688384}
-TREE_SOURCES = ("tree.cu", "kb_device.cuh", "kb_types.h", "kb_launch.h", "kb_spline.cuh", "kb_flow.h")
+TREE_DRAM_CAPTURES = {"5de8928da3ce1dc4": 3238144 + 1705728}
+TREE_SOURCES = ("wick_tree.cu", "kb_wick.cuh", "kb_device.cuh", "kb_types.h", "kb_launch.h", "kb_spline.cuh", "kb_flow.h")
 E2E_REPEATS = 5
 
 
@@ -72,14 +72,16 @@ def reference_flops(n):
 
 
 def tree_flops(n):
-    """FLOPs the Schur-complement tree executes per point: per child of a level-k node
-    of size m = 2(n-k)+1, one reciprocal (~8), the prefix product (6), (m-2) scaled
-    pivot entries (6 each) and (m-2)^2 complex FMAs (8 each); per leaf ~34."""
-    total = 0
-    for k in range(n - 1):
-        m = 2 * (n - k) + 1
-        total += (1 << (k + 1)) * (8 + 6 + 6 * (m - 2) + 8 * (m - 2) ** 2)
-    return total + (1 << n) * 34
+    """FLOPs the elimination tree executes per point: per node with m > 2 vertices left, the
+    pivot's reciprocal and the squared prefix (28), and for each of its two children m scaled
+    entries of its copy (10 each) and m^2 complex FMAs (8 each); per node with two vertices
+    left, its four configurations without division (118)."""
+    if n <= 1:
+        return 30 * n
+    total = (1 << (n - 2)) * 118
+    for m in range(3, n + 1):
+        total += (1 << (n - m)) * (28 + 2 * (10 * m + 8 * m * m))
+    return total
 
 
 class ClockSampler:

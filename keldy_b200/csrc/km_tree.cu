@@ -26,6 +26,10 @@
 // of wick_tree.cu: 256 >> m nodes of level m per warp, from m = 8 (or the order) to m = 3 (one per
 // lane), the last three vertices forward and backward in registers. All levels' nodes stay in
 // shared memory for the way back.
+//
+// Bound: latency, at 8 warps per SM (255 registers; the nodes kept for the way back fill the shared
+// memory). 2^20 points of order 8 8.8 ms (69 for the tree that it replaced), of order 5 1.5 (9.8);
+// of 65,536 points of order 8 (0.67 ms) ncu shows the FP64 pipe 27 % busy, shared memory 52 %.
 #include "kb_wick.cuh"
 
 namespace kb {

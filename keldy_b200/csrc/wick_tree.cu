@@ -31,9 +31,11 @@
 // of a node splitting its children; the last five vertices run in registers. Orders above 8
 // walk the levels above 9 depth first. Warps never wait for each other: no CTA barrier.
 //
-// Bound: latency. Order 8 (2^20 points): 3.3 ms, FP64 pipe 42 % busy, 1,590 instructions per point,
-// of them 800 FP64, shared memory 50 %; the stalls are fixed latencies of dependent FP64
-// instructions and shared-memory loads at 12 warps per SM. Splitting a level's nodes over fewer
+// Bound: latency. Order 8 (2^20 points): 3.15 ms (13.1 for the elimination in the given order, one
+// CTA per sub-batch of points). Of 65,536 points (0.37 ms) ncu shows the FP64 pipe 39 % busy, 1,330
+// instructions per point, shared memory 44 %; the stalls are shared-memory loads (2.2 cycles per
+// issued instruction) and fixed latencies of dependent FP64 instructions (1.8) at 12 warps per SM.
+// Measured when order 8 took 3.6 to 3.8 ms: splitting a level's nodes over fewer
 // lanes with more registers (512 >> m nodes, 255 registers, 8 warps) took 4.6 ms, 15 warps at
 // 128 registers 4.8 (spills), an elimination of both vertices 8 and 7 per step 4.1.
 #include <cuda_runtime.h>
