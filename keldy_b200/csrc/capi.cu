@@ -815,10 +815,11 @@ static ItemDev make_item(const kb_model *m, const kb_integrand *f, int order) {
 // order 8) while the item would have fewer than eight chunks per resident tree warp (at most
 // `limit`), so that the last chunks of a large item leave no warp idle for long: 2^18 points of
 // order 7 in 2,048 chunks of 128 on 1,776 warps were two rounds for 1.15. A smaller group costs:
-// with 8 points per chunk instead of 32, order 8 takes 26 %, order 6 48 % and order 2 three times
+// with 8 points per chunk instead of 32, order 8 takes 18 %, order 6 41 % longer and order 2 2.7 times
 // as long, so below a full group (down to 8 points, 4 from order 6 on, 1 from order 10 on) only
-// while the item would have fewer chunks than an eighth of the warps. It depends on the item
-// alone: a batch adds each item's points in the order of a call of its own.
+// while the item would have fewer chunks than an eighth of the warps (16 items of 4,001 points of
+// order 6 in one call: 139 us; with a quarter of the warps 154, with a sixteenth 164). It depends on
+// the item alone: a batch adds each item's points in the order of a call of its own.
 static int item_chunk(const kb_context *ctx, int order, int64_t n, int most, int64_t limit) {
   int c = most;
   const int64_t warps = (int64_t)ctx->sm_count * ctx->ctas_per_sm * TREE_WARPS;

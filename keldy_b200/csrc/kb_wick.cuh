@@ -52,8 +52,9 @@ __device__ __forceinline__ double2 pivot_rcp(double2 a) {
 }
 
 // The latency of a small call is a chain of round trips to the L2 (300 to 700 cycles each): what
-// follows keeps their number down. 1,000 points of order 2: the kernel took 18,900 cycles, 9,400 of
-// them in the item's search, constants and set-up.
+// follows keeps their number down. 1,000 points of order 2: the kernel took 18,900 cycles, 11,000 of
+// them in the item's search, constants and set-up (now 8,600; the kernel 16 -> 13 us between
+// events).
 
 // The warps take their first chunk by their place (first warps of all CTAs, then second ones) and
 // later ones from the counter, each one chunk ahead of its use. (As plain PTX: atomicAdd's
