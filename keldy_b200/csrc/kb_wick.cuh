@@ -224,7 +224,7 @@ __device__ __noinline__ GroupSetup setup_group(int mode, const double *in, const
   }
   jac *= cj;
   bool dom = it.f.A.spin == it.f.B.spin, sorted = true;
-  if (mine) {
+  if (mine && N > 0) { // (order 0 has no coordinates: u holds what an earlier kernel left there)
     double before = u[lane];
     if (keep && before < 0.0) dom = false;
     for (int j = 1; j < N; ++j) {

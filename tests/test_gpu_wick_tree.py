@@ -58,3 +58,20 @@ def test_chunk_sizes(ctx, oracle, golden, chunk):
             assert abs(s - w) <= 1e-12 * sc, (n, abs(s - w) / sc)
     finally:
         ctx.set_launch(-1, *before)
+
+
+def test_order_0_after_other_kernels(ctx, oracle, golden):
+    """Order 0 is g0(A, B) at every point, whatever the kernels before left in shared memory: the
+    kernel method's nodes, or times below zero (more chunks than resident warps, full groups)."""
+    gm, om = _models(ctx, oracle, golden)
+    rng = np.random.default_rng(9)
+    none = np.zeros((1 << 17, 0))
+    A, B = ENDS[0]
+    want = oracle.integrand(om, A, B, none[:1])[0][0]
+    before = [lambda n=n: gm.integrand_kernel(A, rng.random((8192, n)) * 10.0) for n in (1, 3, 6, 8)]
+    before += [lambda n=n: gm.integrand(A, B, -3.0 * rng.random((1 << 16, n)), keep_u_hypercube=False) for n in (1, 5, 8)]
+    for fill in before:
+        for call in (lambda: gm.integrand(A, B, none), lambda: gm.evaluate_warped(A, B, [], none)[::2]):
+            fill()
+            v, d = call()
+            assert np.all(d == 1) and np.all(np.abs(v - want) <= 1e-12 * abs(want))
