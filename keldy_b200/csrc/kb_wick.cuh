@@ -269,15 +269,17 @@ __device__ __forceinline__ double mesh_position(double dx, double delta, double 
   return fma(fma(-q, delta, dx), rdelta, q);
 }
 
-// Whether every lookup of a point (sorted times, stride st) lies inside the tabulated window. The
-// mesh position grows with the time difference, so the extreme differences decide.
+// Whether every lookup of a point (sorted times, stride st) lies inside the tabulated window, by
+// interp_index's rule: positions whose whole part is 0 .. npts - 1 (2 t_max / delta itself may round
+// above npts - 1). The mesh position grows with the time difference, so the extreme differences
+// decide.
 __device__ __forceinline__ bool in_window(const ItemDev &it, int N, const double *u, int st, double rdelta) {
   const ModelDev &m = it.model;
   const int spin = it.f.A.spin;
   const double hi = u[0], lo = u[(N - 1) * st];
   auto inside = [&](double x) {
     const double a = mesh_position(__dsub_rn(x, m.xmin), m.delta, rdelta);
-    return a >= 0.0 && a <= (double)(m.npts - 1);
+    return a >= 0.0 && a < (double)m.npts;
   };
   bool ok = true;
   for (int j = 0; j < N; ++j) ok = ok && u[j * st] == u[j * st];

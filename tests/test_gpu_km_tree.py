@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from keldy_b200 import capi
+from tests.test_gpu_wick_tree import window_models
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +47,20 @@ def test_guarded_points_among_others(ctx, oracle, n):
         ws, onp, ond, sc, ob, oc, od = oracle.integrate_kernel(oracle.model(10.0, *m), X, chain, n, 151, 7, 1.0, 9.0, seed=4)
         assert (npt, nd, drop) == (onp, ond, od) and np.array_equal(cnt, oc)
         assert np.abs(bins - ob).max() <= 1e-12 * sc and abs(s - ws) <= 1e-12 * sc
+
+
+@pytest.mark.parametrize("interp", [1, 3])
+@pytest.mark.parametrize("tmax,mesh", [(9.0, 1001), (11.0, 2001), (10.0, 2001)])
+def test_window_upper_end(ctx, oracle, tmax, mesh, interp):
+    """Vertices at 0 and t_max, X at t_max: 2 t_max / delta may round above the last mesh point's number."""
+    gm, om, _ = window_models(ctx, oracle, tmax, mesh, interp)
+    rng = np.random.default_rng(4)
+    for n in (1, 2, 4, 7, 9):
+        t = rng.random((3, n)) * tmax
+        t[0, 0], t[1, n - 1] = 0.0, tmax
+        t[2, [0, n - 1]] = 0.0, tmax if n > 1 else 0.0
+        for X in ((tmax, 0, 0, 0, 0), (tmax, 0, 1, 0, 0)):
+            got, dom = gm.integrand_kernel(X, t)
+            want, odom, sc = oracle.integrand_kernel(om, X, t)
+            assert np.array_equal(dom, odom)
+            assert np.all(np.abs(got - want).max(axis=(1, 2)) <= 1e-12 * np.maximum(sc, 1e-300)), n

@@ -75,3 +75,43 @@ def test_order_0_after_other_kernels(ctx, oracle, golden):
             fill()
             v, d = call()
             assert np.all(d == 1) and np.all(np.abs(v - want) <= 1e-12 * abs(want))
+
+
+def window_models(ctx, oracle, tmax, mesh, interp):
+    t = np.linspace(-tmax, tmax, mesh)
+    le = 0.5j * np.exp(-np.abs(t)) + 0.1 * np.sin(t) * np.exp(-np.abs(t))
+    tables = le, -np.conj(le[::-1])
+    gm, om = ctx.model(tmax, *tables), oracle.model(tmax, *tables, interp=interp)
+    gm.set_interpolation(interp)
+    return gm, om, 2.0 * tmax / (mesh - 1)
+
+
+@pytest.mark.parametrize("interp", [1, 3])
+@pytest.mark.parametrize("tmax,mesh", [(9.0, 1001), (11.0, 2001), (10.0, 2001), (14.0, 25001)])
+def test_window_upper_end(ctx, oracle, tmax, mesh, interp):
+    """Time differences of t_max, where 2 t_max / delta may round above the last mesh point's number
+    (not at t_max = 10), and beyond it by less than a mesh step: the window is floor(position) <=
+    npts - 1 for the tree, the pivoted LU and the oracle alike."""
+    gm, om, delta = window_models(ctx, oracle, tmax, mesh, interp)
+    rng = np.random.default_rng(3)
+    for n in (1, 2, 4, 7, 9):
+        t = rng.random((5, n)) * tmax
+        t[0, 0], t[1, n - 1] = 0.0, tmax
+        t[2, [0, n - 1]] = 0.0, tmax if n > 1 else 0.0
+        for A, B in (((tmax, 0, 0, 0, 0), (tmax, 0, 1, 0, 0)), ((tmax, 0, 1, 0, 0), (0.0, 0, 0, 0, 0))):
+            w, dw, sc = oracle.integrand(om, A, B, t)
+            for algo in (capi.ALGO_TREE, capi.ALGO_DIRECT):
+                v, d = gm.integrand(A, B, t, algo=algo)
+                assert np.array_equal(d, dw) and np.all(np.abs(v - w) <= 1e-12 * sc), (n, algo)
+        A, B = (tmax, 0, 0, 0, 0), (0.5 * tmax, 0, 1, 0, 0)
+        t = rng.random((5, n)) * 0.9 * tmax
+        t[1, 0], t[3, n - 1] = -0.4 * delta, -0.7 * delta
+        w, dw, sc = oracle.integrand(om, A, B, t, keep_u_hypercube=False)
+        for algo in (capi.ALGO_TREE, capi.ALGO_DIRECT):
+            v, d = gm.integrand(A, B, t, algo=algo, keep_u_hypercube=False)
+            assert np.array_equal(d, dw) and np.all(np.abs(v - w) <= 1e-12 * sc), (n, algo)
+            t[1, 0] = -1.2 * delta
+            with pytest.raises(capi.KbError) as e:
+                gm.integrand(A, B, t, algo=algo, keep_u_hypercube=False)
+            assert e.value.code == capi.KB_E_RANGE
+            t[1, 0] = -0.4 * delta
