@@ -512,8 +512,8 @@ __device__ __forceinline__ unsigned km_passes(const Launch &L, KmShared &T, int 
       const int ee = have ? e : 0, p = ee / n2, q = ee - p * n2, i = q >> 1; // idle lanes: the first
       const bool ok = have && ((good >> p) & 1u);
       const double j = T.jac[s0 + p], t = T.u[((i + 1) << lgp) + s0 + p];
-      double2 v = ok ? out[ee] : c2(0.0, 0.0);
-      v = c2(v.x * j, v.y * j);
+      double2 v = c2(0.0, 0.0); // (whatever the Jacobian of a point that is not evaluated)
+      if (ok) v = c2(out[ee].x * j, out[ee].y * j);
       if (eval) {
         if (have && !((guarded >> (s0 + p)) & 1u))
           L.out_kvals[(first + s0 + p) * n2 + 2 * T.place[(i << lgp) + s0 + p] + (q & 1)] = v;

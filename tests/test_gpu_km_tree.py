@@ -64,3 +64,16 @@ def test_window_upper_end(ctx, oracle, tmax, mesh, interp):
             want, odom, sc = oracle.integrand_kernel(om, X, t)
             assert np.array_equal(dom, odom)
             assert np.all(np.abs(got - want).max(axis=(1, 2)) <= 1e-12 * np.maximum(sc, 1e-300)), n
+
+
+@pytest.mark.parametrize("n", [1, 3, 6, 9])
+def test_points_outside_with_any_jacobian(ctx, golden, n):
+    """Points outside the domain add nothing, whatever their Jacobian (exp(u_max / w) overflows here, the
+    times are -infinity)."""
+    gm = ctx.model(10.0, golden["table_beta20_lesser"], golden["table_beta20_greater"])
+    item = dict(model=gm, rng=ctx.sobol(n), chain=[(capi.WARPER_EXPONENTIAL, 10.0, 0.01)], A=(10.0, 0, 0, 0, 0), order=n,
+                k_first=1, n_points=100)
+    (s, npt, nd, bins, cnt, drop), = capi.integrate_kernel(ctx, [item], 7, 1.0, 9.0)
+    assert (s, npt, nd, drop) == (0, 100, 0, 0) and not bins.any() and not cnt.any()
+    (s, npt, nd), = [r[:3] for r in capi.integrate_kernel_single_omega(ctx, [item], 0.3)]
+    assert (s, npt, nd) == (0, 100, 0)
