@@ -203,10 +203,11 @@ __device__ __noinline__ GroupSetup setup_group(int mode, const double *in, const
         x = t;
       } else if (wd.kind == KB_WARPER_EXPONENTIAL) {
         // u = u_max - w log(1 + c0 l), so 1 / f1(u) = c1 exp(u / w) = c1 (1 + c0) / (1 + c0 l) without
-        // the exponential (and without the rounding of u in its argument)
+        // the exponential (and without the rounding of u in its argument); c0 = exp(u_max / w) - 1
+        // overflows from u_max = 710 w on: then u = -infinity, 1 / f1 = 0
         const double a = wd.c[0] * x;
         x = wd.u_max - wd.w * log1p(a);
-        f = wd.c[1] * ((1.0 + wd.c[0]) / (1.0 + a));
+        f = isinf(wd.c[0]) ? 1.0 / warper_f1(wd, x) : wd.c[1] * ((1.0 + wd.c[0]) / (1.0 + a));
       } else {
         const double t = warper_Finv(wd, x);
         x = t;

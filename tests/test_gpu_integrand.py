@@ -240,3 +240,20 @@ def test_empty_and_ragged_inputs(ctx, golden):
             assert res[0] == 0 and res[1] == 0
     with pytest.raises(capi.KbError):
         capi.integrate(ctx, [dict(items[1], order=17, rng=ctx.sobol(17))])
+
+
+@pytest.mark.parametrize("w", [0.01, 0.0135, 0.02, 0.1])
+def test_exponential_warper_of_a_short_scale(ctx, oracle, golden, w):
+    """exp(u_max / w) overflows at the first two: every time is -infinity, values and Jacobians are 0.
+    The Jacobian's exponent u / w reaches 500, so its relative error n * 500 * 2^-53 < 1e-12."""
+    le, gr = golden["table_beta20_lesser"], golden["table_beta20_greater"]
+    gm, om = ctx.model(10.0, le, gr), oracle.model(10.0, le, gr)
+    A, B = EXTERNALS[0][1], EXTERNALS[0][2]
+    chain = [(capi.WARPER_EXPONENTIAL, 10.0, w)]
+    li = np.random.default_rng(2).random((40, 3))
+    for algo in (capi.ALGO_TREE, capi.ALGO_DIRECT):
+        v, j, d = gm.evaluate_warped(A, B, chain, li, algo=algo)
+        wv, wj, wd, sc = oracle.evaluate_warped(om, A, B, chain, li)
+        np.testing.assert_array_equal(d, wd)
+        np.testing.assert_allclose(j, wj, rtol=1e-12)
+        assert np.all(np.abs(v - wv) <= 1e-12 * sc)
