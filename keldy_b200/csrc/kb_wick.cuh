@@ -11,10 +11,17 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-// What an entry's value is made of, by its kind: the table, and the copies as a word: the high word
-// of delta's sign (+1, -1: forward minus backward copy is g^> - g^< or the opposite; 0: both copies
-// are one function), bit 0: the backward copy is g^>, bit 1: there is no table. `alt`: for a
-// vertex on the other side of the external time.
+// An entry in the column of its earlier vertex is g^> on that vertex's forward copy and g^< on the
+// backward one, an entry in its row the opposite. A node keeps ONE function S of every entry, the same
+// for the whole matrix (`base`), and delta = the other one - S: one copy of a vertex takes delta in its
+// column and not in its row (copy 0 of the trees: forward where S is g^<), the other in its row and not
+// in its column. The base is the function that is smaller at equal times. The other way round (or with
+// one copy as the base of rows and columns alike) S + delta of a nearly empty or full level cancels:
+// with |g^<| = 1e-3 |g^>| three digits were lost.
+//
+// What an entry's value is made of, by its kind: the table, and the functions as a word: the high word
+// of delta's sign (+1, -1: delta is g^> - g^< or the opposite; 0: both copies are one function), bit 0:
+// S is g^>, bit 1: there is no table. `alt`: for a vertex on the other side of the external time.
 struct EntryKind {
   const double2 *tab;
   unsigned w, alt;
@@ -29,12 +36,13 @@ struct ItemConst {
   const unsigned long long *lookup;
   int last; // first mesh point of the last interval
   int cubic;
+  int greater; // the base is g^>: the trees' copy 0 is the backward one, their sums have the sign (-1)^order
 };
 
 __device__ __forceinline__ double2 cfma(double2 c, double2 a, double2 b) {
   return c2(fma(a.x, b.x, fma(-a.y, b.y, c.x)), fma(a.x, b.y, fma(a.y, b.x, c.y)));
 }
-// s + f d, f = 1 (the forward copy) or 0
+// s + f d, f = 1 (the copy that takes the difference) or 0
 __device__ __forceinline__ double2 copyof(double2 s, double2 d, double f) { return c2(fma(d.x, f, s.x), fma(d.y, f, s.y)); }
 
 // 1 / a for a pivot: the squared modulus' reciprocal by one third-order Newton-Raphson (Householder)
@@ -298,17 +306,16 @@ __device__ __forceinline__ void fill_item(ItemConst &K, const ItemDev &it, doubl
   if (lane >= 4) return;
   const ModelDev &m = it.model;
   const int spin = it.f.A.spin;
-  // A later than the vertex (or at its time): forward copy g^>, backward g^<; earlier: A's branch
-  // decides. B likewise; of two vertices the earlier one's index.
-  constexpr unsigned GREATER = 0x3FF00000u, LESSER = 0xBFF00001u;
+  double2 gl, gg;
+  int b0 = 0;
+  g0_pair(m, m.tab[spin][0][0], 0.0, gl, gg, &b0);
+  const bool greater = cabs1(gg) < cabs1(gl);
+  // A earlier than the vertex: A's branch decides; B likewise; of two vertices the earlier one's index.
   const double2 *tab = m.tab[spin][lane == 2 ? it.f.A.orbital : 0][lane == 3 ? it.f.B.orbital : 0];
-  const unsigned w = (lane & 1) ? LESSER : GREATER, none = tab ? 0u : 2u;
+  const unsigned w = greater ? 0xBFF00001u : 0x3FF00000u, none = tab ? 0u : 2u;
   const unsigned alt = lane == 2 ? (it.f.A.k_idx ? 1u : 0u) : lane == 3 ? (it.f.B.k_idx ? 0u : 1u) : w;
   K.kind[lane] = EntryKind{tab ? tab : no_table, w | none, alt | none};
   if (lane) return;
-  double2 gl, gg;
-  int b0 = 0;
-  g0_pair(m, tab, 0.0, gl, gg, &b0);
   K.eq = c2(gl.x, gl.y - m.alpha);
   K.xmin = m.xmin;
   K.delta = m.delta;
@@ -317,11 +324,11 @@ __device__ __forceinline__ void fill_item(ItemConst &K, const ItemDev &it, doubl
   K.lookup = lookup;
   K.last = m.npts - 2;
   K.cubic = m.interp == 3;
+  K.greater = greater;
 }
 
-// The first `total` entries of a pass's lookup list: S = the copy of Keldysh index 1 (backward) of
-// an entry's earlier vertex, delta = forward copy - S; u: the group's times from the pass's
-// first column. Each entry
+// The first `total` entries of a pass's lookup list: S and delta (EntryKind); u: the group's times
+// from the pass's first column. Each entry
 // is one lookup of g^< and g^> at one time difference; each lane starts GK of them, without a
 // branch between them, before it uses the first, so that their L2 round trips overlap. The
 // gathers do not allocate in the little L1 that shared memory leaves, which then holds the

@@ -10,8 +10,8 @@
 // with respect to r's 2n entries (one per vertex and copy), so one reverse pass over the tree of the
 // direct integrand (wick_tree.cu, whose facts about the vertex matrix hold here) gives them all:
 //
-// * Forward: a node with m vertices left is V's Schur complement S (m x m, the backward copies),
-//   the columns C (the entries to X, copies as S's columns) and E (the unit vector e_q of the
+// * Forward: a node with m vertices left is V's Schur complement S (m x m, one function of every
+//   entry: EntryKind), the columns C (the entries to X, copies as S's rows) and E (the unit vector e_q of the
 //   zeroed vertex q), and the row Q = d e_q^T (d = the zeroed diagonal entry) with its two
 //   corners: by Sherman-Morrison det(W) W^-1 c = det(V) [(1 - d z_q) y + d y_q z], y = V^-1 c,
 //   z = V^-1 e_q, and the corners hold -d y_q and -d z_q. The row r itself is never formed.
@@ -171,7 +171,7 @@ __device__ __forceinline__ void km_level(double2 *buf, const double2 *dl, const 
   for (int q = 0; q < COLS; ++q) {
     const int c = min(c0 + q, m), src = c < m - 1 ? c : c + 1;
     const double2 d = c < m - 1 ? dr[c] : dlC[m - 1];
-    r[q] = copyof(S[m * W + src], d, c == m ? 0.0 : f);
+    r[q] = copyof(S[m * W + src], d, c == m ? 0.0 : 1.0 - f);
   }
 #pragma unroll
   for (int k = 0; k < ROWS; ++k) {
@@ -186,30 +186,31 @@ __device__ __forceinline__ void km_level(double2 *buf, const double2 *dl, const 
 }
 
 // The last two vertices of a node T (rows Q, 1, 2; columns 1, 2, C, E), signed D^2 = D2: adds its
-// terms to o (sums (1, f), (1, b), (2, f), (2, b)) and its h_1, h_2, g to h. With vertex 1 left
-// alone, p, C, E, Q, corners kc, ke: t_1^a = -D^2 p ((1 + ke) C^a - kc E) without a division, and
-// h_1 = -D^2 p (1 + ke) dC_1, g = D^2 Q dC_1 (times the squared pivot p2's share of D^2).
+// terms to o (sums (1, 0), (1, 1), (2, 0), (2, 1)) and its h_1, h_2, g to h. With vertex 1 left
+// alone, p, C, E, Q, corners kc, ke: t_1^a = -+D^2 p ((1 + ke) C^a - kc E) without a division
+// (C^1 = C^0 + dC_1), and h_1 = D^2 p (1 + ke) dC_1, g = -D^2 Q dC_1 (times the squared pivot p2's
+// share of D^2).
 __device__ __forceinline__ void km_leaf2(const double2 (&T)[12], double2 D2, double2 d12, double2 d21, double2 dC1,
                                          double2 dC2, double2 *o, double2 *h, double floor_, bool &guard) {
   const double2 p2 = T[9], ip = pivot_rcp(p2);
   if (!(cabs1(p2) >= floor_)) guard = true;
   const double2 Dn = cmul(D2, cmul(p2, p2));
   const double2 q = cmul(T[1], ip), E2 = T[11];
-  const double2 ke = cfms(T[3], q, E2), one = c2(1.0 + ke.x, ke.y);
+  const double2 ke = cfms(T[3], q, E2), one = c2(1.0 + ke.x, ke.y), nC1 = c2(-dC1.x, -dC1.y);
 #pragma unroll
   for (int a = 0; a < 2; ++a) {
     const double sg = a ? -1.0 : 1.0;
-    const double2 r1 = a ? T[8] : cadd(T[8], d21), c = a ? T[5] : cadd(T[5], d12), Cc = a ? T[10] : cadd(T[10], dC2);
+    const double2 r1 = a ? cadd(T[8], d21) : T[8], c = a ? T[5] : cadd(T[5], d12), Cc = a ? cadd(T[10], dC2) : T[10];
     const double2 L = cmul(c, ip);
     const double2 p1 = cfms(T[4], L, r1), C1 = cfms(T[6], L, Cc), E1 = cfms(T[7], L, E2), Q1 = cfms(T[0], q, r1);
     const double2 kc = cfms(T[2], q, Cc);
     double2 w = cmul(Dn, p1);
     w = c2(sg * w.x, sg * w.y);
-    const double2 u = cmul(w, cfms(cmul(one, C1), kc, E1)), v = cmul(w, cmul(one, dC1)); // -t_1^b, -h_1
-    const double2 ge = cmul(cmul(c2(sg * Dn.x, sg * Dn.y), Q1), cmul(p1, dC1));
+    const double2 u = cmul(w, cfms(cmul(one, C1), kc, E1)), v = cmul(w, cmul(one, nC1)); // -t_1^0, -h_1
+    const double2 ge = cmul(cmul(c2(sg * Dn.x, sg * Dn.y), Q1), cmul(p1, nC1));
     const double2 t2 = cmul(ip, cfms(cmul(v, r1), ge, E2));
-    o[0] = c2(o[0].x - (u.x + v.x), o[0].y - (u.y + v.y));
-    o[1] = cadd(o[1], u);
+    o[0] = c2(o[0].x - u.x, o[0].y - u.y);
+    o[1] = c2(o[1].x + (u.x - v.x), o[1].y + (u.y - v.y));
     o[2 + a] = cadd(o[2 + a], t2);
     h[0] = c2(h[0].x - v.x, h[0].y - v.y);
     h[1] = cadd(h[1], t2);
@@ -226,7 +227,7 @@ __device__ __forceinline__ void km_back(const double2 *buf, const double2 *dl, i
   const int child = lane >> LC;
   const double2 *S = buf + km_base(m) + (child >> 1) * km_sz(m) + m * W;
   const double2 *dr = dl + (m - 1) * (m - 2) + m - 1;
-  const double f = (child & 1) ? 0.0 : 1.0;
+  const double f = (child & 1) ? 1.0 : 0.0; // (its row)
   const double2 ip = pivot_rcp(S[m - 1]);
   double2 s = cmul(g, S[m + 1]);
 #pragma unroll
@@ -294,7 +295,7 @@ __device__ __forceinline__ void km_subtree(KmShared &T, double2 *out, const doub
       double2 r[5];
 #pragma unroll
       for (int q = 0; q < 5; ++q)
-        r[q] = q == 4 ? S[4 * W + 5] : copyof(S[4 * W + (q < 3 ? q : 4)], q < 3 ? dr[q] : dlC[3], f);
+        r[q] = q == 4 ? S[4 * W + 5] : copyof(S[4 * W + (q < 3 ? q : 4)], q < 3 ? dr[q] : dlC[3], 1.0 - f);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const double2 Lf = cmul(i ? copyof(S[i * W + 3], dc[i - 1], f) : S[3], ip);
@@ -311,9 +312,9 @@ __device__ __forceinline__ void km_subtree(KmShared &T, double2 *out, const doub
     for (int a = 0; a < 2; ++a) {
       const double f = a ? 0.0 : 1.0, sg = a ? -1.0 : 1.0;
       double2 r[4], U[12];
-      r[0] = copyof(s[15], dl[4], f);
-      r[1] = copyof(s[16], dl[5], f);
-      r[2] = copyof(s[18], dlC[2], f);
+      r[0] = copyof(s[15], dl[4], 1.0 - f);
+      r[1] = copyof(s[16], dl[5], 1.0 - f);
+      r[2] = copyof(s[18], dlC[2], 1.0 - f);
       r[3] = E3;
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
@@ -342,11 +343,11 @@ __device__ __forceinline__ void km_subtree(KmShared &T, double2 *out, const doub
 #pragma unroll
     for (int e = 0; e < 12; ++e) U[e] = T.buf[lane * km_sz(2) + e];
     km_leaf2(U, D2, dl[0], dl[1], dlC[0], dlC[1], o, hh, floor_, guard);
-  } else { // order 1: t^a = -p C^a (its corners are 0)
+  } else { // order 1: t^a = -+p C^a (its corners are 0)
     const double2 *S = T.buf + lane * km_sz(1) + km_w(1);
-    const double2 b = cmul(S[0], S[1]), fw = cmul(S[0], cadd(S[1], dlC[0]));
-    o[0] = c2(-fw.x, -fw.y);
-    o[1] = b;
+    const double2 t0 = cmul(S[0], S[1]);
+    o[0] = c2(-t0.x, -t0.y);
+    o[1] = cmul(S[0], cadd(S[1], dlC[0]));
   }
   h[0] = hh[0];
   h[1] = hh[1];
@@ -403,7 +404,7 @@ __device__ __forceinline__ void km_step_down(const double2 *S, double2 *o, const
   D2n = cmul(D2, cmul(p, p));
   if (a) D2n = c2(-D2n.x, -D2n.y);
   const int c = min(lane & 15, m), src = c < m - 1 ? c : c + 1; // a column per lane, every other row
-  const double2 r = copyof(S[m * W + src], c < m - 1 ? dr[c] : dlC[m - 1], c == m ? 0.0 : f);
+  const double2 r = copyof(S[m * W + src], c < m - 1 ? dr[c] : dlC[m - 1], c == m ? 0.0 : 1.0 - f);
 #pragma unroll 5
   for (int i = lane >> 4; i < m; i += 2) {
     const double2 Lf = cmul(copyof(S[i * W + m - 1], dc[max(i, 1) - 1], i ? f : 0.0), ip);
@@ -437,7 +438,7 @@ __device__ __noinline__ void km_deep(KmShared &T, double2 *stack, const double2 
       double2 s = cmul(g, R[10]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        s = cfma(s, h[j], copyof(R[j], dr[j], a9 ? 0.0 : 1.0));
+        s = cfma(s, h[j], copyof(R[j], dr[j], a9 ? 1.0 : 0.0));
         H[j] = cadd(H[j], h[j]);
       }
       const double2 t = cmul(c2(-s.x, -s.y), ip);
@@ -450,7 +451,7 @@ __device__ __noinline__ void km_deep(KmShared &T, double2 *stack, const double2 
       const double2 *R = N10 + 10 * km_w(10), *dr = dl + 9 * 8 + 9;
       double2 s = cmul(G, R[11]);
 #pragma unroll
-      for (int j = 0; j < 9; ++j) s = cfma(s, H[j], copyof(R[j], dr[j], a10 ? 0.0 : 1.0));
+      for (int j = 0; j < 9; ++j) s = cfma(s, H[j], copyof(R[j], dr[j], a10 ? 1.0 : 0.0));
       if (lane == 0) T.out[18 + a10] = cmul(c2(-s.x, -s.y), pivot_rcp(R[9]));
       __syncwarp();
     }
@@ -468,6 +469,7 @@ __device__ __forceinline__ unsigned km_passes(const Launch &L, KmShared &T, int 
   const bool eval = L.mode != IN_SOBOL;
   const int nb = L.nbins * 2;
   const double floor_ = T.k.floor_;
+  const int flip = T.k.greater; // the trees' copy 0 is Keldysh index 1
   double2 *dl0 = T.buf + km_delta(N);
   const int dsz = km_delta_sz(N);
   double2 *root = N > 8 ? stack : T.buf + km_base(N);
@@ -509,14 +511,14 @@ __device__ __forceinline__ unsigned km_passes(const Launch &L, KmShared &T, int 
     for (int e0 = 0; e0 < np * n2; e0 += 32) {
       const int e = e0 + lane;
       const bool have = e < np * n2;
-      const int ee = have ? e : 0, p = ee / n2, q = ee - p * n2, i = q >> 1; // idle lanes: the first
+      const int ee = have ? e : 0, p = ee / n2, q = ee - p * n2, i = q >> 1, kk = (q & 1) ^ flip; // idle lanes: the first
       const bool ok = have && ((good >> p) & 1u);
-      const double j = T.jac[s0 + p], t = T.u[((i + 1) << lgp) + s0 + p];
+      const double j = (N & flip) ? -T.jac[s0 + p] : T.jac[s0 + p], t = T.u[((i + 1) << lgp) + s0 + p];
       double2 v = c2(0.0, 0.0); // (whatever the Jacobian of a point that is not evaluated)
       if (ok) v = c2(out[ee].x * j, out[ee].y * j);
       if (eval) {
         if (have && !((guarded >> (s0 + p)) & 1u))
-          L.out_kvals[(first + s0 + p) * n2 + 2 * T.place[(i << lgp) + s0 + p] + (q & 1)] = v;
+          L.out_kvals[(first + s0 + p) * n2 + 2 * T.place[(i << lgp) + s0 + p] + kk] = v;
         continue;
       }
       if (L.km_fourier) {
@@ -530,7 +532,7 @@ __device__ __forceinline__ unsigned km_passes(const Launch &L, KmShared &T, int 
         bin = t == L.bin_xmax ? L.nbins - 1 : min((int)((t - L.bin_xmin) / L.bin_size), L.nbins - 1);
       csum = cadd(csum, v);
       // each bin's lowest lane adds the lanes' terms in order
-      const unsigned same = __match_any_sync(FULL, ok && bin >= 0 ? 2 * bin + (q & 1) : -1 - lane);
+      const unsigned same = __match_any_sync(FULL, ok && bin >= 0 ? 2 * bin + kk : -1 - lane);
       double2 s = v;
       for (unsigned r = same & (same - 1u); __any_sync(FULL, r != 0u); r &= r - 1u) {
         const int from = r ? __ffs(r) - 1 : lane;
@@ -538,7 +540,7 @@ __device__ __forceinline__ unsigned km_passes(const Launch &L, KmShared &T, int 
         if (r) s = cadd(s, w);
       }
       if (ok && bin >= 0 && lane == __ffs(same) - 1) {
-        const size_t b = (size_t)c * nb + 2 * bin + (q & 1);
+        const size_t b = (size_t)c * nb + 2 * bin + kk;
         L.bin_sums[b] = cadd(L.bin_sums[b], s);
         L.bin_counts[b] += (unsigned)__popc(same) << (N - 1);
       }

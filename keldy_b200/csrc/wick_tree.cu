@@ -11,15 +11,15 @@
 //   on its vertex's index.
 // * Gaussian elimination of the vertices, earliest first, keeps that form: the correction
 //   c_i r_j / p holds the eliminated vertex's column and row, which depend on its index alone.
-//   So a node of the elimination tree with m vertices left is ONE (m+1) x (m+1) matrix S (the
-//   backward copies), both children of a node share its pivot p, and the difference of an
-//   entry's two copies is the same number at every node: S^f_ij = S_ij + delta_ij with delta
-//   fixed per point. (A node of both copies, as in an elimination in the given order, is
+//   So a node of the elimination tree with m vertices left is ONE (m+1) x (m+1) matrix S (of every
+//   entry the copy that starts as g^<, or of every entry g^>: EntryKind), both children of a node
+//   share its pivot p, and the difference of an entry's two copies is the same number at every
+//   node: S_ij + delta_ij with delta fixed per point. (A node of both copies, as in an elimination in the given order, is
 //   (2m+1)^2 entries and two pivots.)
 // * The last two vertices need no division. With X, Y the external entries of the latest
 //   vertex, its two configurations differ only in them, so the external corner and the
 //   square of the leaf's own terms cancel before anything is rounded:
-//     sum_{a1} = -D^2 p2 p1' (X_f Y_f - X_b Y_b)', and p2 times each factor is a polynomial
+//     sum_{a1} = -D^2 p2 p1' (X_0 Y_0 - X_1 Y_1)', and p2 times each factor is a polynomial
 //   of the 3 x 3 matrix's entries (leaf2).
 //
 // Cost: sum_m 2^(n-m) (m+1)^2 complex multiply-adds, ~15 * 2^n (the elimination in the given
@@ -155,7 +155,7 @@ __device__ __forceinline__ void build_roots(const ItemConst &K, int N, int np, c
 
 // Nodes of a level, and the lanes of a node, are numbered so that a point's nodes stay in its
 // own lanes: with m vertices left, node lane >> (m-3), whose low bit is the copy of vertex m+1
-// that led to it (1: backward).
+// that led to it (0: delta in its column, 1: delta in its row).
 
 // Level 8 (node S, 9 x 9) to level 7: half a row of its child per lane.
 __device__ __forceinline__ void level8(const double2 *S, double2 *buf, const double2 *dl, double2 D2, double2 *D2c,
@@ -170,7 +170,7 @@ __device__ __forceinline__ void level8(const double2 *S, double2 *buf, const dou
   const double2 Lf = cmul(copyof(S[i * W + 8], dc[i], f), ip);
   double2 *o = buf + node_base(7) + child * node_sz(7) + i * WC + j0;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) o[q] = cfms(S[i * W + j0 + q], Lf, copyof(S[8 * W + j0 + q], dr[j0 + q], f));
+  for (int q = 0; q < 4; ++q) o[q] = cfms(S[i * W + j0 + q], Lf, copyof(S[8 * W + j0 + q], dr[j0 + q], 1.0 - f));
 }
 
 // Level 7 to level 6: a row of its child per lane.
@@ -186,7 +186,7 @@ __device__ __forceinline__ void level7(double2 *buf, const double2 *dl, const do
     const double2 Lf = cmul(copyof(S[i * W + 7], dc[i], f), ip);
     double2 *o = buf + node_base(6) + child * node_sz(6) + i * WC;
 #pragma unroll
-    for (int j = 0; j < 7; ++j) o[j] = cfms(S[i * W + j], Lf, copyof(S[7 * W + j], dr[j], f));
+    for (int j = 0; j < 7; ++j) o[j] = cfms(S[i * W + j], Lf, copyof(S[7 * W + j], dr[j], 1.0 - f));
   } else {
     D2c[child] = cmul(D2p[child >> 1], cmul(p, p));
   }
@@ -205,7 +205,7 @@ __device__ __forceinline__ void level6(double2 *buf, const double2 *dl, const do
   if (l == 0) D2c[child] = cmul(D2p[child >> 1], cmul(p, p));
   double2 r[3];
 #pragma unroll
-  for (int j = 0; j < 3; ++j) r[j] = copyof(S[6 * W + j0 + j], dr[j0 + j], f);
+  for (int j = 0; j < 3; ++j) r[j] = copyof(S[6 * W + j0 + j], dr[j0 + j], 1.0 - f);
   double2 *o = buf + node_base(5) + child * node_sz(5) + i0 * WC + j0;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -217,37 +217,37 @@ __device__ __forceinline__ void level6(double2 *buf, const double2 *dl, const do
 
 // The last two vertices of a node T (3 x 3: external, latest vertex 1, vertex 2), all four
 // configurations. With c = (T02, T12), r = (T20, T21) of vertex 2's copy, after its elimination
-//   p2 p1' = T11 p2 - c1 r1 = q,  p2 (X_f Y_f - X_b Y_b) = p2 K - c0 r1 dY - c1 r0 dX,
-// (X, Y = T01, T10; dX, dY their differences; K = X dY + dX (Y + dY)), and the two leaves of
+//   p2 p1' = T11 p2 - c1 r1 = q,  p2 (X_0 Y_0 - X_1 Y_1) = p2 K + c0 r1 dY - c1 r0 dX,
+// (X, Y = T01, T10; X_0 = X + dX, Y_1 = Y + dY; K = dX Y - X dY), and the two leaves of
 // vertex 1 sum to -D^2 q times that: no division, the external corner drops out. Returns
-// q_b (...)_b - q_f (...)_f. d2: vertex 2's differences {c0, c1, r0, r1}; g2 = d2[0] dY,
+// q_1 (...)_1 - q_0 (...)_0. d2: vertex 2's differences {c0, c1, r0, r1}; g2 = d2[0] dY,
 // h2 = dX d2[2]. SCALE: also the sum of |term| of the four leaves, without the factor D^2.
 template <bool SCALE>
 __device__ __forceinline__ double2 leaf2(const double2 (&T)[9], double2 dX, double2 dY, const double2 (&d2)[4],
                                          double2 g2, double2 h2, double &scale, double floor_, bool &guard) {
-  const double2 K = cfma(cmul(T[1], dY), dX, cadd(T[3], dY));
+  const double2 K = cfms(cmul(dX, T[3]), T[1], dY);
   const double2 P = cmul(T[4], T[8]), Q = cmul(T[8], K);
   const double2 g = cmul(T[2], dY), h = cmul(dX, T[6]);
-  const double2 tb = cmul(cfms(P, T[5], T[7]), cfms(cfms(Q, g, T[7]), h, T[5]));
   const double2 c1 = cadd(T[5], d2[1]), r1 = cadd(T[7], d2[3]);
-  const double2 tf = cmul(cfms(P, c1, r1), cfms(cfms(Q, cadd(g, g2), r1), cadd(h, h2), c1));
+  const double2 t1 = cmul(cfms(P, T[5], r1), cfms(cfma(Q, g, r1), cadd(h, h2), T[5]));
+  const double2 t0 = cmul(cfms(P, c1, T[7]), cfms(cfma(Q, cadd(g, g2), T[7]), h, c1));
   if constexpr (SCALE) {
     if (!(cabs1(T[8]) >= floor_)) guard = true;
     const double2 ip = pivot_rcp(T[8]);
 #pragma unroll
     for (int a2 = 0; a2 < 2; ++a2) {
-      const double2 c0 = a2 ? T[2] : cadd(T[2], d2[0]), r0 = a2 ? T[6] : cadd(T[6], d2[2]);
-      const double2 k1 = a2 ? T[5] : c1, s1 = a2 ? T[7] : r1;
+      const double2 c0 = a2 ? T[2] : cadd(T[2], d2[0]), r0 = a2 ? cadd(T[6], d2[2]) : T[6];
+      const double2 k1 = a2 ? T[5] : c1, s1 = a2 ? r1 : T[7];
       const double2 q = cfms(P, k1, s1), sg = cfms(cmul(T[8], T[0]), c0, r0);
 #pragma unroll
       for (int a1 = 0; a1 < 2; ++a1) {
-        const double2 X = a1 ? T[1] : cadd(T[1], dX), Y = a1 ? T[3] : cadd(T[3], dY);
+        const double2 X = a1 ? T[1] : cadd(T[1], dX), Y = a1 ? cadd(T[3], dY) : T[3];
         const double2 xi = cfms(cmul(T[8], X), c0, s1), et = cfms(cmul(T[8], Y), k1, r0);
         scale += cabs(cmul(cmul(q, ip), cfms(cmul(q, sg), xi, et)));
       }
     }
   }
-  return c2(tb.x - tf.x, tb.y - tf.y);
+  return c2(t1.x - t0.x, t1.y - t0.y);
 }
 
 // The last three vertices of a node s (4 x 4, in registers), all eight configurations, times
@@ -267,7 +267,7 @@ __device__ __forceinline__ double2 leaf3(const double2 (&s)[16], const double2 *
   for (int a = 0; a < 2; ++a) {
     double2 r[3], T[9];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) r[j] = a ? s[12 + j] : cadd(s[12 + j], dl[9 + j]);
+    for (int j = 0; j < 3; ++j) r[j] = a ? cadd(s[12 + j], dl[9 + j]) : s[12 + j];
     T[0] = c2(0.0, 0.0);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -296,12 +296,12 @@ __device__ __forceinline__ double2 level5(double2 (&s)[16], const double2 *buf, 
   const double2 p5 = S[5 * W + 5], i5 = pivot_rcp(p5);
   double2 r5[5], r4[4];
 #pragma unroll
-  for (int j = 0; j < 5; ++j) r5[j] = copyof(S[5 * W + j], dl[25 + j], f5);
+  for (int j = 0; j < 5; ++j) r5[j] = copyof(S[5 * W + j], dl[25 + j], 1.0 - f5);
   const double2 L54 = cmul(copyof(S[4 * W + 5], dl[24], f5), i5);
   const double2 p4 = cfms(S[4 * W + 4], L54, r5[4]), i4 = pivot_rcp(p4);
   if (!(cabs1(p5) >= floor_) || !(cabs1(p4) >= floor_)) guard = true;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) r4[j] = copyof(cfms(S[4 * W + j], L54, r5[j]), dl[16 + j], f4);
+  for (int j = 0; j < 4; ++j) r4[j] = copyof(cfms(S[4 * W + j], L54, r5[j]), dl[16 + j], 1.0 - f4);
   s[0] = c2(0.0, 0.0);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -325,7 +325,7 @@ __device__ __forceinline__ double2 level4(double2 (&s)[16], const double2 *buf, 
   if (!(cabs1(p) >= floor_)) guard = true;
   double2 r[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) r[j] = copyof(S[20 + j], dl[16 + j], f);
+  for (int j = 0; j < 4; ++j) r[j] = copyof(S[20 + j], dl[16 + j], 1.0 - f);
   s[0] = c2(0.0, 0.0);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -381,7 +381,7 @@ __device__ __forceinline__ void step_down(const double2 *S, double2 *o, const do
   const double2 *dc = dl + m * (m - 1), *dr = dl + m * m;
   const double f = (PAIR ? half : a) ? 0.0 : 1.0;
   const int col = min(j, m - 1); // idle lanes repeat the last column's loads
-  const double2 r = copyof(S[m * W + col], dr[col], f);
+  const double2 r = copyof(S[m * W + col], dr[col], 1.0 - f);
   if (!(cabs1(p) >= floor_)) guard = true;
   const double2 ip = pivot_rcp(p);
   D2n = cmul(D2, cmul(p, p));
@@ -518,14 +518,13 @@ __device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int order
           if (!(cabs1(s[8]) >= floor_)) guard = true;
           v = leaf2<SCALE>(s, dl[0], dl[1], d2, cmul(d2[0], dl[1]), cmul(dl[0], d2[2]), scale, floor_, guard);
         }
-      } else if (lane < np) { // order 1: -p (X_f Y_f - X_b Y_b)
+      } else if (lane < np) { // order 1: -p (X_0 Y_0 - X_1 Y_1)
         const double2 *S = T.buf + lane * node_sz(1), *dl = dl0 + lane * dsz;
         const double2 dX = dl[0], dY = dl[1];
-        v = cmul(S[3], cfma(cmul(S[1], dY), dX, cadd(S[2], dY)));
-        v = c2(-v.x, -v.y);
+        v = cmul(S[3], cfms(cmul(S[1], dY), dX, S[2]));
         if (SCALE) {
-          const double2 xb = S[1], yb = S[2], xf = cadd(xb, dX), yf = cadd(yb, dY);
-          scale = cabs(cmul(S[3], cfms(cmul(S[3], S[0]), xf, yf))) + cabs(cmul(S[3], cfms(cmul(S[3], S[0]), xb, yb)));
+          const double2 X = S[1], Y = S[2], z = cmul(S[3], S[0]);
+          scale = cabs(cmul(S[3], cfms(z, cadd(X, dX), Y))) + cabs(cmul(S[3], cfms(z, X, cadd(Y, dY))));
         }
       }
       const unsigned gm = __ballot_sync(FULL, guard);
@@ -668,7 +667,8 @@ __global__ void __launch_bounds__(TREE_WARPS * 32, TREE_CTAS_PER_SM) tree_kernel
         if (SCALE) T.fscale[lane] = cabs(v);
       }
       __syncwarp();
-      const double2 fv = mine ? T.fval[lane] : c2(0.0, 0.0);
+      double2 fv = mine ? T.fval[lane] : c2(0.0, 0.0);
+      if (N & T.k.greater) fv = c2(-fv.x, -fv.y);
       const bool ok = mine && dom;
       const bool fb = ok && (((guarded >> lane) & 1u) || !isfinite(fv.x) || !isfinite(fv.y));
       if (EVAL) {

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from keldy_b200 import capi
-from tests.test_gpu_wick_tree import window_models
+from tests.test_gpu_wick_tree import one_sided_models, window_models
 
 pytestmark = pytest.mark.gpu
 
@@ -77,3 +77,15 @@ def test_points_outside_with_any_jacobian(ctx, golden, n):
     assert (s, npt, nd, drop) == (0, 100, 0, 0) and not bins.any() and not cnt.any()
     (s, npt, nd), = [r[:3] for r in capi.integrate_kernel_single_omega(ctx, [item], 0.3)]
     assert (s, npt, nd) == (0, 100, 0)
+
+
+@pytest.mark.parametrize("ratio,small", [(1e-1, "lesser"), (1e-1, "greater"), (1e-5, "lesser")])
+def test_nearly_empty_and_full_levels(ctx, oracle, ratio, small):
+    """(At a ratio of 1e-5 the other way the elimination without pivoting itself is off by 1e-12.)"""
+    gm, om = one_sided_models(ctx, oracle, ratio, small)
+    for n in (1, 2, 3, 4, 5, 6, 7, 8, 9):
+        t = np.random.default_rng(n).random((40 if n < 8 else 8, n)) * 10.0
+        X = (10.0, 0, 0, 0, 0) if n % 2 else (6.0, 0, 1, 0, 0)
+        got, dom = gm.integrand_kernel(X, t)
+        want, odom, sc = oracle.integrand_kernel(om, X, t)
+        assert np.array_equal(dom, odom) and np.all(np.abs(got - want).max(axis=(1, 2)) <= 1e-12 * sc), n

@@ -115,3 +115,25 @@ def test_window_upper_end(ctx, oracle, tmax, mesh, interp):
                 gm.integrand(A, B, t, algo=algo, keep_u_hypercube=False)
             assert e.value.code == capi.KB_E_RANGE
             t[1, 0] = -0.4 * delta
+
+
+def one_sided_models(ctx, oracle, ratio, small):
+    """A nearly empty (small: "lesser") or full level: one of g^<, g^> `ratio` times the other."""
+    t = np.linspace(-10, 10, 2001)
+    big, little = np.exp(-np.abs(t) * (1 + 0.3j * np.sign(t))), ratio * np.exp(-0.5 * np.abs(t)) * np.cos(t)
+    tables = (1j * little, -1j * big) if small == "lesser" else (1j * big, -1j * little)
+    return ctx.model(10.0, *tables), oracle.model(10.0, *tables)
+
+
+@pytest.mark.parametrize("small", ["lesser", "greater"])
+@pytest.mark.parametrize("ratio", [1e-1, 1e-3, 1e-5])
+def test_nearly_empty_and_full_levels(ctx, oracle, ratio, small):
+    """The small function's entries keep their digits beside the other's."""
+    gm, om = one_sided_models(ctx, oracle, ratio, small)
+    for n in (1, 2, 3, 4, 5, 6, 7, 8, 9):
+        t = np.random.default_rng(n).random((40 if n < 8 else 8, n)) * 10.0
+        for A, B in ENDS[:2]:
+            v, d, gsc = gm.integrand(A, B, t, algo=capi.ALGO_TREE, want_scale=True)
+            w, dw, sc = oracle.integrand(om, A, B, t)
+            assert np.array_equal(d, dw) and np.all(np.abs(v - w) <= 1e-12 * sc), n
+            np.testing.assert_allclose(gsc, sc, rtol=1e-9)
