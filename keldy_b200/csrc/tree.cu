@@ -11,6 +11,7 @@
 // (pivot = first maximum of |re|+|im|, as LAPACK's zgetf2). It serves models whose
 // spin-down tables differ from spin-up ones, points whose tree pivots fall below the
 // guard, and cross-checks.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdio.h>
 
@@ -50,38 +51,34 @@ __device__ __forceinline__ double spline_flow_point(const double *knots, int N, 
   return jac;
 }
 
-// Inputs of np points (thread p < np): vertex times into u[j*np+p], Jacobian and
-// domain flag. keep: drop points with a negative time (keep_u_hypercube).
-__device__ void load_points(const Launch &L, const ItemDev &it, int N, int np, long long gp0, double *u,
-                            double *jac_out, int *flag_out, bool keep) {
-  int p = threadIdx.x;
-  if (p >= np) return;
-  long long gp = gp0 + p;
-  double *x = u + p;
+// Inputs of point gp (by the calling thread): vertex times into x (stride st), Jacobian and domain
+// flag (0: inside). keep: drop points with a negative time (keep_u_hypercube).
+__device__ void load_point(const Launch &L, const ItemDev &it, int N, long long gp, double *x, int st, bool keep,
+                           double &jac_out, int &flag_out) {
   double jac = 1.0;
   if (L.mode == IN_SOBOL) {
     if (it.flow_x) { // Sobol point already mapped by the learned flow
-      for (int j = 0; j < N; ++j) x[j * np] = it.flow_x[gp * N + j];
+      for (int j = 0; j < N; ++j) x[j * st] = it.flow_x[gp * N + j];
       jac = it.flow_jac[gp];
     } else {
       uint32_t k = it.k_first + (uint32_t)gp;
-      for (int j = 0; j < N; ++j) x[j * np] = sobol_coord(it.rng, k, j);
-      if (it.spline_knots) jac = spline_flow_point(it.spline_knots, N, x, np);
-      if (it.ar_spline) jac = ar_spline_point(it.ar_spline, N, x, np);
+      for (int j = 0; j < N; ++j) x[j * st] = sobol_coord(it.rng, k, j);
+      if (it.spline_knots) jac = spline_flow_point(it.spline_knots, N, x, st);
+      if (it.ar_spline) jac = ar_spline_point(it.ar_spline, N, x, st);
     }
-    jac *= chain_reverse(it.chain, it.chain_len, 0, N, x, np);
+    jac *= chain_reverse(it.chain, it.chain_len, 0, N, x, st);
   } else {
     long long src = L.index ? (long long)L.index[gp] : gp;
-    for (int j = 0; j < N; ++j) x[j * np] = L.in[src * N + j];
-    if (L.mode == IN_LI) jac = chain_reverse(it.chain, it.chain_start, 0, N, x, np);
+    for (int j = 0; j < N; ++j) x[j * st] = L.in[src * N + j];
+    if (L.mode == IN_LI) jac = chain_reverse(it.chain, it.chain_start, 0, N, x, st);
   }
   int dom = 1;
   if (it.f.A.spin != it.f.B.spin) dom = 0;
   if (keep)
     for (int j = 0; j < N; ++j)
-      if (x[j * np] < 0.0) dom = 0;
-  jac_out[p] = jac;
-  flag_out[p] = dom ? 0 : 1;
+      if (x[j * st] < 0.0) dom = 0;
+  jac_out = jac;
+  flag_out = dom ? 0 : 1;
 }
 
 // Bin of the earliest vertex time (binner_t::in_bounds and coord2index, binner.hpp:163-176:
@@ -380,12 +377,6 @@ __device__ __forceinline__ void direct_point(DirectShared &D, const ItemDev &it,
   __syncthreads();
 }
 
-__device__ void direct_load_point(const Launch &L, const ItemDev &it, int N, long long gp, bool keep,
-                                  DirectShared &D) {
-  load_points(L, it, N, 1, gp, D.u, D.jac, D.flag, keep);
-  __syncthreads();
-}
-
 // Modes: IN_TIMES / IN_LI (every point, or the points of L.index), IN_SOBOL (per-chunk
 // partial sums, as the tree kernel).
 __global__ void __launch_bounds__(NT) direct_kernel(Launch L) {
@@ -416,7 +407,8 @@ __global__ void __launch_bounds__(NT) direct_kernel(Launch L) {
     }
     for (int p = 0; p < ccount; ++p) {
       long long gp = cfirst + p;
-      direct_load_point(L, it, N, gp, keep, D);
+      if (tid == 0) load_point(L, it, N, gp, D.u, 1, keep, D.jac[0], D.flag[0]);
+      __syncthreads();
       double2 f;
       double sc;
       direct_point(D, it, N, eval && L.out_scale != nullptr, f, sc, &s_bad);
@@ -481,53 +473,94 @@ __device__ __forceinline__ int next_guarded(const Launch &L, long long first, in
 }
 
 // Points the tree marked in a chunk's fb_mask, evaluated with keldy's algorithm and
-// added to that chunk's partial sum in point order.
-__global__ void __launch_bounds__(NT) fallback_kernel(Launch L) {
+// added to that chunk's partial sum in point order. A cluster of FB_CTAS blocks per chunk: block r
+// takes the guarded points r, r + FB_CTAS, ... of the chunk, sets them up at once (a thread per
+// point) and leaves their values in block 0's shared memory, which adds them in point order. Where
+// every point is guarded (a zero diagonal, alpha = Im g^<(0)) this pass is the call: 4,096
+// points of order 6 take 674 us, with a block per chunk and each point set up by itself 1,135, in
+// clusters of four blocks 677; 32,768 points 4.1 ms, in clusters of four 5.2.
+constexpr int FB_CTAS = 2;
+constexpr int FB_MINE = CHUNK_POINTS / FB_CTAS; // a block's points of a chunk, at most
+static_assert(NT == CHUNK_POINTS, "a thread per point of a chunk");
+// In the place of the other spin's matrix, which these points do not need (more shared memory would
+// leave the factorisations' local arrays little L1).
+struct GuardedShared {
+  double u[MAX_ORDER * FB_MINE], jac[FB_MINE]; // this block's points
+  int flag[FB_MINE];
+  // block 0: values, Jacobians and bins of the cluster's points; two sets, so that one barrier per
+  // chunk keeps the next chunk's values from those still being added
+  double2 f[2 * CHUNK_POINTS];
+  double j[2 * CHUNK_POINTS];
+  int b[2 * CHUNK_POINTS];
+};
+static_assert(sizeof(GuardedShared) <= sizeof(DirectShared::G2), "the other spin's matrix holds the points");
+__global__ void __launch_bounds__(NT, 4) __cluster_dims__(FB_CTAS, 1, 1) fallback_kernel(Launch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   DirectShared &D = *reinterpret_cast<DirectShared *>(smem_raw);
   __shared__ int s_bad;
-  const int tid = threadIdx.x;
-  if (tid == 0) s_bad = 0;
-  __syncthreads();
-  // block b takes chunks b, b + grid, ...; it looks at NT of them at once, as guarded points are
-  // rare (one by one, 8,192 chunks without any took 14 us)
   __shared__ unsigned s_found[NT / 32];
-  const long long step = gridDim.x;
-  int k = -1;
-  for (long long c0 = blockIdx.x; c0 < L.n_chunks;) {
-    k = next_guarded(L, c0, gridDim.x, k, s_found);
+  GuardedShared &S = *reinterpret_cast<GuardedShared *>(D.G2);
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int tid = threadIdx.x, rank = (int)cluster.block_rank();
+  GuardedShared &S0 = *cluster.map_shared_rank(&S, 0);
+  if (tid == 0) s_bad = 0;
+  cluster.sync(); // block 0 runs
+  // cluster b takes chunks b, b + clusters, ...; it looks at NT of them at once, as guarded points are
+  // rare (one by one, 8,192 chunks without any took 14 us)
+  const int step = gridDim.x / FB_CTAS;
+  int k = -1, set = 0;
+  for (long long c0 = blockIdx.x / FB_CTAS; c0 < L.n_chunks;) {
+    k = next_guarded(L, c0, step, k, s_found);
     if (k < 0) {
-      c0 += NT * step;
+      c0 += (long long)NT * step;
       continue;
     }
-    const int c = (int)(c0 + k * step);
-    ChunkPartial pr = L.partials[c];
+    const int c = (int)(c0 + (long long)k * step);
     const int item = find_item(L.chunk_offsets, L.n_items, c);
     const ItemDev &it = L.items[item];
+    const int N = it.order;
     const long long cfirst = (long long)(c - L.chunk_offsets[item]) * it.chunk_points;
-    for (int bit = 0; bit < it.chunk_points; ++bit) {
-      unsigned long long w = pr.fb_mask[bit >> 6];
-      if (!((w >> (bit & 63)) & 1ull)) continue;
-      direct_load_point(L, it, it.order, cfirst + bit, true, D);
+    const unsigned long long w0 = L.partials[c].fb_mask[0], w1 = L.partials[c].fb_mask[1], w = tid < 64 ? w0 : w1;
+    const int low = __popcll(w0), total = low + __popcll(w1);
+    const unsigned long long below = (1ull << (tid & 63)) - 1ull;
+    const int q = __popcll(w & below) + (tid >= 64 ? low : 0); // this thread's point among the guarded ones
+    __syncthreads();
+    if (((w >> (tid & 63)) & 1ull) && q % FB_CTAS == rank) {
+      const int p = q / FB_CTAS;
+      load_point(L, it, N, cfirst + tid, S.u + p, FB_MINE, true, S.jac[p], S.flag[p]);
+    }
+    __syncthreads();
+    for (int p = 0; p * FB_CTAS + rank < total; ++p) {
+      if (tid < N) D.u[tid] = S.u[tid * FB_MINE + p];
+      if (tid == 0) D.flag[0] = S.flag[p];
+      __syncthreads();
       double2 f;
       double sc;
-      direct_point(D, it, it.order, false, f, sc, &s_bad);
+      direct_point(D, it, N, false, f, sc, &s_bad);
       if (tid == 0) {
-        f = apply_cutoff(f, it.f.cutoff);
-        pr.sum_re += f.x * D.jac[0];
-        pr.sum_im += f.y * D.jac[0];
-        if (L.nbins) { // counted by the tree kernel; the value is added here
-          const int bin = time_bin(L, D.u, 1, it.order);
-          if (bin >= 0) {
-            double2 &bs = L.bin_sums[(size_t)c * L.nbins + bin];
-            bs = c2(bs.x + f.x * D.jac[0], bs.y + f.y * D.jac[0]);
-          }
-        }
+        const int o = set * CHUNK_POINTS + p * FB_CTAS + rank;
+        S0.f[o] = apply_cutoff(f, it.f.cutoff);
+        S0.j[o] = S.jac[p];
+        if (L.nbins) S0.b[o] = time_bin(L, D.u, 1, N);
       }
       __syncthreads();
     }
-    if (tid == 0) L.partials[c] = pr;
-    __syncthreads();
+    cluster.sync();
+    if (rank == 0 && tid == 0) {
+      double2 sum = c2(L.partials[c].sum_re, L.partials[c].sum_im);
+      for (int o = set * CHUNK_POINTS, e = o + total; o < e; ++o) {
+        const double2 f = S.f[o];
+        const double j = S.j[o];
+        sum = c2(fma(f.x, j, sum.x), fma(f.y, j, sum.y)); // (explicit: with and without bins the same sums)
+        if (L.nbins && S.b[o] >= 0) { // counted by the tree kernel; the value is added here
+          double2 &bs = L.bin_sums[(size_t)c * L.nbins + S.b[o]];
+          bs = c2(fma(f.x, j, bs.x), fma(f.y, j, bs.y));
+        }
+      }
+      L.partials[c].sum_re = sum.x;
+      L.partials[c].sum_im = sum.y;
+    }
+    set ^= 1;
   }
   if (tid == 0 && s_bad) atomicOr(L.err, 1);
 }
@@ -758,7 +791,7 @@ __global__ void __launch_bounds__(KM_THREADS) km_fallback_kernel(Launch L) {
     for (int bit = 0; bit < it.chunk_points; ++bit) {
       if (!((pr.fb_mask[bit >> 6] >> (bit & 63)) & 1ull)) continue;
       __syncthreads();
-      load_points(L, it, N, 1, cfirst + bit, K.u, K.jac, K.flag, keep);
+      if (tid == 0) load_point(L, it, N, cfirst + bit, K.u, 1, keep, K.jac[0], K.flag[0]);
       __syncthreads();
       const double2 s = kernel_point(K, it, N, &s_bad);
       if (tid < n2) K.S[tid] = s;
@@ -879,7 +912,7 @@ cudaError_t launch_direct(const Launch &L, int grid, cudaStream_t st) {
 }
 
 cudaError_t launch_fallback(const Launch &L, int grid, cudaStream_t st) {
-  fallback_kernel<<<grid, NT, direct_smem_bytes(), st>>>(L);
+  fallback_kernel<<<(grid + FB_CTAS - 1) / FB_CTAS * FB_CTAS, NT, direct_smem_bytes(), st>>>(L);
   return cudaGetLastError();
 }
 

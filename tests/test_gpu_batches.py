@@ -63,3 +63,23 @@ def test_groups_of_several_quads(ctx, oracle, order):
     w, onp, ond, sc = oracle.integrate(oracle.model(10.0, *_tables("plain")), A, B, EXPONENTIAL, order, npts, seed=5)
     assert (npt, nd, nfb) == (onp, ond, 0) and nd > npts // 2
     assert abs(s - w) <= 1e-12 * sc
+
+
+@pytest.mark.parametrize("chunk", [1, 5, 33, 64, 128])
+@pytest.mark.parametrize("order,npts", [(2, 1), (2, 6), (3, 131), (5, 300), (7, 66)])
+def test_guarded_points_of_a_chunk(ctx, oracle, order, npts, chunk):
+    """The pivoted-LU pass over chunks with one, some and all points guarded (those outside the domain
+    are not), sums and bins; sums of a call and of the allocation-free call are the same."""
+    gm, om = ctx.model(10.0, *_tables("guarded")), oracle.model(10.0, *_tables("guarded"))
+    before = ctx.get_launch(order)
+    try:
+        ctx.set_launch(-1, chunk)
+        for chain in (INVERSE, EXPONENTIAL):
+            item = _item(gm, ctx.sobol(order), order, npts, 4, chain)
+            (s, npt, nd, nfb, bins, counts, dropped), = capi.integrate_binned(ctx, [item], 9, 0.5, 9.0)
+            w, onp, ond, sc, ob, oc, od = oracle.integrate_binned(om, A, B, chain, order, npts, 9, 0.5, 9.0, seed=3)
+            assert (npt, nd, nfb, dropped) == (onp, ond, ond, od) and np.array_equal(counts, oc)
+            assert abs(s - w) <= 1e-12 * sc and np.abs(bins - ob).max() <= 1e-12 * sc
+            assert capi.integrate_noalloc(ctx, [item]) == capi.integrate(ctx, [item]) == [(s, npt, nd, nfb)]
+    finally:
+        ctx.set_launch(-1, *before)
