@@ -1278,6 +1278,7 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
   if (n_work == 0) return KB_OK;
   std::vector<ItemDev> items((size_t)n_work);
   std::vector<long long> offs(1, 0);
+  bool lu = false; // some points are known to go to the pivoted LU
   for (int i = 0; i < n_work; ++i) {
     int tree = 0;
     kb_work w = work[i];
@@ -1287,8 +1288,10 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
     if (st) return st;
     KB_CHECK(work[i].order <= KM_MAX_ORDER, "the kernel method runs orders 1..10");
     KB_CHECK(!work[i].flow, "the kernel method does not take a learned flow");
+    // (a model whose spins differ: every point goes to the pivoted LU, a block per chunk)
     const int64_t cp = items[(size_t)i].chunk_points =
-        item_chunk(ctx, work[i].order, items[(size_t)i].n_points, CHUNK_POINTS, INT64_MAX);
+        tree ? item_chunk(ctx, work[i].order, items[(size_t)i].n_points, CHUNK_POINTS, INT64_MAX) : 16;
+    lu = lu || (!tree && items[(size_t)i].n_points > 0);
     offs.push_back(offs.back() + (items[(size_t)i].n_points + cp - 1) / cp);
   }
   const long long nchunks = offs.back();
@@ -1354,11 +1357,15 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
     return KB_OK;
   };
   ctx->last_launches = 1;
+  if (lu) {
+    KB_CUDA(launch_km_fallback(L, ctx->sm_count * 4, st));
+    ctx->last_launches++;
+  }
   int rc = finish();
   if (rc) return rc;
   bool guarded = false;
   for (size_t j = 0; j < ni; ++j) guarded = guarded || reinterpret_cast<const kb_accum *>(host.data() + a_acc)[j].n_fallback;
-  if (guarded) {
+  if (guarded && !lu) {
     KB_CUDA(cudaMemsetAsync(place<kb_accum>(buf, a_acc), 0, ni * sizeof(kb_accum), st));
     KB_CUDA(launch_km_fallback(L, ctx->sm_count * 4, st));
     ctx->last_launches++;
@@ -1427,7 +1434,7 @@ int kb_integrand_kernel_eval(kb_context *ctx, const kb_model *m, const kb_gf_ind
   if (count == 0) return KB_OK;
   ItemDev it = make_item(m, &f, order);
   it.n_points = count;
-  it.chunk_points = item_chunk(ctx, order, count, 32, INT64_MAX);
+  it.chunk_points = it.spin_symmetric ? item_chunk(ctx, order, count, 32, INT64_MAX) : 16;
   std::lock_guard<std::mutex> lk(ctx->mu);
   KB_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;

@@ -89,3 +89,23 @@ def test_nearly_empty_and_full_levels(ctx, oracle, ratio, small):
         got, dom = gm.integrand_kernel(X, t)
         want, odom, sc = oracle.integrand_kernel(om, X, t)
         assert np.array_equal(dom, odom) and np.all(np.abs(got - want).max(axis=(1, 2)) <= 1e-12 * sc), n
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 7])
+@pytest.mark.parametrize("npts", [1, 15, 17, 100])
+def test_models_whose_spins_differ(ctx, oracle, golden, n, npts):
+    """Every point goes to the pivoted LU, set up 16 at a time: sums, bins and values."""
+    tables = [golden[f"table_{k}_{s}"] for k in ("beta20", "T0") for s in ("lesser", "greater")]
+    gm, om = ctx.model(10.0, *tables[:2], 0.0, *tables[2:]), oracle.model(10.0, *tables[:2], 0.0, *tables[2:])
+    X = (10.0, 0, 0, 0, 0)
+    chain = [(capi.WARPER_PLASMA_UV, 10.0, 0.0), (capi.WARPER_INVERSE, 10.0, 2.0)]
+    item = dict(model=gm, rng=ctx.sobol(n), chain=chain, A=X, order=n, k_first=5, n_points=npts)
+    (s, npt, nd, bins, cnt, drop), = capi.integrate_kernel(ctx, [item], 7, 1.0, 9.0)
+    ws, onp, ond, sc, ob, oc, od = oracle.integrate_kernel(om, X, chain, n, npts, 7, 1.0, 9.0, seed=4)
+    assert (npt, nd, drop) == (onp, ond, od) and np.array_equal(cnt, oc)
+    assert np.abs(bins - ob).max() <= 1e-12 * sc and abs(s - ws) <= 1e-12 * sc
+    t = np.random.default_rng(n).random((npts, n)) * 10.0
+    t[::3, 0] *= -1.0
+    got, dom = gm.integrand_kernel(X, t)
+    want, odom, sc = oracle.integrand_kernel(om, X, t)
+    assert np.array_equal(dom, odom) and np.all(np.abs(got - want).max(axis=(1, 2)) <= 1e-12 * sc)
