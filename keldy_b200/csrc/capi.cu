@@ -846,6 +846,12 @@ struct Block {
 size_t tree_scratch(int grid, int max_order) {
   return max_order > 9 ? (size_t)grid * PTS_SLOT * sizeof(double) : 0;
 }
+// What an evaluation call uploads in one piece ahead of its points, and reads back.
+struct EvalHead {
+  ItemDev it;
+  long long offs[2];
+  int counter, flagged, err, pad;
+};
 template <typename T> T *place(const DevBuf &b, size_t at) {
   return reinterpret_cast<T *>(static_cast<unsigned char *>(b.p) + at);
 }
@@ -872,22 +878,18 @@ static int run_eval(kb_context *ctx, ItemDev it, int mode, int64_t count, const 
   long long offs[2] = {0, nchunks};
   const int grid = (int)std::min<long long>(nchunks, use_tree ? ctx->tree_grid : ctx->sm_count * 4);
   const size_t inbytes = (size_t)count * N * sizeof(double);
-  struct Head { // uploaded in one piece
-    ItemDev it;
-    long long offs[2];
-    int counter, flagged, err, pad;
-  } head;
+  EvalHead head;
   memset(&head, 0, sizeof(head));
   head.it = it;
   memcpy(head.offs, offs, sizeof(offs));
   Block B;
-  const size_t a_head = B.take(sizeof(Head)), a_in = B.take(inbytes), a_val = B.take(count * sizeof(double2)),
+  const size_t a_head = B.take(sizeof(head)), a_in = B.take(inbytes), a_val = B.take(count * sizeof(double2)),
                a_jac = B.take(count * sizeof(double)), a_dom = B.take(count * sizeof(int)),
                a_flag = B.take(count * sizeof(int)), a_scale = B.take(scale ? count * sizeof(double) : 0),
                a_pts = B.take(use_tree ? tree_scratch(grid, N) : 0);
   DevBuf buf;
   KB_CUDA(buf.alloc(B.size, st));
-  Head *dh = place<Head>(buf, a_head);
+  EvalHead *dh = place<EvalHead>(buf, a_head);
   KB_CUDA(cudaMemcpyAsync(dh, &head, sizeof(head), cudaMemcpyHostToDevice, st));
   if (inbytes) KB_CUDA(cudaMemcpyAsync(place<double>(buf, a_in), in_host, inbytes, cudaMemcpyHostToDevice, st));
   Launch L;
@@ -1439,46 +1441,56 @@ int kb_integrand_kernel_eval(kb_context *ctx, const kb_model *m, const kb_gf_ind
   KB_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t s = ctx->stream;
   const long long nchunks = (count + it.chunk_points - 1) / it.chunk_points;
-  long long offs[2] = {0, nchunks};
-  DevBuf ditem, doff, dcnt, din, dout, ddom, dpart;
-  KB_CUDA(ditem.alloc(sizeof(ItemDev), s));
-  KB_CUDA(dpart.alloc((size_t)nchunks * sizeof(ChunkPartial), s));
-  KB_CUDA(doff.alloc(sizeof(offs), s));
-  KB_CUDA(dcnt.alloc(sizeof(int), s));
-  KB_CUDA(din.alloc((size_t)count * order * sizeof(double), s));
-  KB_CUDA(dout.alloc((size_t)count * 2 * order * sizeof(double2), s));
-  KB_CUDA(ddom.alloc((size_t)count * sizeof(int), s));
-  KB_CUDA(cudaMemcpyAsync(ditem.p, &it, sizeof(ItemDev), cudaMemcpyHostToDevice, s));
-  KB_CUDA(cudaMemcpyAsync(doff.p, offs, sizeof(offs), cudaMemcpyHostToDevice, s));
-  KB_CUDA(cudaMemcpyAsync(din.p, times, (size_t)count * order * sizeof(double), cudaMemcpyHostToDevice, s));
-  KB_CUDA(cudaMemsetAsync(dcnt.p, 0, sizeof(int), s));
-  KB_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), s));
+  const int kgrid = (int)std::min<long long>(nchunks, (long long)ctx->sm_count * KM_CTAS_PER_SM);
+  const size_t inbytes = (size_t)count * order * sizeof(double), outbytes = (size_t)count * 2 * order * sizeof(double2);
+  EvalHead head;
+  memset(&head, 0, sizeof(head));
+  head.it = it;
+  head.offs[1] = nchunks;
+  Block B;
+  const size_t a_head = B.take(sizeof(head)), a_in = B.take(inbytes), a_out = B.take(outbytes),
+               a_dom = B.take(count * sizeof(int)), a_part = B.take((size_t)nchunks * sizeof(ChunkPartial)),
+               a_pts = B.take((size_t)kgrid * KM_SLOT * sizeof(double));
+  DevBuf buf;
+  KB_CUDA(buf.alloc(B.size, s));
+  EvalHead *dh = place<EvalHead>(buf, a_head);
+  KB_CUDA(cudaMemcpyAsync(dh, &head, sizeof(head), cudaMemcpyHostToDevice, s));
+  KB_CUDA(cudaMemcpyAsync(place<double>(buf, a_in), times, inbytes, cudaMemcpyHostToDevice, s));
   Launch L;
   memset(&L, 0, sizeof(L));
-  L.items = ditem.as<ItemDev>();
+  L.items = &dh->it;
   L.n_items = 1;
   L.any_cubic = items_any_cubic(&it, 1);
-  L.chunk_offsets = doff.as<long long>();
+  L.chunk_offsets = dh->offs;
   L.n_chunks = (int)nchunks;
-  L.chunk_counter = dcnt.as<int>();
+  L.chunk_counter = &dh->counter;
   L.mode = IN_TIMES;
   L.keep_u_hypercube = keep_u_hypercube;
-  L.in = din.as<double>();
-  L.partials = dpart.as<ChunkPartial>();
-  L.out_kvals = dout.as<double2>();
-  L.out_dom = ddom.as<int>();
-  L.err = ctx->d_err;
-  const int kgrid = (int)std::min<long long>(nchunks, (long long)ctx->sm_count * KM_CTAS_PER_SM);
-  DevBuf dpts;
-  KB_CUDA(dpts.alloc((size_t)kgrid * KM_SLOT * sizeof(double), s));
-  L.pts = dpts.as<double>();
+  L.in = place<double>(buf, a_in);
+  L.partials = place<ChunkPartial>(buf, a_part);
+  L.out_kvals = place<double2>(buf, a_out);
+  L.out_dom = place<int>(buf, a_dom);
+  L.n_flagged = &dh->flagged;
+  L.err = &dh->err;
+  L.pts = place<double>(buf, a_pts);
   KB_CUDA(launch_km_tree(L, kgrid, s));
-  KB_CUDA(launch_km_fallback(L, (int)std::min<long long>(nchunks, ctx->sm_count * 4), s));
-  int err = 0;
-  KB_CUDA(cudaMemcpyAsync(out, dout.p, (size_t)count * 2 * order * sizeof(double2), cudaMemcpyDeviceToHost, s));
-  if (in_domain) KB_CUDA(cudaMemcpyAsync(in_domain, ddom.p, (size_t)count * sizeof(int), cudaMemcpyDeviceToHost, s));
-  KB_CUDA(cudaMemcpyAsync(&err, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  KB_CUDA(cudaStreamSynchronize(s));
+  auto fallback = [&]() { return launch_km_fallback(L, (int)std::min<long long>(nchunks, ctx->sm_count * 4), s); };
+  if (!it.spin_symmetric) KB_CUDA(fallback());
+  auto download = [&]() -> int {
+    KB_CUDA(cudaMemcpyAsync(&head, dh, sizeof(head), cudaMemcpyDeviceToHost, s));
+    KB_CUDA(cudaMemcpyAsync(out, L.out_kvals, outbytes, cudaMemcpyDeviceToHost, s));
+    if (in_domain) KB_CUDA(cudaMemcpyAsync(in_domain, L.out_dom, count * sizeof(int), cudaMemcpyDeviceToHost, s));
+    KB_CUDA(cudaStreamSynchronize(s));
+    return KB_OK;
+  };
+  int rc = download();
+  if (rc) return rc;
+  if (it.spin_symmetric && head.flagged) { // the points the tree marked
+    KB_CUDA(fallback());
+    rc = download();
+    if (rc) return rc;
+  }
+  const int err = head.err;
   if (err & 1) return fail(KB_E_RANGE, "g0 evaluated outside its tabulated time window");
   return KB_OK;
 }

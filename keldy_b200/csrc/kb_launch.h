@@ -56,7 +56,7 @@ struct Launch {
   int *out_dom;
   double *out_scale;
   int *out_flag;        // tree: 1 = point needs the pivoted-LU kernel
-  int *n_flagged;       // tree: their number is added here
+  int *n_flagged;       // IN_TIMES / IN_LI, both trees: the number of such points is added here
   // gridDim.x * PTS_SLOT doubles of scratch (tree kernel) or KM_SLOT (kernel-method tree)
   double *pts;
   // IN_SOBOL

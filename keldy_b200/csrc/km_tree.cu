@@ -659,6 +659,7 @@ __global__ void __launch_bounds__(KM_WARPS * 32, KM_CTAS_PER_SM) km_tree_kernel(
       pr.fb_mask[1] = fbm[1];
       L.partials[c] = pr;
       if (!eval && L.nbins) L.bin_dropped[c] = ndrop;
+      if (eval && nfb) atomicAdd(L.n_flagged, (int)nfb);
     }
   }
   if (__any_sync(FULL, bad) && lane == 0) atomicOr(L.err, 1);

@@ -109,3 +109,18 @@ def test_models_whose_spins_differ(ctx, oracle, golden, n, npts):
     got, dom = gm.integrand_kernel(X, t)
     want, odom, sc = oracle.integrand_kernel(om, X, t)
     assert np.array_equal(dom, odom) and np.all(np.abs(got - want).max(axis=(1, 2)) <= 1e-12 * sc)
+
+
+@pytest.mark.parametrize("n,count", [(1, 40), (2, 1), (3, 33), (5, 70)])
+def test_values_of_guarded_points(ctx, oracle, n, count):
+    """Every point of the domain goes to the pivoted LU (g(0) = 0) after the tree has counted them."""
+    t = np.linspace(-10, 10, 2001)
+    le = 1j * t * np.exp(-t * t / 8) + 0.2 * np.sin(t)
+    tables = le, -np.conj(le[::-1])
+    gm, om = ctx.model(10.0, *tables), oracle.model(10.0, *tables)
+    u = np.random.default_rng(n).random((count, n)) * 10.0
+    u[1::4, 0] *= -1.0
+    for X in ((10.0, 0, 0, 0, 0), (6.0, 0, 1, 0, 0)):
+        got, dom = gm.integrand_kernel(X, u)
+        want, odom, sc = oracle.integrand_kernel(om, X, u)
+        assert np.array_equal(dom, odom) and np.all(np.abs(got - want).max(axis=(1, 2)) <= 1e-12 * sc)
