@@ -829,6 +829,15 @@ static int item_chunk(const kb_context *ctx, int order, int64_t n, int most, int
   return c;
 }
 
+// The largest chunks that still spread an item over the CTAs: the context's chunk size of the order,
+// halved (down to 8) while the item would have fewer chunks than half the resident tree CTAs.
+static int coarse_chunk(const kb_context *ctx, int order, int64_t n) {
+  int c = ctx->chunk_points[order];
+  const int64_t want = (int64_t)ctx->sm_count * ctx->ctas_per_sm / 2;
+  while (c > 8 && (n + c - 1) / c < want) c >>= 1;
+  return c;
+}
+
 } // extern "C"
 
 // Places in one device block: an allocation, an upload and a download per call instead of one per
@@ -1061,6 +1070,20 @@ struct TimeBins {
   uint64_t *dropped; // [n_work], added to
 };
 
+// Every chunk holds a call's time bins. Where those of all chunks would take more than BIN_BYTES (most of
+// what the memory pool keeps from call to call: beyond, each call maps its memory anew, 8 us per MB), the
+// items' chunks are grown to coarse(item): 300 items of 2^18 points with 4,096 bins take 50 GB instead of
+// 200. Such a call adds an item's points in another order than a call of its own may.
+constexpr size_t BIN_BYTES = KB_POOL_KEEP_BYTES / 4 * 3;
+template <class Coarse>
+void limit_bins(std::vector<ItemDev> &items, size_t nb, Coarse coarse) {
+  size_t bytes = 0;
+  for (const ItemDev &it : items)
+    bytes += (size_t)((it.n_points + it.chunk_points - 1) / it.chunk_points) * nb * (sizeof(double2) + sizeof(unsigned));
+  if (bytes <= BIN_BYTES) return;
+  for (ItemDev &it : items) it.chunk_points = std::max(it.chunk_points, coarse(it));
+}
+
 // One batched pass over `items`: two groups (tree / pivoted LU), each one persistent
 // launch over its items, heaviest orders first. Sums are added to acc[acc_index[i]]
 // (and to the time bins of that work item when `bins` is given), the kernels' error bits to err.
@@ -1076,11 +1099,10 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
     std::stable_sort(ids.begin(), ids.end(), [&](int a, int b) { return items[(size_t)a].order > items[(size_t)b].order; });
     std::vector<ItemDev> sorted;
     std::vector<long long> offs(1, 0);
-    for (int i : ids) {
-      sorted.push_back(items[(size_t)i]);
-      const long long cp = items[(size_t)i].chunk_points;
-      offs.push_back(offs.back() + (items[(size_t)i].n_points + cp - 1) / cp);
-    }
+    for (int i : ids) sorted.push_back(items[(size_t)i]);
+    if (bins)
+      limit_bins(sorted, (size_t)bins->nbins, [&](const ItemDev &it) { return coarse_chunk(ctx, it.order, it.n_points); });
+    for (const ItemDev &it : sorted) offs.push_back(offs.back() + (it.n_points + it.chunk_points - 1) / it.chunk_points);
     const long long nchunks = offs.back();
     if (nchunks > INT32_MAX) return fail(KB_E_INVALID, "too many points in one kb_integrate call");
     const int tgrid = (int)std::min<long long>(nchunks, (long long)ctx->sm_count * ctx->ctas_per_sm);
@@ -1291,11 +1313,12 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
     KB_CHECK(work[i].order <= KM_MAX_ORDER, "the kernel method runs orders 1..10");
     KB_CHECK(!work[i].flow, "the kernel method does not take a learned flow");
     // (a model whose spins differ: every point goes to the pivoted LU, a block per chunk)
-    const int64_t cp = items[(size_t)i].chunk_points =
+    items[(size_t)i].chunk_points =
         tree ? item_chunk(ctx, work[i].order, items[(size_t)i].n_points, CHUNK_POINTS, INT64_MAX) : 16;
     lu = lu || (!tree && items[(size_t)i].n_points > 0);
-    offs.push_back(offs.back() + (items[(size_t)i].n_points + cp - 1) / cp);
   }
+  if (bins) limit_bins(items, 2 * (size_t)bins->nbins, [](const ItemDev &) { return 16; });
+  for (const ItemDev &it : items) offs.push_back(offs.back() + (it.n_points + it.chunk_points - 1) / it.chunk_points);
   const long long nchunks = offs.back();
   if (nchunks > INT32_MAX) return fail(KB_E_INVALID, "too many points in one call");
   if (nchunks == 0) return KB_OK;
@@ -1933,7 +1956,7 @@ constexpr size_t NOALLOC_OFFS_OFF = NOALLOC_ITEMS_OFF + sizeof(ItemDev) * KB_NOA
 constexpr size_t NOALLOC_ACC_OFF = ((NOALLOC_OFFS_OFF + sizeof(long long) * (KB_NOALLOC_MAX_ITEMS + 1)) + 255) / 256 * 256;
 constexpr size_t NOALLOC_CNT_OFF = NOALLOC_ACC_OFF + sizeof(kb_accum) * 2 * KB_NOALLOC_MAX_ITEMS;
 constexpr size_t NOALLOC_PART_OFF = (NOALLOC_CNT_OFF + sizeof(int) + 255) / 256 * 256;
-// An item's chunks number at most its chunks in the documented unit (noalloc_unit), or twice
+// An item's chunks number at most its chunks in the documented unit (coarse_chunk), or twice
 // NOALLOC_SPLIT_CHUNKS where item_chunk split a small item further.
 constexpr int64_t NOALLOC_SPLIT_CHUNKS = 888;
 constexpr size_t NOALLOC_PARTIALS = KB_NOALLOC_MAX_CHUNKS + KB_NOALLOC_MAX_ITEMS * 2 * NOALLOC_SPLIT_CHUNKS;
@@ -1946,15 +1969,6 @@ constexpr size_t NOALLOC_B200_TREE_CTAS = 148 * 4;
 static_assert(NOALLOC_PTS_SLOTS >= NOALLOC_B200_TREE_CTAS, "scratch too small for one set-up slot per resident CTA");
 
 static __device__ __align__(256) unsigned char kb_noalloc_scratch[KB_NOALLOC_SCRATCH_BYTES];
-
-// The unit of the call's documented chunk limit: the context's chunk size of the order, halved
-// (down to 8) while the item would have fewer chunks than half the resident tree CTAs.
-int noalloc_unit(const kb_context *ctx, int order, int64_t n) {
-  int c = ctx->chunk_points[order];
-  const int64_t want = (int64_t)ctx->sm_count * ctx->ctas_per_sm / 2;
-  while (c > 8 && (n + c - 1) / c < want) c >>= 1;
-  return c;
-}
 
 std::mutex g_noalloc_mu;
 unsigned char *g_noalloc_addr[NOALLOC_MAX_DEVICES] = {};
@@ -2008,7 +2022,7 @@ extern "C" int kb_integrate_noalloc(kb_context *ctx, const kb_work *work, int n_
     group_of[i] = it.spin_symmetric ? 0 : 1;
     // kb_integrate's rule for a small item's scheduling chunks, but at most as many as the array holds
     it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order], NOALLOC_SPLIT_CHUNKS);
-    const int64_t unit = noalloc_unit(ctx, w.order, w.n_points);
+    const int64_t unit = coarse_chunk(ctx, w.order, w.n_points);
     chunks_total += (w.n_points + unit - 1) / unit;
   }
   if (chunks_total > KB_NOALLOC_MAX_CHUNKS)

@@ -110,3 +110,15 @@ def test_bins_with_guarded_pivots(ctx, oracle):
         assert nfb > 0 and nd == ond
         assert np.array_equal(counts, ocounts) and dropped == odropped
         assert np.abs(bins - obins).max() <= 1e-12 * sc
+
+
+def test_bins_of_many_items_fit(ctx, golden):
+    """300 items of 2^18 points with 4,096 bins: 50 GB of bins in chunks of 128 points, more than the
+    device holds in chunks of 32. One item alone (2,048 chunks of 128 points) gives the same counts."""
+    gm = ctx.model(10.0, golden["table_beta20_lesser"], golden["table_beta20_greater"])
+    item = _item(gm, ctx.sobol(1), PLASMA_EXP, 1, 1 << 18)
+    res = capi.integrate_binned(ctx, [item] * 300, 4096, 0.0, 10.0)
+    one, = capi.integrate_binned(ctx, [item], 4096, 0.0, 10.0)
+    for r in res:
+        assert r[1:4] == one[1:4] and r[6] == one[6] and np.array_equal(r[5], one[5])
+        assert r[0] == one[0] and np.array_equal(r[4], one[4])
