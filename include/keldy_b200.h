@@ -379,7 +379,8 @@ int kb_integrand_kernel_eval(kb_context *ctx, const kb_model *m, const kb_gf_ind
  * KB_NOALLOC_MAX_ITEMS work items and KB_NOALLOC_MAX_CHUNKS scheduling chunks per call
  * (8,388,608 points with the default 128-point chunks; KB_E_INVALID beyond). The chunk
  * size and CTAs per SM are the context's launch shape (kb_context_set_launch), as in
- * kb_integrate; the tree grid is also capped at the per-CTA slots the array holds (more
+ * kb_integrate; a call of more than 179,200 chunks of kb_integrate's (many items of 10^5 points and
+ * more) runs in larger ones, so that its sums may differ from kb_integrate's in rounding. The tree grid is also capped at the per-CTA slots the array holds (more
  * than the 592 resident CTAs of a B200). All calls share the array: calls that overlap on
  * the GPU race. The first call on a device looks up the array's device address
  * (cudaGetSymbolAddress); make it before any stream capture. */

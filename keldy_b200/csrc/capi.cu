@@ -1956,8 +1956,9 @@ constexpr size_t NOALLOC_OFFS_OFF = NOALLOC_ITEMS_OFF + sizeof(ItemDev) * KB_NOA
 constexpr size_t NOALLOC_ACC_OFF = ((NOALLOC_OFFS_OFF + sizeof(long long) * (KB_NOALLOC_MAX_ITEMS + 1)) + 255) / 256 * 256;
 constexpr size_t NOALLOC_CNT_OFF = NOALLOC_ACC_OFF + sizeof(kb_accum) * 2 * KB_NOALLOC_MAX_ITEMS;
 constexpr size_t NOALLOC_PART_OFF = (NOALLOC_CNT_OFF + sizeof(int) + 255) / 256 * 256;
-// An item's chunks number at most its chunks in the documented unit (coarse_chunk), or twice
-// NOALLOC_SPLIT_CHUNKS where item_chunk split a small item further.
+// The array holds kb_integrate's chunks of most calls. Where it does not, item_chunk's splits stop at
+// NOALLOC_SPLIT_CHUNKS: an item's chunks then number at most its chunks in the documented unit
+// (coarse_chunk), or twice NOALLOC_SPLIT_CHUNKS where item_chunk split it further.
 constexpr int64_t NOALLOC_SPLIT_CHUNKS = 888;
 constexpr size_t NOALLOC_PARTIALS = KB_NOALLOC_MAX_CHUNKS + KB_NOALLOC_MAX_ITEMS * 2 * NOALLOC_SPLIT_CHUNKS;
 constexpr size_t NOALLOC_PTS_OFF =
@@ -1996,7 +1997,7 @@ extern "C" int kb_integrate_noalloc(kb_context *ctx, const kb_work *work, int n_
   if (n_work == 0) return KB_OK;
   ItemDev items[KB_NOALLOC_MAX_ITEMS];
   int group_of[KB_NOALLOC_MAX_ITEMS];
-  long long chunks_total = 0;
+  long long chunks_total = 0, partials = 0;
   for (int i = 0; i < n_work; ++i) {
     const kb_work &w = work[i];
     int st = check_integrand(w.m, &w.f, w.order);
@@ -2020,14 +2021,17 @@ extern "C" int kb_integrate_noalloc(kb_context *ctx, const kb_work *work, int n_
     it.k_first = w.k_first;
     it.n_points = w.n_points;
     group_of[i] = it.spin_symmetric ? 0 : 1;
-    // kb_integrate's rule for a small item's scheduling chunks, but at most as many as the array holds
-    it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order], NOALLOC_SPLIT_CHUNKS);
+    it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order], INT64_MAX); // as kb_integrate
+    partials += (w.n_points + it.chunk_points - 1) / it.chunk_points;
     const int64_t unit = coarse_chunk(ctx, w.order, w.n_points);
     chunks_total += (w.n_points + unit - 1) / unit;
   }
   if (chunks_total > KB_NOALLOC_MAX_CHUNKS)
     return fail(KB_E_INVALID, "kb_integrate_noalloc: more than KB_NOALLOC_MAX_CHUNKS (65,536) scheduling chunks in "
                               "one call (8,388,608 points with the default 128-point chunks)");
+  for (int i = 0; i < n_work && partials > (long long)NOALLOC_PARTIALS; ++i)
+    items[i].chunk_points =
+        item_chunk(ctx, work[i].order, work[i].n_points, ctx->chunk_points[work[i].order], NOALLOC_SPLIT_CHUNKS);
   std::lock_guard<std::mutex> lk(ctx->mu);
   KB_CUDA(cudaSetDevice(ctx->device));
   unsigned char *base = nullptr;

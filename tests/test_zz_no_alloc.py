@@ -83,3 +83,17 @@ def test_noalloc_limits(ctx):
     with pytest.raises(capi.KbError) as e:
         capi.integrate_noalloc(ctx, [items[0]] * (capi.NOALLOC_MAX_ITEMS + 1))
     assert e.value.code == capi.KB_E_INVALID
+
+
+def test_noalloc_mid_sized_items(ctx):
+    """Items of the sizes where kb_integrate splits its chunks most: the same chunks, so equal sums. A
+    call of more chunks than the array holds runs in larger ones."""
+    _, le, gr = flatband(1.0, 0.2, 0.5, 20.0, 10.0, 4001)
+    m = ctx.model(10.0, le, gr)
+    items = [dict(model=m, rng=ctx.sobol(n), chain=PLASMA_EXP, A=(10.0, 0, 0), B=(10.0, 0, 1), order=n, k_first=1 + n,
+                  n_points=p) for n, p in ((1, (1 << 17) + 5), (2, 1 << 18), (3, 30011), (9, 28001))]
+    assert capi.integrate_noalloc(ctx, items) == capi.integrate(ctx, items)
+    many = [dict(items[0], n_points=1 << 17)] * capi.NOALLOC_MAX_ITEMS
+    want, sc = capi.integrate(ctx, many[:1])[0], _scale(ctx, many[0])
+    for s, n, d, fb in capi.integrate_noalloc(ctx, many):
+        assert (n, d, fb) == want[1:] and abs(s - want[0]) <= 1e-12 * sc
