@@ -413,11 +413,14 @@ int kb_plan_result(kb_context *ctx, kb_plan *plan, kb_accum *acc);
 int kb_plan_set_k_first(kb_context *ctx, kb_plan *plan, int item, uint32_t k_first);
 
 /* Launch shape of the tree kernel: points per scheduling chunk for `order` (1..128;
- * order -1 sets every order) and resident CTAs per SM (1 to 4; 0 keeps the value). A work
- * item's chunks are halved down to a full group of points (32, 16 above order 8) while it has
- * fewer than eight per resident warp, and further (down to 8 points, 4 from order 6 on) while
- * it has fewer than an eighth of the warps, so that it spreads over the GPU; the chunking
- * depends on the item alone. */
+ * order -1 sets every order) and resident CTAs per SM (1 to 4; 0 keeps the value). 128, the
+ * default, lets the library choose: chunks halved from 128 down to a full group of points (32,
+ * 16 above order 8) while a work item has fewer than eight per resident warp. Any chunks are
+ * halved further (down to 8 points, 4 at orders 6 to 8, 2 at order 9, 1 above) while the item
+ * has fewer than an eighth of the warps, so that it spreads over the GPU. The chunking depends
+ * on the item alone, except in a call whose time bins would take more than 192 MiB (a bin
+ * takes 20 bytes per chunk): its chunks are at most halved (down to 8 points) while the item has
+ * fewer than half the resident CTAs. */
 int kb_context_set_launch(kb_context *ctx, int order, int chunk_points, int ctas_per_sm);
 int kb_context_get_launch(kb_context *ctx, int order, int *chunk_points, int *ctas_per_sm);
 

@@ -1,8 +1,8 @@
 """Autotuner of the tree kernel's launch shape.
 
 For each perturbation order it times a plan (one CUDA-graph launch) of a flat-band
-workload over the candidate scheduling-chunk sizes and resident CTAs per SM, and keeps
-the fastest. Results are cached per GPU model in ~/.cache/keldy_b200/ (or
+workload over the candidate scheduling-chunk sizes (128: the library's choice per work item)
+and resident CTAs per SM, and keeps the fastest. Results are cached per GPU model in ~/.cache/keldy_b200/ (or
 $KELDY_B200_CACHE) and applied to a context with `apply`.
 """
 from __future__ import annotations
@@ -18,9 +18,9 @@ TIE = 0.01
 
 
 def _points(order):
-    """Points of a tuning run: 2^20 up to order 8 (over a dozen 128-point chunks per resident
-    CTA of a B200's 592, so that the last partial wave does not favour small chunks);
-    fewer at the costly high orders."""
+    """Points of a tuning run: 2^20 up to order 8 (nine 64-point chunks, which the library chooses
+    there, per resident warp of a B200's 1,776, so that the last partial wave does not favour
+    small chunks); fewer at the costly high orders."""
     return {9: 1 << 18, 10: 1 << 17, 11: 1 << 16, 12: 1 << 15}.get(order, 1 << 20 if order <= 8 else 1 << 14)
 
 

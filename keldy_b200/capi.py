@@ -399,8 +399,8 @@ class Context:
         check(self.L.kb_context_set_timing(self.h, int(enable)))
 
     def set_launch(self, order=-1, chunk_points=128, ctas_per_sm=0):
-        """Tree-kernel launch shape: points per scheduling chunk of `order` (-1: all) and
-        resident CTAs per SM (0 keeps the current value)."""
+        """Tree-kernel launch shape: points per scheduling chunk of `order` (-1: all; 128: the
+        library's choice per item) and resident CTAs per SM (0 keeps the current value)."""
         check(self.L.kb_context_set_launch(self.h, order, chunk_points, ctas_per_sm))
 
     def get_launch(self, order):

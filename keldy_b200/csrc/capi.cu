@@ -810,8 +810,7 @@ static ItemDev make_item(const kb_model *m, const kb_integrand *f, int order) {
   return it;
 }
 
-// Points per scheduling chunk of a work item of n points: `most` (the context's chunk size for
-// its order, autotuned or kb_context_set_launch), halved down to a full group (32 points, 16 above
+// Points per scheduling chunk of a work item of n points: `most`, halved down to a full group (32 points, 16 above
 // order 8) while the item would have fewer than eight chunks per resident tree warp (at most
 // `limit`), so that the last chunks of a large item leave no warp idle for long: 2^18 points of
 // order 7 in 2,048 chunks of 128 on 1,776 warps were two rounds for 1.15. A smaller group costs:
@@ -827,6 +826,13 @@ static int item_chunk(const kb_context *ctx, int order, int64_t n, int most, int
   while (c > full && (n + c - 1) / c < std::min(8 * warps, limit)) c >>= 1;
   while (c > least && (n + c - 1) / c < warps / 8) c >>= 1;
   return c;
+}
+
+// The same for an integration: a chunk size below 128 that the caller set for the order
+// (kb_context_set_launch, the autotuner) is taken as it is, but for items too small to spread.
+static int order_chunk(const kb_context *ctx, int order, int64_t n, int64_t limit = INT64_MAX) {
+  const int set = ctx->chunk_points[order];
+  return item_chunk(ctx, order, n, set, set == CHUNK_POINTS ? limit : 0);
 }
 
 // The largest chunks that still spread an item over the CTAs: the context's chunk size of the order,
@@ -1243,7 +1249,7 @@ int work_item(kb_context *ctx, const kb_work &w, int algo, ItemDev &it, int &tre
   it.rng = sobol_dev(w.rng);
   it.k_first = w.k_first;
   it.n_points = w.n_points;
-  it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order], INT64_MAX);
+  it.chunk_points = order_chunk(ctx, w.order, w.n_points);
   if (w.flow && w.flow->layout.kind == FLOW_KIND_SPLINE) it.spline_knots = w.flow->knots; // mapped in line
   if (w.flow && w.flow->layout.kind == FLOW_KIND_AR_SPLINE) it.ar_spline = w.flow->master; // mapped in line
   if (algo == KB_ALGO_TREE && !it.spin_symmetric)
@@ -2021,7 +2027,7 @@ extern "C" int kb_integrate_noalloc(kb_context *ctx, const kb_work *work, int n_
     it.k_first = w.k_first;
     it.n_points = w.n_points;
     group_of[i] = it.spin_symmetric ? 0 : 1;
-    it.chunk_points = item_chunk(ctx, w.order, w.n_points, ctx->chunk_points[w.order], INT64_MAX); // as kb_integrate
+    it.chunk_points = order_chunk(ctx, w.order, w.n_points); // as kb_integrate
     partials += (w.n_points + it.chunk_points - 1) / it.chunk_points;
     const int64_t unit = coarse_chunk(ctx, w.order, w.n_points);
     chunks_total += (w.n_points + unit - 1) / unit;
@@ -2030,8 +2036,7 @@ extern "C" int kb_integrate_noalloc(kb_context *ctx, const kb_work *work, int n_
     return fail(KB_E_INVALID, "kb_integrate_noalloc: more than KB_NOALLOC_MAX_CHUNKS (65,536) scheduling chunks in "
                               "one call (8,388,608 points with the default 128-point chunks)");
   for (int i = 0; i < n_work && partials > (long long)NOALLOC_PARTIALS; ++i)
-    items[i].chunk_points =
-        item_chunk(ctx, work[i].order, work[i].n_points, ctx->chunk_points[work[i].order], NOALLOC_SPLIT_CHUNKS);
+    items[i].chunk_points = order_chunk(ctx, work[i].order, work[i].n_points, NOALLOC_SPLIT_CHUNKS);
   std::lock_guard<std::mutex> lk(ctx->mu);
   KB_CUDA(cudaSetDevice(ctx->device));
   unsigned char *base = nullptr;

@@ -67,3 +67,19 @@ def test_autotune_small(ctx, tmp_path):
     autotune.apply(ctx, table)
     assert ctx.get_launch(8)[0] == table[8]["chunk_points"]
     ctx.set_launch(-1, 128, 2)
+
+
+def test_chunk_sizes_take_effect(ctx, model):
+    """A chunk size below 128 is taken as it is: chunks of 32 and of 64 points add the points in another
+    order, so not all sums can be the same bit for bit (and stay within rounding)."""
+    sums = {}
+    items = [dict(it, n_points=1 << 17) for it in _items(ctx, model)[:5]]
+    try:
+        for c in (32, 64):
+            ctx.set_launch(-1, c, 4)
+            sums[c] = [r[0] for r in capi.integrate(ctx, items)]
+    finally:
+        ctx.set_launch(-1, 128, 2)
+    assert sums[32] != sums[64]
+    for a, b, it in zip(sums[32], sums[64], items):
+        assert abs(a - b) <= 1e-12 * _scale(it)
