@@ -1110,7 +1110,7 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
       limit_bins(sorted, (size_t)bins->nbins, [&](const ItemDev &it) { return coarse_chunk(ctx, it.order, it.n_points); });
     for (const ItemDev &it : sorted) offs.push_back(offs.back() + (it.n_points + it.chunk_points - 1) / it.chunk_points);
     const long long nchunks = offs.back();
-    if (nchunks > INT32_MAX) return fail(KB_E_INVALID, "too many points in one kb_integrate call");
+    if (nchunks > MAX_CHUNKS) return fail(KB_E_INVALID, "too many points in one kb_integrate call");
     const int tgrid = (int)std::min<long long>(nchunks, (long long)ctx->sm_count * ctx->ctas_per_sm);
     const size_t ni = sorted.size(), nb = bins ? (size_t)bins->nbins : 0;
     // one block: the upload (items, chunk offsets, the scheduling counter, zeroed sums and error
@@ -1326,7 +1326,7 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
   if (bins) limit_bins(items, 2 * (size_t)bins->nbins, [](const ItemDev &) { return 16; });
   for (const ItemDev &it : items) offs.push_back(offs.back() + (it.n_points + it.chunk_points - 1) / it.chunk_points);
   const long long nchunks = offs.back();
-  if (nchunks > INT32_MAX) return fail(KB_E_INVALID, "too many points in one call");
+  if (nchunks > MAX_CHUNKS) return fail(KB_E_INVALID, "too many points in one call");
   if (nchunks == 0) return KB_OK;
   std::lock_guard<std::mutex> lk(ctx->mu);
   KB_CUDA(cudaSetDevice(ctx->device));
@@ -1743,7 +1743,7 @@ int kb_plan_create(kb_context *ctx, const kb_work *work, int n_work, int algo, k
       p->where_pos[(size_t)g.ids[(size_t)j]] = j;
     }
     g.n_chunks = offs.back();
-    if (g.n_chunks > INT32_MAX) {
+    if (g.n_chunks > MAX_CHUNKS) {
       plan_free(p);
       return fail(KB_E_INVALID, "too many points in one plan");
     }

@@ -23,6 +23,9 @@ struct ChunkPartial {
 };
 
 constexpr int CHUNK_POINTS = 128; // points per scheduling chunk (<= 128: two 64-bit masks)
+// Chunks of a launch, at most: the chunk counter and the numbers made from it (ints) run past the last
+// chunk, by two for each resident warp (fewer than 2^14).
+constexpr long long MAX_CHUNKS = INT32_MAX - (1 << 16);
 // The tree kernel (wick_tree.cu): warps of a CTA, resident CTAs per SM (12 warps: 168 registers
 // per thread and 19 KB of shared memory per warp), and the complex entries of a warp's global
 // scratch (L2-resident): the nodes of orders 9..16 above level 8, sum_{m=9..16} (m+1)^2 + 2 * 81.

@@ -83,3 +83,19 @@ def test_chunk_sizes_take_effect(ctx, model):
     assert sums[32] != sums[64]
     for a, b, it in zip(sums[32], sums[64], items):
         assert abs(a - b) <= 1e-12 * _scale(it)
+
+
+def test_more_chunks_than_the_counter_counts(ctx, model):
+    """2^31 - 1 chunks of one point: the chunk counter would overflow past the last one. Refused before
+    anything is allocated or launched."""
+    item = dict(_items(ctx, model)[0], k_first=1, n_points=(1 << 31) - 1)
+    before = capi.device_allocations()
+    try:
+        ctx.set_launch(-1, 1, 4)
+        for call in (lambda: capi.integrate(ctx, [item]), lambda: capi.Plan(ctx, [item])):
+            with pytest.raises(capi.KbError) as e:
+                call()
+            assert e.value.code == capi.KB_E_INVALID and "too many points" in str(e.value)
+    finally:
+        ctx.set_launch(-1, 128, 2)
+    assert capi.device_allocations() == before
