@@ -148,7 +148,8 @@ struct Pipe {
   uint32_t tmem;       // TMEM base
   uint32_t mphase;     // parity of the next MMA completion (all threads)
   uint32_t wphase[3];  // parity of the next fill of each slot (thread 0)
-  int pending[3];      // fill issued and not yet waited (thread 0)
+  int pending[3];      // fill issued and not yet seen complete (thread 0)
+  int open;            // products issued and not yet seen complete (thread 0)
   const uint16_t *img; // global weight images
 };
 
@@ -190,21 +191,27 @@ __device__ bool mma_step(Pipe &P, int wslot, const Mma &m0, const Mma &m1, int n
   if (threadIdx.x == 0) {
     tc_fence_after();
     if (wslot >= 0 && P.pending[wslot]) {
-      if (!mbar_wait(P.wbar[wslot], P.wphase[wslot])) bad = 1;
-      P.wphase[wslot] ^= 1;
-      P.pending[wslot] = 0;
+      if (mbar_wait(P.wbar[wslot], P.wphase[wslot])) {
+        P.wphase[wslot] ^= 1;
+        P.pending[wslot] = 0;
+      } else {
+        bad = 1;
+      }
     }
     if (!bad) {
       issue_mma(m0);
       if (n > 1) issue_mma(m1);
       umma_commit(P.mbar);
+      P.open = 1;
     }
   }
   if (__syncthreads_or(bad)) return false;
   const int tmo = mbar_wait(P.mbar, P.mphase) ? 0 : 1;
-  P.mphase ^= 1;
   tc_fence_after();
-  return !__syncthreads_or(tmo);
+  if (__syncthreads_or(tmo)) return false;
+  P.mphase ^= 1;
+  P.open = 0;
+  return true;
 }
 
 __device__ __forceinline__ unsigned char *row_ptr(unsigned char *buf, int t) {
@@ -294,6 +301,7 @@ __device__ void pipe_init(Pipe &P, unsigned char *base, int n_act, SmemHead *&he
     P.pending[j] = 0;
   }
   P.mphase = 0;
+  P.open = 0;
   P.img = img;
   if (threadIdx.x == 0) {
     mbar_init(P.mbar, 1);
@@ -307,9 +315,11 @@ __device__ void pipe_init(Pipe &P, unsigned char *base, int n_act, SmemHead *&he
   P.tmem = head->tmem_slot;
 }
 
-// Waits for fills still in flight, then frees the TMEM columns.
+// Waits for fills and products still in flight (once more, where a wait ran out), then frees the
+// TMEM columns.
 __device__ void pipe_finish(Pipe &P, uint32_t ncols, int *err) {
   if (threadIdx.x == 0) {
+    if (P.open && !mbar_wait(P.mbar, P.mphase)) atomicOr(err, FLOW_ERR_TIMEOUT);
     for (int j = 0; j < 3; ++j)
       if (P.pending[j]) {
         if (!mbar_wait(P.wbar[j], P.wphase[j])) atomicOr(err, FLOW_ERR_TIMEOUT);
@@ -349,6 +359,7 @@ __global__ void __launch_bounds__(NT, 2)
     P.pending[j] = 0;
   }
   P.mphase = 0;
+  P.open = 0;
   P.img = f.img;
   if (threadIdx.x == 0) {
     mbar_init(P.mbar, 1);
@@ -601,12 +612,12 @@ __global__ void __launch_bounds__(TRAIN_NT, 1)
       // during the layer above, their logits take one product
       if (l + 1 < FLOW_LAYERS) {
         const int tmo = (mbar_wait(hbar[0], hphase) && mbar_wait(hbar[1], hphase)) ? 0 : 1;
-        hphase ^= 1;
-        hpending = 0;
-        if (__syncthreads_or(tmo)) {
+        if (__syncthreads_or(tmo)) { // the loads stay pending: waited for once more on the way out
           ok = false;
           break;
         }
+        hphase ^= 1;
+        hpending = 0;
         const Mma none = {}, m = {P.tmem, act_addr(P, 2), w_addr(P, 2), 0, 0, 0};
         if (!(ok = mma_step(P, 2, m, none, 1))) break;
       }
