@@ -1090,6 +1090,18 @@ void limit_bins(std::vector<ItemDev> &items, size_t nb, Coarse coarse) {
   for (ItemDev &it : items) it.chunk_points = std::max(it.chunk_points, coarse(it));
 }
 
+// Adds a pass's times to the call's, from events around its integrand (0, 1), pivoted-LU (1, 2) and
+// reduction launches (2, 3); the pass that follows for guarded points has no integrand launch.
+int add_times(kb_context *ctx, bool integrand) {
+  if (!ctx->timing) return KB_OK;
+  float ms = 0;
+  for (int i = integrand ? 0 : 1; i < 3; ++i) {
+    KB_CUDA(cudaEventElapsedTime(&ms, ctx->ev[i], ctx->ev[i + 1]));
+    ctx->last_ms[i] += ms;
+  }
+  return KB_OK;
+}
+
 // One batched pass over `items`: two groups (tree / pivoted LU), each one persistent
 // launch over its items, heaviest orders first. Sums are added to acc[acc_index[i]]
 // (and to the time bins of that work item when `bins` is given), the kernels' error bits to err.
@@ -1175,6 +1187,7 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
     };
     ctx->last_launches++;
     int rc = finish();
+    if (!rc) rc = add_times(ctx, true);
     if (rc) return rc;
     // guarded points are rare: their pass is launched when the sums say that there are some (the
     // launch is a seventh of a small call), and the sums are formed again with them
@@ -1182,9 +1195,11 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
     for (size_t j = 0; j < ni; ++j) guarded = guarded || reinterpret_cast<const kb_accum *>(host.data() + a_acc)[j].n_fallback;
     if (group == 0 && guarded) {
       KB_CUDA(cudaMemsetAsync(place<kb_accum>(buf, a_acc), 0, ni * sizeof(kb_accum), st));
+      if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[1], st));
       KB_CUDA(launch_fallback(L, ctx->sm_count * 4, st));
       ctx->last_launches++;
       rc = finish();
+      if (!rc) rc = add_times(ctx, false);
       if (rc) return rc;
     }
     const kb_accum *part = reinterpret_cast<const kb_accum *>(host.data() + a_acc);
@@ -1192,15 +1207,6 @@ int run_integrate(kb_context *ctx, const std::vector<ItemDev> &items, const std:
     const unsigned long long *hbc = reinterpret_cast<const unsigned long long *>(host.data() + a_oc);
     const unsigned long long *hbd = reinterpret_cast<const unsigned long long *>(host.data() + a_od);
     err |= *reinterpret_cast<const int *>(host.data() + a_err);
-    if (ctx->timing) {
-      float a = 0, b = 0, c = 0;
-      KB_CUDA(cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[1]));
-      KB_CUDA(cudaEventElapsedTime(&b, ctx->ev[1], ctx->ev[2]));
-      KB_CUDA(cudaEventElapsedTime(&c, ctx->ev[2], ctx->ev[3]));
-      ctx->last_ms[0] += a;
-      ctx->last_ms[1] += b;
-      ctx->last_ms[2] += c;
-    }
     for (size_t j = 0; j < ids.size(); ++j) {
       const int w = acc_index[(size_t)ids[j]];
       kb_accum &a = acc[w];
@@ -1377,30 +1383,35 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
   KB_CUDA(launch_km_tree(L, kgrid, st));
   if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[1], st));
   auto finish = [&]() -> int { // as run_integrate's
+    if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[2], st));
     KB_CUDA(launch_reduce(L, place<kb_accum>(buf, a_acc), st));
     if (nb)
       KB_CUDA(launch_reduce_bins(L, place<double2>(buf, a_os), place<unsigned long long>(buf, a_oc),
                                  place<unsigned long long>(buf, a_od), st));
-    if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[2], st));
+    if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[3], st));
     ctx->last_launches += nb ? 2 : 1;
     KB_CUDA(cudaMemcpyAsync(host.data() + a_acc, place<unsigned char>(buf, a_acc), down_end - a_acc, cudaMemcpyDeviceToHost, st));
     KB_CUDA(cudaStreamSynchronize(st));
     return KB_OK;
   };
   ctx->last_launches = 1;
+  ctx->last_ms[0] = ctx->last_ms[1] = ctx->last_ms[2] = 0.0;
   if (lu) {
     KB_CUDA(launch_km_fallback(L, ctx->sm_count * 4, st));
     ctx->last_launches++;
   }
   int rc = finish();
+  if (!rc) rc = add_times(ctx, true);
   if (rc) return rc;
   bool guarded = false;
   for (size_t j = 0; j < ni; ++j) guarded = guarded || reinterpret_cast<const kb_accum *>(host.data() + a_acc)[j].n_fallback;
   if (guarded && !lu) {
     KB_CUDA(cudaMemsetAsync(place<kb_accum>(buf, a_acc), 0, ni * sizeof(kb_accum), st));
+    if (ctx->timing) KB_CUDA(cudaEventRecord(ctx->ev[1], st));
     KB_CUDA(launch_km_fallback(L, ctx->sm_count * 4, st));
     ctx->last_launches++;
     rc = finish();
+    if (!rc) rc = add_times(ctx, false);
     if (rc) return rc;
   }
   const kb_accum *part = reinterpret_cast<const kb_accum *>(host.data() + a_acc);
@@ -1408,14 +1419,6 @@ int integrate_kernel_impl(kb_context *ctx, const kb_work *work, int n_work, cons
   const unsigned long long *hbc = reinterpret_cast<const unsigned long long *>(host.data() + a_oc);
   const unsigned long long *hbd = reinterpret_cast<const unsigned long long *>(host.data() + a_od);
   const int err = *reinterpret_cast<const int *>(host.data() + a_err);
-  if (ctx->timing) {
-    float a = 0, c = 0;
-    KB_CUDA(cudaEventElapsedTime(&a, ctx->ev[0], ctx->ev[1]));
-    KB_CUDA(cudaEventElapsedTime(&c, ctx->ev[1], ctx->ev[2]));
-    ctx->last_ms[0] = a;
-    ctx->last_ms[1] = 0.0;
-    ctx->last_ms[2] = c;
-  }
   if (err & 1) return fail(KB_E_RANGE, "g0 evaluated outside its tabulated time window");
   for (int w = 0; w < n_work; ++w) {
     acc[w].sum_re += part[(size_t)w].sum_re;

@@ -83,3 +83,19 @@ def test_guarded_points_of_a_chunk(ctx, oracle, order, npts, chunk):
             assert capi.integrate_noalloc(ctx, [item]) == capi.integrate(ctx, [item]) == [(s, npt, nd, nfb)]
     finally:
         ctx.set_launch(-1, *before)
+
+
+def test_times_of_a_call_with_guarded_points(ctx):
+    """The pivoted-LU time is its launch's own: for 40 points beside 2^18 ordinary ones with 4,096 bins
+    less than the sums over the bins (168 MB), which are formed before it and after it."""
+    rng = ctx.sobol(2)
+    items = [_item(ctx.model(10.0, *_tables(k)), rng, 2, n, 1, EXPONENTIAL) for k, n in (("plain", 1 << 18), ("guarded", 40))]
+    ctx.set_timing(True)
+    try:
+        for _ in range(3):
+            res = capi.integrate_binned(ctx, items, 4096, 0.0, 10.0)
+            integrand, lu, sums, launches = ctx.last_timing()
+    finally:
+        ctx.set_timing(False)
+    assert res[1][3] == 40 and launches == 6
+    assert 0.0 < lu < sums and integrand > 0.0
