@@ -11,6 +11,9 @@ QMC sum. Synthetic g0 tables built on the host from the model's closed form.
 
     python bench.py [--gpus N --steps K --warmup W] [--impl reference]
 
+The result is one JSON line of about 2 KB on stdout; what explains it (sources of the figures, runs,
+the batched series, launch shapes and the further measurements) is one JSON line on stderr.
+
 Under torchrun each rank takes its own contiguous block of Sobol indices (weak
 scaling); the per-rank sums are combined with one all_reduce, as keldy's
 integrator::reduce_result does.
@@ -39,6 +42,22 @@ GAMMA, EPS_D, BIAS, BETA, T_MAX, NPTS = 1.0, 0.0, 0.0, 50.0, 20.0, 40001
 TREE_DRAM_CAPTURES = {"5de8928da3ce1dc4": 3238144 + 1705728}
 TREE_SOURCES = ("wick_tree.cu", "kb_wick.cuh", "kb_device.cuh", "kb_types.h", "kb_launch.h", "kb_spline.cuh", "kb_flow.h")
 E2E_REPEATS = 5
+# What of a result goes to stderr: every key but these, and these keys' explanations.
+RESULT_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+               "vs_baseline", "dtype", "data", "impl", "config", "e2e", "gpu_launches", "roofline", "fallback_points",
+               "clocks", "cpu_baseline")
+EXPLANATIONS = {"e2e": ("statistic", "runs_evals_per_s"), "roofline": ("traffic_source", "peak_source")}
+
+
+def split_result(result):
+    """(the stdout line's object, the stderr line's object) of a result."""
+    line = {k: result[k] for k in RESULT_KEYS if k in result}
+    details = {k: v for k, v in result.items() if k not in line}
+    for k, names in EXPLANATIONS.items():
+        if k in line:
+            details[k] = {n: line[k][n] for n in names if n in line[k]}
+            line[k] = {n: v for n, v in line[k].items() if n not in names}
+    return line, details
 
 
 def _code_only(text):
@@ -669,6 +688,8 @@ def run_ours(args, rank, world, local_rank):
             line["learned_vs_plain"] = measure_learned(ctx, model, A, B, chain)
         if cpu is not None:
             line["cpu_baseline"] = {k: cpu[k] for k in ("value", "unit", "cores", "kind", "sample")}
+        line, details = split_result(line)
+        print(json.dumps(details), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     if world > 1:
         import torch.distributed as dist

@@ -50,3 +50,21 @@ def test_no_cpu_path_without_device():
     with pytest.raises(capi.KbError) as e:
         capi.Context(0)
     assert e.value.code in (capi.KB_E_NODEVICE, capi.KB_E_CUDA)
+
+
+def test_bench_line_is_short():
+    """The benchmark's result stays one short line on stdout, whatever explains it; nothing is lost."""
+    import json
+    import bench
+    result = {k: 1.234567890123456 for k in bench.RESULT_KEYS if k not in ("config", "e2e", "roofline", "clocks", "impl")}
+    result["config"] = bench.workload_config(8, 1 << 20)
+    result["e2e"] = {"value": 1.0, "unit": "evals/s", "h2d_bytes_per_step": 1, "d2h_bytes_per_step": 40,
+                     "statistic": "s" * 100, "runs_evals_per_s": [1.0] * 5}
+    result["roofline"] = {"bound": "fp64", "achieved": 1.0, "frac": 1.0, "traffic_source": "t" * 300,
+                          "numerator": "n" * 200, "peak_source": "p" * 200}
+    result["clocks"] = {"sm_mhz": 1965.0, "sm_max_mhz": 1965.0, "reasons": []}
+    result["learned_vs_plain"] = {"x": list(range(5000))}
+    line, details = bench.split_result(result)
+    assert len(json.dumps(line)) < 2500
+    for k, v in result.items():
+        assert line.get(k, details.get(k)) == v or {**line[k], **details[k]} == v
