@@ -111,27 +111,4 @@ struct ItemDev {
   const float *ar_spline;
 };
 
-// One chunk of points of one item, processed by one CTA iteration.
-struct ChunkDev {
-  int item;
-  int order;
-  int64_t first; // offset of the first point within the item
-  int count;
-};
-
-// Per-chunk partial sums (deterministic reduction afterwards).
-struct PartialDev {
-  double sum_re;
-  double sum_im;
-  unsigned long long n_in_domain;
-  unsigned long long n_fallback;
-};
-
-// A point the tree handed to the pivoted-LU kernel.
-struct FallbackDev {
-  int item;
-  int pad;
-  int64_t index; // point offset within the item
-};
-
 } // namespace kb

@@ -92,62 +92,54 @@ __device__ __forceinline__ int time_bin(const Launch &L, const double *u, int st
   return min((int)((t - L.bin_xmin) / L.bin_size), L.nbins - 1);
 }
 
-// G (row-major, M = 2N+1) of np points: G[p*M*M + r*M + c]. Out-of-domain points get
-// the identity (their values are discarded; this keeps every pivot finite).
-// Items per point: the N(N-1) ordered vertex pairs, the N external-row and N
-// external-column entries (one table lookup each: g^< and g^> at one time difference),
-// the N diagonal blocks (g(0)) and the corner. Each thread computes the lookup positions
-// of GK items before issuing their loads, so that GK L2 round trips overlap.
+// G (row-major, M = 2N+1) of a point inside the domain.
+// Items: the N(N-1) ordered vertex pairs, the N external-row and N external-column entries
+// (one table lookup each: g^< and g^> at one time difference), the N diagonal blocks (g(0))
+// and the corner. Each thread computes the lookup positions of GK items before issuing
+// their loads, so that GK L2 round trips overlap.
 template <bool CUBIC, int GK>
-__device__ void build_G(const ItemDev &it, int N, int np, const double *u, const int *flag, double2 *buf,
-                        int spin, int *bad) {
+__device__ void build_G(const ItemDev &it, int N, const double *u, double2 *G, int spin, int *bad) {
   const ModelDev &m = it.model;
   const int M = 2 * N + 1;
-  const int npair = N * (N - 1), nlook = npair + 2 * N, per = nlook + N + 1;
+  const int npair = N * (N - 1), nlook = npair + 2 * N, total = nlook + N + 1;
   const kb_gf_index &A = it.f.A, &B = it.f.B;
   const double2 *t00 = m.tab[spin][0][0];
   const double2 *trow = m.tab[spin][A.orbital][0];
   const double2 *tcol = m.tab[spin][0][B.orbital];
-  const int total = np * per;
-  // r / per and q / (N - 1) as a multiply-high by 2^32 / d rounded up (exact for the
-  // quotients here: r < 2^16, d <= 289); mn1 wraps to 0 for N - 1 = 1 (q / 1 = q)
-  const unsigned mper = 0xFFFFFFFFu / (unsigned)per + 1u;
+  // q / (N - 1) as a multiply-high by 2^32 / (N - 1) rounded up (exact for the quotients here);
+  // mn1 wraps to 0 for N - 1 = 1 (q / 1 = q)
   const unsigned mn1 = N > 1 ? 0xFFFFFFFFu / (unsigned)(N - 1) + 1u : 0u;
+  auto pair = [&](int q, int &i, int &j) {
+    i = mn1 ? (int)__umulhi((unsigned)q, mn1) : q;
+    const int r = q - i * (N - 1);
+    j = r + (r >= i ? 1 : 0);
+  };
   for (int base = threadIdx.x; base < total; base += GK * blockDim.x) {
-    int kind[GK], pi[GK], qi[GK], ix[GK];
+    int kind[GK], ix[GK];
     double wt[GK], dt[GK];
     const double2 *tb[GK];
 #pragma unroll
     for (int k = 0; k < GK; ++k) {
-      const int r = base + k * blockDim.x;
-      kind[k] = 0; // 0: none, 1: pair, 2: row, 3: col, 4: diagonal, 5: corner, 6: out of domain
+      const int q = base + k * blockDim.x;
+      kind[k] = 0; // 0: none, 1: pair, 2: row, 3: col, 4: diagonal, 5: corner
       tb[k] = nullptr;
       ix[k] = 0;
       wt[k] = 0.0;
       dt[k] = 0.0;
-      pi[k] = 0;
-      qi[k] = 0;
-      if (r >= total) continue;
-      const int p = (int)__umulhi((unsigned)r, mper), q = r - p * per;
-      pi[k] = p;
-      qi[k] = q;
-      const double *x = u + p;
-      if (flag[p] & 1) {
-        kind[k] = 6;
-        continue;
-      }
+      if (q >= total) continue;
       if (q < npair) {
-        const int i = mn1 ? (int)__umulhi((unsigned)q, mn1) : q, r2 = q - i * (N - 1), j = r2 + (r2 >= i ? 1 : 0);
+        int i, j;
+        pair(q, i, j);
         kind[k] = 1;
-        dt[k] = x[i * np] - x[j * np];
+        dt[k] = u[i] - u[j];
         tb[k] = t00;
       } else if (q < npair + N) {
         kind[k] = 2;
-        dt[k] = A.time - x[(q - npair) * np];
+        dt[k] = A.time - u[q - npair];
         tb[k] = trow;
       } else if (q < nlook) {
         kind[k] = 3;
-        dt[k] = x[(q - npair - N) * np] - B.time;
+        dt[k] = u[q - npair - N] - B.time;
         tb[k] = tcol;
       } else if (q < nlook + N) {
         kind[k] = 4;
@@ -173,12 +165,10 @@ __device__ void build_G(const ItemDev &it, int N, int np, const double *u, const
     }
 #pragma unroll
     for (int k = 0; k < GK; ++k) {
-      if (kind[k] == 0) continue;
-      double2 *G = buf + (size_t)pi[k] * M * M;
-      const int q = qi[k];
-      const double *x = u + pi[k];
+      const int q = base + k * blockDim.x;
       if (kind[k] == 1) {
-        const int i = mn1 ? (int)__umulhi((unsigned)q, mn1) : q, r2 = q - i * (N - 1), j = r2 + (r2 >= i ? 1 : 0);
+        int i, j;
+        pair(q, i, j);
         double2 *g = G + (2 * i) * M + 2 * j;
         const double d = dt[k];
         const bool later = (d != 0.0) ? (d > 0.0) : (i > j);
@@ -188,16 +178,14 @@ __device__ void build_G(const ItemDev &it, int N, int np, const double *u, const
         g[M] = gg[k];                     // backward-forward
       } else if (kind[k] == 2) {
         const int j = q - npair;
-        const double uj = x[j * np];
         double2 *row = G + (2 * N) * M + 2 * j;
-        row[0] = compare_3way(A.time, A.k_idx, N, uj, 0, j) > 0 ? gg[k] : gl[k];
-        row[1] = compare_3way(A.time, A.k_idx, N, uj, 1, j) > 0 ? gg[k] : gl[k];
+        row[0] = compare_3way(A.time, A.k_idx, N, u[j], 0, j) > 0 ? gg[k] : gl[k];
+        row[1] = compare_3way(A.time, A.k_idx, N, u[j], 1, j) > 0 ? gg[k] : gl[k];
       } else if (kind[k] == 3) {
         const int j = q - npair - N;
-        const double uj = x[j * np];
         double2 *col = G + (2 * j) * M + 2 * N;
-        col[0] = compare_3way(uj, 0, j, B.time, B.k_idx, N) > 0 ? gg[k] : gl[k];
-        col[M] = compare_3way(uj, 1, j, B.time, B.k_idx, N) > 0 ? gg[k] : gl[k];
+        col[0] = compare_3way(u[j], 0, j, B.time, B.k_idx, N) > 0 ? gg[k] : gl[k];
+        col[M] = compare_3way(u[j], 1, j, B.time, B.k_idx, N) > 0 ? gg[k] : gl[k];
       } else if (kind[k] == 4) {
         const int i = q - nlook;
         double2 *g = G + (2 * i) * M + 2 * i;
@@ -208,40 +196,17 @@ __device__ void build_G(const ItemDev &it, int N, int np, const double *u, const
         g[M] = gg[k];
       } else if (kind[k] == 5) {
         G[(2 * N) * M + 2 * N] = c2(0.0, 0.0);
-      } else { // out of domain: identity blocks, zero externals
-        const double2 z = c2(0.0, 0.0), one = c2(1.0, 0.0);
-        if (q < npair) {
-          const int i = mn1 ? (int)__umulhi((unsigned)q, mn1) : q, r2 = q - i * (N - 1), j = r2 + (r2 >= i ? 1 : 0);
-          double2 *g = G + (2 * i) * M + 2 * j;
-          g[0] = g[1] = g[M] = g[M + 1] = z;
-        } else if (q < npair + N) {
-          double2 *row = G + (2 * N) * M + 2 * (q - npair);
-          row[0] = row[1] = z;
-        } else if (q < nlook) {
-          double2 *col = G + (2 * (q - npair - N)) * M + 2 * N;
-          col[0] = col[M] = z;
-        } else if (q < nlook + N) {
-          const int i = q - nlook;
-          double2 *g = G + (2 * i) * M + 2 * i;
-          g[0] = g[M + 1] = one;
-          g[1] = g[M] = z;
-        } else {
-          G[(2 * N) * M + 2 * N] = one;
-        }
       }
     }
   }
 }
 
-// build_G with the model's interpolation chosen once per call; ANY_CUBIC = false compiles
-// the linear lookup only (launches whose models all interpolate linearly).
-template <bool ANY_CUBIC, int GK = 2>
-__device__ void build_G_any(const ItemDev &it, int N, int np, const double *u, const int *flag, double2 *buf,
-                            int spin, int *bad) {
-  if (ANY_CUBIC && it.model.interp == 3)
-    build_G<true, GK>(it, N, np, u, flag, buf, spin, bad);
+// build_G with the model's interpolation.
+__device__ void build_G_model(const ItemDev &it, int N, const double *u, double2 *G, int spin, int *bad) {
+  if (it.model.interp == 3)
+    build_G<true, 2>(it, N, u, G, spin, bad);
   else
-    build_G<false, GK>(it, N, np, u, flag, buf, spin, bad);
+    build_G<false, 2>(it, N, u, G, spin, bad);
 }
 
 __device__ __forceinline__ double2 apply_cutoff(double2 f, double cutoff) {
@@ -330,10 +295,10 @@ __device__ __forceinline__ void direct_point(DirectShared &D, const ItemDev &it,
   }
   const int M = 2 * N + 1;
   const int spin = it.f.A.spin;
-  build_G_any<true>(it, N, 1, D.u, D.flag, D.G1, spin, bad);
+  build_G_model(it, N, D.u, D.G1, spin, bad);
   const double2 *G2 = D.G1;
   if (!it.spin_symmetric) {
-    build_G_any<true>(it, N, 1, D.u, D.flag, D.G2, 1 - spin, bad);
+    build_G_model(it, N, D.u, D.G2, 1 - spin, bad);
     G2 = D.G2;
   }
   __syncthreads();
