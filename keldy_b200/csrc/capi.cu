@@ -846,8 +846,8 @@ static int coarse_chunk(const kb_context *ctx, int order, int64_t n) {
 
 } // extern "C"
 
-// Places in one device block: an allocation, an upload and a download per call instead of one per
-// array (each costs the host 2 to 5 us, most of a small call).
+// Places in one device block: an allocation per call instead of one per array, and in the integration
+// calls one upload and one download (each costs the host 2 to 5 us, most of a small call).
 namespace {
 struct Block {
   size_t size = 0;

@@ -476,8 +476,8 @@ __global__ void __launch_bounds__(NT, 2)
 
 // ------------------------------------------------------------ training step
 // TMEM columns: [0,128) working accumulator, [128,256) dW1, [256,384) dW2, [384,512) dW3.
-// Bound: a CTA's chain of 71 products per tile, each waited for, with an epilogue between two: a
-// batch of 8,192 points is 64 tiles, so the chain's length is the step's time. Four threads per
+// Bound: a CTA's chain of 41 waited steps per tile (58 products: 18 forward, 5 logits again, 35 gradients
+// in 18 steps), with an epilogue between two: a batch of 8,192 points is 64 tiles, so the chain's length is the step's time. Four threads per
 // point (warps w, w + 4, w + 8, w + 12 on TMEM lane quadrant w) take one slot, or a quarter of an
 // epilogue's columns, each: with one thread per point a step of 8,192 points took 248 us, with two
 // 152 us, with four 150 us. The coordinates and their gradients that the other threads made

@@ -498,7 +498,7 @@ __device__ __forceinline__ unsigned group_values(WarpShared<SCALE> &T, int order
                 __syncwarp();
               }
             }
-            if (!pair_at) { // orders 15 and 16: level 8's node from global scratch
+            if (!pair_at) { // orders 14 to 16: level 8's node from global scratch
               for (int e = lane; e < 81; e += 32) T.buf[node_base(8) + e] = pair8[81 * (tr & 1) + e];
               __syncwarp();
             }

@@ -137,3 +137,18 @@ def test_nearly_empty_and_full_levels(ctx, oracle, ratio, small):
             w, dw, sc = oracle.integrand(om, A, B, t)
             assert np.array_equal(d, dw) and np.all(np.abs(v - w) <= 1e-12 * sc), n
             np.testing.assert_allclose(gsc, sc, rtol=1e-9)
+
+
+@pytest.mark.parametrize("interp", [1, 3])
+@pytest.mark.parametrize("n,count", [(10, 3), (13, 3), (14, 3), (15, 2), (16, 2)])
+def test_depth_first_layouts(ctx, oracle, golden, n, count, interp):
+    """Where the depth-first levels' nodes lie changes at orders 10 (level 9's node leaves shared memory),
+    14 (level 8's pair as well, and level 9's is back) and 16 (neither); several points per group."""
+    le, gr = golden["table_beta20_lesser"], golden["table_beta20_greater"]
+    gm, om = ctx.model(10.0, le, gr, 0.4), oracle.model(10.0, le, gr, 0.4, interp=interp)
+    gm.set_interpolation(interp)
+    A, B = ENDS[n % 2]
+    t = np.random.default_rng(n).random((count, n)) * 10.0
+    v, d = gm.integrand(A, B, t, algo=capi.ALGO_TREE)
+    w, dw, sc = oracle.integrand(om, A, B, t)
+    assert np.array_equal(d, dw) and np.all(np.abs(v - w) <= 1e-12 * sc)
