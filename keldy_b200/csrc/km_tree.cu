@@ -28,7 +28,7 @@
 // shared memory for the way back.
 //
 // Bound: latency, at 8 warps per SM (255 registers; the nodes kept for the way back fill the shared
-// memory). 2^20 points of order 8 8.8 ms (69 for the tree that it replaced), of order 5 1.5 (9.8);
+// memory). 2^20 points of order 8 8.9 ms (69 for the tree that it replaced), of order 5 1.6 (9.8);
 // of 65,536 points of order 8 (0.67 ms) ncu shows the FP64 pipe 27 % busy, shared memory 52 %.
 #include "kb_wick.cuh"
 
@@ -154,7 +154,7 @@ __device__ __forceinline__ void km_level(double2 *buf, const double2 *dl, const 
   const double2 *S = buf + km_base(m) + (child >> 1) * km_sz(m);
   double2 *o = buf + km_base(m - 1) + child * km_sz(m - 1);
   const double2 *dc = dl + (m - 1) * (m - 2), *dr = dc + m - 1; // entries (i, m) and (m, j)
-  const double f = (child & 1) ? 0.0 : 1.0;
+  const double f = (child & 1) ? 0.0 : 1.0, fr = (child & 1) ? 1.0 : 0.0;
   const double2 p = S[m * W + m - 1], ip = pivot_rcp(p);
   if (!(cabs1(p) >= floor_)) guard = true;
   if (l == (1 << LC) - 1) {
@@ -171,7 +171,7 @@ __device__ __forceinline__ void km_level(double2 *buf, const double2 *dl, const 
   for (int q = 0; q < COLS; ++q) {
     const int c = min(c0 + q, m), src = c < m - 1 ? c : c + 1;
     const double2 d = c < m - 1 ? dr[c] : dlC[m - 1];
-    r[q] = copyof(S[m * W + src], d, c == m ? 0.0 : 1.0 - f);
+    r[q] = copyof(S[m * W + src], d, c == m ? 0.0 : fr);
   }
 #pragma unroll
   for (int k = 0; k < ROWS; ++k) {
@@ -287,7 +287,7 @@ __device__ __forceinline__ void km_subtree(KmShared &T, double2 *out, const doub
       constexpr int W = km_w(4);
       const double2 *S = T.buf + (lane >> 1) * km_sz(4);
       const double2 *dc = dl + 6, *dr = dl + 9;
-      const double f = (lane & 1) ? 0.0 : 1.0;
+      const double f = (lane & 1) ? 0.0 : 1.0, fr = (lane & 1) ? 1.0 : 0.0;
       const double2 p = S[4 * W + 3], ip = pivot_rcp(p);
       if (!(cabs1(p) >= floor_)) guard = true;
       D2 = cmul(T.D2[lane >> 1], cmul(p, p));
@@ -295,7 +295,7 @@ __device__ __forceinline__ void km_subtree(KmShared &T, double2 *out, const doub
       double2 r[5];
 #pragma unroll
       for (int q = 0; q < 5; ++q)
-        r[q] = q == 4 ? S[4 * W + 5] : copyof(S[4 * W + (q < 3 ? q : 4)], q < 3 ? dr[q] : dlC[3], 1.0 - f);
+        r[q] = q == 4 ? S[4 * W + 5] : copyof(S[4 * W + (q < 3 ? q : 4)], q < 3 ? dr[q] : dlC[3], fr);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const double2 Lf = cmul(i ? copyof(S[i * W + 3], dc[i - 1], f) : S[3], ip);
@@ -310,11 +310,11 @@ __device__ __forceinline__ void km_subtree(KmShared &T, double2 *out, const doub
     double2 h3 = c2(0.0, 0.0), t3f = c2(0.0, 0.0);
 #pragma unroll 1
     for (int a = 0; a < 2; ++a) {
-      const double f = a ? 0.0 : 1.0, sg = a ? -1.0 : 1.0;
+      const double f = a ? 0.0 : 1.0, fr = a ? 1.0 : 0.0, sg = a ? -1.0 : 1.0;
       double2 r[4], U[12];
-      r[0] = copyof(s[15], dl[4], 1.0 - f);
-      r[1] = copyof(s[16], dl[5], 1.0 - f);
-      r[2] = copyof(s[18], dlC[2], 1.0 - f);
+      r[0] = copyof(s[15], dl[4], fr);
+      r[1] = copyof(s[16], dl[5], fr);
+      r[2] = copyof(s[18], dlC[2], fr);
       r[3] = E3;
 #pragma unroll
       for (int i = 0; i < 3; ++i) {
@@ -398,13 +398,13 @@ __device__ __forceinline__ void km_step_down(const double2 *S, double2 *o, const
                                              int lane, double2 D2, double2 &D2n, double floor_, bool &guard) {
   const int W = km_w(m), WC = km_w(m - 1);
   const double2 *dc = dl + (m - 1) * (m - 2), *dr = dc + m - 1;
-  const double f = a ? 0.0 : 1.0;
+  const double f = a ? 0.0 : 1.0, fr = a ? 1.0 : 0.0;
   const double2 p = S[m * W + m - 1], ip = pivot_rcp(p);
   if (!(cabs1(p) >= floor_)) guard = true;
   D2n = cmul(D2, cmul(p, p));
   if (a) D2n = c2(-D2n.x, -D2n.y);
   const int c = min(lane & 15, m), src = c < m - 1 ? c : c + 1; // a column per lane, every other row
-  const double2 r = copyof(S[m * W + src], c < m - 1 ? dr[c] : dlC[m - 1], c == m ? 0.0 : 1.0 - f);
+  const double2 r = copyof(S[m * W + src], c < m - 1 ? dr[c] : dlC[m - 1], c == m ? 0.0 : fr);
 #pragma unroll 5
   for (int i = lane >> 4; i < m; i += 2) {
     const double2 Lf = cmul(copyof(S[i * W + m - 1], dc[max(i, 1) - 1], i ? f : 0.0), ip);
