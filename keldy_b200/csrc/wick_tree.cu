@@ -31,8 +31,8 @@
 // of a node splitting its children; the last five vertices run in registers. Orders above 8
 // walk the levels above 9 depth first. Warps never wait for each other: no CTA barrier.
 //
-// Bound: latency. Order 8 (2^20 points): 3.15 ms (13.1 for the elimination in the given order, one
-// CTA per sub-batch of points). Of 65,536 points (0.37 ms) ncu shows the FP64 pipe 39 % busy, 1,330
+// Bound: latency. Order 8 (2^20 points): 3.17 ms (13.1 for the elimination in the given order, one
+// CTA per sub-batch of points). Of 65,536 points (0.37 ms) ncu shows the FP64 pipe 39 % busy, 1,335
 // instructions per point, shared memory 44 %; the stalls are shared-memory loads (2.2 cycles per
 // issued instruction) and fixed latencies of dependent FP64 instructions (1.8) at 12 warps per SM.
 // Measured when order 8 took 3.6 to 3.8 ms: splitting a level's nodes over fewer
