@@ -257,3 +257,54 @@ def test_exponential_warper_of_a_short_scale(ctx, oracle, golden, w):
         np.testing.assert_array_equal(d, wd)
         np.testing.assert_allclose(j, wj, rtol=1e-12)
         assert np.all(np.abs(v - wv) <= 1e-12 * sc)
+
+
+def _extended(le, gr, tmax, u):
+    """The integrand for A = (t_max, forward), B = (t_max, backward) at times u, and the sum of its |terms|, in
+    80-bit arithmetic: the table positions as the kernels form them (rounded to double), the rest exact to 2^-60."""
+    from itertools import permutations
+    count, n = u.shape
+    C, mesh = np.clongdouble, len(le)
+    perms = {k: [(p, (-1) ** sum(p[j] > p[i] for i in range(k) for j in range(i))) for p in permutations(range(k))]
+             for k in (n, n + 1)}
+
+    def det(m):
+        return sum(s * np.prod([m[:, i, p[i]] for i in range(m.shape[1])], axis=0) for p, s in perms[m.shape[1]])
+
+    full = np.concatenate([u, np.full((count, 1), tmax)], axis=1)
+    dt = full[:, :, None] - full[:, None, :]
+    a = (dt + tmax) / (2.0 * tmax / (mesh - 1))
+    i = np.clip(np.floor(a).astype(np.int64), 0, mesh - 2)
+    w = (a - i).astype(np.longdouble)
+    less, great = [(1 - w) * g.astype(C)[i] + w * g.astype(C)[i + 1] for g in (le, gr)]
+    later, eq = dt > 0, np.arange(n + 1)
+    later[:, n, :], later[:, :, n] = True, False
+    fwd, bwd = np.where(later, great, less), np.where(later, less, great)
+    fwd[:, eq, eq] = bwd[:, eq, eq] = less[:, eq, eq]
+    g = [[fwd, less], [great, bwd]]  # [branch of i][branch of j][p][i][j]
+    total, scale = np.zeros(count, C), np.zeros(count, np.longdouble)
+    for cfg in range(1 << n):
+        b = [(cfg >> k) & 1 for k in range(n)]
+        m = np.zeros((count, n + 1, n + 1), C)
+        for r in range(n + 1):
+            for c in range(n + 1):
+                if r < n or c < n:
+                    m[:, r, c] = g[b[r] if r < n else 0][b[c] if c < n else 1][:, r, c]
+        term = det(m) * det(m[:, :n, :n])
+        total += -term if sum(b) & 1 else term
+        scale += np.abs(term)
+    return total, scale
+
+
+@pytest.mark.parametrize("algo", [capi.ALGO_TREE, capi.ALGO_DIRECT])
+@pytest.mark.parametrize("n", [1, 2, 3, 4])
+def test_integrand_vs_extended_precision(ctx, golden, n, algo):
+    """A few units in the last place of the sum of |terms|: a lookup rounds four times, a determinant has n + 1
+    pivots whose reciprocals and updates round about eight times each, pivots are at least 0.29 of the largest
+    entry; two determinants: 16 (n + 1) / 0.29 * 2^-53, 6e-15 (n + 1)."""
+    for name in ("T0", "beta20"):
+        le, gr = golden[f"table_{name}_lesser"], golden[f"table_{name}_greater"]
+        u = np.random.default_rng(n).random((200 if n < 4 else 60, n)) * 10.0
+        v, d = ctx.model(10.0, le, gr).integrand((10.0, 0, 0), (10.0, 0, 1), u, algo=algo)
+        w, sc = _extended(le, gr, 10.0, u)
+        assert np.all(d == 1) and np.all(np.abs(v - w) <= 6e-15 * (n + 1) * sc)
